@@ -519,6 +519,24 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
   std::vector<PairEntry<double>> td(NPAIR);
   const int W = p->n_type - 1;
   double rl_max = 0.;
+  // Largest error of a distance from the coarse fixed-point differences of the screening and list
+  // tests (each axis truncated to 512 units: 2^32 per box length in x, y, 2^30 per width in z),
+  // twice over for the FP32 arithmetic.  Below ~500 sigma of box the 2e-4 margin covers it.
+  double fx_err = 0.;
+  for (auto& s : ctx->sys) {
+    double e2 = 0.;
+    for (int d = 0; d < 3; ++d) {
+      const double e = 512. * s.boundary[d] / (d < 2 ? 4294967296.0 : 1073741824.0);
+      e2 += e * e;
+    }
+    fx_err = std::max(fx_err, 2. * std::sqrt(e2));
+  }
+  // cut-off^2 -> FP32 threshold of those tests
+  auto fx_margin = [&](double rc2) {
+    if (rc2 <= 0.) return 0.f;
+    const double r = std::sqrt(rc2) + fx_err;
+    return (float)std::max(rc2 * 1.0002, r * r);
+  };
   for (int i = 0; i < MAXT; ++i)
     for (int j = 0; j < MAXT; ++j) {
       PairEntry<double> e;
@@ -559,8 +577,8 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
       g.range2 = (float)e.range2; g.eps4 = (float)e.eps4; g.sig2 = (float)e.sig2; g.shift = (float)e.shift;
       g.inv_rc = (float)e.inv_rc; g.rlist2 = (float)e.rlist2; g.dpd_rc2 = (float)e.dpd_rc2;
       g.inv_dpd_rc = (float)e.inv_dpd_rc; g.qq = (float)e.qq; g.flags = e.flags;
-      g.screen2 = (float)(e.screen2 * 1.0002);
-      g.rlist2 = (float)(e.rlist2 * 1.0002);
+      g.screen2 = fx_margin(e.screen2);
+      g.rlist2 = fx_margin(e.rlist2);
     }
   if (rl_max <= 0.) rl_max = 1.0 + skin;
   ctx->rl_max = rl_max;
@@ -573,8 +591,8 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
         if (e.screen2 > 0.) { slo = std::min(slo, e.screen2); shi = std::max(shi, e.screen2); }
       }
     const bool uni = hi > 0. && hi == lo && shi == slo;
-    C.rl2_uni_f = uni ? (float)(hi * 1.0002) : 0.f;
-    C.scr2_uni_f = uni ? (float)(shi * 1.0002) : 0.f;
+    C.rl2_uni_f = uni ? fx_margin(hi) : 0.f;
+    C.scr2_uni_f = uni ? fx_margin(shi) : 0.f;
   }
   // ---- replicas -------------------------------------------------------------------------------
   ctx->hreps.resize(n_rep);
@@ -714,8 +732,9 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
   for (auto d : dst) DA(*d, Nn);
   for (int k = 0; k < 9; ++k) DA(S.tmp[k], Nn);
   DA(S.tag, Nn); DA(S.info, Nn); DA(S.tmp_tag, Nn); DA(S.tmp_info, Nn); DA(S.slot_of_tag, Nn);
+  DA(S.pfx, Nn);  // (the FP64 mode: for the list build and the pair kernel's screening)
   if (S.mixed) {
-    DA(S.pfx, Nn); DA(S.vf, Nn); DA(S.f4, Nn);
+    DA(S.vf, Nn); DA(S.f4, Nn);
     DA(S.pfx_alt, Nn); DA(S.vf_alt, Nn);
   } else {
     DA(S.pd, Nn); DA(S.vd, Nn);
@@ -764,7 +783,8 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
   S.reps = ctx->dreps;
   S.tabf = ctx->dtabf;
   S.tabd = ctx->dtabd;
-  S.rl2_uni = S.mixed ? C.rl2_uni_f : 0.f;
+  S.rl2_uni = C.rl2_uni_f;
+  S.fx_err = (float)fx_err;
   S.nl_h = nl_h;
   S.nl_hx = nl_hx;
   if (ctx->opt.pair_schedule < 0 || ctx->opt.pair_schedule > 1)

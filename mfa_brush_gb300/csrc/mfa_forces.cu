@@ -473,7 +473,7 @@ __device__ __forceinline__ real_t<MIXED> pair_fs(const DevState& s, const SimCon
 //           that the integrator reads;
 //   BONDED  (FUSED only) the particle's bonded terms (bonded_of) in the same thread, which saves
 //           the bonded kernel's launch and its read-modify-write of the force;
-//   UNI     (MIXED only) one screening cut-off for every type pair (SimConst::scr2_uni_f).
+//   UNI     one screening cut-off for every type pair (SimConst::scr2_uni_f).
 // Without FUSED the forces are added to (accumulate) or stored in the FP64 force arrays.
 // Virial (EFLAG): each visit of a pair adds half of F_ij (x) (r_i - r_j) (the other visit adds the
 // other half); a pair with a fixed wall bead, which has no list of its own, counts in full.
@@ -500,11 +500,17 @@ __global__ void __launch_bounds__(128, MIXED ? (PERSIST ? 8 : ((INTEG && !EFLAG)
   static_assert(!BONDED || FUSED, "bonded terms are fused only into the fused form");
   static_assert(!INTEG || (FUSED && !PERSIST), "the integration is fused into the fused form");
   __shared__ PairEntry<real> tab[NPAIR];
+  __shared__ float scr[MIXED ? 1 : NPAIR];  // FP64: the FP32 screening thresholds
   // FUSED: the particle's FP64 total, in shared memory while the pair loop runs (registers are
   // scarce there; it is touched once per batch)
   __shared__ double ftot[FUSED ? 3 : 1][FUSED ? 128 : 1];
   for (int k = threadIdx.x; k < NPAIR; k += blockDim.x) {
-    if constexpr (MIXED) tab[k] = s.tabf[k]; else tab[k] = s.tabd[k];
+    if constexpr (MIXED) {
+      tab[k] = s.tabf[k];
+    } else {
+      tab[k] = s.tabd[k];
+      scr[k] = s.tabf[k].screen2;
+    }
   }
   __shared__ int tile_sh;
   const int ntile = (s.N + blockDim.x - 1) / blockDim.x;
@@ -567,13 +573,12 @@ __global__ void __launch_bounds__(128, MIXED ? (PERSIST ? 8 : ((INTEG && !EFLAG)
     const int n = __ldg(&s.nn[i]);
     const int p0 = R.p0;
     // own position / velocity
-    int4 qi;
+    const int4 qi = __ldg(&s.pfx[i]);
     dbl4 pi;
     real vix, viy, viz;
     int tag_i;
     real ux = 0, uy = 0, uz = 0;
     if constexpr (MIXED) {
-      qi = __ldg(&s.pfx[i]);
       float4 v4 = __ldg(&s.vf[i]);
       vix = v4.x; viy = v4.y; viz = v4.z;
       tag_i = __float_as_int(v4.w) - p0;
@@ -613,21 +618,21 @@ __global__ void __launch_bounds__(128, MIXED ? (PERSIST ? 8 : ((INTEG && !EFLAG)
     // gathers
     int* const jl = pair_pool + threadIdx.x;
     int k = 0;
-    // screening against the largest cut-off of the type pair; MIXED uses the coarse conversion
-    // (512 fixed-point units of resolution, inside the 2e-4 margin of screen2)
-    const float cx = ux * 512.f, cy = uy * 512.f, cz = uz * 512.f;
+    // screening against the largest cut-off of the type pair, in FP32 on the fixed-point views in
+    // both precisions, with the coarse conversion (512 fixed-point units of resolution, inside the
+    // 2e-4 margin of screen2); the evaluation then tests the exact distance
+    const float cx = R.ufx_f[0] * 512.f, cy = R.ufx_f[1] * 512.f, cz = R.ufx_f[2] * 512.f;
     auto screen = [&](int j) -> bool {
-      if constexpr (MIXED) {
-        const int4 qj = __ldg(&s.pfx[j]);
-        const float dx = i2f_coarse(fx_diff(qi.x, qj.x), 9) * cx;
-        const float dy = i2f_coarse(fx_diff(qi.y, qj.y), 9) * cy;
-        const float dz = i2f_coarse(fx_diff(qi.z, qj.z), 9) * cz;
-        return dx * dx + dy * dy + dz * dz < (UNI ? C.scr2_uni_f : tab[ti * MAXT + info_type(qj.w)].screen2);
-      } else {
-        real dx, dy, dz;
-        const int wj = delta(j, dx, dy, dz);
-        return dx * dx + dy * dy + dz * dz < tab[ti * MAXT + info_type(wj)].screen2;
-      }
+      const int4 qj = __ldg(&s.pfx[j]);
+      const float dx = i2f_coarse(fx_diff(qi.x, qj.x), 9) * cx;
+      const float dy = i2f_coarse(fx_diff(qi.y, qj.y), 9) * cy;
+      const float dz = i2f_coarse(fx_diff(qi.z, qj.z), 9) * cz;
+      const int tt = ti * MAXT + info_type(qj.w);
+      float lim;
+      if constexpr (UNI) lim = C.scr2_uni_f;
+      else if constexpr (MIXED) lim = tab[tt].screen2;
+      else lim = scr[tt];
+      return dx * dx + dy * dy + dz * dz < lim;
     };
     while (k < n) {
       int m = 0;
@@ -820,8 +825,10 @@ void launch_pair(const DevState& s, const SimConst& C, cudaStream_t st, bool acc
     if (eflag) k_pair<true, true><<<g, B, 0, st>>>(s, C, true, acc);
     else k_pair<true, false><<<g, B, 0, st>>>(s, C, true, acc);
   } else {
-    if (eflag) k_pair<false, true><<<g, B, 0, st>>>(s, C, accumulate, acc);
-    else k_pair<false, false><<<g, B, 0, st>>>(s, C, accumulate, acc);
+    using KernT = void (*)(DevState, SimConst, bool, Acc, int);
+    const KernT kd[2][2] = {{k_pair<false, false>, k_pair<false, true>},
+                            {k_pair<false, false, false, false, true>, k_pair<false, true, false, false, true>}};
+    kd[uni ? 1 : 0][eflag ? 1 : 0]<<<g, B, 0, st>>>(s, C, accumulate, acc, 0);
   }
 }
 

@@ -26,8 +26,8 @@ __device__ __forceinline__ void store_views(const DevState& s, int i, const RepD
   q.y = to_fx_periodic(y, R.sfx[1]);
   q.z = to_fx_z(z, R.sfx[2]);
   q.w = w;
+  s.pfx[i] = q;
   if (s.mixed) {
-    s.pfx[i] = q;
     s.vf[i] = make_float4((float)vx, (float)vy, (float)vz, __int_as_float(t));
   } else {
     s.pd[i] = mk_dbl4(x, y, z, __longlong_as_double((long long)w));

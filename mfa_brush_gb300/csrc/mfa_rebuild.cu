@@ -25,14 +25,13 @@
 
 namespace mfa {
 
-
-__device__ __forceinline__ void cell_coords(const RepDesc& R, double x, double y, double z, int& ix, int& iy,
-                                            int& iz) {
-  ix = (int)(x * R.inv_lc[0]);
-  iy = (int)(y * R.inv_lc[1]);
-  iz = (int)(z * R.inv_lc[2]);
-  ix = min(max(ix, 0), R.nc[0] - 1);
-  iy = min(max(iy, 0), R.nc[1] - 1);
+// Cell of a fixed-point position on the replica's list grid: one integer multiply per axis (x, y
+// wrap with the fixed point; z is clamped to the grid).  Shared by the binning and the list build
+// of both precisions, so they agree to the bit.
+__device__ __forceinline__ void cell_coords(const RepDesc& R, const int4& q, int& ix, int& iy, int& iz) {
+  ix = (int)(((unsigned long long)(unsigned)q.x * (unsigned)R.nc[0]) >> 32);
+  iy = (int)(((unsigned long long)(unsigned)q.y * (unsigned)R.nc[1]) >> 32);
+  iz = (int)(((long long)q.z * R.nc[2]) >> 30);
   iz = min(max(iz, 0), R.nc[2] - 1);
 }
 
@@ -156,8 +155,7 @@ __global__ void k_bin(DevState s) {
   const int i = s.reps[rr].p0 + loc;
   int w = s.info[i];
   const RepDesc& R = s.reps[info_rep(w)];
-  int ix, iy, iz;
-  if (s.mixed) {  // the list builder's integer formula on the fixed-point view
+  if (s.mixed) {
     // (x, y need no check: the fixed-point view wraps them; the integrator flags NaN); the z
     // check in FP32, as FP64 compares and the cell-height division issue on the FP64 pipe
     const double zd = s.rz[i];
@@ -165,21 +163,14 @@ __global__ void k_bin(DevState s) {
     if (!(z >= R.zlim_f[0] && z <= R.zlim_f[1]))  // also false for NaN
       atomicOr(s.status, (__double_as_longlong(zd) & 0x7FF0000000000000ll) == 0x7FF0000000000000ll ? ST_NAN
                                                                                                 : ST_OUT_OF_BOX);
-    const int4 q = s.pfx[i];
-    ix = (int)(((unsigned long long)(unsigned)q.x * (unsigned)R.nc[0]) >> 32);
-    iy = (int)(((unsigned long long)(unsigned)q.y * (unsigned)R.nc[1]) >> 32);
-    iz = (int)(((long long)q.z * R.nc[2]) >> 30);
-    iz = min(max(iz, 0), R.nc[2] - 1);
   } else {
     const double lz = 1. / R.inv_lc[2];
-    double x = s.rx[i], y = s.ry[i], z = s.rz[i];
-    if (!(isfinite(x) && isfinite(y) && isfinite(z))) {
-      atomicOr(s.status, ST_NAN);
-      x = y = z = 0.;
-    }
-    if (z < -lz || z > R.L[2] + lz) atomicOr(s.status, ST_OUT_OF_BOX);
-    cell_coords(R, x, y, z, ix, iy, iz);
+    const double x = s.rx[i], y = s.ry[i], z = s.rz[i];
+    if (!(isfinite(x) && isfinite(y) && isfinite(z))) atomicOr(s.status, ST_NAN);
+    else if (z < -lz || z > R.L[2] + lz) atomicOr(s.status, ST_OUT_OF_BOX);
   }
+  int ix, iy, iz;
+  cell_coords(R, s.pfx[i], ix, iy, iz);
   const int c = R.cell_off + (iz * R.nc[1] + iy) * R.nc[0] + ix;
   s.cell_of[i] = c;
   // Particles are still nearly sorted by cell, so neighbouring lanes share cells: the lanes of one
@@ -402,8 +393,8 @@ __device__ __forceinline__ int4 write_views(const DevState& s, int i, const RepD
   q.y = to_fx_periodic(y, R.sfx[1]);
   q.z = to_fx_z(z, R.sfx[2]);
   q.w = w;
+  s.pfx[i] = q;
   if (s.mixed) {
-    s.pfx[i] = q;
     s.vf[i] = make_float4(d2f_fast(vx), d2f_fast(vy), d2f_fast(vz), __int_as_float(t));
   } else {
     s.pd[i] = mk_dbl4(x, y, z, __longlong_as_double((long long)w));
@@ -435,7 +426,11 @@ __global__ void k_copyback(DevState s) {
   }
 }
 
-// Full Verlet list: every mobile particle lists all j (mobile or wall) with r^2 < (rc_ij+skin)^2.
+// Full Verlet list: every mobile particle lists all j (mobile or wall) with r^2 < (rc_ij+skin)^2,
+// decided in FP32 on the fixed-point positions with a 2e-4 margin in both precisions (the FP64 mode
+// keeps the fixed-point view for this and for the pair kernel's screening; with candidate tests in
+// FP64, issued at 1/64 of the FP32 rate, ten steps of a 7200-particle FP64 channel took 1434 us,
+// with these 1000, and ten of a batch of 242 k particles 9.73 ms against 6.65).
 // One thread per particle.  Cells are at least 1/H of the list cut-off wide (H = 2 by default),
 // and the (2H+1)^3 cells around a particle are walked as (2H+1)^2 x-rows: the cells of a row are
 // consecutive in the sorted order unless the row wraps in x, so a row is one contiguous slot range
@@ -453,27 +448,24 @@ __global__ void k_copyback(DevState s) {
 // coalesced; a particle with more neighbours writes the rest straight to the list)
 constexpr int NL_STAGE = 32;
 
-template <bool MIXED, bool UNI, int H, int HX = H>
+template <bool UNI, int H, int HX = H>
 __global__ void __launch_bounds__(NL_BLOCK, 8) k_nlist(DevState s) {
   const int nwl = *s.wl_n;
   const int nchunks = s.wl_k[nwl];
   if ((int)blockIdx.x >= nchunks) return;
   __shared__ int nl_sh[NL_BLOCK * (NL_STAGE | 1)];
   __shared__ float rl2f[NPAIR];
-  __shared__ double rl2d[NPAIR];
   __shared__ float rlmax[MAXT];
   __shared__ int blk_max;
   __shared__ int chunk;
   const int cap = s.nbr_cap;
   int* mine = nl_sh + threadIdx.x * (NL_STAGE | 1);
-  for (int k = threadIdx.x; k < NPAIR; k += blockDim.x) {
-    rl2d[k] = s.tabd[k].rlist2;
-    rl2f[k] = s.tabf ? s.tabf[k].rlist2 : 0.f;
-  }
+  for (int k = threadIdx.x; k < NPAIR; k += blockDim.x) rl2f[k] = s.tabf[k].rlist2;
   if (threadIdx.x < MAXT) {  // largest list cut-off of each type, with the culling margin
-    double m = 0.;
-    for (int t = 0; t < MAXT; ++t) m = fmax(m, s.tabd[threadIdx.x * MAXT + t].rlist2);
-    rlmax[threadIdx.x] = (float)m * 1.0004f;
+    float m = 0.f;
+    for (int t = 0; t < MAXT; ++t) m = fmaxf(m, s.tabf[threadIdx.x * MAXT + t].rlist2);
+    m = sqrtf(m) + s.fx_err;
+    rlmax[threadIdx.x] = m * m * 1.0002f;
   }
   for (;;) {
   // the next chunk from the queue (chunks differ in cost: a queue keeps the blocks busy)
@@ -495,35 +487,19 @@ __global__ void __launch_bounds__(NL_BLOCK, 8) k_nlist(DevState s) {
     const RepDesc& R = s.reps[info_rep(w)];
     const int ti = info_type(w);
     int ix, iy, iz;
-    int4 qi = make_int4(0, 0, 0, 0);
-    double x = 0., y = 0., z = 0.;
-    if (MIXED) {
-      qi = s.pfx[i];
-      ix = (int)(((unsigned long long)(unsigned)qi.x * (unsigned)R.nc[0]) >> 32);
-      iy = (int)(((unsigned long long)(unsigned)qi.y * (unsigned)R.nc[1]) >> 32);
-      iz = (int)(((long long)qi.z * R.nc[2]) >> 30);
-      iz = min(max(iz, 0), R.nc[2] - 1);
-    } else {
-      x = s.rx[i]; y = s.ry[i]; z = s.rz[i];
-      cell_coords(R, x, y, z, ix, iy, iz);
-    }
+    const int4 qi = s.pfx[i];
+    cell_coords(R, qi, ix, iy, iz);
     // coarse conversion (512 fixed-point units); rl2f carries a 2e-4 margin
     const float ux = R.ufx_f[0] * 512.f, uy = R.ufx_f[1] * 512.f, uz = R.ufx_f[2] * 512.f;
     const int nx = R.nc[0];
     // Row culling and x trimming: a cell is skipped when its distance from the particle, taken
-    // from the cell edges, is beyond the largest list cut-off of the particle's type times 1.0004
-    // (the candidate test below has a 1.0002 margin; the coarse position is off by < 1e-5 sigma).
+    // from the cell edges, is beyond the largest list cut-off of the particle's type, the candidate
+    // test's margin included, plus the error of the coarse position and 1e-4 of itself
     // (no FP64 and no conversion instructions here: both run on the slow FP64 pipe)
-    float px, py, pz;  // position in cell units
-    if (MIXED) {
-      px = (__int_as_float(0x4B000000 | ((unsigned)qi.x >> 9)) - 8388608.0f) * R.cpu_f[0];
-      py = (__int_as_float(0x4B000000 | ((unsigned)qi.y >> 9)) - 8388608.0f) * R.cpu_f[1];
-      pz = i2f_coarse(qi.z, 9) * R.cpu_f[2];
-    } else {
-      px = (float)(x * R.inv_lc[0]);
-      py = (float)(y * R.inv_lc[1]);
-      pz = (float)(z * R.inv_lc[2]);
-    }
+    // position in cell units
+    const float px = (__int_as_float(0x4B000000 | ((unsigned)qi.x >> 9)) - 8388608.0f) * R.cpu_f[0];
+    const float py = (__int_as_float(0x4B000000 | ((unsigned)qi.y >> 9)) - 8388608.0f) * R.cpu_f[1];
+    const float pz = i2f_coarse(qi.z, 9) * R.cpu_f[2];
     const float lx = R.lc_f[0], ly = R.lc_f[1], lz = R.lc_f[2];
     const float rl2max = rlmax[ti];
     const float rl_uni = s.rl2_uni;  // UNI: one list cut-off for every pair (2e-4 margin included)
@@ -574,22 +550,11 @@ __global__ void __launch_bounds__(NL_BLOCK, 8) k_nlist(DevState s) {
           // 2 / 4 / 8 measured 0.6 / 2.9 / 3.8 % slower on a rebuild of 256 brush replicas
 #pragma unroll 1
           for (int j = sb[g]; j < se[g]; ++j) {
-            int wj;
-            bool hit;
-            if (MIXED) {
-              const int4 qj = s.pfx[j];
-              wj = qj.w;
-              const float ddx = i2f_coarse(fx_diff(qi.x, qj.x), 9) * ux;
-              const float ddy = i2f_coarse(fx_diff(qi.y, qj.y), 9) * uy;
-              const float ddz = i2f_coarse(fx_diff(qi.z, qj.z), 9) * uz;
-              hit = ddx * ddx + ddy * ddy + ddz * ddz < (UNI ? rl_uni : rl2f[ti * MAXT + info_type(wj)]);
-            } else {
-              wj = s.info[j];
-              const double ddx = mic_ref(x - s.rx[j], R.L[0], R.invL[0]);
-              const double ddy = mic_ref(y - s.ry[j], R.L[1], R.invL[1]);
-              const double ddz = z - s.rz[j];
-              hit = ddx * ddx + ddy * ddy + ddz * ddz < rl2d[ti * MAXT + info_type(wj)];
-            }
+            const int4 qj = s.pfx[j];
+            const float ddx = i2f_coarse(fx_diff(qi.x, qj.x), 9) * ux;
+            const float ddy = i2f_coarse(fx_diff(qi.y, qj.y), 9) * uy;
+            const float ddz = i2f_coarse(fx_diff(qi.z, qj.z), 9) * uz;
+            const bool hit = ddx * ddx + ddy * ddy + ddz * ddz < (UNI ? rl_uni : rl2f[ti * MAXT + info_type(qj.w)]);
             if (hit && j != i) {
               if (cnt < NL_STAGE) mine[cnt] = j;
               else if (cnt < cap) s.nbr[(size_t)cnt * s.Np + i] = j;  // rare: past the staged rows
@@ -651,15 +616,14 @@ void launch_rebuild(const DevState& s, cudaStream_t st, bool force) {
   k_sort_cells<<<gC, B, 0, st>>>(s);
   k_permute<<<gN, B, 0, st>>>(s);
   k_copyback<<<gN, B, 0, st>>>(s);
-  const int var = s.mixed ? (s.rl2_uni > 0.f ? 2 : 1) : 0;
+  const int uni = s.rl2_uni > 0.f ? 1 : 0;
   using KernT = void (*)(DevState);
-  const KernT kerns[3][3] = {{k_nlist<false, false, 1>, k_nlist<true, false, 1>, k_nlist<true, true, 1>},
-                             {k_nlist<false, false, 2>, k_nlist<true, false, 2>, k_nlist<true, true, 2>},
-                             {k_nlist<false, false, 3>, k_nlist<true, false, 3>, k_nlist<true, true, 3>}};
+  const KernT kerns[3][2] = {{k_nlist<false, 1>, k_nlist<true, 1>},
+                             {k_nlist<false, 2>, k_nlist<true, 2>},
+                             {k_nlist<false, 3>, k_nlist<true, 3>}};
   // cells finer along x alone (with 3x3 rows in y, z)
-  const KernT kx[2][3] = {{k_nlist<false, false, 1, 2>, k_nlist<true, false, 1, 2>, k_nlist<true, true, 1, 2>},
-                          {k_nlist<false, false, 1, 3>, k_nlist<true, false, 1, 3>, k_nlist<true, true, 1, 3>}};
-  const KernT kern = (s.nl_hx != s.nl_h) ? kx[s.nl_hx - 2][var] : kerns[s.nl_h - 1][var];
+  const KernT kx[2][2] = {{k_nlist<false, 1, 2>, k_nlist<true, 1, 2>}, {k_nlist<false, 1, 3>, k_nlist<true, 1, 3>}};
+  const KernT kern = (s.nl_hx != s.nl_h) ? kx[s.nl_hx - 2][uni] : kerns[s.nl_h - 1][uni];
   const int gl = std::min((s.N + NL_BLOCK - 1) / NL_BLOCK, s.nsm * 8);
   kern<<<gl, NL_BLOCK, 0, st>>>(s);
   k_clear_flags<<<1, 256, 0, st>>>(s.rebuild_flag, s.nrep, s.rebuilds, s.rep_rebuilds);

@@ -46,6 +46,7 @@ struct DevState {
   int ncell_tot;
   // control words
   float rl2_uni;  // SimConst::rl2_uni_f (0: per-pair list cut-offs)
+  float fx_err;   // largest distance error of the coarse fixed-point differences, in sigma
   int nl_h;       // list-build cells per list cut-off; the search covers (2 nl_h + 1)^3 cells
   int nl_hx;      // the same along x alone (nl_h unless list_cells_x; only with nl_h 1)
   int pair_persist;  // mfa_options.pair_schedule
