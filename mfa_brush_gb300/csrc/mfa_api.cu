@@ -223,6 +223,30 @@ void fill_virial(const mfa_ctx* ctx, const double* acc, int rep, mfa_virial* o) 
   o->step = ctx->sys[rep].s_time + ctx->host_steps;
 }
 
+// The tables of the FP64 noise (NoiseTab), from their definitions.
+NoiseTab noise_tables() {
+  NoiseTab t;
+  const long double pi = 3.14159265358979323846264338327950288L;
+  for (int k = 0; k < 256; ++k) {
+    const long double f = (1.L + (k + 0.5L) / 256.L) / (k < 128 ? 1.L : 2.L);
+    const long double c = (k == 0 || k == 255) ? 1.L : roundl(2048.L / f) / 2048.L;
+    t.lg[k] = make_double2((double)c, (double)(2.L * logl(c)));
+  }
+  for (int e = 0; e < 32; ++e) t.ln2[e] = (double)(2.L * e * logl(2.L));
+  for (int k = 0; k < 1024; ++k)
+    t.cs[k] = make_double2((double)cosl(2.L * pi * k / 1024.L), (double)sinl(2.L * pi * k / 1024.L));
+  return t;
+}
+
+int upload_noise_tables(mfa_ctx* ctx) {
+  static const NoiseTab t = noise_tables();  // constants: once per process (0.7 ms on the Arm host)
+  NoiseTab* d = nullptr;
+  DA(d, 1);
+  CK(cudaMemcpy(d, &t, sizeof t, cudaMemcpyHostToDevice));
+  ctx->S.noise = d;
+  return MFA_OK;
+}
+
 // ewald_k(0) (ewald_k.f90:37-124): the k-vectors in the reference's enumeration order, G(k),
 // and the list of charged particles, of replica rep (the particles p0 .. p0 + n_mon_tot - 1 of the
 // batch; a_type holds the whole batch).
@@ -783,6 +807,7 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
   S.reps = ctx->dreps;
   S.tabf = ctx->dtabf;
   S.tabd = ctx->dtabd;
+  if (!S.mixed) RET(upload_noise_tables(ctx));
   S.rl2_uni = C.rl2_uni_f;
   S.fx_err = (float)fx_err;
   S.nl_h = nl_h;

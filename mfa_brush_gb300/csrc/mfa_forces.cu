@@ -386,88 +386,106 @@ constexpr int PAIR_G = 2;
 
 // Force factor fs of the pair (i, j) along d = r_i - r_j (LJ with the switch-on clamp, DPD with the
 // pair's Philox noise, real-space Coulomb), fluid_fluid.f90:97-261, dpd_forces.f90:45-115,
-// ewald_real.f90:15-33; with EFLAG the pair's share `half` of its energies.
-template <bool MIXED, bool EFLAG>
-__device__ __forceinline__ real_t<MIXED> pair_fs(const DevState& s, const SimConst& C,
-                                                 const PairEntry<real_t<MIXED>>& e, real_t<MIXED> dx,
-                                                 real_t<MIXED> dy, real_t<MIXED> dz, int wj, int j,
-                                                 real_t<MIXED> vix, real_t<MIXED> viy, real_t<MIXED> viz, int tag_i,
-                                                 int p0, uint32_t nkey, real_t<MIXED> r2min,
-                                                 real_t<MIXED> half, real_t<MIXED>& e_lj, real_t<MIXED>& e_c) {
-  using real = real_t<MIXED>;
-  (void)wj;
-  const real sig = cst<MIXED>(C.sig, C.sig_f), gam = cst<MIXED>(C.gamma, C.gamma_f);
-  const real coul_rc2 = cst<MIXED>(C.coul_rc2, C.coul_rc2_f);
-  const real r2raw = dx * dx + dy * dy + dz * dz;
+// ewald_real.f90:15-33; with EFLAG the pair's share `half` of its energies.  FP32 (pair_fs) and
+// FP64 (pair_fs64) forms.
+template <bool EFLAG>
+__device__ __forceinline__ float pair_fs(const DevState& s, const SimConst& C, const PairEntry<float>& e, float dx,
+                                         float dy, float dz, int j, float vix, float viy, float viz, int tag_i,
+                                         int p0, uint32_t nkey, float r2min, float half, float& e_lj, float& e_c) {
+  const float r2raw = dx * dx + dy * dy + dz * dz;
   const int fl = e.flags;
-  real r2 = r2raw;
+  float r2 = r2raw;
   const bool in_lj = r2raw < e.range2;
-  real fs = 0;  // force factor along d = r_i - r_j
+  float fs = 0;  // force factor along d = r_i - r_j
   if (in_lj) {
     r2 = r2raw < r2min ? r2min : r2raw;
-    // MIXED: the hardware reciprocal (2 ulp) instead of the IEEE division sequence
-    real inv_r2;
-    if constexpr (MIXED) inv_r2 = __fdividef(1.f, r2); else inv_r2 = (real)1 / r2;
-    const real s2 = e.sig2 * inv_r2;
-    const real s6 = s2 * s2 * s2;
-    const real s12 = s6 * s6;
-    fs = e.eps4 * ((real)12 * s12 - (real)6 * s6) * inv_r2;
+    // the hardware reciprocal (2 ulp) instead of the IEEE division sequence
+    const float inv_r2 = __fdividef(1.f, r2);
+    const float s2 = e.sig2 * inv_r2;
+    const float s6 = s2 * s2 * s2;
+    const float s12 = s6 * s6;
+    fs = e.eps4 * (12.f * s12 - 6.f * s6) * inv_r2;
     if (EFLAG) e_lj += half * e.eps4 * ((s12 - s6) - e.shift);
   }
   const bool dpd = (in_lj && (fl & PF_DPD_LJ)) || ((fl & PF_DPD_OWN) && r2 < e.dpd_rc2);
   if (dpd) {
-    real vjx, vjy, vjz;
-    int tag_j;
-    if constexpr (MIXED) {
-      float4 v4 = __ldg(&s.vf[j]);
-      vjx = v4.x; vjy = v4.y; vjz = v4.z;
-      tag_j = __float_as_int(v4.w) - p0;
-    } else {
-      dbl4 v4 = s.vd[j];
-      vjx = v4.x; vjy = v4.y; vjz = v4.z;
-      tag_j = (int)__double_as_longlong(v4.w) - p0;
-    }
-    real r, ir;
-    if constexpr (MIXED) {  // one hardware reciprocal square root (2 ulp)
-      ir = rsqrtf(r2);
-      r = r2 * ir;
-    } else {
-      r = sqrt(r2);
-      ir = (real)1 / r;
-    }
-    real wr, wd;
+    const float4 v4 = __ldg(&s.vf[j]);
+    const int tag_j = __float_as_int(v4.w) - p0;
+    const float ir = rsqrtf(r2);  // one hardware reciprocal square root (2 ulp)
+    const float r = r2 * ir;
+    float wr, wd;
     if (C.dpd_weight1) {
       wr = wd = 1;
     } else {
-      wr = (real)1 - r * ((fl & PF_DPD_OWN) ? e.inv_dpd_rc : e.inv_rc);
+      wr = 1.f - r * ((fl & PF_DPD_OWN) ? e.inv_dpd_rc : e.inv_rc);
       wd = wr * wr;
     }
-    real g;
-    if constexpr (MIXED) g = pair_gauss_f(nkey, tag_i, tag_j);
-    else g = pair_gauss_d(nkey, tag_i, tag_j);
-    const real rdot = ((vix - vjx) * dx + (viy - vjy) * dy + (viz - vjz) * dz) * ir;
-    fs += (sig * wr * g - gam * wd * rdot) * ir;
+    const float g = pair_gauss_f(nkey, tag_i, tag_j);
+    const float rdot = ((vix - v4.x) * dx + (viy - v4.y) * dy + (viz - v4.z) * dz) * ir;
+    fs += (C.sig_f * wr * g - C.gamma_f * wd * rdot) * ir;
   }
   if (fl & PF_COUL) {
-    const bool in_c = (coul_rc2 > 0) ? (r2raw < coul_rc2) : in_lj;
+    const bool in_c = (C.coul_rc2_f > 0) ? (r2raw < C.coul_rc2_f) : in_lj;
     if (in_c) {
-      const real rc2 = in_lj ? r2 : r2raw;
-      const real r = sqrt(rc2), ir = (real)1 / r;
-      const real qq = e.qq;
-      const real sqa = cst<MIXED>(C.sqrt_alpha, C.sqrt_alpha_f);
-      const real ec = erfc(sqa * r);
+      const float rc2 = in_lj ? r2 : r2raw;
+      const float r = sqrtf(rc2), ir = 1.f / r;
+      const float qq = e.qq, sqa = C.sqrt_alpha_f;
+      const float ec = erfcf(sqa * r);
       if (EFLAG) e_c += half * qq * ec * ir;
-      const real isp = cst<MIXED>(C.inv_sqrt_pi, C.inv_sqrt_pi_f), ac = cst<MIXED>(C.alpha_c, C.alpha_c_f);
-      fs += (qq * sqa * isp * (real)2 * exp(-ac * rc2) * ir + qq * ec * ir * ir) * ir;
+      fs += (qq * sqa * C.inv_sqrt_pi_f * 2.f * expf(-C.alpha_c_f * rc2) * ir + qq * ec * ir * ir) * ir;
     }
   }
   return fs;
 }
 
-// The pair kernel.  Template switches:
-//   MIXED   FP32 pair arithmetic on the fixed-point views (else FP64 throughout);
+template <bool EFLAG>
+__device__ __forceinline__ double pair_fs64(const DevState& s, const SimConst& C, const PairEntry<double>& e,
+                                            double dx, double dy, double dz, int j, double vix, double viy,
+                                            double viz, int tag_i, int p0, uint32_t nkey, double r2min, double half,
+                                            double& e_lj, double& e_c) {
+  const double r2raw = dx * dx + dy * dy + dz * dz;
+  const int fl = e.flags;
+  const bool in_lj = r2raw < e.range2;
+  const double r2 = (in_lj && r2raw < r2min) ? r2min : r2raw;
+  const bool dpd = (in_lj && (fl & PF_DPD_LJ)) || ((fl & PF_DPD_OWN) && r2 < e.dpd_rc2);
+  const bool in_c = (fl & PF_COUL) && ((C.coul_rc2 > 0) ? (r2raw < C.coul_rc2) : in_lj);
+  double fs = 0;
+  if (!(in_lj || dpd || in_c)) return fs;
+  const double ir = rsqrt64(r2);  // the only root and division of the pair
+  if (in_lj) {
+    const double inv_r2 = ir * ir;
+    const double s2 = e.sig2 * inv_r2;
+    const double s6 = s2 * s2 * s2;
+    const double s12 = s6 * s6;
+    fs = e.eps4 * (12. * s12 - 6. * s6) * inv_r2;
+    if (EFLAG) e_lj += half * e.eps4 * ((s12 - s6) - e.shift);
+  }
+  if (dpd) {
+    const dbl4 v4 = s.vd[j];
+    const int tag_j = (int)__double_as_longlong(v4.w) - p0;
+    double wr, wd;
+    if (C.dpd_weight1) {
+      wr = wd = 1;
+    } else {
+      wr = 1. - r2 * ir * ((fl & PF_DPD_OWN) ? e.inv_dpd_rc : e.inv_rc);
+      wd = wr * wr;
+    }
+    const double g = pair_gauss_d(s.noise, nkey, tag_i, tag_j);
+    const double rdot = ((vix - v4.x) * dx + (viy - v4.y) * dy + (viz - v4.z) * dz) * ir;
+    fs += (C.sig * wr * g - C.gamma * wd * rdot) * ir;
+  }
+  if (in_c) {
+    const double r = r2 * ir, qq = e.qq, ec = erfc(C.sqrt_alpha * r);
+    if (EFLAG) e_c += half * qq * ec * ir;
+    fs += (qq * C.sqrt_alpha * C.inv_sqrt_pi * 2. * exp(-C.alpha_c * r2) * ir + qq * ec * ir * ir) * ir;
+  }
+  return fs;
+}
+
+// The pair kernel of the mixed mode: FP32 pair arithmetic on the fixed-point views.  Template
+// switches:
 //   EFLAG   energies and the virial into the accumulators;
-//   FUSED   the fused mixed-precision step (MIXED only): FP32 partial sums over each batch of kept
+//   FUSED   the fused mixed-precision step: FP32 partial sums over each batch of kept
 //           pairs are added to an FP64 per-particle total, together with the bonded, wall and body
 //           forces of the particle, and the total is stored (rounded to FP32) in the force array
 //           that the integrator reads;
@@ -487,31 +505,23 @@ __device__ __forceinline__ real_t<MIXED> pair_fs(const DevState& s, const SimCon
 //           of blockDim.x particles from a queue (s.pair_q[0], one atomic ticket per tile, no
 //           waiting) and the last block to finish resets the queue for the next launch.  Compiled
 //           for 8 resident blocks per SM (64 registers): at 9 the tile loop spills.
-template <bool MIXED, bool EFLAG, bool FUSED = false, bool BONDED = false, bool UNI = false, bool PERSIST = false,
+template <bool EFLAG, bool FUSED = false, bool BONDED = false, bool UNI = false, bool PERSIST = false,
           bool INTEG = false>
 // Resident blocks per SM: 10 for the kernel with the integration in its tail (48 registers and a
 // 52-byte spill; 0.558 against 0.584 ms per step at 9 blocks, 56 registers; 11 or 12 blocks leave
 // 40 registers and spill 124 bytes: 0.579 ms), 9 for the other fused forms, 8 for the persistent
 // schedule (its tile loop spills at 9).
-__global__ void __launch_bounds__(128, MIXED ? (PERSIST ? 8 : ((INTEG && !EFLAG) ? 10 : 9)) : 4) k_pair(DevState s, SimConst C, bool accumulate,
-                                                                             Acc acc, int bmask = 0) {
-  using real = real_t<MIXED>;
-  static_assert(!FUSED || MIXED, "the fused form is the mixed-precision one");
+__global__ void __launch_bounds__(128, PERSIST ? 8 : ((INTEG && !EFLAG) ? 10 : 9)) k_pair(DevState s, SimConst C,
+                                                                                          bool accumulate, Acc acc,
+                                                                                          int bmask = 0) {
+  using real = float;
   static_assert(!BONDED || FUSED, "bonded terms are fused only into the fused form");
   static_assert(!INTEG || (FUSED && !PERSIST), "the integration is fused into the fused form");
   __shared__ PairEntry<real> tab[NPAIR];
-  __shared__ float scr[MIXED ? 1 : NPAIR];  // FP64: the FP32 screening thresholds
   // FUSED: the particle's FP64 total, in shared memory while the pair loop runs (registers are
   // scarce there; it is touched once per batch)
   __shared__ double ftot[FUSED ? 3 : 1][FUSED ? 128 : 1];
-  for (int k = threadIdx.x; k < NPAIR; k += blockDim.x) {
-    if constexpr (MIXED) {
-      tab[k] = s.tabf[k];
-    } else {
-      tab[k] = s.tabd[k];
-      scr[k] = s.tabf[k].screen2;
-    }
-  }
+  for (int k = threadIdx.x; k < NPAIR; k += blockDim.x) tab[k] = s.tabf[k];
   __shared__ int tile_sh;
   const int ntile = (s.N + blockDim.x - 1) / blockDim.x;
   for (int pass = 0;; ++pass) {
@@ -560,7 +570,7 @@ __global__ void __launch_bounds__(128, MIXED ? (PERSIST ? 8 : ((INTEG && !EFLAG)
   // variant with bonded terms, of the bonded virial partials after it: the batch is dead once
   // the pair loop ends, and a barrier separates the two uses, so the variant keeps room for L1.
   constexpr int JL_WORDS = PAIR_BATCH * 128;
-  constexpr int BV_WORDS = (EFLAG && BONDED) ? 128 * (int)(sizeof(BondVir<real_t<MIXED>>) / 4) : 0;
+  constexpr int BV_WORDS = (EFLAG && BONDED) ? 128 * (int)(sizeof(BondVir<real>) / 4) : 0;
   __shared__ __align__(16) int pair_pool[JL_WORDS > BV_WORDS ? JL_WORDS : BV_WORDS];
   real fx = 0, fy = 0, fz = 0;        // the current batch (FUSED), else the whole sum
   real e_lj = 0, e_c = 0;
@@ -574,38 +584,17 @@ __global__ void __launch_bounds__(128, MIXED ? (PERSIST ? 8 : ((INTEG && !EFLAG)
     const int p0 = R.p0;
     // own position / velocity
     const int4 qi = __ldg(&s.pfx[i]);
-    dbl4 pi;
-    real vix, viy, viz;
-    int tag_i;
-    real ux = 0, uy = 0, uz = 0;
-    if constexpr (MIXED) {
-      float4 v4 = __ldg(&s.vf[i]);
-      vix = v4.x; viy = v4.y; viz = v4.z;
-      tag_i = __float_as_int(v4.w) - p0;
-      ux = R.ufx_f[0]; uy = R.ufx_f[1]; uz = R.ufx_f[2];
-    } else {
-      pi = s.pd[i];
-      dbl4 v4 = s.vd[i];
-      vix = v4.x; viy = v4.y; viz = v4.z;
-      tag_i = (int)__double_as_longlong(v4.w) - p0;
-    }
-    const double L0 = R.L[0], L1 = R.L[1], iL0 = R.invL[0], iL1 = R.invL[1];
+    const float4 vi = __ldg(&s.vf[i]);
+    const int tag_i = __float_as_int(vi.w) - p0;
+    const float ux = R.ufx_f[0], uy = R.ufx_f[1], uz = R.ufx_f[2];
     const uint32_t nkey = pair_key(R.seed, step);  // the replica's noise key of this step
     const int* __restrict__ nb = s.nbr + i;
     auto delta = [&](int j, real& dx, real& dy, real& dz) -> int {
-      if constexpr (MIXED) {
-        const int4 qj = __ldg(&s.pfx[j]);
-        dx = i2f_fast(fx_diff(qi.x, qj.x)) * ux;
-        dy = i2f_fast(fx_diff(qi.y, qj.y)) * uy;
-        dz = i2f_fast(fx_diff(qi.z, qj.z)) * uz;
-        return qj.w;
-      } else {
-        const dbl4 pj = s.pd[j];
-        dx = mic_ref(pi.x - pj.x, L0, iL0);
-        dy = mic_ref(pi.y - pj.y, L1, iL1);
-        dz = pi.z - pj.z;
-        return (int)__double_as_longlong(pj.w);
-      }
+      const int4 qj = __ldg(&s.pfx[j]);
+      dx = i2f_fast(fx_diff(qi.x, qj.x)) * ux;
+      dy = i2f_fast(fx_diff(qi.y, qj.y)) * uy;
+      dz = i2f_fast(fx_diff(qi.z, qj.z)) * uz;
+      return qj.w;
     };
     // Two phases per batch: (1) screen list entries with the cheap distance test and keep the
     // ones inside any interaction range, (2) evaluate LJ + DPD + Coulomb on the kept pairs only.
@@ -618,21 +607,15 @@ __global__ void __launch_bounds__(128, MIXED ? (PERSIST ? 8 : ((INTEG && !EFLAG)
     // gathers
     int* const jl = pair_pool + threadIdx.x;
     int k = 0;
-    // screening against the largest cut-off of the type pair, in FP32 on the fixed-point views in
-    // both precisions, with the coarse conversion (512 fixed-point units of resolution, inside the
-    // 2e-4 margin of screen2); the evaluation then tests the exact distance
-    const float cx = R.ufx_f[0] * 512.f, cy = R.ufx_f[1] * 512.f, cz = R.ufx_f[2] * 512.f;
+    // screening against the largest cut-off of the type pair, with the coarse conversion (512
+    // fixed-point units of resolution, inside the margin of screen2)
+    const float cx = ux * 512.f, cy = uy * 512.f, cz = uz * 512.f;
     auto screen = [&](int j) -> bool {
       const int4 qj = __ldg(&s.pfx[j]);
       const float dx = i2f_coarse(fx_diff(qi.x, qj.x), 9) * cx;
       const float dy = i2f_coarse(fx_diff(qi.y, qj.y), 9) * cy;
       const float dz = i2f_coarse(fx_diff(qi.z, qj.z), 9) * cz;
-      const int tt = ti * MAXT + info_type(qj.w);
-      float lim;
-      if constexpr (UNI) lim = C.scr2_uni_f;
-      else if constexpr (MIXED) lim = tab[tt].screen2;
-      else lim = scr[tt];
-      return dx * dx + dy * dy + dz * dz < lim;
+      return dx * dx + dy * dy + dz * dz < (UNI ? C.scr2_uni_f : tab[ti * MAXT + info_type(qj.w)].screen2);
     };
     while (k < n) {
       int m = 0;
@@ -671,17 +654,12 @@ __global__ void __launch_bounds__(128, MIXED ? (PERSIST ? 8 : ((INTEG && !EFLAG)
         const PairEntry<real>& e = tab[ti * MAXT + info_type(wj)];
         // half of each mobile pair (both ends sum it); a fixed wall bead has no list of its own
         const real half = info_mobile(wj) ? (real)0.5 : (real)1;
-        const real fs = pair_fs<MIXED, EFLAG>(s, C, e, dx, dy, dz, wj, j, vix, viy, viz, tag_i, p0, nkey,
-                                              r2min, half, e_lj, e_c);
-        if constexpr (MIXED) {  // unmerged products and sums: alike with and without energies
-          fx = __fadd_rn(fx, __fmul_rn(fs, dx));
-          fy = __fadd_rn(fy, __fmul_rn(fs, dy));
-          fz = __fadd_rn(fz, __fmul_rn(fs, dz));
-        } else {
-          fx += fs * dx;
-          fy += fs * dy;
-          fz += fs * dz;
-        }
+        const real fs = pair_fs<EFLAG>(s, C, e, dx, dy, dz, j, vi.x, vi.y, vi.z, tag_i, p0, nkey, r2min, half,
+                                       e_lj, e_c);
+        // unmerged products and sums: alike with and without energies
+        fx = __fadd_rn(fx, __fmul_rn(fs, dx));
+        fy = __fadd_rn(fy, __fmul_rn(fs, dy));
+        fz = __fadd_rn(fz, __fmul_rn(fs, dz));
         if (EFLAG) sym_add(wv, half * fs, dx, dy, dz);
       }
       if constexpr (FUSED) {  // the batch's FP32 partial into the FP64 total
@@ -712,7 +690,7 @@ __global__ void __launch_bounds__(128, MIXED ? (PERSIST ? 8 : ((INTEG && !EFLAG)
     if (active) {
       if constexpr (BONDED) {
         real fb[3] = {0, 0, 0};
-        hb = bonded_of<MIXED, EFLAG>(s, C, bmask, i, w, fb, eb, &bv);
+        hb = bonded_of<true, EFLAG>(s, C, bmask, i, w, fb, eb, &bv);
         fxd += f2d_fast(fb[0]);
         fyd += f2d_fast(fb[1]);
         fzd += f2d_fast(fb[2]);
@@ -783,6 +761,162 @@ __global__ void __launch_bounds__(128, MIXED ? (PERSIST ? 8 : ((INTEG && !EFLAG)
   }
 }
 
+// The pair kernel of the FP64 mode.  The FP64 pipe bounds it (an FP64 instruction of a warp holds it
+// for 16 clocks however many lanes are active), so (1) the list is screened in FP32 on the fixed-point
+// view, (2) the kept pairs of a warp's 32 particles are put together and evaluated 32 at a time, a
+// lane per pair whoever owns it (a thread per particle left half of the lanes idle: the kept counts
+// of neighbours differ), and (3) the roots, divisions and noise are those of mfa_dev.cuh.  The
+// products go back through shared memory and each owner adds its own in list order, so the sums do
+// not depend on which lane evaluated a pair.  A warp on a replica boundary evaluates each lane's own
+// pairs instead, so that the energy sums (by lane) stay with their replica.
+constexpr int P64_BATCH = 8;  // kept pairs per particle and round
+struct Pair64Warp {           // shared memory of a warp
+  double own[6][32];          // its particles' positions and half-step velocities
+  double f[3][32 * P64_BATCH];  // force of each kept pair on its owner
+  int tag[32], type[32];
+  int j[32 * P64_BATCH];
+  unsigned char who[32 * P64_BATCH];
+};
+
+template <bool EFLAG, bool UNI>
+__global__ void __launch_bounds__(128, 4) k_pair64(DevState s, SimConst C, bool accumulate, Acc acc) {
+  extern __shared__ __align__(16) unsigned char sh_raw[];
+  __shared__ PairEntry<double> tab[NPAIR];
+  __shared__ float scr[NPAIR];
+  for (int k = threadIdx.x; k < NPAIR; k += blockDim.x) {
+    tab[k] = s.tabd[k];
+    scr[k] = s.tabf[k].screen2;
+  }
+  __syncthreads();
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  Pair64Warp& W = reinterpret_cast<Pair64Warp*>(sh_raw)[threadIdx.x >> 5];
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool inside = i < s.N;
+  const int w = __ldg(&s.info[min(i, s.N - 1)]);  // (the lanes past the end take the last replica)
+  const bool active = inside && info_mobile(w);
+  const int rep = info_rep(w);
+  const bool one = __all_sync(FULL, rep == __shfl_sync(FULL, rep, 0));
+  const RepDesc& R = s.reps[rep];
+  const long long step = R.s_time + *s.steps_done;
+  const double r2min = C.force_switch_on ? r2min_of(C, step) : 0.;
+  const int p0 = R.p0, ti = info_type(w);
+  const uint32_t nkey = pair_key(R.seed, step);
+  const double L0 = R.L[0], L1 = R.L[1], iL0 = R.invL[0], iL1 = R.invL[1];
+  const int n = active ? __ldg(&s.nn[i]) : 0;
+  const int* __restrict__ nb = s.nbr + i;
+  int4 qi = make_int4(0, 0, 0, 0);
+  if (active) {
+    qi = __ldg(&s.pfx[i]);
+    const dbl4 x = s.pd[i], v = s.vd[i];
+    W.own[0][lane] = x.x; W.own[1][lane] = x.y; W.own[2][lane] = x.z;
+    W.own[3][lane] = v.x; W.own[4][lane] = v.y; W.own[5][lane] = v.z;
+    W.tag[lane] = (int)__double_as_longlong(v.w) - p0;
+    W.type[lane] = ti;
+  }
+  const float cx = R.ufx_f[0] * 512.f, cy = R.ufx_f[1] * 512.f, cz = R.ufx_f[2] * 512.f;
+  auto screen = [&](int j) -> bool {  // as the mixed kernel's
+    const int4 qj = __ldg(&s.pfx[j]);
+    const float dx = i2f_coarse(fx_diff(qi.x, qj.x), 9) * cx;
+    const float dy = i2f_coarse(fx_diff(qi.y, qj.y), 9) * cy;
+    const float dz = i2f_coarse(fx_diff(qi.z, qj.z), 9) * cz;
+    return dx * dx + dy * dy + dz * dz < (UNI ? C.scr2_uni_f : scr[ti * MAXT + info_type(qj.w)]);
+  };
+  double fx = 0., fy = 0., fz = 0., e_lj = 0., e_c = 0.;
+  double wv[6] = {0., 0., 0., 0., 0., 0.};  // EFLAG: pair virial, xx yy zz xy xz yz
+  int k = 0;
+  while (__any_sync(FULL, k < n)) {
+    // the lane's next kept pairs, at most P64_BATCH, first in its own row of W.j
+    int m = 0;
+    while (k < n && m < P64_BATCH) {
+      constexpr int G = 4;  // entries whose loads are in flight together
+      if (k + G <= n && m <= P64_BATCH - G) {
+        int jg[G];
+        bool hg[G];
+#pragma unroll
+        for (int u = 0; u < G; ++u) jg[u] = __ldg(nb + (size_t)(k + u) * s.Np);
+#pragma unroll
+        for (int u = 0; u < G; ++u) hg[u] = screen(jg[u]);
+#pragma unroll
+        for (int u = 0; u < G; ++u)
+          if (hg[u]) W.j[lane * P64_BATCH + m++] = jg[u];
+        k += G;
+      } else {
+        const int j = __ldg(nb + (size_t)k * s.Np);
+        ++k;
+        if (screen(j)) W.j[lane * P64_BATCH + m++] = j;
+      }
+    }
+    // then together: owner after owner, each in list order
+    int at = m;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(FULL, at, o);
+      if (lane >= o) at += y;
+    }
+    const int total = __shfl_sync(FULL, at, 31);
+    at -= m;
+    int mine[P64_BATCH];
+#pragma unroll
+    for (int t = 0; t < P64_BATCH; ++t) mine[t] = (t < m) ? W.j[lane * P64_BATCH + t] : 0;
+    __syncwarp();
+#pragma unroll
+    for (int t = 0; t < P64_BATCH; ++t)
+      if (t < m) {
+        W.j[at + t] = mine[t];
+        W.who[at + t] = (unsigned char)lane;
+      }
+    __syncwarp();
+    const int rounds = one ? (total + 31) >> 5 : (int)__reduce_max_sync(FULL, (unsigned)m);
+    for (int t = 0; t < rounds; ++t) {
+      const int q = one ? 32 * t + lane : at + t;
+      if (one ? q < total : t < m) {
+        const int j = W.j[q], o = W.who[q];
+        const dbl4 pj = s.pd[j];
+        const double dx = mic_fast(W.own[0][o] - pj.x, L0, iL0);
+        const double dy = mic_fast(W.own[1][o] - pj.y, L1, iL1);
+        const double dz = W.own[2][o] - pj.z;
+        const int wj = (int)__double_as_longlong(pj.w);
+        // half of each mobile pair (both ends sum it); a fixed wall bead has no list of its own
+        const double half = info_mobile(wj) ? 0.5 : 1.;
+        const double fs = pair_fs64<EFLAG>(s, C, tab[W.type[o] * MAXT + info_type(wj)], dx, dy, dz, j, W.own[3][o],
+                                           W.own[4][o], W.own[5][o], W.tag[o], p0, nkey, r2min, half, e_lj, e_c);
+        W.f[0][q] = fs * dx;
+        W.f[1][q] = fs * dy;
+        W.f[2][q] = fs * dz;
+        if (EFLAG) sym_add(wv, half * fs, dx, dy, dz);
+      }
+    }
+    __syncwarp();
+    for (int t = 0; t < m; ++t) {
+      fx += W.f[0][at + t];
+      fy += W.f[1][at + t];
+      fz += W.f[2][at + t];
+    }
+    __syncwarp();
+  }
+  if (inside) {
+    if (!accumulate) {
+      s.fx[i] = fx;
+      s.fy[i] = fy;
+      s.fz[i] = fz;
+    } else if (active) {
+      s.fx[i] += fx;
+      s.fy[i] += fy;
+      s.fz[i] += fz;
+    }
+  }
+  if (EFLAG) {
+    int sl[8];
+    double v[8];
+    sl[0] = O_VFF; v[0] = e_lj;
+    sl[1] = O_VCOUL; v[1] = e_c;
+    sym_slots(sl + 2, v + 2, O_VIR + 9 * V_PAIR, wv);
+    // (a warp of one replica: every lane has evaluated pairs, the ends' lanes too)
+    obs_push<double, 8>(acc, sl, v, rep, one ? true : active);
+  }
+}
+
 void launch_pair(const DevState& s, const SimConst& C, cudaStream_t st, bool accumulate, bool eflag, Acc acc,
                  int block, int bonded_mask, bool integ) {
   // 32, 64 or 128 threads per block (the kernel is compiled for at most 128); anything else
@@ -793,22 +927,22 @@ void launch_pair(const DevState& s, const SimConst& C, cudaStream_t st, bool acc
   if (s.mixed && !accumulate) {  // the fused step
     using KernT = void (*)(DevState, SimConst, bool, Acc, int);
     // [bonded][uni][eflag]
-    const KernT ks[2][2][2] = {{{k_pair<true, false, true>, k_pair<true, true, true>},
-                                {k_pair<true, false, true, false, true>, k_pair<true, true, true, false, true>}},
-                               {{k_pair<true, false, true, true>, k_pair<true, true, true, true>},
-                                {k_pair<true, false, true, true, true>, k_pair<true, true, true, true, true>}}};
+    const KernT ks[2][2][2] = {{{k_pair<false, true>, k_pair<true, true>},
+                                {k_pair<false, true, false, true>, k_pair<true, true, false, true>}},
+                               {{k_pair<false, true, true>, k_pair<true, true, true>},
+                                {k_pair<false, true, true, true>, k_pair<true, true, true, true>}}};
     // the persistent schedule for the steps without energies: [bonded][uni]
-    const KernT kp[2][2] = {{k_pair<true, false, true, false, false, true>, k_pair<true, false, true, false, true, true>},
-                            {k_pair<true, false, true, true, false, true>, k_pair<true, false, true, true, true, true>}};
+    const KernT kp[2][2] = {{k_pair<false, true, false, false, true>, k_pair<false, true, false, true, true>},
+                            {k_pair<false, true, true, false, true>, k_pair<false, true, true, true, true>}};
     // with the step's integration in the tail: [eflag][bonded][uni]
-    const KernT ki[2][2][2] = {{{k_pair<true, false, true, false, false, false, true>,
-                                 k_pair<true, false, true, false, true, false, true>},
-                                {k_pair<true, false, true, true, false, false, true>,
-                                 k_pair<true, false, true, true, true, false, true>}},
-                               {{k_pair<true, true, true, false, false, false, true>,
-                                 k_pair<true, true, true, false, true, false, true>},
-                                {k_pair<true, true, true, true, false, false, true>,
-                                 k_pair<true, true, true, true, true, false, true>}}};
+    const KernT ki[2][2][2] = {{{k_pair<false, true, false, false, false, true>,
+                                 k_pair<false, true, false, true, false, true>},
+                                {k_pair<false, true, true, false, false, true>,
+                                 k_pair<false, true, true, true, false, true>}},
+                               {{k_pair<true, true, false, false, false, true>,
+                                 k_pair<true, true, false, true, false, true>},
+                                {k_pair<true, true, true, false, false, true>,
+                                 k_pair<true, true, true, true, false, true>}}};
     const int bi = bonded_mask ? 1 : 0, ui = uni ? 1 : 0;
     if (integ) {
       ki[eflag ? 1 : 0][bi][ui]<<<g, B, 0, st>>>(s, C, false, acc, bonded_mask);
@@ -822,13 +956,16 @@ void launch_pair(const DevState& s, const SimConst& C, cudaStream_t st, bool acc
       ks[bi][ui][eflag ? 1 : 0]<<<g, B, 0, st>>>(s, C, false, acc, bonded_mask);
     }
   } else if (s.mixed) {  // the drop-in: added to the FP64 force
-    if (eflag) k_pair<true, true><<<g, B, 0, st>>>(s, C, true, acc);
-    else k_pair<true, false><<<g, B, 0, st>>>(s, C, true, acc);
+    if (eflag) k_pair<true><<<g, B, 0, st>>>(s, C, true, acc);
+    else k_pair<false><<<g, B, 0, st>>>(s, C, true, acc);
   } else {
-    using KernT = void (*)(DevState, SimConst, bool, Acc, int);
-    const KernT kd[2][2] = {{k_pair<false, false>, k_pair<false, true>},
-                            {k_pair<false, false, false, false, true>, k_pair<false, true, false, false, true>}};
-    kd[uni ? 1 : 0][eflag ? 1 : 0]<<<g, B, 0, st>>>(s, C, accumulate, acc, 0);
+    using KernT = void (*)(DevState, SimConst, bool, Acc);
+    const KernT kd[2][2] = {{k_pair64<false, false>, k_pair64<true, false>},
+                            {k_pair64<false, true>, k_pair64<true, true>}};
+    // the warps are independent: one per block while that leaves SMs without a full block of four
+    const int B64 = (block == 32 || block == 64 || block == 128) ? block : (s.N < 128 * 4 * s.nsm ? 32 : 128);
+    kd[uni ? 1 : 0][eflag ? 1 : 0]<<<(s.N + B64 - 1) / B64, B64, B64 / 32 * sizeof(Pair64Warp), st>>>(s, C, accumulate,
+                                                                                                   acc);
   }
 }
 

@@ -66,6 +66,7 @@ struct DevState {
   const RepDesc* reps;
   const PairEntry<float>* tabf;
   const PairEntry<double>* tabd;
+  const NoiseTab* noise;  // FP64 mode
 };
 
 // energy accumulators: slot-major [NOBS][nrep]
