@@ -125,6 +125,7 @@ int check_status(mfa_ctx* ctx) {
   CK(cudaStreamSynchronize(ctx->st));
   unsigned s = ctx->h_status[0];
   note_list_count(ctx);
+  if (s & ST_BARRIER) return fail(ctx, MFA_ERR_CUDA, "the cell sort's grid barrier timed out");
   if (s & ST_NAN) return fail(ctx, MFA_ERR_NAN, "non-finite position detected");
   if (s & ST_OUT_OF_BOX) return fail(ctx, MFA_ERR_OUT_OF_BOX, "a particle left the channel");
   if (s & ST_NLIST_OVERFLOW) {
@@ -159,13 +160,12 @@ __global__ void k_clear_overflow(unsigned* status) {
 }
 
 // rebuild of the flagged replicas (all of them when forced); counts and clears the flags
-constexpr int kRebuildLaunches = 11;
 void rebuild(mfa_ctx* ctx, bool force) {
   launch_rebuild(ctx->S, ctx->st, force);
-  ctx->launches += kRebuildLaunches;
+  ctx->launches += rebuild_launches();
 }
 
-// Graph form of the skin check: the IF body (the eleven rebuild kernels) runs only on steps whose
+// Graph form of the skin check: the IF body (the rebuild kernels) runs only on steps whose
 // position update raised the flag of some replica; other steps launch nothing.
 __global__ void k_cond_rebuild(const int* flag, cudaGraphConditionalHandle h) {
   cudaGraphSetConditional(h, flag[0] ? 1u : 0u);
@@ -623,7 +623,7 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
   ctx->v_coul_self.assign(n_rep, 0.);
   ctx->v_ww.assign(n_rep, 0.);
   ctx->v_ff_walls.assign(n_rep, 0.);
-  int cell_off = 0, p0 = 0;
+  int cell_off = 0, row_off = 0, plane_off = 0, p0 = 0;
   double dens_max = 0.;
   // list-build cells per list cut-off: as asked, else the fewest (the largest cells: fewest rows
   // to walk) that every replica's box holds 2h+1 of in x and y
@@ -668,7 +668,7 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
       R.nc[d] = nc;
       R.inv_lc[d] = (double)nc / s.boundary[d];
       R.lc_f[d] = (float)(s.boundary[d] / nc);
-      R.cpu_f[d] = (float)(512. * nc / ((d < 2) ? 4294967296.0 : 1073741824.0));
+      R.L_f[d] = (float)s.boundary[d];
       if (d == 2) {
         R.zlim_f[0] = (float)(-s.boundary[2] / nc);
         R.zlim_f[1] = (float)(s.boundary[2] + s.boundary[2] / nc);
@@ -677,6 +677,10 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
     R.ncell = R.nc[0] * R.nc[1] * R.nc[2];
     R.cell_off = cell_off;
     cell_off += R.ncell;
+    R.row_off = row_off;
+    row_off += R.nc[1] * R.nc[2];
+    R.plane_off = plane_off;
+    plane_off += R.nc[2];
     R.p0 = p0;
     R.n_part = s.n_part;
     R.n_mon_tot = s.n_mon_tot;
@@ -764,12 +768,22 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
     DA(S.pd, Nn); DA(S.vd, Nn);
   }
   DA(S.ref, Nn);
+  DA(S.lp, Nn);
   DA(S.nn, Nn);
   DA(S.cell_of, Nn); DA(S.rank, Nn); DA(S.perm, Nn);
   S.ncell_tot = cell_off;
-  DA(S.cell_count, cell_off + 1);  // zero between rebuilds: k_bin counts up, k_sort_cells zeroes
+  DA(S.cell_count, cell_off + 1);  // (this and the row and plane counts: zero between rebuilds)
+  DA(S.row_count, row_off);
+  DA(S.plane_count, plane_off);
+  // room for the tags of a cell: the mean of the densest replica and three standard deviations of
+  // independent particles (a liquid's are smaller; a denser cell costs that rebuild two passes more)
+  {
+    double mean = 0.;
+    for (const RepDesc& R : ctx->hreps) mean = std::max(mean, (double)R.n_part / R.ncell);
+    S.bucket_cap = ((int)std::ceil(mean + 3. * std::sqrt(mean) + 2.) + 3) / 4 * 4;
+  }
+  DA(S.bucket, (size_t)cell_off * S.bucket_cap);
   DA(S.cell_start, cell_off + 1);
-  DA(S.scan_blk, 2 * 256);  // the cell-start scan's block sums and offsets
   DA(S.rebuild_flag, 1 + n_rep);
   DA(S.steps_alt, 1);
   S.sync_alt = 0;
@@ -779,9 +793,9 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
   DA(S.wl_p, n_rep + 1);
   DA(S.wl_c, n_rep + 1);
   DA(S.wl_k, n_rep + 1);
-  DA(S.wl_n, 2);
+  DA(S.wl_y, n_rep + 1);
+  DA(S.wl_n, 5);
   CK(cudaDeviceGetAttribute(&S.nsm, cudaDevAttrMultiProcessorCount, ctx->device));
-  DA(S.cell_rep, cell_off);
   DA(S.rebuilds, 1);
   DA(S.rep_rebuilds, n_rep);
   DA(S.status, 2);  // [0] status bits, [1] largest list count of the rebuilds so far
@@ -835,12 +849,10 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
   CK(cudaMemsetAsync(S.rebuild_flag, 0, sizeof(int) * (1 + n_rep), st));
   CK(cudaMemsetAsync(S.cell_count, 0, sizeof(int) * (cell_off + 1), st));
   CK(cudaMemsetAsync(S.pair_q, 0, sizeof(int) * 2, st));
-  {
-    std::vector<int> cr(std::max(cell_off, 1));
-    for (int r = 0; r < n_rep; ++r)
-      for (int c = 0; c < ctx->hreps[r].ncell; ++c) cr[ctx->hreps[r].cell_off + c] = r;
-    CK(cudaMemcpy(S.cell_rep, cr.data(), sizeof(int) * cell_off, cudaMemcpyHostToDevice));
-  }
+  CK(cudaMemsetAsync(S.wl_n, 0, sizeof(int) * 5, st));
+  CK(cudaMemsetAsync(S.row_count, 0, sizeof(int) * row_off, st));
+  CK(cudaMemsetAsync(S.plane_count, 0, sizeof(int) * plane_off, st));
+  CK(cudaMemcpyAsync(S.cell_start + cell_off, &ctx->N, sizeof(int), cudaMemcpyHostToDevice, st));  // the last cell's end
   CK(cudaMemsetAsync(S.rep_rebuilds, 0, sizeof(long long) * n_rep, st));
   CK(cudaMemsetAsync(S.status, 0, 2 * sizeof(unsigned), st));
   CK(cudaMemsetAsync(S.steps_done, 0, sizeof(long long), st));
@@ -1232,7 +1244,7 @@ static long long issue_steps(mfa_ctx* ctx, int n, int phase, bool prof, bool obs
       L += 1;  // the rebuild body's launches are not counted: they run only when triggered
     } else {
       launch_rebuild(Sr, st, false);
-      L += kRebuildLaunches;
+      L += rebuild_launches();
     }
     const bool split = prof || (obs && ef);
     if (fused_at(k)) {  // forces and this step's integration in one kernel; the views move across

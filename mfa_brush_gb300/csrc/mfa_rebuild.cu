@@ -3,20 +3,21 @@
 // Replaces the reference's neighbour bookkeeping: the linked cells of cell_list.f90:56-268
 // (BIN_TYPE 2, rebuilt incrementally every step) and the skin-based Verlet lists of
 // binning.f90 / check_skin.f90 (BIN_TYPE 0, rebuilt when a particle moved > skin/2).  Here the
-// list is rebuilt when the position kernel has raised `rebuild_flag` (displacement > skin/2):
+// list is rebuilt when the position kernel has raised `rebuild_flag` (displacement > skin/2), by
+// two kernels.  k_sort, a cooperative launch whose phases a grid barrier separates:
 //   1. bin:      cell of every particle on the replica's list grid (cell edge >= r_cut_max+skin),
-//                per-cell counts with one atomic per particle;
-//   2. scan:     cell starts from the counts of the rebuilt replicas' cells (three kernels);
-//   3. place:    particle -> (cell start + atomic rank);
-//   4. order:    each cell's segment sorted by tag (cells hold a handful of particles), so the
-//                final order (replica, cell, tag) and every later FP sum order are deterministic;
-//   5. permute:  FP64 state gathered into the new order, views and rebuild references rewritten;
-//   6. list:     full neighbour list over the 27 surrounding cells (x,y periodic, z bounded).
+//                counts per cell, cell row and cell plane, the particle's tag into its cell's bucket;
+//   2. starts:   a warp per row of cells: the planes and rows before it, then a scan along the row;
+//   3. permute:  a particle's slot is its cell's start plus the number of smaller tags in the bucket:
+//                the FP64 state goes there (the final order (replica, cell, tag) and every later
+//                FP sum order are deterministic);
+//   4. back:     the state in the new order, views and rebuild references rewritten.
+// and k_nlist, the full neighbour list over the surrounding cells (x,y periodic, z bounded).
 // The decision is per replica, as the reference decides per system: the position kernel raises the
-// flag of the replica whose particle moved.  k_worklist lists the flagged replicas with prefix sums
-// of their particles, cells and list chunks, and every kernel after it strides over that work on a
-// grid of fixed size; the other replicas' slots, cells and lists stay as they are (a replica's
-// slots are one fixed range, its cells one fixed range, and its lists name only its own slots).
+// flag of the replica whose particle moved.  Every block lists the flagged replicas with prefix sums
+// of their particles and cells, and the phases stride over that work; the other replicas' slots,
+// cells and lists stay as they are (a replica's slots are one fixed range, its cells one fixed range,
+// and its lists name only its own slots).
 // In a captured CUDA graph the sequence sits in the body of a conditional node that runs only on
 // steps where some replica is flagged.
 #include <algorithm>
@@ -36,123 +37,30 @@ __device__ __forceinline__ void cell_coords(const RepDesc& R, const int4& q, int
 }
 
 // ---- work list ------------------------------------------------------------------------------
-// The kernels of a rebuild stride over the work of the listed replicas only (their particles,
-// cells or list-builder chunks) on grids of a fixed size, so a rebuild of a few replicas costs
-// little more than their own work.
-constexpr int WL_THREADS = 1024;
-// particles per block of the list builder (one chunk of a replica's slots)
-constexpr int NL_BLOCK = 128;
+// particles per chunk of the list builder (a warp's, consecutive slots of one replica)
+constexpr int NL_CHUNK = 32;
+constexpr int SORT_T = 512;      // threads per block of k_sort
+constexpr int SORT_PER_SM = 2;   // its blocks per SM (3 or 4: 0.5-2 % slower steps, fewer registers)
+constexpr int WL_SHARED = 1024;  // replicas whose work list fits in shared memory
 
-// The replicas to rebuild (flagged, or all when forced) and the prefix sums of their particles,
-// cells and list chunks: one block, a scan over the replicas in chunks of its threads.
-__global__ void __launch_bounds__(WL_THREADS) k_worklist(DevState s, bool force) {
-  __shared__ int sc[4][WL_THREADS / 32];
-  __shared__ int carry[4];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const bool any = force || s.rebuild_flag[0] != 0;
-  if (threadIdx.x < 4) carry[threadIdx.x] = 0;
-  __syncthreads();
-  for (int base = 0; base < s.nrep && any; base += WL_THREADS) {
-    const int r = base + threadIdx.x;
-    const bool sel = r < s.nrep && (force || s.rebuild_flag[1 + r] != 0);
-    int v[4] = {0, 0, 0, 0};
-    if (sel) {
-      const RepDesc& R = s.reps[r];
-      v[0] = 1; v[1] = R.n_part; v[2] = R.ncell; v[3] = (R.n_part + NL_BLOCK - 1) / NL_BLOCK;
-    }
-    int x[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {  // inclusive warp scans
-      x[q] = v[q];
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x[q], o);
-        if (lane >= o) x[q] += y;
-      }
-      if (lane == 31) sc[q][wid] = x[q];
-    }
-    __syncthreads();
-    if (wid == 0) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int t = sc[q][lane];
-        int u = t;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int y = __shfl_up_sync(0xffffffffu, u, o);
-          if (lane >= o) u += y;
-        }
-        sc[q][lane] = u - t;  // exclusive warp offsets
-      }
-    }
-    __syncthreads();
-    int ex[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) ex[q] = carry[q] + sc[q][wid] + x[q] - v[q];
-    if (sel) {
-      s.wl_rep[ex[0]] = r;
-      s.wl_p[ex[0]] = ex[1];
-      s.wl_c[ex[0]] = ex[2];
-      s.wl_k[ex[0]] = ex[3];
-    }
-    __syncthreads();
-    if (threadIdx.x == WL_THREADS - 1 || r == s.nrep - 1)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) carry[q] = ex[q] + v[q];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    const int n = any ? carry[0] : 0;
-    s.wl_n[0] = n;
-    s.wl_n[1] = 0;  // the list builder's chunk queue
-    s.cell_start[s.ncell_tot] = s.N;  // the end of the last cell
-    s.wl_p[n] = any ? carry[1] : 0;
-    s.wl_c[n] = any ? carry[2] : 0;
-    s.wl_k[n] = any ? carry[3] : 0;
-  }
-}
+// The replicas to rebuild (n of them) in ascending order and the prefix sums over them of their
+// particles, cells, rows of cells and list chunks.
+struct WorkList {
+  int *rep, *p, *c, *y, *k;
+  int n;
+};
 
-// Work item g of a prefix array pre (n listed replicas) -> its replica r and index loc inside it:
-// the last k with pre[k] <= g, found by a binary search.
-__device__ __forceinline__ int wl_find(const int* __restrict__ pre, int n, int g) {
+// Work item g of a prefix array pre (n listed replicas): the last k with pre[k] <= g.
+__device__ __forceinline__ int wl_find(const int* pre, int n, int g) {
   int lo = 0, hi = n - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
-    if (__ldg(&pre[mid]) <= g) lo = mid; else hi = mid - 1;
+    if (pre[mid] <= g) lo = mid; else hi = mid - 1;
   }
   return lo;
 }
-__device__ __forceinline__ void wl_map(const int* __restrict__ pre, const int* __restrict__ list, int n, int g,
-                                       int& r, int& loc) {
-  const int k = wl_find(pre, n, g);
-  r = __ldg(&list[k]);
-  loc = g - __ldg(&pre[k]);
-}
-// The same for the lanes of a warp that hold consecutive items (a grid-stride loop): the first
-// active lane searches, the others step forward from its replica.
-__device__ __forceinline__ int wl_map_warp(const int* __restrict__ pre, const int* __restrict__ list, int n, int g,
-                                           int& r, int& loc) {
-  const unsigned m = __activemask();
-  const int leader = __ffs(m) - 1;
-  int k = 0;
-  if ((int)(threadIdx.x & 31) == leader) k = wl_find(pre, n, g);
-  k = __shfl_sync(m, k, leader);
-  while (k + 1 < n && __ldg(&pre[k + 1]) <= g) ++k;
-  r = __ldg(&list[k]);
-  loc = g - __ldg(&pre[k]);
-  return k;  // the position in the list
-}
-
-#define WL_FOR(pre, g)                                                                             \
-  const int wl_cnt_ = *s.wl_n;                                                                     \
-  const int wl_tot_ = s.pre[wl_cnt_];                                                              \
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < wl_tot_; g += gridDim.x * blockDim.x)
-
-__global__ void k_bin(DevState s) {
-  WL_FOR(wl_p, g) {
-  int rr, loc;
-  wl_map_warp(s.wl_p, s.wl_rep, wl_cnt_, g, rr, loc);
-  const int i = s.reps[rr].p0 + loc;
+// Particle i of a rebuilt replica into its cell: the cell's count and the particle's rank in it.
+__device__ __forceinline__ void bin_particle(const DevState& s, int i) {
   int w = s.info[i];
   const RepDesc& R = s.reps[info_rep(w)];
   if (s.mixed) {
@@ -171,185 +79,65 @@ __global__ void k_bin(DevState s) {
   }
   int ix, iy, iz;
   cell_coords(R, s.pfx[i], ix, iy, iz);
-  const int c = R.cell_off + (iz * R.nc[1] + iy) * R.nc[0] + ix;
+  const int row = iz * R.nc[1] + iy, c = R.cell_off + row * R.nc[0] + ix;
   s.cell_of[i] = c;
-  // Particles are still nearly sorted by cell, so neighbouring lanes share cells: the lanes of one
-  // cell take consecutive ranks from a single atomicAdd (k_sort_cells orders each cell by tag
-  // afterwards, so the order of the ranks does not matter).
-  const unsigned grp = __match_any_sync(__activemask(), c);  // the lanes still here
-  const int lane = threadIdx.x & 31, leader = __ffs(grp) - 1;
+  // Particles are still nearly sorted by cell, so neighbouring lanes share cells, rows and planes:
+  // the lanes of one cell take consecutive ranks from a single atomicAdd (the buckets are ordered by
+  // tag afterwards, so the order of the ranks does not matter), those of a row or plane one sum.
+  const unsigned here = __activemask();
+  const int lane = threadIdx.x & 31;
+  const unsigned gc = __match_any_sync(here, c), gr = __match_any_sync(here, R.row_off + row),
+                 gz = __match_any_sync(here, R.plane_off + iz);
+  const int leader = __ffs(gc) - 1;
   int base = 0;
-  if (lane == leader) base = atomicAdd(&s.cell_count[c], __popc(grp));
-  base = __shfl_sync(grp, base, leader);
-  s.rank[i] = base + __popc(grp & ((1u << lane) - 1u));
-  }
+  if (lane == leader) base = atomicAdd(&s.cell_count[c], __popc(gc));
+  if (lane == __ffs(gr) - 1) atomicAdd(&s.row_count[R.row_off + row], __popc(gr));
+  if (lane == __ffs(gz) - 1) atomicAdd(&s.plane_count[R.plane_off + iz], __popc(gz));
+  base = __shfl_sync(gc, base, leader);
+  const int rank = base + __popc(gc & ((1u << lane) - 1u));
+  s.rank[i] = rank;
+  if (rank < s.bucket_cap) s.bucket[(size_t)c * s.bucket_cap + rank] = s.tag[i];
+  else s.wl_n[3] = 1;  // a cell denser than its bucket: this rebuild orders the cells the long way
 }
 
-// ---- cell starts of the listed replicas ---------------------------------------------------------
-// The cells of the listed replicas, one after another in list order, form one sequence g; E[g] is
-// the exclusive prefix sum of their counts.  A replica's counts sum to its particle count, so E at
-// the first cell of the k-th listed replica is wl_p[k], and the start of cell g is
-// p0 + E[g] - wl_p[k].  The starts of the other replicas' cells stay as they were, and the first
-// cell of every replica starts at its p0, so cell_start[c + 1] ends every cell c.  Three kernels on
-// a fixed grid of SCAN_BLOCKS blocks: each block's share of the sequence is summed, the block sums
-// are scanned, and each block scans its share again from its offset and writes the starts.
-constexpr int SCAN_BLOCKS = 256;
-constexpr int SCAN_T = 1024;
-
-__device__ __forceinline__ void scan_share(const DevState& s, int& lo, int& hi) {
-  const int tot = s.wl_c[*s.wl_n];
-  const int seg = ((tot + SCAN_BLOCKS - 1) / SCAN_BLOCKS + SCAN_T - 1) / SCAN_T * SCAN_T;
-  lo = min(tot, (int)blockIdx.x * seg);
-  hi = min(tot, lo + seg);
-}
-
-// block sum of v (all threads); the total in every thread
-__device__ __forceinline__ int block_sum_int(int v, int* red) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  __syncthreads();
-  if (lane == 0) red[wid] = v;
-  __syncthreads();
-  int t = 0;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-  return t;
-}
-
-__global__ void __launch_bounds__(SCAN_T) k_wscan_sum(DevState s) {
-  __shared__ int red[SCAN_T / 32];
-  int lo, hi;
-  scan_share(s, lo, hi);
-  const int n = *s.wl_n;
+// The starts of the cells of one row (a warp): the particles of the planes and rows before it in
+// its replica, then a scan along the row.
+__device__ __forceinline__ void row_starts(const DevState& s, const RepDesc& R, int row) {
+  const int lane = threadIdx.x & 31, iz = row / R.nc[1];
   int v = 0;
-  for (int g = lo + threadIdx.x; g < hi; g += SCAN_T) {
-    int r, c;
-    wl_map_warp(s.wl_c, s.wl_rep, n, g, r, c);
-    v += s.cell_count[s.reps[r].cell_off + c];
-  }
-  v = block_sum_int(v, red);
-  if (threadIdx.x == 0) s.scan_blk[blockIdx.x] = v;
-}
-
-// exclusive scan of the SCAN_BLOCKS block sums (one block)
-__global__ void __launch_bounds__(SCAN_T) k_wscan_blocks(DevState s) {
-  __shared__ int warp_tot[32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int v = threadIdx.x < SCAN_BLOCKS ? s.scan_blk[threadIdx.x] : 0;
-  int x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) warp_tot[wid] = x;
-  __syncthreads();
-  if (wid == 0) {
-    const int t = warp_tot[lane];
-    int u = t;
+  for (int z = lane; z < iz; z += 32) v += s.plane_count[R.plane_off + z];
+  for (int y = iz * R.nc[1] + lane; y < row; y += 32) v += s.row_count[R.row_off + y];
+  int at = R.p0 + (int)__reduce_add_sync(0xffffffffu, (unsigned)v);
+  const int c0 = R.cell_off + row * R.nc[0];
+  for (int b = 0; b < R.nc[0]; b += 32) {
+    const int n = b + lane < R.nc[0] ? s.cell_count[c0 + b + lane] : 0;
+    int x = n;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, u, o);
-      if (lane >= o) u += y;
+      const int u = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += u;
     }
-    warp_tot[lane] = u - t;
-  }
-  __syncthreads();
-  if (threadIdx.x < SCAN_BLOCKS) s.scan_blk[SCAN_BLOCKS + threadIdx.x] = x - v + warp_tot[wid];
-}
-
-__global__ void __launch_bounds__(SCAN_T) k_wscan_write(DevState s) {
-  __shared__ int warp_tot[32];
-  __shared__ int carry;
-  int lo, hi;
-  scan_share(s, lo, hi);
-  const int n = *s.wl_n;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (threadIdx.x == 0) carry = s.scan_blk[SCAN_BLOCKS + blockIdx.x];
-  __syncthreads();
-  for (int base = lo; base < hi; base += SCAN_T) {
-    const int g = base + threadIdx.x;
-    int r = 0, c = 0, k = 0, v = 0;
-    if (g < hi) {
-      k = wl_map_warp(s.wl_c, s.wl_rep, n, g, r, c);
-      v = s.cell_count[s.reps[r].cell_off + c];
-    }
-    int x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    if (lane == 31) warp_tot[wid] = x;
-    __syncthreads();
-    if (wid == 0) {
-      const int t = warp_tot[lane];
-      int u = t;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, u, o);
-        if (lane >= o) u += y;
-      }
-      warp_tot[lane] = u - t;
-    }
-    __syncthreads();
-    const int e = carry + warp_tot[wid] + x - v;  // E[g]
-    if (g < hi) s.cell_start[s.reps[r].cell_off + c] = s.reps[r].p0 + e - s.wl_p[k];
-    __syncthreads();
-    if (threadIdx.x == SCAN_T - 1) carry = e + v;
-    __syncthreads();
+    if (b + lane < R.nc[0]) s.cell_start[c0 + b + lane] = at + x - n;
+    at += __shfl_sync(0xffffffffu, x, 31);
   }
 }
 
-__global__ void k_place(DevState s) {
-  WL_FOR(wl_p, g) {
-    int r, loc;
-    wl_map_warp(s.wl_p, s.wl_rep, wl_cnt_, g, r, loc);
-    const int i = s.reps[r].p0 + loc;
-    s.perm[s.cell_start[s.cell_of[i]] + s.rank[i]] = i;
+// The slot of particle i (tag t) in the new order, from its cell's bucket of tags.
+__device__ __forceinline__ int bucket_slot(const DevState& s, int i, int t) {
+  const int c = s.cell_of[i], n = s.cell_count[c];
+  const int4* b = reinterpret_cast<const int4*>(s.bucket + (size_t)c * s.bucket_cap);  // (a multiple of 4)
+  int less = 0;
+  for (int k = 0; k < n; k += 4) {
+    const int4 q = b[k >> 2];
+    less += (q.x < t) + (k + 1 < n && q.y < t) + (k + 2 < n && q.z < t) + (k + 3 < n && q.w < t);
   }
+  return s.cell_start[c] + less;
 }
 
-// compare-exchange of (tag, slot) pairs by tag
-__device__ __forceinline__ void cmpx(int (&t)[8], int (&p)[8], int i, int j) {
-  if (t[j] < t[i]) {
-    const int u = t[i], q = p[i];
-    t[i] = t[j]; p[i] = p[j];
-    t[j] = u; p[j] = q;
-  }
-}
-
-__global__ void k_sort_cells(DevState s) {
-  WL_FOR(wl_c, g) {
-  int r, lc;
-  wl_map_warp(s.wl_c, s.wl_rep, wl_cnt_, g, r, lc);
-  const int c = s.reps[r].cell_off + lc;
-  int b = s.cell_start[c], n = s.cell_count[c];
-  s.cell_count[c] = 0;  // the last reader of the count: zero again for the next rebuild's k_bin
-  if (n <= 1) continue;
-  if (n <= 8) {
-    // a cell of up to 8: all its slots and tags loaded at once (two dependent loads, not a chain
-    // per element), sorted in registers by a fixed network (Batcher's odd-even merge for 8, its
-    // 4-input form for up to 4) with the unused places padded by the largest tag
-    int p[8], t[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) p[k] = k < n ? s.perm[b + k] : 0;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) t[k] = k < n ? s.tag[p[k]] : 0x7fffffff;
-    cmpx(t, p, 0, 1); cmpx(t, p, 2, 3); cmpx(t, p, 0, 2); cmpx(t, p, 1, 3); cmpx(t, p, 1, 2);
-    if (n > 4) {
-      cmpx(t, p, 4, 5); cmpx(t, p, 6, 7); cmpx(t, p, 4, 6); cmpx(t, p, 5, 7); cmpx(t, p, 5, 6);
-      // merge of the two sorted halves
-      cmpx(t, p, 0, 4); cmpx(t, p, 1, 5); cmpx(t, p, 2, 6); cmpx(t, p, 3, 7);
-      cmpx(t, p, 2, 4); cmpx(t, p, 3, 5);
-      cmpx(t, p, 1, 2); cmpx(t, p, 3, 4); cmpx(t, p, 5, 6);
-    }
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-      if (k < n) s.perm[b + k] = p[k];
-    continue;
-  }
-  for (int k = 1; k < n; ++k) {  // insertion sort by tag
+// The slots of cell c ordered by tag (a rebuild with a cell denser than its bucket).
+__device__ __forceinline__ void sort_cell(const DevState& s, int c) {
+  const int b = s.cell_start[c], n = s.cell_count[c];
+  for (int k = 1; k < n; ++k) {
     int p = s.perm[b + k];
     int t = s.tag[p];
     int m = k - 1;
@@ -359,30 +147,27 @@ __global__ void k_sort_cells(DevState s) {
     }
     s.perm[b + m + 1] = p;
   }
-  }
 }
 
-__global__ void k_permute(DevState s) {
-  WL_FOR(wl_p, g) {
-  int r, loc;
-  wl_map_warp(s.wl_p, s.wl_rep, wl_cnt_, g, r, loc);
-  const int i = s.reps[r].p0 + loc;
-  int o = s.perm[i];
-  s.tmp[0][i] = s.rx[o];
-  s.tmp[1][i] = s.ry[o];
-  s.tmp[2][i] = s.rz[o];
-  s.tmp[3][i] = s.vx[o];
-  s.tmp[4][i] = s.vy[o];
-  s.tmp[5][i] = s.vz[o];
-  const int wo = s.info[o];
+// The state of slot o to slot to(o) of the new order; the loads are issued before the slot is known.
+template <typename F>
+__device__ __forceinline__ void permute_slot(const DevState& s, int o, F to) {
+  const double x = s.rx[o], y = s.ry[o], z = s.rz[o], vx = s.vx[o], vy = s.vy[o], vz = s.vz[o];
+  const int wo = s.info[o], t = s.tag[o];
+  const int i = to(t);
+  s.tmp[0][i] = x;
+  s.tmp[1][i] = y;
+  s.tmp[2][i] = z;
+  s.tmp[3][i] = vx;
+  s.tmp[4][i] = vy;
+  s.tmp[5][i] = vz;
   if (s.permute_accel || !info_mobile(wo)) {
     s.tmp[6][i] = s.ax[o];
     s.tmp[7][i] = s.ay[o];
     s.tmp[8][i] = s.az[o];
   }
-  s.tmp_tag[i] = s.tag[o];
+  s.tmp_tag[i] = t;
   s.tmp_info[i] = wo;
-  }
 }
 
 // Writes the pair-kernel views of slot i and returns the fixed-point position (w in q.w).
@@ -403,11 +188,8 @@ __device__ __forceinline__ int4 write_views(const DevState& s, int i, const RepD
   return q;
 }
 
-__global__ void k_copyback(DevState s) {
-  WL_FOR(wl_p, g) {
-  int rr, loc;
-  wl_map_warp(s.wl_p, s.wl_rep, wl_cnt_, g, rr, loc);
-  const int i = s.reps[rr].p0 + loc;
+// Slot i of the new order back into the state, with its views and its position of this rebuild.
+__device__ __forceinline__ void copyback_slot(const DevState& s, int i) {
   double x = s.tmp[0][i], y = s.tmp[1][i], z = s.tmp[2][i];
   double vx = s.tmp[3][i], vy = s.tmp[4][i], vz = s.tmp[5][i];
   s.rx[i] = x; s.ry[i] = y; s.rz[i] = z;
@@ -421,201 +203,463 @@ __global__ void k_copyback(DevState s) {
   s.slot_of_tag[t] = i;
   const RepDesc& R = s.reps[info_rep(w)];
   int4 q = write_views(s, i, R, x, y, z, vx, vy, vz, w, t);
+  // the list builder's view: sigma from the fixed point (so that it wraps alike), to 512 units
+  s.lp[i] = make_float4((__int_as_float(0x4B000000 | ((unsigned)q.x >> 9)) - 8388608.0f) * (512.f * R.ufx_f[0]),
+                        (__int_as_float(0x4B000000 | ((unsigned)q.y >> 9)) - 8388608.0f) * (512.f * R.ufx_f[1]),
+                        i2f_coarse(q.z, 9) * (512.f * R.ufx_f[2]), __int_as_float(w));
   q.w = 0;
   s.ref[i] = q;
+}
+
+// Grid barrier of a cooperative launch: every block arrives at the k-th barrier (k = 1, 2, ..) on a
+// counter that the list builder's end sets back to zero.  The wait is bounded (about a second):
+// then the status word gets ST_BARRIER and the kernel returns.
+__device__ __forceinline__ bool grid_barrier(const DevState& s, int k) {
+  __shared__ bool ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned* cnt = reinterpret_cast<unsigned*>(s.wl_n + 4);
+    const unsigned target = (unsigned)k * gridDim.x;
+    unsigned seen, old;
+    __threadfence();
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(cnt) : "memory");
+    seen = old + 1;
+    for (int t = 0; t < (1 << 21) && seen < target; ++t)
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(cnt) : "memory");
+    ok = seen >= target;
+    if (!ok) atomicOr(s.status, ST_BARRIER);
+    __threadfence();
+  }
+  __syncthreads();
+  return ok;
+}
+
+// block-wide exclusive scan of v; the block's total in `total`
+__device__ __forceinline__ int block_scan_excl(int v, int* sh, int& total) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  int x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  __syncthreads();  // sh may still be read from the call before
+  if (lane == 31) sh[wid] = x;
+  __syncthreads();
+  int off = 0, t = 0;
+  for (int q = 0; q < nw; ++q) {
+    const int y = sh[q];
+    off += q < wid ? y : 0;
+    t += y;
+  }
+  total = t;
+  return off + x - v;
+}
+
+// The work list of the flagged replicas (all when forced), by one block into L.
+__device__ __forceinline__ void make_worklist(const DevState& s, bool force, WorkList& L, int* sh) {
+  int n = 0, at[4] = {0, 0, 0, 0};
+  for (int base = 0; base < s.nrep; base += SORT_T) {
+    const int r = base + threadIdx.x;
+    const bool sel = r < s.nrep && (force || s.rebuild_flag[1 + r] != 0);
+    int v[4] = {0, 0, 0, 0};
+    if (sel) {
+      const RepDesc& R = s.reps[r];
+      v[0] = R.n_part; v[1] = R.ncell; v[2] = R.nc[1] * R.nc[2]; v[3] = (R.n_part + NL_CHUNK - 1) / NL_CHUNK;
+    }
+    int tn, t[4], e[4];
+    const int en = block_scan_excl(sel ? 1 : 0, sh, tn);
+    if (tn == 0) continue;  // (uniform)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) e[q] = at[q] + block_scan_excl(v[q], sh, t[q]);
+    if (sel) {
+      L.rep[n + en] = r;
+      L.p[n + en] = e[0]; L.c[n + en] = e[1]; L.y[n + en] = e[2]; L.k[n + en] = e[3];
+    }
+    n += tn;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) at[q] += t[q];
+  }
+  if (threadIdx.x == 0) { L.p[n] = at[0]; L.c[n] = at[1]; L.y[n] = at[2]; L.k[n] = at[3]; }
+  L.n = n;
+  __syncthreads();
+}
+
+// The sort of the flagged replicas, see the top of the file.  Its passes over memory are short: with
+// a kernel each (ten of them) their launches and ramps took most of the time of a rebuild of a few
+// replicas; with a cluster of eight blocks per replica instead of the whole grid the phases of one
+// large replica took 100 us.  With the list builder below, a rebuild of a 6400-particle channel went
+// from 79 to 36 us, of 32 brush replicas (447 k particles) from 188 to 159, of 256 (4.66 M) from 1451
+// to 1336, and a step's rebuild of the flagged ones of these 256 from 229 to 197 us.
+__global__ void __launch_bounds__(SORT_T, SORT_PER_SM) k_sort(DevState s, bool force) {
+  if (!force && s.rebuild_flag[0] == 0) {  // (the same for every block: the list builder's end clears it)
+    if (blockIdx.x == 0 && threadIdx.x == 0) s.wl_n[0] = s.wl_k[0] = 0;
+    return;
+  }
+  __shared__ int wl[5][WL_SHARED + 1];
+  __shared__ int sh[SORT_T / 32];
+  WorkList L;
+  int bar = 0;
+  if (s.nrep <= WL_SHARED) {  // every block makes its own
+    L.rep = wl[0]; L.p = wl[1]; L.c = wl[2]; L.y = wl[3]; L.k = wl[4];
+    make_worklist(s, force, L, sh);
+    if (blockIdx.x == 0)  // the list builder's copy
+      for (int q = threadIdx.x; q <= L.n; q += SORT_T) {
+        s.wl_k[q] = L.k[q];
+        if (q < L.n) s.wl_rep[q] = L.rep[q];
+      }
+  } else {
+    L.rep = s.wl_rep; L.p = s.wl_p; L.c = s.wl_c; L.y = s.wl_y; L.k = s.wl_k;
+    if (blockIdx.x == 0) {
+      make_worklist(s, force, L, sh);
+      if (threadIdx.x == 0) s.wl_n[0] = L.n;
+    }
+    if (!grid_barrier(s, ++bar)) return;
+    L.n = s.wl_n[0];
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    s.wl_n[0] = L.n;
+    s.wl_n[1] = 0;  // the list builder's chunk queue
+  }
+  // every block takes one contiguous share of the particles, cells and rows in each phase
+  auto share = [&](int total, int unit, int& lo, int& hi) {
+    const int per = ((total + unit - 1) / unit + gridDim.x - 1) / gridDim.x * unit;
+    lo = min(total, (int)blockIdx.x * per);
+    hi = min(total, lo + per);
+  };
+  // f(list position k, item g) for the thread's items of a share, k found once and then stepped on
+  auto each = [&](const int* pre, int lo, int hi, auto f) {
+    int g = lo + threadIdx.x;
+    if (g >= hi) return;
+    int k = wl_find(pre, L.n, g);
+    for (; g < hi; g += SORT_T) {
+      while (k + 1 < L.n && pre[k + 1] <= g) ++k;
+      f(k, g - pre[k]);
+    }
+  };
+  int plo, phi, clo, chi, ylo, yhi;
+  share(L.p[L.n], 32, plo, phi);
+  share(L.c[L.n], 32, clo, chi);
+  share(L.y[L.n], 1, ylo, yhi);
+  each(L.p, plo, phi, [&](int k, int g) { bin_particle(s, s.reps[L.rep[k]].p0 + g); });
+  if (!grid_barrier(s, ++bar)) return;
+  const bool dense = *(volatile int*)(s.wl_n + 3) != 0;
+  for (int g = ylo + (threadIdx.x >> 5); g < yhi; g += SORT_T / 32) {
+    const int k = wl_find(L.y, L.n, g);
+    row_starts(s, s.reps[L.rep[k]], g - L.y[k]);
+  }
+  if (!grid_barrier(s, ++bar)) return;
+  if (!dense) {
+    each(L.p, plo, phi, [&](int k, int g) {
+      const int i = s.reps[L.rep[k]].p0 + g;
+      permute_slot(s, i, [&](int t) { return bucket_slot(s, i, t); });
+    });
+  } else {
+    each(L.p, plo, phi, [&](int k, int g) {
+      const int i = s.reps[L.rep[k]].p0 + g;
+      s.perm[s.cell_start[s.cell_of[i]] + s.rank[i]] = i;
+    });
+    if (!grid_barrier(s, ++bar)) return;
+    each(L.c, clo, chi, [&](int k, int g) { sort_cell(s, s.reps[L.rep[k]].cell_off + g); });
+    if (!grid_barrier(s, ++bar)) return;
+    each(L.p, plo, phi, [&](int k, int g) {
+      const int i = s.reps[L.rep[k]].p0 + g;
+      permute_slot(s, s.perm[i], [&](int) { return i; });
+    });
+  }
+  if (!grid_barrier(s, ++bar)) return;
+  each(L.p, plo, phi, [&](int k, int g) { copyback_slot(s, s.reps[L.rep[k]].p0 + g); });
+  // the counts back to zero for the next binning
+  each(L.c, clo, chi, [&](int k, int g) { s.cell_count[s.reps[L.rep[k]].cell_off + g] = 0; });
+  each(L.y, ylo, yhi, [&](int k, int g) {
+    const RepDesc& R = s.reps[L.rep[k]];
+    s.row_count[R.row_off + g] = 0;
+    if (g % R.nc[1] == 0) s.plane_count[R.plane_off + g / R.nc[1]] = 0;
+  });
+}
+
+// The end of a rebuild, in the list builder's last block to finish: counts it (when some replica was
+// flagged) and the flagged replicas' rebuilds, and clears the flags.
+__device__ __forceinline__ void rebuild_done(const DevState& s) {
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(s.wl_n + 2, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  int* flag = s.rebuild_flag;
+  const bool any = flag[0] != 0;
+  __syncthreads();
+  for (int r = threadIdx.x; r < s.nrep && any; r += blockDim.x) {
+    if (flag[1 + r]) {
+      s.rep_rebuilds[r] += 1;
+      flag[1 + r] = 0;
+    }
+  }
+  if (threadIdx.x == 0) {
+    s.wl_n[2] = s.wl_n[3] = s.wl_n[4] = 0;
+    if (any) {
+      *s.rebuilds += 1;
+      flag[0] = 0;
+    }
   }
 }
 
 // Full Verlet list: every mobile particle lists all j (mobile or wall) with r^2 < (rc_ij+skin)^2,
-// decided in FP32 on the fixed-point positions with a 2e-4 margin in both precisions (the FP64 mode
-// keeps the fixed-point view for this and for the pair kernel's screening; with candidate tests in
-// FP64, issued at 1/64 of the FP32 rate, ten steps of a 7200-particle FP64 channel took 1434 us,
-// with these 1000, and ten of a batch of 242 k particles 9.73 ms against 6.65).
-// One thread per particle.  Cells are at least 1/H of the list cut-off wide (H = 2 by default),
-// and the (2H+1)^3 cells around a particle are walked as (2H+1)^2 x-rows: the cells of a row are
-// consecutive in the sorted order unless the row wraps in x, so a row is one contiguous slot range
-// (two when it wraps).
-// Rows whose y/z distance from the particle exceeds the largest list cut-off of its type are
-// skipped, and each kept row is trimmed in x to the cells within that cut-off, which removes
-// about half of the candidates.  Each thread stages its first NL_STAGE entries in shared memory
-// (row stride NL_STAGE|1 keeps the banks distinct) and the block writes them out row by row: the
-// k-th neighbours of 128 consecutive particles are 128 consecutive ints of nbr, so every store is
-// coalesced (scattered 4-byte stores into the column-major list cost read-modify-writes in HBM).
-// The fixed staging size keeps the shared memory (17 KB per block) independent of the list
-// capacity, so eight blocks fit on an SM.  The blocks take chunks of the replicas being rebuilt
-// from a queue.
-// entries per particle staged in shared memory (the first NL_STAGE rows of the list are written
-// coalesced; a particle with more neighbours writes the rest straight to the list)
-constexpr int NL_STAGE = 32;
+// decided in FP32 with a margin (fx_margin in mfa_api.cu) on an FP32 view of the positions, in both
+// precisions.  Cells are at least 1/H of the list cut-off wide (1/HX along x), and the cells around a
+// particle are walked as (2H+1)^2 x-rows: the cells of a row are consecutive in the sorted order
+// unless the row wraps in x, so a row is one contiguous slot range (two when it wraps).  Rows whose
+// y/z distance from the particle exceeds the largest list cut-off of its type are skipped, and each
+// kept row is trimmed in x to the cells within that cut-off, which removes about half of the
+// candidates.  A range lies in one periodic image, so its shift goes into the particle's
+// coordinates once and a candidate costs three subtractions, three products and a compare (with
+// integer minimum images and conversions per candidate it took twice the instructions).
+//
+// The list's order is by row, then by slot, whichever way it is built:
+//   a thread per particle, when there are particles enough to fill the GPU with NL_G lanes each (2048
+//     threads per SM; the least work, as the lanes of a warp walk nearly the same rows);
+//   NL_G lanes per particle, when there are not: one or a few replicas flagged, where a thread's walk
+//     of ~80 candidates one after the other is 36 us of latency, and this is 14.  The lanes set up a
+//     row each, take the candidates of a row side by side and place the hits by a ballot.  (With
+//     four or sixteen times as many particles built this way the steps of 64 and 256 brush replicas
+//     took 4 and 10 % longer.)
+// Bound by the latency of the candidates' loads and by issue (60 % active, 19 of 32 lanes).  Short
+// lists gain nothing from unrolled candidate loops, long ones 2 %.
+// Each lane (group) stages its first NL_STAGE entries in shared memory and the warp writes them out
+// row by row: the k-th neighbours of 32 consecutive particles are 32 consecutive ints of nbr
+// (scattered 4-byte stores into the column-major list cost read-modify-writes in HBM).
+constexpr int NL_T = 128;    // threads per block
+constexpr int NL_STAGE = 32;  // staged entries per particle (later ones go straight to the list)
+constexpr int NL_G = 8;      // lanes per particle of the second form
+
+struct NlRow {  // slot ranges of a row, the second when it wraps in x
+  int b0, e0, b1, e1;
+  float x0, x1, y;  // the particle's coordinates in the image of each range
+};
+
+// exact for small integers, without a conversion instruction
+__device__ __forceinline__ float nl_float(int v) { return i2f_coarse(v, 0); }
+// squared gap to a cell edge, d the distance before it (0 when the particle is past it)
+__device__ __forceinline__ float nl_gap2(float d) {
+  d = fmaxf(d, 0.f);
+  return d * d;
+}
+
+template <int H, int HX>
+__device__ __forceinline__ NlRow nl_row(const DevState& s, const RepDesc& R, int row, float4 q, int ix, int iy, int iz,
+                                        float rl2max) {
+  NlRow r = {0, 0, 0, 0, q.x, q.x, q.y};
+  const int dz = row / (2 * H + 1) - H, dy = row - (dz + H) * (2 * H + 1) - H;
+  const int cz = iz + dz;
+  int cy = iy + dy;
+  if (cz < 0 || cz >= R.nc[2]) return r;
+  const float lx = R.lc_f[0], ly = R.lc_f[1], lz = R.lc_f[2];
+  const float rem2 = rl2max - (dz > 0 ? nl_gap2(nl_float(cz) * lz - q.z) : (dz < 0 ? nl_gap2(q.z - nl_float(cz + 1) * lz) : 0.f)) -
+                     (dy > 0 ? nl_gap2(nl_float(cy) * ly - q.y) : (dy < 0 ? nl_gap2(q.y - nl_float(cy + 1) * ly) : 0.f));
+  if (rem2 <= 0.f) return r;  // the whole row is beyond the list cut-off
+  const int nx = R.nc[0];
+  int xa = ix, xb = ix;
+#pragma unroll
+  for (int k = 1; k <= HX; ++k) {
+    xa -= nl_gap2(q.x - nl_float(ix - k + 1) * lx) < rem2;
+    xb += nl_gap2(nl_float(ix + k) * lx - q.x) < rem2;
+  }
+  if (cy < 0) { cy += R.nc[1]; r.y += R.L_f[1]; }
+  else if (cy >= R.nc[1]) { cy -= R.nc[1]; r.y -= R.L_f[1]; }
+  const int* __restrict__ st = s.cell_start + R.cell_off + (cz * R.nc[1] + cy) * nx;
+  // (cell_start[c + 1] ends cell c; there is one entry past the last cell)
+  if (xa < 0) {
+    r.b0 = st[0]; r.e0 = st[xb + 1];
+    r.b1 = st[nx + xa]; r.e1 = st[nx];
+    r.x1 += R.L_f[0];
+  } else if (xb >= nx) {
+    r.b0 = st[xa]; r.e0 = st[nx];
+    r.b1 = st[0]; r.e1 = st[xb - nx + 1];
+    r.x1 -= R.L_f[0];
+  } else {
+    r.b0 = st[xa]; r.e0 = st[xb + 1];
+  }
+  return r;
+}
 
 template <bool UNI, int H, int HX = H>
-__global__ void __launch_bounds__(NL_BLOCK, 8) k_nlist(DevState s) {
-  const int nwl = *s.wl_n;
-  const int nchunks = s.wl_k[nwl];
-  if ((int)blockIdx.x >= nchunks) return;
-  __shared__ int nl_sh[NL_BLOCK * (NL_STAGE | 1)];
+__global__ void __launch_bounds__(NL_T, 8) k_nlist(DevState s) {
+  constexpr int NR = (2 * H + 1) * (2 * H + 1);
+  const int nwl = s.wl_n[0], nchunks = s.wl_k[nwl];
+  const int lane = threadIdx.x & 31, warp = (blockIdx.x * NL_T + threadIdx.x) >> 5, nwarps = gridDim.x * (NL_T / 32);
+  __shared__ int nl_sh[NL_T * (NL_STAGE | 1)];
   __shared__ float rl2f[NPAIR];
   __shared__ float rlmax[MAXT];
-  __shared__ int blk_max;
-  __shared__ int chunk;
-  const int cap = s.nbr_cap;
-  int* mine = nl_sh + threadIdx.x * (NL_STAGE | 1);
-  for (int k = threadIdx.x; k < NPAIR; k += blockDim.x) rl2f[k] = s.tabf[k].rlist2;
-  if (threadIdx.x < MAXT) {  // largest list cut-off of each type, with the culling margin
-    float m = 0.f;
-    for (int t = 0; t < MAXT; ++t) m = fmaxf(m, s.tabf[threadIdx.x * MAXT + t].rlist2);
-    m = sqrtf(m) + s.fx_err;
-    rlmax[threadIdx.x] = m * m * 1.0002f;
-  }
-  for (;;) {
-  // the next chunk from the queue (chunks differ in cost: a queue keeps the blocks busy)
-  __syncthreads();
-  if (threadIdx.x == 0) chunk = atomicAdd(s.wl_n + 1, 1);
-  __syncthreads();
-  const int ch = chunk;
-  if (ch >= nchunks) break;
-  int rc, kc;  // the chunk's replica and its index there (the same for the whole block)
-  wl_map(s.wl_k, s.wl_rep, nwl, ch, rc, kc);
-  const int i0 = s.reps[rc].p0 + kc * NL_BLOCK, i1 = min(s.reps[rc].p0 + s.reps[rc].n_part, i0 + NL_BLOCK);
-  const int i = i0 + threadIdx.x;
-  const bool doit = i < i1;
-  const int w = doit ? s.info[i] : 0;
-  if (threadIdx.x == 0) blk_max = 0;
-  __syncthreads();
-  int cnt = 0, found = 0;  // entries stored, neighbours found (more when the list overflows)
-  if (doit && info_mobile(w)) {
-    const RepDesc& R = s.reps[info_rep(w)];
-    const int ti = info_type(w);
-    int ix, iy, iz;
-    const int4 qi = s.pfx[i];
-    cell_coords(R, qi, ix, iy, iz);
-    // coarse conversion (512 fixed-point units); rl2f carries a 2e-4 margin
-    const float ux = R.ufx_f[0] * 512.f, uy = R.ufx_f[1] * 512.f, uz = R.ufx_f[2] * 512.f;
-    const int nx = R.nc[0];
-    // Row culling and x trimming: a cell is skipped when its distance from the particle, taken
-    // from the cell edges, is beyond the largest list cut-off of the particle's type, the candidate
-    // test's margin included, plus the error of the coarse position and 1e-4 of itself
-    // (no FP64 and no conversion instructions here: both run on the slow FP64 pipe)
-    // position in cell units
-    const float px = (__int_as_float(0x4B000000 | ((unsigned)qi.x >> 9)) - 8388608.0f) * R.cpu_f[0];
-    const float py = (__int_as_float(0x4B000000 | ((unsigned)qi.y >> 9)) - 8388608.0f) * R.cpu_f[1];
-    const float pz = i2f_coarse(qi.z, 9) * R.cpu_f[2];
-    const float lx = R.lc_f[0], ly = R.lc_f[1], lz = R.lc_f[2];
-    const float rl2max = rlmax[ti];
-    const float rl_uni = s.rl2_uni;  // UNI: one list cut-off for every pair (2e-4 margin included)
-    auto fl = [](int v) { return i2f_coarse(v, 0); };  // exact for small integers
-    auto gap2 = [](float d, float l) {  // squared gap of d cell widths (0 when the particle is past the edge)
-      d = fmaxf(d, 0.f) * l;
-      return d * d;
-    };
-    float gxp[HX], gxm[HX];  // squared gaps to the cells ix + k and ix - k, k = 1..HX
-#pragma unroll
-    for (int k = 1; k <= HX; ++k) {
-      gxp[k - 1] = gap2(fl(ix + k) - px, lx);
-      gxm[k - 1] = gap2(px - fl(ix - k + 1), lx);
+  if (nchunks > 0) {
+    for (int k = threadIdx.x; k < NPAIR; k += NL_T) rl2f[k] = s.tabf[k].rlist2;
+    if (threadIdx.x < MAXT) {  // largest list cut-off of each type, with the culling margin
+      float m = 0.f;
+      for (int t = 0; t < MAXT; ++t) m = fmaxf(m, s.tabf[threadIdx.x * MAXT + t].rlist2);
+      m = sqrtf(m) + s.fx_err;
+      rlmax[threadIdx.x] = m * m * 1.0002f;
     }
-    for (int dz = -H; dz <= H; ++dz) {
-      const int cz = iz + dz;
-      if (cz < 0 || cz >= R.nc[2]) continue;
-      const float rz2 = rl2max - ((dz > 0) ? gap2(fl(cz) - pz, lz) : (dz < 0 ? gap2(pz - fl(cz + 1), lz) : 0.f));
-      for (int dy = -H; dy <= H; ++dy) {
-        int cy = iy + dy;
-        const float rem2 = rz2 - ((dy > 0) ? gap2(fl(cy) - py, ly) : (dy < 0 ? gap2(py - fl(cy + 1), ly) : 0.f));
-        if (rem2 <= 0.f) continue;  // the whole row is beyond the list cut-off
-        int xa = ix, xb = ix;
+    __syncthreads();
+    const unsigned FULL = 0xffffffffu;
+    const int cap = s.nbr_cap;
+    const float rl_uni = s.rl2_uni;  // UNI: one list cut-off for every pair
+    int most = 0;  // neighbours found (more than the capacity when the list overflows)
+    auto hit_of = [&](float x, float y, float z, float4 c, int ti) {
+      const float dx = x - c.x, dy = y - c.y, dz = z - c.z;
+      return dx * dx + dy * dy + dz * dz < (UNI ? rl_uni : rl2f[ti * MAXT + info_type(__float_as_int(c.w))]);
+    };
+    if ((long long)nchunks * NL_CHUNK * NL_G > (long long)s.nsm * 2048) {
+      // ---- a thread per particle, chunks from a queue (they differ in cost)
+      int* mine = nl_sh + threadIdx.x * (NL_STAGE | 1);  // odd stride: distinct banks
+      for (;;) {
+        int ch = 0;
+        if (lane == 0) ch = atomicAdd(s.wl_n + 1, 1);
+        ch = __shfl_sync(FULL, ch, 0);
+        if (ch >= nchunks) break;
+        const int lk = wl_find(s.wl_k, nwl, ch);
+        const RepDesc& R = s.reps[s.wl_rep[lk]];
+        const int loc = (ch - s.wl_k[lk]) * NL_CHUNK + lane, i = R.p0 + loc;
+        const bool doit = loc < R.n_part;
+        int cnt = 0;
+        if (doit) {
+          const float4 q = s.lp[i];
+          const int w = __float_as_int(q.w);
+          if (info_mobile(w)) {
+            const int ti = info_type(w);
+            int ix, iy, iz;
+            cell_coords(R, s.pfx[i], ix, iy, iz);
+            const float rl2max = rlmax[ti];
+            const float lx = R.lc_f[0], ly = R.lc_f[1], lz = R.lc_f[2];
+            const int nx = R.nc[0], ny = R.nc[1];
+            float gxm[HX], gxp[HX];  // squared gaps to the cells ix - k and ix + k
 #pragma unroll
-        for (int k = 0; k < HX; ++k) {
-          xa -= gxm[k] < rem2;
-          xb += gxp[k] < rem2;
-        }
-        cy += (cy < 0) ? R.nc[1] : 0;
-        cy -= (cy >= R.nc[1]) ? R.nc[1] : 0;
-        const int row = R.cell_off + (cz * R.nc[1] + cy) * nx;
-        // x-runs of cells xa..xb: one contiguous slot range, or two when the row wraps; the
-        // scan has one entry past the last cell, so cell_start[c + 1] ends cell c
-        int xa0, xb0, xa1 = 0, xb1 = -1;
-        if (xa < 0) { xa0 = 0; xb0 = xb; xa1 = nx + xa; xb1 = nx - 1; }
-        else if (xb >= nx) { xa0 = xa; xb0 = nx - 1; xa1 = 0; xb1 = xb - nx; }
-        else { xa0 = xa; xb0 = xb; }
-        const int nseg = (xb1 >= xa1) ? 2 : 1;
-        int sb[2], se[2];
-        sb[0] = s.cell_start[row + xa0];
-        se[0] = s.cell_start[row + xb0 + 1];
-        if (nseg == 2) {
-          sb[1] = s.cell_start[row + xa1];
-          se[1] = s.cell_start[row + xb1 + 1];
-        }
-        for (int g = 0; g < nseg; ++g) {
-          // not unrolled: the rows are short (a few candidates in 3x3x3 cells), and unrolling by
-          // 2 / 4 / 8 measured 0.6 / 2.9 / 3.8 % slower on a rebuild of 256 brush replicas
-#pragma unroll 1
-          for (int j = sb[g]; j < se[g]; ++j) {
-            const int4 qj = s.pfx[j];
-            const float ddx = i2f_coarse(fx_diff(qi.x, qj.x), 9) * ux;
-            const float ddy = i2f_coarse(fx_diff(qi.y, qj.y), 9) * uy;
-            const float ddz = i2f_coarse(fx_diff(qi.z, qj.z), 9) * uz;
-            const bool hit = ddx * ddx + ddy * ddy + ddz * ddz < (UNI ? rl_uni : rl2f[ti * MAXT + info_type(qj.w)]);
-            if (hit && j != i) {
-              if (cnt < NL_STAGE) mine[cnt] = j;
-              else if (cnt < cap) s.nbr[(size_t)cnt * s.Np + i] = j;  // rare: past the staged rows
-              ++cnt;
+            for (int k = 1; k <= HX; ++k) {
+              gxm[k - 1] = nl_gap2(q.x - nl_float(ix - k + 1) * lx);
+              gxp[k - 1] = nl_gap2(nl_float(ix + k) * lx - q.x);
+            }
+            for (int cz = max(iz - H, 0); cz <= min(iz + H, R.nc[2] - 1); ++cz) {
+              const float rz2 = rl2max - (cz > iz ? nl_gap2(nl_float(cz) * lz - q.z)
+                                                  : (cz < iz ? nl_gap2(q.z - nl_float(cz + 1) * lz) : 0.f));
+              for (int dy = -H; dy <= H; ++dy) {
+                int cy = iy + dy;
+                const float rem2 = rz2 - (dy > 0 ? nl_gap2(nl_float(cy) * ly - q.y)
+                                                 : (dy < 0 ? nl_gap2(q.y - nl_float(cy + 1) * ly) : 0.f));
+                if (rem2 <= 0.f) continue;  // the whole row is beyond the list cut-off
+                int xa = ix, xb = ix;
+#pragma unroll
+                for (int k = 0; k < HX; ++k) {
+                  xa -= gxm[k] < rem2;
+                  xb += gxp[k] < rem2;
+                }
+                float y = q.y;
+                if (cy < 0) { cy += ny; y += R.L_f[1]; }
+                else if (cy >= ny) { cy -= ny; y -= R.L_f[1]; }
+                const int* __restrict__ st = s.cell_start + R.cell_off + (cz * ny + cy) * nx;
+                // (cell_start[c + 1] ends cell c; there is one entry past the last cell)
+                int b = st[max(xa, 0)], e = st[min(xb, nx - 1) + 1], b1 = 0, e1 = 0;
+                float x = q.x, x1 = q.x;
+                if (xa < 0) { b1 = st[nx + xa]; e1 = st[nx]; x1 += R.L_f[0]; }
+                else if (xb >= nx) { b1 = st[0]; e1 = st[xb - nx + 1]; x1 -= R.L_f[0]; }
+                // (one loop for both ranges and every lane: with a loop per kind of row the lanes of a
+                // warp that walk different kinds take turns, 17 % slower on 256 brush replicas)
+                for (int g = 0; g < 2; ++g) {
+#pragma unroll(UNI ? 1 : 2)
+                  for (int j = b; j < e; ++j) {
+                    const bool hit = hit_of(x, y, q.z, s.lp[j], ti) && j != i;
+                    mine[min(cnt, NL_STAGE)] = j;  // kept when it hits; the last word takes the rest
+                    if (hit && cnt >= NL_STAGE && cnt < cap) s.nbr[(size_t)cnt * s.Np + i] = j;
+                    cnt += hit;
+                  }
+                  b = b1; e = e1; x = x1;
+                }
+              }
             }
           }
         }
+        most = max(most, cnt);
+        const int kept = min(cnt, cap), rows = min((int)__reduce_max_sync(FULL, (unsigned)kept), NL_STAGE);
+        for (int k = 0; k < rows; ++k)
+          if (k < kept) s.nbr[(size_t)k * s.Np + i] = mine[k];
+        if (doit) s.nn[i] = kept;
+      }
+    } else {
+      // ---- NL_G lanes per particle
+      constexpr int PW = 32 / NL_G;  // particles of a warp at a time
+      const int q8 = lane & (NL_G - 1), grp = lane / NL_G;
+      int* mine = nl_sh + (threadIdx.x / NL_G) * (NL_STAGE | 1);
+      const int units = nchunks * (NL_CHUNK / PW);
+      for (int u = warp; u < units; u += nwarps) {
+        const int ch = u / (NL_CHUNK / PW);
+        const int lk = wl_find(s.wl_k, nwl, ch);
+        const RepDesc& R = s.reps[s.wl_rep[lk]];
+        const int loc = (ch - s.wl_k[lk]) * NL_CHUNK + (u % (NL_CHUNK / PW)) * PW + grp, i = R.p0 + loc;
+        const bool doit = loc < R.n_part;
+        const float4 q = s.lp[doit ? i : R.p0];
+        const int w = __float_as_int(q.w), ti = info_type(w);
+        const bool walk = doit && info_mobile(w);
+        int ix = 0, iy = 0, iz = 0;
+        if (walk) cell_coords(R, s.pfx[i], ix, iy, iz);
+        const float rl2max = rlmax[ti];
+        int cnt = 0;
+        for (int rb = 0; rb < NR; rb += NL_G) {  // each lane sets up a row
+          NlRow r = {0, 0, 0, 0, 0.f, 0.f, 0.f};
+          if (walk && rb + q8 < NR) r = nl_row<H, HX>(s, R, rb + q8, q, ix, iy, iz, rl2max);
+          const bool any1 = __any_sync(FULL, r.e1 > r.b1);
+          for (int o = 0; o < NL_G && rb + o < NR; ++o) {
+            for (int g = 0; g < (any1 ? 2 : 1); ++g) {
+              const int b = __shfl_sync(FULL, g ? r.b1 : r.b0, o, NL_G), e = __shfl_sync(FULL, g ? r.e1 : r.e0, o, NL_G);
+              const float x = __shfl_sync(FULL, g ? r.x1 : r.x0, o, NL_G), y = __shfl_sync(FULL, r.y, o, NL_G);
+              const int it = ((int)__reduce_max_sync(FULL, (unsigned)(e - b)) + NL_G - 1) / NL_G;
+              for (int t = 0; t < it; ++t) {
+                const int j = b + t * NL_G + q8;
+                bool hit = false;
+                if (j < e) hit = hit_of(x, y, q.z, s.lp[j], ti) && j != i;
+                const unsigned bits = (__ballot_sync(FULL, hit) >> (grp * NL_G)) & ((1u << NL_G) - 1u);
+                if (hit) {
+                  const int k = cnt + __popc(bits & ((1u << q8) - 1u));
+                  if (k < NL_STAGE) mine[k] = j;
+                  else if (k < cap) s.nbr[(size_t)k * s.Np + i] = j;
+                }
+                cnt += __popc(bits);
+              }
+            }
+          }
+        }
+        most = max(most, cnt);
+        const int kept = min(cnt, cap);
+        __syncwarp();
+        // (consecutive lanes take consecutive particles of one list row)
+        const int pi = lane % PW;
+        const int kp = __shfl_sync(FULL, kept, pi * NL_G), ip = __shfl_sync(FULL, i, pi * NL_G);
+        const int* from = nl_sh + ((threadIdx.x & ~31) / NL_G + pi) * (NL_STAGE | 1);
+        for (int k = lane / PW; k < min(kp, NL_STAGE); k += NL_G) s.nbr[(size_t)k * s.Np + ip] = from[k];
+        if (doit && q8 == 0) s.nn[i] = kept;
+        __syncwarp();  // the staging area is the next particles'
       }
     }
-    found = cnt;
-    if (cnt > cap) {
-      atomicOr(s.status, ST_NLIST_OVERFLOW);
-      cnt = cap;
+    // the true count, so that the host grows the capacity past it
+    most = (int)__reduce_max_sync(FULL, (unsigned)most);
+    if (lane == 0 && (unsigned)most > *(volatile unsigned*)(s.status + 1)) {
+      atomicMax(s.status + 1, (unsigned)most);
+      if (most > cap) atomicOr(s.status, ST_NLIST_OVERFLOW);
     }
   }
-  atomicMax(&blk_max, found);  // the true count, so that the host grows the capacity past it
-  __syncthreads();
-  if (threadIdx.x == 0) atomicMax(s.status + 1, (unsigned)blk_max);  // largest count, for the host
-  const int mx = min(blk_max, NL_STAGE);
-  if (doit) {
-    for (int k = 0; k < mx; ++k)
-      if (k < cnt) s.nbr[(size_t)k * s.Np + i] = mine[k];
-    s.nn[i] = cnt;
-  }
-  __syncthreads();  // the staging area and blk_max are reused by the next chunk
-  }
+  rebuild_done(s);
 }
 
-
-// End of a rebuild: counts it (when some replica was flagged) and the flagged replicas' rebuilds,
-// then clears the flags.
-__global__ void k_clear_flags(int* flag, int nrep, long long* rebuilds, long long* rep_rebuilds) {
-  const bool any = flag[0] != 0;
-  __syncthreads();
-  for (int r = threadIdx.x; r < nrep; r += blockDim.x) {
-    if (flag[1 + r]) {
-      rep_rebuilds[r] += 1;
-      flag[1 + r] = 0;
-    }
-  }
-  if (threadIdx.x == 0 && any) {
-    *rebuilds += 1;
-    flag[0] = 0;
-  }
-}
+int rebuild_launches() { return 2; }
 
 void launch_rebuild(const DevState& s, cudaStream_t st, bool force) {
-  const int B = 256;
-  // fixed grids that stride over the work list: a few waves of the GPU, at most what the largest
-  // work (every particle or cell) fills
-  const int gN = std::min((s.N + B - 1) / B, s.nsm * 8);
-  const int gC = std::min((s.ncell_tot + B - 1) / B, s.nsm * 8);
-  k_worklist<<<1, WL_THREADS, 0, st>>>(s, force);
-  k_bin<<<gN, B, 0, st>>>(s);
-  k_wscan_sum<<<SCAN_BLOCKS, SCAN_T, 0, st>>>(s);
-  k_wscan_blocks<<<1, SCAN_T, 0, st>>>(s);
-  k_wscan_write<<<SCAN_BLOCKS, SCAN_T, 0, st>>>(s);
-  k_place<<<gN, B, 0, st>>>(s);
-  k_sort_cells<<<gC, B, 0, st>>>(s);
-  k_permute<<<gN, B, 0, st>>>(s);
-  k_copyback<<<gN, B, 0, st>>>(s);
+  // two blocks per SM at most (what is resident together), no more than the particles fill
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(std::min((s.N + SORT_T - 1) / SORT_T, s.nsm * SORT_PER_SM));
+  cfg.blockDim = dim3(SORT_T);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k_sort, s, force);
   const int uni = s.rl2_uni > 0.f ? 1 : 0;
   using KernT = void (*)(DevState);
   const KernT kerns[3][2] = {{k_nlist<false, 1>, k_nlist<true, 1>},
@@ -624,9 +668,8 @@ void launch_rebuild(const DevState& s, cudaStream_t st, bool force) {
   // cells finer along x alone (with 3x3 rows in y, z)
   const KernT kx[2][2] = {{k_nlist<false, 1, 2>, k_nlist<true, 1, 2>}, {k_nlist<false, 1, 3>, k_nlist<true, 1, 3>}};
   const KernT kern = (s.nl_hx != s.nl_h) ? kx[s.nl_hx - 2][uni] : kerns[s.nl_h - 1][uni];
-  const int gl = std::min((s.N + NL_BLOCK - 1) / NL_BLOCK, s.nsm * 8);
-  kern<<<gl, NL_BLOCK, 0, st>>>(s);
-  k_clear_flags<<<1, 256, 0, st>>>(s.rebuild_flag, s.nrep, s.rebuilds, s.rep_rebuilds);
+  const int gl = std::min((s.N * NL_G + NL_T - 1) / NL_T, s.nsm * 8);
+  kern<<<gl, NL_T, 0, st>>>(s);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -37,12 +37,15 @@ struct DevState {
   dbl4* pd;
   dbl4* vd;
   int4* ref;   // fixed-point position at the last rebuild
+  float4* lp;  // FP32 position (sigma, wrapped) and info at the last rebuild, the list builder's view
   // neighbour list
   int *nn, *nbr;
   int nbr_cap;
   // cells
   int *cell_of, *rank, *perm, *cell_count, *cell_start;
-  int* scan_blk;              // [2 * 256] block sums and offsets of the cell-start scan
+  int *row_count, *plane_count;  // particles per row (y, z) and plane (z) of list cells (0 between rebuilds)
+  int* bucket;                // [ncell_tot][bucket_cap] tags of each list cell during a sort
+  int bucket_cap;             // (a multiple of 4)
   int ncell_tot;
   // control words
   float rl2_uni;  // SimConst::rl2_uni_f (0: per-pair list cut-offs)
@@ -52,11 +55,11 @@ struct DevState {
   int pair_persist;  // mfa_options.pair_schedule
   int* pair_q;       // [2] the persistent pair kernel's queue: next tile, blocks finished
   int* rebuild_flag;          // [1 + nrep]: [0] some replica needs a rebuild, [1 + r] replica r does
-  int* cell_rep;              // [ncell_tot] replica of each list cell
-  // work list of a rebuild (k_worklist): the replicas to rebuild in ascending order (wl_rep), the
-  // prefix sums over them of their particles (wl_p), cells (wl_c) and list-builder chunks (wl_k),
-  // each [nrep + 1], their number (wl_n[0]) and the list builder's chunk queue (wl_n[1])
-  int *wl_rep, *wl_p, *wl_c, *wl_k, *wl_n;
+  // work list of a rebuild: the replicas to rebuild in ascending order (wl_rep), the prefix sums over
+  // them of their particles (wl_p), cells (wl_c), rows (wl_y) and list-builder chunks (wl_k), each
+  // [nrep + 1]; wl_n: their number, the list builder's chunk queue and its finished blocks, whether
+  // a cell is denser than its bucket, the sort's barrier counter (the last three 0 between rebuilds)
+  int *wl_rep, *wl_p, *wl_c, *wl_y, *wl_k, *wl_n;
   int nsm;                    // streaming multiprocessors of the device (grids of the rebuild)
   long long* rebuilds;        // [1] rebuild events (any replica)
   long long* rep_rebuilds;    // [nrep] rebuilds of each replica
@@ -148,6 +151,7 @@ __device__ __forceinline__ void sym_add(T* w6, T c, T dx, T dy, T dz) {
 // Rebuilds the replicas whose flag is set (every replica when `force`), then counts the rebuild
 // and clears the flags.
 void launch_rebuild(const DevState& s, cudaStream_t st, bool force);
+int rebuild_launches();  // kernels of one rebuild
 // The skin test's outcome for replica `rep` (check_skin.f90:11-24 decides per system).
 __device__ __forceinline__ void flag_rebuild(const DevState& s, int rep) {
   s.rebuild_flag[1 + rep] = 1;
