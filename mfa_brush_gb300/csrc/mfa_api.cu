@@ -39,6 +39,7 @@ struct mfa_ctx {
   std::vector<double> v_coul_self, v_ww;
   std::vector<double> v_ff_walls;  // LJ energy of the fixed wall beads among themselves (WALL 1)
   std::vector<KSpace> Ks;  // k-space of each replica (its own box, k-set and charged particles)
+  KSpaceBatch KB = {};     // the same for the launches
   bool kspace = false;
   bool fuse_integ = false;  // mfa_step runs the integration of its plain steps in the pair kernel
   unsigned* h_status = nullptr;  // pinned: [0] status bits, [1] largest list count seen
@@ -317,6 +318,7 @@ int setup_kspace(mfa_ctx* ctx, const int32_t* a_type, int rep) {
   // force chunks of whole rows: KS_FR for the dense kernel; for the one-k-at-a-time kernel as
   // many as let its shared-memory tables fit (the X table alone grows with nxm)
   const bool dense = kspace_dense(K, ctx->S.mixed);
+  K.dense = dense ? 1 : 0;
   std::vector<int> chunk_row;
   for (int frows = KS_FR;; frows /= 2) {
     chunk_row.clear();
@@ -889,6 +891,11 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
       int r = setup_kspace(ctx, a_type, rep);
       if (r != MFA_OK) return r;
     }
+    ctx->KB = kspace_batch(ctx->Ks, S.mixed);
+    KSpace* dks = nullptr;
+    DA(dks, n_rep);
+    CK(cudaMemcpy(dks, ctx->Ks.data(), sizeof(KSpace) * n_rep, cudaMemcpyHostToDevice));
+    ctx->KB.d = dks;
   }
   if (ctx->opt.separate_integrator < 0 || ctx->opt.separate_integrator > 1)
     return fail(ctx, MFA_ERR_ARG, "separate_integrator must be 0 or 1");
@@ -1085,8 +1092,7 @@ int mfa_ewald_k(mfa_ctx* ctx, int32_t mode, double* v) {
   if (!ctx->kspace) return fail(ctx, MFA_ERR_STATE, "ewald_k: not a charged system");
   int r;
   if ((r = zero_call_slot(ctx, O_VCOULK)) || (r = zero_call_group(ctx, V_KSPACE))) return r;
-  for (const KSpace& K : ctx->Ks) launch_kspace(ctx->S, ctx->C, K, ctx->st, true, acc_of(ctx->acc_call, ctx->nrep));
-  ctx->launches += 4 * (long long)ctx->Ks.size();
+  ctx->launches += launch_kspace(ctx->S, ctx->C, ctx->KB, ctx->st, true, acc_of(ctx->acc_call, ctx->nrep));
   CK(cudaGetLastError());
   return read_call_slot(ctx, O_VCOULK, v, 0.);
 }
@@ -1096,8 +1102,7 @@ int mfa_dipolar_correction(mfa_ctx* ctx, double* v) {
   if (!ctx->kspace) return fail(ctx, MFA_ERR_STATE, "dipolar_correction: not a charged system");
   int r;
   if ((r = zero_call_slot(ctx, O_VDIP)) || (r = zero_call_group(ctx, V_DIP))) return r;
-  for (const KSpace& K : ctx->Ks) launch_dipolar(ctx->S, ctx->C, K, ctx->st, true, acc_of(ctx->acc_call, ctx->nrep));
-  ctx->launches += 2 * (long long)ctx->Ks.size();
+  ctx->launches += launch_dipolar(ctx->S, ctx->C, ctx->KB, ctx->st, true, acc_of(ctx->acc_call, ctx->nrep));
   CK(cudaGetLastError());
   return read_call_slot(ctx, O_VDIP, v, 0.);
 }
@@ -1256,13 +1261,7 @@ static long long issue_steps(mfa_ctx* ctx, int n, int phase, bool prof, bool obs
       launch_pair(S, C, st, false, ef, acc, ctx->opt.block_size, S.mixed ? mask : 0);
       L += 1;
       if (mask && !S.mixed) { launch_bonded(S, C, st, mask, ef, acc, true); L += 1; }
-      if (ctx->kspace) {
-        for (const KSpace& K : ctx->Ks) {
-          launch_kspace(S, C, K, st, ef, acc, true);
-          launch_dipolar(S, C, K, st, ef, acc, true);
-          L += 7;
-        }
-      }
+      if (ctx->kspace) L += launch_kspace_step(S, C, ctx->KB, st, ef, acc);
       if (k < n && !split) {
         launch_integrate(S, C, st, 2, true, ef, acc);
         L += 1;
@@ -1790,10 +1789,7 @@ int mfa_kernel_times(mfa_ctx* ctx, int32_t nsteps, float* mean_ms, int32_t* laun
     mark(1);
     if (mask && !S.mixed) { launch_bonded(Sk, C, st, mask, ef, acc, true); mark(2); }
     if (ctx->kspace) {
-      for (const KSpace& K : ctx->Ks) {
-        launch_kspace(Sk, C, K, st, ef, acc, true);
-        launch_dipolar(Sk, C, K, st, ef, acc, true);
-      }
+      launch_kspace_step(Sk, C, ctx->KB, st, ef, acc);
       mark(4);
     }
     launch_integrate(Sk, C, st, k < nsteps ? 2 : 1, true, ef, acc);

@@ -24,8 +24,14 @@
 //                 Im(conj(Y Z) S) to F_y, F_z; rows added with Kahan compensation;
 //   k_ks_force:   the same per row, one k at a time from shared memory (FP64, or nxm > 15);
 //   k_ks_force_sum: the chunk partials in a fixed order, times -8 pi q / V, into the force array.
-// dipolar_correction.f90:20-33 (Yeh-Berkowitz slab term) is k_ks_dipole + k_ks_dipole_force, FP64.
-// Every sum has a fixed order, so a charged run is reproducible bit for bit.
+// dipolar_correction.f90:20-33 (Yeh-Berkowitz slab term), FP64: the moment in blocks of its own of
+// k_ks_tables, the force in k_ks_force_sum.
+// Every sum has a fixed order, so a charged run is reproducible bit for bit.  A batch runs each
+// kernel once for all replicas (the last grid dimension; the blocks past a replica's own extent
+// leave): launched replica by replica, 7 kernels each, twelve small charged channels spent 825 us a
+// step in launches one behind the other.  A replica's work is divided as it is alone, so its sums
+// are those of the replica run alone.
+#include <algorithm>
 #include <type_traits>
 
 #include "mfa_state.cuh"
@@ -67,28 +73,6 @@ __device__ __forceinline__ const kcplx<MIXED>* ktab(const KSpace& K) {
   if constexpr (MIXED) return K.tabf; else return K.tabd;
 }
 
-template <bool MIXED>
-__global__ void k_ks_tables(DevState s, KSpace K) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= K.nq * K.ncol) return;
-  const int col = idx / K.nq, p = idx - col * K.nq;
-  const int i = s.slot_of_tag[K.qtag[p]];
-  double u;
-  if (col <= K.nxm) u = (double)col * K.cx * s.rx[i];
-  else if (col <= K.nxm + 1 + K.nym) u = (double)(col - K.nxm - 1) * K.cy * s.ry[i];
-  else u = (double)(col - K.nxm - K.nym - 2) * K.cz * s.rz[i];
-  u -= rint(u);  // turns in [-1/2, 1/2]
-  if constexpr (MIXED) {
-    float sn, cs;
-    sincospif(2.f * (float)u, &sn, &cs);
-    K.tabf[idx] = make_float2(cs, sn);
-  } else {
-    double sn, cs;
-    sincospi(2. * u, &sn, &cs);
-    K.tabd[idx] = make_double2(cs, sn);
-  }
-}
-
 constexpr int KS_TILE = 32;  // particles per shared-memory tile of k_ks_rho (one per lane)
 
 // rho(row, nx) = sum_p A(p, row) X(p, nx), A = q Y(ny) Z(nz), with X(p, -n) = conj X(p, n): the
@@ -110,7 +94,10 @@ constexpr int KS_AS = KS_RB + 2;  // A row stride (8-byte slots; 16-byte aligned
 static_assert(KS_TILE * KS_XS * sizeof(float2) % 16 == 0, "the A rows follow the X rows 16-byte aligned");
 
 template <bool MIXED>
-__global__ void __launch_bounds__(KS_RHO_T, MIXED ? 3 : 1) k_ks_rho(KSpace K) {
+__global__ void __launch_bounds__(KS_RHO_T, MIXED ? 3 : 1) k_ks_rho(const KSpace* __restrict__ Ks, int nz) {
+  const KSpace K = Ks[blockIdx.z / nz];
+  const int zs = blockIdx.z % nz;
+  if ((int)blockIdx.x * KS_RB >= K.nrows || (int)blockIdx.y >= K.npchunks || zs * KS_SL > K.nxm || K.nq == 0) return;
   using real = kreal<MIXED>;
   using Cx = kcplx<MIXED>;
   extern __shared__ __align__(16) unsigned char shraw[];
@@ -122,7 +109,7 @@ __global__ void __launch_bounds__(KS_RHO_T, MIXED ? 3 : 1) k_ks_rho(KSpace K) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4;
   constexpr int NW = KS_RHO_T / 32;
   constexpr int RL = KS_RW / 2;  // rows per lane
-  const int slot = blockIdx.z * KS_SL + (lane & (KS_SL - 1));  // |nx| of the lane
+  const int slot = zs * KS_SL + (lane & (KS_SL - 1));  // |nx| of the lane
   const int r0 = warp * KS_RW + half * RL;                      // the lane's first row
   const bool act = r0 < nr;
   for (int r = threadIdx.x; r < nr; r += KS_RHO_T) {
@@ -145,7 +132,7 @@ __global__ void __launch_bounds__(KS_RHO_T, MIXED ? 3 : 1) k_ks_rho(KSpace K) {
       if constexpr (MIXED) q = K.qvalf[pq]; else q = K.qval[pq];
 #pragma unroll
       for (int i = 0; i < KS_SL / NW; ++i) {  // slot columns warp + NW i
-        const int n = blockIdx.z * KS_SL + warp + NW * i;
+        const int n = zs * KS_SL + warp + NW * i;
         Cx xv;
         xv.x = 0;
         xv.y = 0;
@@ -252,23 +239,24 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
   return b;
 }
 
-// Block sum of v (all threads), then the last block of the grid to finish adds the per-block
+// Block sum of v (all threads), then the last of `blocks` blocks to finish adds the per-block
 // partials: each of its threads a strided subset in order, then a block sum; a fixed order for
 // a given grid.  Returns true in thread 0 of that block, with the total in `total`.
-__device__ __forceinline__ bool grid_sum_last(double v, double* part, unsigned* ticket, double& total) {
+__device__ __forceinline__ bool grid_sum_last(double v, double* part, unsigned* ticket, unsigned blocks,
+                                              double& total) {
   __shared__ double red[32];
   __shared__ bool last;
   const double b = block_sum(v, red);
   if (threadIdx.x == 0) {
     part[blockIdx.x] = b;
     __threadfence();
-    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    last = atomicAdd(ticket, 1u) == blocks - 1;
   }
   __syncthreads();
   if (!last) return false;
   __threadfence();
   double t = 0.;
-  for (unsigned k = threadIdx.x; k < gridDim.x; k += blockDim.x) t += ((volatile double*)part)[k];
+  for (unsigned k = threadIdx.x; k < blocks; k += blockDim.x) t += ((volatile double*)part)[k];
   t = block_sum(t, red);
   if (threadIdx.x != 0) return false;
   total = t;
@@ -276,9 +264,10 @@ __device__ __forceinline__ bool grid_sum_last(double v, double* part, unsigned* 
   return true;
 }
 
-// The same for NV values at once; part holds gridDim.x x NV partials.
+// The same for NV values at once; part holds blocks x NV partials.
 template <int NV>
-__device__ __forceinline__ bool grid_sum_last_n(const double* v, double* part, unsigned* ticket, double* total) {
+__device__ __forceinline__ bool grid_sum_last_n(const double* v, double* part, unsigned* ticket, unsigned blocks,
+                                                double* total) {
   __shared__ double red[32];
   __shared__ bool last;
   double b[NV];
@@ -288,7 +277,7 @@ __device__ __forceinline__ bool grid_sum_last_n(const double* v, double* part, u
 #pragma unroll
     for (int c = 0; c < NV; ++c) part[(size_t)blockIdx.x * NV + c] = b[c];
     __threadfence();
-    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    last = atomicAdd(ticket, 1u) == blocks - 1;
   }
   __syncthreads();
   if (!last) return false;
@@ -296,7 +285,7 @@ __device__ __forceinline__ bool grid_sum_last_n(const double* v, double* part, u
   double t[NV];
 #pragma unroll
   for (int c = 0; c < NV; ++c) t[c] = 0.;
-  for (unsigned k = threadIdx.x; k < gridDim.x; k += blockDim.x)
+  for (unsigned k = threadIdx.x; k < blocks; k += blockDim.x)
 #pragma unroll
     for (int c = 0; c < NV; ++c) t[c] += ((volatile double*)part)[(size_t)k * NV + c];
 #pragma unroll
@@ -308,18 +297,66 @@ __device__ __forceinline__ bool grid_sum_last_n(const double* v, double* part, u
   return true;
 }
 
+// parts of the sum that a launch covers
+constexpr int KS_RECIP = 1, KS_DIPOLE = 2;
+constexpr int KS_TAB_T = 256;  // threads of a k_ks_tables block
+__host__ __device__ inline int ks_dipole_blocks(int nq) {
+  return nq > 0 ? (nq + KS_TAB_T - 1) / KS_TAB_T < KS_RED_MAX ? (nq + KS_TAB_T - 1) / KS_TAB_T : KS_RED_MAX : 0;
+}
+
+// Blocks 0 .. ks_dipole_blocks - 1 of a replica: the dipole moment; the blocks from dblk on: the tables.
+template <bool MIXED>
+__global__ void __launch_bounds__(KS_TAB_T) k_ks_tables(DevState s, const KSpace* __restrict__ Ks, int dblk, int what,
+                                                        double pi, Acc acc, bool eflag) {
+  const KSpace& K = Ks[blockIdx.y];
+  if ((int)blockIdx.x < dblk) {
+    const int nb = ks_dipole_blocks(K.nq);
+    if (!(what & KS_DIPOLE) || (int)blockIdx.x >= nb) return;
+    double m = 0.;
+    for (int p = blockIdx.x * KS_TAB_T + threadIdx.x; p < K.nq; p += nb * KS_TAB_T)
+      m += K.qval[p] * (s.rz[s.slot_of_tag[K.qtag[p]]] - K.lz_half);
+    double tot;
+    if (grid_sum_last(m, K.red_part + 7 * KS_RED_MAX, K.ticket + 1, nb, tot)) {
+      K.mz[0] = tot;
+      if (eflag) acc.col(O_VDIP)[K.rep] += 2. * pi * tot * tot * K.inv_V;
+    }
+    return;
+  }
+  const int idx = (blockIdx.x - dblk) * KS_TAB_T + threadIdx.x;
+  if (!(what & KS_RECIP) || K.nk == 0 || idx >= K.nq * K.ncol) return;
+  const int col = idx / K.nq, p = idx - col * K.nq;
+  const int i = s.slot_of_tag[K.qtag[p]];
+  double u;
+  if (col <= K.nxm) u = (double)col * K.cx * s.rx[i];
+  else if (col <= K.nxm + 1 + K.nym) u = (double)(col - K.nxm - 1) * K.cy * s.ry[i];
+  else u = (double)(col - K.nxm - K.nym - 2) * K.cz * s.rz[i];
+  u -= rint(u);  // turns in [-1/2, 1/2]
+  if constexpr (MIXED) {
+    float sn, cs;
+    sincospif(2.f * (float)u, &sn, &cs);
+    K.tabf[idx] = make_float2(cs, sn);
+  } else {
+    double sn, cs;
+    sincospi(2. * u, &sn, &cs);
+    K.tabd[idx] = make_double2(cs, sn);
+  }
+}
+
 // Thread (k, g) of a block of 32 k x 8 groups sums the chunk partials c = g, g + 8, ..; the
 // eight group sums are then added in group order: a fixed order for every k.  With energies, the
 // reciprocal-space virial sum over k of u_k (delta_ab - 2 k_a k_b (1/k^2 + 1/(4 alpha_c))) as well
 // (u_k = G |rho|^2, the k's term of the energy), the derivative of the energy under a deformation
 // of the cell.
 template <bool MIXED>
-__global__ void __launch_bounds__(256) k_ks_rho_sum(KSpace K, double pi4, double fac_alpha, Acc acc, bool eflag) {
+__global__ void __launch_bounds__(256) k_ks_rho_sum(const KSpace* __restrict__ Ks, double pi4, double fac_alpha, Acc acc,
+                                                    bool eflag) {
+  const KSpace K = Ks[blockIdx.y];
+  const int nkb = (K.nk + 31) / 32, blocks = min(KS_RED_MAX, nkb);  // blocks of this replica
+  if ((int)blockIdx.x >= blocks || K.nq == 0) return;
   __shared__ double2 part[8][32];
   const int kl = threadIdx.x & 31, g = threadIdx.x >> 5;
   double u[7] = {0., 0., 0., 0., 0., 0., 0.};  // energy, then the virial xx yy zz xy xz yz
-  const int nkb = (K.nk + 31) / 32;
-  for (int kb = blockIdx.x; kb < nkb; kb += gridDim.x) {
+  for (int kb = blockIdx.x; kb < nkb; kb += blocks) {
     const int k = kb * 32 + kl;
     double re = 0., im = 0.;
     if (k < K.nk) {
@@ -365,8 +402,9 @@ __global__ void __launch_bounds__(256) k_ks_rho_sum(KSpace K, double pi4, double
     }
     __syncthreads();
   }
+  if (!eflag) return;
   double tot[7];
-  if (grid_sum_last_n<7>(u, K.red_part, K.ticket, tot) && eflag) {
+  if (grid_sum_last_n<7>(u, K.red_part, K.ticket, blocks, tot)) {
     const double sc = pi4 * K.inv_V;
     acc.col(O_VCOULK)[K.rep] += tot[0] * sc;
     const int idx[6] = {0, 4, 8, 1, 2, 5};
@@ -388,7 +426,9 @@ struct KD<false> {
 };
 
 template <bool MIXED>
-__global__ void __launch_bounds__(KS_FB) k_ks_force(KSpace K) {
+__global__ void __launch_bounds__(KS_FB) k_ks_force(const KSpace* __restrict__ Ks) {
+  const KSpace K = Ks[blockIdx.z];
+  if (K.dense || (int)blockIdx.x * KS_FB >= K.nq || (int)blockIdx.y >= K.nkchunks) return;
   using real = kreal<MIXED>;
   using Cx = kcplx<MIXED>;
   using real2 = kcplx<MIXED>;
@@ -493,7 +533,9 @@ __global__ void __launch_bounds__(KS_FB) k_ks_force(KSpace K) {
 // of their slot range (frow), so that the rows of a chunk share a narrow window of slots; slots
 // outside the window are skipped (a branch uniform over the block).
 template <int QF>
-__global__ void __launch_bounds__(KS_FB) k_ks_force_dense(KSpace K) {
+__global__ void __launch_bounds__(KS_FB) k_ks_force_dense(const KSpace* __restrict__ Ks) {
+  const KSpace K = Ks[blockIdx.z];
+  if (!K.dense || (int)blockIdx.x * KS_FB >= K.nq || (int)blockIdx.y >= K.nkchunks) return;
   constexpr int NF = 4 * QF;  // folded slots |n| = 0 .. NF - 1
   extern __shared__ __align__(16) unsigned char shraw[];
   float4* Wd = reinterpret_cast<float4*>(shraw);              // [KS_FR][NF][2]
@@ -578,31 +620,36 @@ __global__ void __launch_bounds__(KS_FB) k_ks_force_dense(KSpace K) {
   o[2] = (double)fz - (double)cz;
 }
 
-// F_i = -(8 pi q_i / V) * sum over k-chunks in a fixed order, added to the FP64 force array or,
-// in the fused mixed-precision step, to the FP32 one.
-__global__ void k_ks_force_sum(DevState s, KSpace K, double pi8, bool to_f4) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= K.nq) return;
-  double f[3] = {0., 0., 0.};
-  for (int c = 0; c < K.nkchunks; ++c)
-    for (int d = 0; d < 3; ++d) f[d] += K.fpart[((size_t)c * K.nq + p) * 3 + d];
+// F_i = -(8 pi q_i / V) * sum over k-chunks in a fixed order, and the slab term's -4 pi q_i M_z / V
+// along z, added to the FP64 force array or, in the fused mixed-precision step, to the FP32 one.  A
+// thread per component: the partials of a chunk are read in order.
+__global__ void __launch_bounds__(128) k_ks_force_sum(DevState s, const KSpace* __restrict__ Ks, double pi, int what,
+                                                      bool to_f4) {
+  const KSpace K = Ks[blockIdx.y];
+  const int idx = blockIdx.x * 128 + threadIdx.x;
+  if (idx >= 3 * K.nq) return;
+  const int p = idx / 3, d = idx - 3 * p;
   const int i = s.slot_of_tag[K.qtag[p]];
-  const double qf = -pi8 * K.qval[p] * K.inv_V;
-  if (to_f4) {
-    float4 g = s.f4[i];
-    g.x += (float)(qf * f[0]);
-    g.y += (float)(qf * f[1]);
-    g.z += (float)(qf * f[2]);
-    s.f4[i] = g;
-  } else {
-    s.fx[i] += qf * f[0];
-    s.fy[i] += qf * f[1];
-    s.fz[i] += qf * f[2];
+  const double q = K.qval[p];
+  double* fd = d == 0 ? s.fx : (d == 1 ? s.fy : s.fz);
+  float* f4 = reinterpret_cast<float*>(s.f4 + i) + d;
+  if ((what & KS_RECIP) && K.nk > 0) {
+    double f = 0.;
+#pragma unroll 8
+    for (int c = 0; c < K.nkchunks; ++c) f += K.fpart[(size_t)c * K.nq * 3 + idx];
+    const double qf = -(8. * pi) * q * K.inv_V;
+    if (to_f4) *f4 += (float)(qf * f);
+    else fd[i] += qf * f;
+  }
+  if ((what & KS_DIPOLE) && d == 2) {
+    const double f = -4. * pi * q * K.mz[0] * K.inv_V;
+    if (to_f4) *f4 += (float)f;
+    else fd[i] += f;
   }
 }
 
 namespace {
-size_t rho_smem(const KSpace& K, bool mixed) {
+size_t rho_smem(bool mixed) {
   return (size_t)KS_TILE * (KS_XS + KS_AS) * (mixed ? sizeof(float2) : sizeof(double2)) +
          (size_t)KS_RB * sizeof(int2);
 }
@@ -613,16 +660,16 @@ size_t force_smem(const KSpace& K, bool mixed) {
 }
 // groups of four folded slots |nx| = 0 .. nxm of k_ks_force_dense
 int dense_qf(const KSpace& K) { return (K.nxm + 4) / 4; }
-size_t dense_smem(const KSpace& K) {
-  return (size_t)KS_FR * (4 * dense_qf(K) * 2 * sizeof(float4) + sizeof(int2) + sizeof(float2));
+size_t dense_smem(int qf) {
+  return (size_t)KS_FR * (4 * qf * 2 * sizeof(float4) + sizeof(int2) + sizeof(float2));
 }
 constexpr int KS_DENSE_QX_MAX = 8;  // the register-resident X of k_ks_force_dense: nxm <= 15
 
 template <int QF>
-void launch_dense(const KSpace& K, dim3 g, cudaStream_t st) {
-  k_ks_force_dense<QF><<<g, KS_FB, dense_smem(K), st>>>(K);
+void launch_dense(const KSpace* Ks, size_t shm, dim3 g, cudaStream_t st) {
+  k_ks_force_dense<QF><<<g, KS_FB, shm, st>>>(Ks);
 }
-typedef void (*dense_launcher)(const KSpace&, dim3, cudaStream_t);
+typedef void (*dense_launcher)(const KSpace*, size_t, dim3, cudaStream_t);
 const dense_launcher kDense[5] = {nullptr, launch_dense<1>, launch_dense<2>, launch_dense<3>, launch_dense<4>};
 bool use_dense(const KSpace& K, bool mixed) { return mixed && K.qx <= KS_DENSE_QX_MAX; }
 }  // namespace
@@ -631,7 +678,7 @@ bool kspace_dense(const KSpace& K, bool mixed) { return use_dense(K, mixed); }
 size_t kspace_force_smem(const KSpace& K, bool mixed) { return force_smem(K, mixed); }
 
 int kspace_prepare(const KSpace& K, bool mixed) {
-  const size_t a = rho_smem(K, mixed), b = use_dense(K, mixed) ? dense_smem(K) : force_smem(K, mixed);
+  const size_t a = rho_smem(mixed), b = use_dense(K, mixed) ? dense_smem(dense_qf(K)) : force_smem(K, mixed);
   if (a > KS_SMEM_MAX || b > KS_SMEM_MAX) return (int)cudaErrorInvalidConfiguration;
   // The opt-in is a property of the kernel for the whole process, not of a context: set it to the
   // largest allowed size once, so that no context lowers it below another's needs (occupancy
@@ -644,62 +691,92 @@ int kspace_prepare(const KSpace& K, bool mixed) {
   return (int)e;  // dense_smem stays below 48 KB: 32 rows x 16 folded slots x 32 B + 512 B
 }
 
-void launch_kspace(const DevState& s, const SimConst& C, const KSpace& K, cudaStream_t st, bool eflag, Acc acc,
-                   bool fused) {
-  if (K.nk == 0 || K.nq == 0) return;
+KSpaceBatch kspace_batch(const std::vector<KSpace>& Ks, bool mixed) {
+  KSpaceBatch B = {};
+  B.n = (int)Ks.size();
+  for (const KSpace& K : Ks) {
+    if (K.nq == 0) continue;  // no charges: every block of this replica leaves
+    B.dip = std::max(B.dip, ks_dipole_blocks(K.nq));
+    B.tab = std::max(B.tab, K.nk ? (K.nq * K.ncol + KS_TAB_T - 1) / KS_TAB_T : 0);
+    B.nq = std::max(B.nq, K.nq);
+    if (K.nk == 0) continue;
+    B.rows = std::max(B.rows, (K.nrows + KS_RB - 1) / KS_RB);
+    B.pchunks = std::max(B.pchunks, K.npchunks);
+    B.nz = std::max(B.nz, (K.nxm + KS_SL) / KS_SL);
+    B.sum = std::max(B.sum, std::min(KS_RED_MAX, (K.nk + 31) / 32));
+    const int fb = (K.nq + KS_FB - 1) / KS_FB;
+    if (use_dense(K, mixed)) {
+      B.dense_p = std::max(B.dense_p, fb);
+      B.dense_k = std::max(B.dense_k, K.nkchunks);
+      B.qf = std::max(B.qf, dense_qf(K));
+    } else {
+      B.force_p = std::max(B.force_p, fb);
+      B.force_k = std::max(B.force_k, K.nkchunks);
+      B.force_shm = std::max(B.force_shm, force_smem(K, mixed));
+    }
+  }
+  return B;
+}
+
+static int launch_ks(const DevState& s, const SimConst& C, KSpaceBatch B, cudaStream_t st, int what, bool eflag,
+                     Acc acc, bool to_f4) {
+  if (B.nq == 0) return 0;
+  const int most = 65535 / std::max(B.nz, 1);  // the last grid dimension holds nz per replica
+  if (B.n > most) {
+    KSpaceBatch A = B;
+    A.n = most;
+    B.d += most;
+    B.n -= most;
+    return launch_ks(s, C, A, st, what, eflag, acc, to_f4) + launch_ks(s, C, B, st, what, eflag, acc, to_f4);
+  }
   const double pi = (double)3.1415926536f;  // mfa_common.f90:315 (single-precision literal)
-  const int nt = K.nq * K.ncol;
-  if (s.mixed) k_ks_tables<true><<<(nt + 255) / 256, 256, 0, st>>>(s, K);
-  else k_ks_tables<false><<<(nt + 255) / 256, 256, 0, st>>>(s, K);
-  const dim3 g1((K.nrows + KS_RB - 1) / KS_RB, K.npchunks, (K.nxm + KS_SL) / KS_SL);
-  const size_t shm1 = rho_smem(K, s.mixed);
-  if (s.mixed) k_ks_rho<true><<<g1, KS_RHO_T, shm1, st>>>(K);
-  else k_ks_rho<false><<<g1, KS_RHO_T, shm1, st>>>(K);
-  const int gs = std::min(KS_RED_MAX, (K.nk + 31) / 32);
-  const double fac_alpha = 1. / (4. * C.alpha_c);
-  if (s.mixed) k_ks_rho_sum<true><<<gs, 256, 0, st>>>(K, 4. * pi, fac_alpha, acc, eflag);
-  else k_ks_rho_sum<false><<<gs, 256, 0, st>>>(K, 4. * pi, fac_alpha, acc, eflag);
-  const dim3 g2((K.nq + KS_FB - 1) / KS_FB, K.nkchunks);
-  if (use_dense(K, s.mixed)) {
-    kDense[dense_qf(K)](K, g2, st);
-  } else {
-    const size_t shm2 = force_smem(K, s.mixed);
-    if (s.mixed) k_ks_force<true><<<g2, KS_FB, shm2, st>>>(K);
-    else k_ks_force<false><<<g2, KS_FB, shm2, st>>>(K);
+  const bool recip = (what & KS_RECIP) && B.rows > 0;
+  const int dblk = (what & KS_DIPOLE) ? B.dip : 0, tblk = recip ? B.tab : 0;
+  int launches = 0;
+  if (dblk + tblk > 0) {
+    const dim3 g(dblk + tblk, B.n);
+    if (s.mixed) k_ks_tables<true><<<g, KS_TAB_T, 0, st>>>(s, B.d, dblk, what, pi, acc, eflag);
+    else k_ks_tables<false><<<g, KS_TAB_T, 0, st>>>(s, B.d, dblk, what, pi, acc, eflag);
+    ++launches;
   }
-  k_ks_force_sum<<<(K.nq + 127) / 128, 128, 0, st>>>(s, K, 8. * pi, fused && s.mixed);
+  if (recip) {
+    const dim3 g1(B.rows, B.pchunks, B.nz * B.n), g2(B.sum, B.n);
+    const size_t shm1 = rho_smem(s.mixed);
+    const double fac_alpha = 1. / (4. * C.alpha_c);
+    if (s.mixed) {
+      k_ks_rho<true><<<g1, KS_RHO_T, shm1, st>>>(B.d, B.nz);
+      k_ks_rho_sum<true><<<g2, 256, 0, st>>>(B.d, 4. * pi, fac_alpha, acc, eflag);
+    } else {
+      k_ks_rho<false><<<g1, KS_RHO_T, shm1, st>>>(B.d, B.nz);
+      k_ks_rho_sum<false><<<g2, 256, 0, st>>>(B.d, 4. * pi, fac_alpha, acc, eflag);
+    }
+    launches += 2;
+    if (B.dense_p) {
+      kDense[B.qf](B.d, dense_smem(B.qf), dim3(B.dense_p, B.dense_k, B.n), st);
+      ++launches;
+    }
+    if (B.force_p) {
+      const dim3 g3(B.force_p, B.force_k, B.n);
+      if (s.mixed) k_ks_force<true><<<g3, KS_FB, B.force_shm, st>>>(B.d);
+      else k_ks_force<false><<<g3, KS_FB, B.force_shm, st>>>(B.d);
+      ++launches;
+    }
+  }
+  k_ks_force_sum<<<dim3((3 * B.nq + 127) / 128, B.n), 128, 0, st>>>(s, B.d, pi, what, to_f4);
+  return launches + 1;
 }
 
-__global__ void __launch_bounds__(256) k_ks_dipole(DevState s, KSpace K, double pi, Acc acc, bool eflag) {
-  double m = 0.;
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < K.nq; p += gridDim.x * blockDim.x) {
-    const int i = s.slot_of_tag[K.qtag[p]];
-    m += K.qval[p] * (s.rz[i] - K.lz_half);
-  }
-  double tot;
-  if (grid_sum_last(m, K.red_part + 7 * KS_RED_MAX, K.ticket + 1, tot)) {
-    K.mz[0] = tot;
-    if (eflag) acc.col(O_VDIP)[K.rep] += 2. * pi * tot * tot * K.inv_V;
-  }
+int launch_kspace(const DevState& s, const SimConst& C, const KSpaceBatch& B, cudaStream_t st, bool eflag, Acc acc) {
+  return launch_ks(s, C, B, st, KS_RECIP, eflag, acc, false);
 }
 
-__global__ void k_ks_dipole_force(DevState s, KSpace K, double pi, bool to_f4) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= K.nq) return;
-  const int i = s.slot_of_tag[K.qtag[p]];
-  const double f = -4. * pi * K.qval[p] * K.mz[0] * K.inv_V;
-  if (to_f4) s.f4[i].z += (float)f;
-  else s.fz[i] += f;
+int launch_dipolar(const DevState& s, const SimConst& C, const KSpaceBatch& B, cudaStream_t st, bool eflag, Acc acc) {
+  return launch_ks(s, C, B, st, KS_DIPOLE, eflag, acc, false);
 }
 
-void launch_dipolar(const DevState& s, const SimConst& C, const KSpace& K, cudaStream_t st, bool eflag, Acc acc,
-                    bool fused) {
-  (void)C;
-  if (K.nq == 0) return;
-  const double pi = (double)3.1415926536f;
-  const int g = std::min(KS_RED_MAX, (K.nq + 255) / 256);
-  k_ks_dipole<<<g, 256, 0, st>>>(s, K, pi, acc, eflag);
-  k_ks_dipole_force<<<(K.nq + 255) / 256, 256, 0, st>>>(s, K, pi, fused && s.mixed);
+int launch_kspace_step(const DevState& s, const SimConst& C, const KSpaceBatch& B, cudaStream_t st, bool eflag,
+                       Acc acc) {
+  return launch_ks(s, C, B, st, KS_RECIP | KS_DIPOLE, eflag, acc, s.mixed);
 }
 
 }  // namespace mfa

@@ -1,5 +1,7 @@
 // mfa_state.cuh -- device state of one context and the kernel launchers (host-callable).
 #pragma once
+#include <vector>
+
 #include "mfa_dev.cuh"
 
 namespace mfa {
@@ -245,6 +247,7 @@ struct KSpace {
   double* red_part;     // [8*KS_RED_MAX]: rho_sum energy and virial (7 per block), dipole moment
   unsigned* ticket;     // [2] zero between launches
   int rep;
+  int dense;            // 1: the force in the dense kernel (kspace_dense)
   int plain;            // 1: FP32 sums without Kahan compensation (mfa_options.kspace_plain_sums)
 };
 constexpr int KS_FB = 128;       // particles per force block
@@ -257,11 +260,19 @@ bool kspace_dense(const KSpace& K, bool mixed);
 size_t kspace_force_smem(const KSpace& K, bool mixed);
 // host-side preparation of the kernels (shared-memory opt-in); returns a CUDA error
 int kspace_prepare(const KSpace& K, bool mixed);
-// fused: the mixed-precision fused step adds into the FP32 force array, otherwise into FP64
-void launch_kspace(const DevState& s, const SimConst& C, const KSpace& K, cudaStream_t st, bool eflag, Acc acc,
-                   bool fused = false);
-void launch_dipolar(const DevState& s, const SimConst& C, const KSpace& K, cudaStream_t st, bool eflag, Acc acc,
-                    bool fused = false);
+// The k-spaces of a batch and the largest extents of each kernel's grid over them.
+struct KSpaceBatch {
+  const KSpace* d;  // [n] in device memory
+  int n, nq, dip, tab, rows, pchunks, nz, sum, dense_p, dense_k, qf, force_p, force_k;
+  size_t force_shm;
+};
+KSpaceBatch kspace_batch(const std::vector<KSpace>& Ks, bool mixed);
+// ewald_k and dipolar_correction into the FP64 force array; both at once, as the fused step takes
+// them (mixed: into the FP32 force array).  They return the kernels launched.
+int launch_kspace(const DevState& s, const SimConst& C, const KSpaceBatch& B, cudaStream_t st, bool eflag, Acc acc);
+int launch_dipolar(const DevState& s, const SimConst& C, const KSpaceBatch& B, cudaStream_t st, bool eflag, Acc acc);
+int launch_kspace_step(const DevState& s, const SimConst& C, const KSpaceBatch& B, cudaStream_t st, bool eflag,
+                       Acc acc);
 
 // implicit 9-3 walls (fluid_wall.f90:93-121): the bottom wall's F_z in fb, the top wall's in ft,
 // e = energy of both walls
