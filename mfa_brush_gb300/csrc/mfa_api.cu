@@ -313,6 +313,8 @@ int setup_kspace(mfa_ctx* ctx, const int32_t* a_type, int rep) {
     krow[k] = (int)rows.size() - 1;
   }
   K.nrows = (int)rows.size();
+  for (int r = 0; r < K.nrows; r += KS_RB)
+    K.zc_max = std::max(K.zc_max, rows[std::min(r + KS_RB, K.nrows) - 1].w - rows[r].w + 1);
   // slots of a row: nx = -nxm .. -nxm + 4 qx - 1 (the dense slot table of the force kernel)
   K.qx = (2 * nx + 1 + 3) / 4;
   // force chunks of whole rows: KS_FR for the dense kernel; for the one-k-at-a-time kernel as
@@ -891,7 +893,7 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
       int r = setup_kspace(ctx, a_type, rep);
       if (r != MFA_OK) return r;
     }
-    ctx->KB = kspace_batch(ctx->Ks, S.mixed);
+    ctx->KB = kspace_batch(ctx->Ks, S.mixed, S.nsm);
     KSpace* dks = nullptr;
     DA(dks, n_rep);
     CK(cudaMemcpy(dks, ctx->Ks.data(), sizeof(KSpace) * n_rep, cudaMemcpyHostToDevice));

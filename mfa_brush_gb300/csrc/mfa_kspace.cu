@@ -73,25 +73,55 @@ __device__ __forceinline__ const kcplx<MIXED>* ktab(const KSpace& K) {
   if constexpr (MIXED) return K.tabf; else return K.tabd;
 }
 
+// Two FP32 multiply-adds in one instruction (each rounded as fmaf rounds): the sums below are bound by
+// instruction issue, and a packed one takes one slot for two.
+__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)),
+        "l"(reinterpret_cast<unsigned long long&>(c)));
+  return d;
+}
+
+// (a - ca) + (b - cb) with the compensations ca, cb of sums a, b: rounded sum and remainder (Knuth)
+__device__ __forceinline__ float2 two_sum(float a, float b, float ca, float cb) {
+  const float h = __fadd_rn(a, b), t = __fsub_rn(h, a);
+  const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(h, t)), __fsub_rn(b, t));
+  return make_float2(h, __fsub_rn(e, __fadd_rn(ca, cb)));
+}
+
+// a column of the tables into shared memory, asynchronously
+template <typename Cx>
+__device__ __forceinline__ void cp_async(Cx* to, const Cx* from) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from),
+               "n"(sizeof(Cx))
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
 constexpr int KS_TILE = 32;  // particles per shared-memory tile of k_ks_rho (one per lane)
 
 // rho(row, nx) = sum_p A(p, row) X(p, nx), A = q Y(ny) Z(nz), with X(p, -n) = conj X(p, n): the
 // four real sums P1 = sum a c, P2 = sum b d, P3 = sum a d, P4 = sum b c over A = a + ib,
 // X(p, n) = c + id give both rho(row, n) = (P1 - P2, P3 + P4) and rho(row, -n) = (P1 + P2,
-// P4 - P3).  A block takes KS_RB rows, 16 slots n = 16 z .. 16 z + 15 (blockIdx.z) and a chunk of
-// particles.  Lane l owns slot n = 16 z + (l & 15); warp w owns rows 8 w .. 8 w + 7, four of them
-// per half-warp (l >> 4).  Per particle a lane reads its X (the half-warps share the 16 slots)
-// and its four A (two 16-byte loads, one address per half-warp) for 16 FMAs, which cover up to
-// eight k: half the products of a slot per signed nx.  Slots outside a row's k-range are
-// computed and not stored.  The staging stores, one particle per lane, use odd (X) or 4 mod 32
-// word (A) row strides.
+// P4 - P3).  A block takes KS_RB rows, 16 slots n = 16 z .. 16 z + 15 and a chunk of
+// particles, in tiles of 32.  Lane l owns slot n = 16 z + (l & 15); warp w owns rows 8 w .. 8 w + 7,
+// four of them per half-warp (l >> 4).  Per particle a lane reads its X (the half-warps share the 16
+// slots) and its four A (two 16-byte loads, one address per half-warp) for 16 multiply-adds, packed
+// by two in FP32 (P1, P2 from (a, b) (c, d), P3, P4 from (a, b) (d, c)), which cover up to eight k.
+// Slots outside a row's k-range are computed and not stored.  The table columns that the block's
+// rows and slots use are copied a tile ahead (cp.async); the A of a tile is formed from them.  (Read
+// from global memory when the tile began, their latency stood before every tile: with the packed
+// sums 57 -> 39 us on the charged brush.)
 constexpr int KS_RHO_T = 256;  // threads of a k_ks_rho block (8 warps)
 constexpr int KS_RW = 8;       // rows per warp (four per half-warp)
-constexpr int KS_RB = 64;      // rows per block
 constexpr int KS_SL = 16;      // |nx| slots per block
-constexpr int KS_XS = KS_SL + 1;  // X row stride (8-byte slots)
-constexpr int KS_AS = KS_RB + 2;  // A row stride (8-byte slots; 16-byte aligned rows)
-static_assert(KS_TILE * KS_XS * sizeof(float2) % 16 == 0, "the A rows follow the X rows 16-byte aligned");
+constexpr int KS_CS = KS_TILE + 1;  // column stride (odd: 16 slots of one particle are 16 banks apart)
+constexpr int KS_AS = KS_RB + 2;  // A row stride (16-byte aligned rows)
+static_assert(KS_TILE * KS_AS * sizeof(float2) % 16 == 0, "the columns follow the A rows 16-byte aligned");
 
 template <bool MIXED>
 __global__ void __launch_bounds__(KS_RHO_T, MIXED ? 3 : 1) k_ks_rho(const KSpace* __restrict__ Ks, int nz) {
@@ -101,127 +131,153 @@ __global__ void __launch_bounds__(KS_RHO_T, MIXED ? 3 : 1) k_ks_rho(const KSpace
   using real = kreal<MIXED>;
   using Cx = kcplx<MIXED>;
   extern __shared__ __align__(16) unsigned char shraw[];
-  Cx* Xs = reinterpret_cast<Cx*>(shraw);              // [KS_TILE][KS_XS]
-  Cx* As = Xs + KS_TILE * KS_XS;                      // [KS_TILE][KS_AS] (16-byte aligned: 32 x 17 x 8 B)
-  int2* rc = reinterpret_cast<int2*>(As + KS_TILE * KS_AS);  // [KS_RB] signed Y column, Z column
+  Cx* As = reinterpret_cast<Cx*>(shraw);              // [KS_TILE][KS_AS]
+  int2* rc = reinterpret_cast<int2*>(As + KS_TILE * KS_AS);  // [KS_RB] signed Y column, Z column (of a tile)
+  Cx* cols = reinterpret_cast<Cx*>(rc + KS_RB);       // two tiles of columns: 16 X, the Y, the block's Z
   const Cx* tab = ktab<MIXED>(K);
   const int rbeg = blockIdx.x * KS_RB, nr = min(KS_RB, K.nrows - rbeg);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4;
   constexpr int NW = KS_RHO_T / 32;
   constexpr int RL = KS_RW / 2;  // rows per lane
   const int slot = zs * KS_SL + (lane & (KS_SL - 1));  // |nx| of the lane
-  const int r0 = warp * KS_RW + half * RL;                      // the lane's first row
+  const int r0 = warp * KS_RW + half * RL;             // the lane's first row
   const bool act = r0 < nr;
+  // (rows come kz outer: the block's Z columns are one range)
+  const int zlo = K.rows[rbeg].w, nzc = K.rows[rbeg + nr - 1].w - zlo + 1, ncols = KS_SL + K.nym + 1 + nzc;
   for (int r = threadIdx.x; r < nr; r += KS_RHO_T) {
     const int4 R = K.rows[rbeg + r];
-    const int yc = K.nxm + 1 + abs(R.z);
-    rc[r] = make_int2(R.z < 0 ? -yc : yc, K.nxm + K.nym + 2 + R.w);
+    const int yc = KS_SL + abs(R.z);
+    rc[r] = make_int2(R.z < 0 ? -yc : yc, KS_SL + K.nym + 1 + R.w - zlo);
   }
   const int p_beg = blockIdx.y * K.pchunk, p_end = min(K.nq, p_beg + K.pchunk);
+  auto fetch = [&](int t0, int buf) {
+    const int pq = t0 + lane;
+    if (pq < p_end) {
+      Cx* to = cols + buf * ncols * KS_CS + lane;
+      for (int c = warp; c < ncols; c += NW) {
+        const int n = zs * KS_SL + c;  // X column
+        const int col = c < KS_SL ? n : (c < KS_SL + K.nym + 1 ? K.nxm + 1 + c - KS_SL
+                                                               : K.nxm + K.nym + 2 + zlo + c - KS_SL - K.nym - 1);
+        if (c >= KS_SL || n <= K.nxm) cp_async(to + c * KS_CS, tab + (size_t)col * K.nq + pq);
+      }
+    }
+    cp_async_commit();
+  };
+  // (X slots past nxm are never fetched: zero in both tiles)
+  for (int c = K.nxm + 1 - zs * KS_SL + warp; c < KS_SL; c += NW) {
+    Cx zero;
+    zero.x = zero.y = 0;
+    if (c >= 0) cols[c * KS_CS + lane] = cols[(ncols + c) * KS_CS + lane] = zero;
+  }
   real s[4][RL], c[4][RL];  // sums P1..P4 across tiles and their compensations
 #pragma unroll
   for (int a = 0; a < 4; ++a)
 #pragma unroll
     for (int i = 0; i < RL; ++i) s[a][i] = c[a][i] = 0;
-  for (int t0 = p_beg; t0 < p_end; t0 += KS_TILE) {
+  fetch(p_beg, 0);
+  int buf = 0;
+  for (int t0 = p_beg; t0 < p_end; t0 += KS_TILE, buf ^= 1) {
     const int nt = min(KS_TILE, p_end - t0);
-    __syncthreads();
+    real q = 0;
     if (lane < nt) {
-      const int pq = t0 + lane;
-      real q;
-      if constexpr (MIXED) q = K.qvalf[pq]; else q = K.qval[pq];
+      if constexpr (MIXED) q = K.qvalf[t0 + lane]; else q = K.qval[t0 + lane];
+    }
+    cp_async_wait<0>();
+    __syncthreads();  // this tile's columns are here; the A and columns of the tile before are used up
+    fetch(t0 + KS_TILE, buf ^ 1);  // (nothing past the last tile)
+    const Cx* col = cols + buf * ncols * KS_CS;
+    if (lane < nt) {
 #pragma unroll
-      for (int i = 0; i < KS_SL / NW; ++i) {  // slot columns warp + NW i
-        const int n = zs * KS_SL + warp + NW * i;
-        Cx xv;
-        xv.x = 0;
-        xv.y = 0;
-        if (n <= K.nxm) xv = tab[(size_t)n * K.nq + pq];
-        Xs[lane * KS_XS + warp + NW * i] = xv;
-      }
-#pragma unroll
-      for (int h = 0; h < KS_RB / NW; h += 4) {  // rows warp + NW (h .. h+3)
-        Cx yv[4], zv[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int r = warp + NW * (h + i);
-          if (r < nr) {
-            const int2 R = rc[r];
-            yv[i] = tab[(size_t)abs(R.x) * K.nq + pq];
-            zv[i] = tab[(size_t)R.y * K.nq + pq];
-          }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int r = warp + NW * (h + i);
-          if (r < nr) {
-            if (rc[r].x < 0) yv[i].y = -yv[i].y;
-            Cx A;
-            cmul(yv[i], zv[i], A);
-            A.x *= q;
-            A.y *= q;
-            As[lane * KS_AS + r] = A;
-          }
+      for (int h = 0; h < KS_RB / NW; ++h) {
+        const int r = warp + NW * h;
+        if (r < nr) {
+          const int2 R = rc[r];
+          Cx y = col[abs(R.x) * KS_CS + lane];
+          const Cx z = col[R.y * KS_CS + lane];
+          if (R.x < 0) y.y = -y.y;
+          Cx A;
+          cmul(y, z, A);
+          A.x *= q;
+          A.y *= q;
+          As[lane * KS_AS + r] = A;
         }
       }
     }
     __syncthreads();
     if (act) {
       // plain sums over the tile's particles, compensated sums across tiles
-      real t[4][RL];
+      const Cx* xs = col + (lane & (KS_SL - 1)) * KS_CS;
+      if constexpr (MIXED) {
+        float2 t01[RL], t23[RL];
 #pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int i = 0; i < RL; ++i) t[a][i] = 0;
-#pragma unroll 1
-      for (int p = 0; p < nt; ++p) {
-        const Cx x = Xs[p * KS_XS + (lane & (KS_SL - 1))];
-        Cx A[RL];
-        if constexpr (MIXED) {
+        for (int i = 0; i < RL; ++i) t01[i] = t23[i] = make_float2(0.f, 0.f);
+#pragma unroll 2
+        for (int p = 0; p < nt; ++p) {
+          const float2 x = xs[p], xr = make_float2(x.y, x.x);
           const float4* A4 = reinterpret_cast<const float4*>(As + p * KS_AS + r0);
 #pragma unroll
           for (int i = 0; i < RL / 2; ++i) {
             const float4 u = A4[i];
-            A[2 * i] = make_float2(u.x, u.y);
-            A[2 * i + 1] = make_float2(u.z, u.w);
+            const float2 a = make_float2(u.x, u.y), b = make_float2(u.z, u.w);
+            t01[2 * i] = ffma2(a, x, t01[2 * i]);
+            t23[2 * i] = ffma2(a, xr, t23[2 * i]);
+            t01[2 * i + 1] = ffma2(b, x, t01[2 * i + 1]);
+            t23[2 * i + 1] = ffma2(b, xr, t23[2 * i + 1]);
           }
-        } else {
-#pragma unroll
-          for (int i = 0; i < RL; ++i) A[i] = As[p * KS_AS + r0 + i];
         }
 #pragma unroll
         for (int i = 0; i < RL; ++i) {
-          t[0][i] = fma(A[i].x, x.x, t[0][i]);
-          t[1][i] = fma(A[i].y, x.y, t[1][i]);
-          t[2][i] = fma(A[i].x, x.y, t[2][i]);
-          t[3][i] = fma(A[i].y, x.x, t[3][i]);
+          ksum<MIXED>(s[0][i], c[0][i], t01[i].x, K.plain);
+          ksum<MIXED>(s[1][i], c[1][i], t01[i].y, K.plain);
+          ksum<MIXED>(s[2][i], c[2][i], t23[i].x, K.plain);
+          ksum<MIXED>(s[3][i], c[3][i], t23[i].y, K.plain);
         }
+      } else {
+        real t[4][RL];
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+          for (int i = 0; i < RL; ++i) t[a][i] = 0;
+#pragma unroll 1
+        for (int p = 0; p < nt; ++p) {
+          const Cx x = xs[p];
+#pragma unroll
+          for (int i = 0; i < RL; ++i) {
+            const Cx A = As[p * KS_AS + r0 + i];
+            t[0][i] = fma(A.x, x.x, t[0][i]);
+            t[1][i] = fma(A.y, x.y, t[1][i]);
+            t[2][i] = fma(A.x, x.y, t[2][i]);
+            t[3][i] = fma(A.y, x.x, t[3][i]);
+          }
+        }
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+          for (int i = 0; i < RL; ++i) ksum<MIXED>(s[a][i], c[a][i], t[a][i], K.plain);
       }
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int i = 0; i < RL; ++i) ksum<MIXED>(s[a][i], c[a][i], t[a][i], K.plain);
     }
   }
   if (act && slot <= K.nxm) {
-    double* o = K.rho_part + (size_t)blockIdx.y * 2 * K.nk;
 #pragma unroll
     for (int i = 0; i < RL; ++i) {
       const int r = r0 + i;
       if (r < nr) {
         const int4 R = K.rows[rbeg + r];
-        const double p1 = (double)s[0][i] - (double)c[0][i], p2 = (double)s[1][i] - (double)c[1][i];
-        const double p3 = (double)s[2][i] - (double)c[2][i], p4 = (double)s[3][i] - (double)c[3][i];
         const int lo = K.kn[R.x].x;  // the row's first nx
-        const int kp = R.x + slot - lo;
-        if (kp >= R.x && kp < R.y) {
-          o[2 * kp] = p1 - p2;
-          o[2 * kp + 1] = p3 + p4;
-        }
-        const int km = R.x - slot - lo;
-        if (slot > 0 && km >= R.x && km < R.y) {
-          o[2 * km] = p1 + p2;
-          o[2 * km + 1] = p4 - p3;
+        const int kp = R.x + slot - lo, km = R.x - slot - lo;
+        const bool hp = kp >= R.x && kp < R.y, hm = slot > 0 && km >= R.x && km < R.y;
+        if constexpr (MIXED) {
+          // P +- P' as an unevaluated FP32 sum (48 bits): FP64 here, all blocks at their ends at
+          // once, took a quarter of the kernel
+          float4* o = reinterpret_cast<float4*>(K.rho_part) + (size_t)blockIdx.y * K.nk;
+          const float2 a = two_sum(s[0][i], -s[1][i], c[0][i], -c[1][i]), b = two_sum(s[2][i], s[3][i], c[2][i], c[3][i]);
+          const float2 e = two_sum(s[0][i], s[1][i], c[0][i], c[1][i]), f = two_sum(s[3][i], -s[2][i], c[3][i], -c[2][i]);
+          if (hp) o[kp] = make_float4(a.x, a.y, b.x, b.y);
+          if (hm) o[km] = make_float4(e.x, e.y, f.x, f.y);
+        } else {
+          double2* o = reinterpret_cast<double2*>(K.rho_part) + (size_t)blockIdx.y * K.nk;
+          if (hp) o[kp] = make_double2(s[0][i] - s[1][i], s[2][i] + s[3][i]);
+          if (hm) o[km] = make_double2(s[0][i] + s[1][i], s[3][i] - s[2][i]);
         }
       }
     }
@@ -326,16 +382,22 @@ __global__ void __launch_bounds__(KS_TAB_T) k_ks_tables(DevState s, const KSpace
   if (!(what & KS_RECIP) || K.nk == 0 || idx >= K.nq * K.ncol) return;
   const int col = idx / K.nq, p = idx - col * K.nq;
   const int i = s.slot_of_tag[K.qtag[p]];
-  double u;
-  if (col <= K.nxm) u = (double)col * K.cx * s.rx[i];
-  else if (col <= K.nxm + 1 + K.nym) u = (double)(col - K.nxm - 1) * K.cy * s.ry[i];
-  else u = (double)(col - K.nxm - K.nym - 2) * K.cz * s.rz[i];
-  u -= rint(u);  // turns in [-1/2, 1/2]
+  int n = col, ax = 0;
+  if (col > K.nxm + 1 + K.nym) { n = col - K.nxm - K.nym - 2; ax = 2; }
+  else if (col > K.nxm) { n = col - K.nxm - 1; ax = 1; }
+  // the phase of n = 1 in turns as a 64-bit fixed point (2^-58), times n with wrap-around: its top 32
+  // bits are the phase in [-1/2, 1/2) turns.  One FP64 product; in FP64 the products, the reduction
+  // and the conversions of a column bound this kernel.
+  double t = (ax == 0 ? K.cx * s.rx[i] : (ax == 1 ? K.cy * s.ry[i] : K.cz * s.rz[i]));
+  if ((__double2hiint(t) & 0x7FFFFFFF) >= 0x40200000) t -= rint(t);  // (8 turns away: not wrapped yet)
   if constexpr (MIXED) {
+    const unsigned long long ph = (unsigned long long)round_bits(t * 288230376151711744.0) * (unsigned)n << 6;
     float sn, cs;
-    sincospif(2.f * (float)u, &sn, &cs);
+    sincospif(i2f_fast((int)(ph >> 32)) * (2.f / 4294967296.f), &sn, &cs);
     K.tabf[idx] = make_float2(cs, sn);
   } else {
+    double u = (double)n * t;
+    u -= rint(u);  // turns in [-1/2, 1/2]
     double sn, cs;
     sincospi(2. * u, &sn, &cs);
     K.tabd[idx] = make_double2(cs, sn);
@@ -362,9 +424,15 @@ __global__ void __launch_bounds__(256) k_ks_rho_sum(const KSpace* __restrict__ K
     if (k < K.nk) {
 #pragma unroll 4
       for (int c = g; c < K.npchunks; c += 8) {
-        const double2 v = reinterpret_cast<const double2*>(K.rho_part + (size_t)c * 2 * K.nk)[k];
-        re += v.x;
-        im += v.y;
+        if constexpr (MIXED) {
+          const float4 v = reinterpret_cast<const float4*>(K.rho_part)[(size_t)c * K.nk + k];
+          re += f2d_fast(v.x) + f2d_fast(v.y);
+          im += f2d_fast(v.z) + f2d_fast(v.w);
+        } else {
+          const double2 v = reinterpret_cast<const double2*>(K.rho_part)[(size_t)c * K.nk + k];
+          re += v.x;
+          im += v.y;
+        }
       }
     }
     part[g][kl] = make_double2(re, im);
@@ -532,10 +600,13 @@ __global__ void __launch_bounds__(KS_FB) k_ks_force(const KSpace* __restrict__ K
 // table (k_ks_rho_sum's (W, kx W) per signed slot) while staging it.  The rows are taken in order
 // of their slot range (frow), so that the rows of a chunk share a narrow window of slots; slots
 // outside the window are skipped (a branch uniform over the block).
-template <int QF>
+// A thread takes PP particles KS_FB apart: with one, the broadcast loads of the slots bound the kernel (L1
+// at 83 %); two share them (68 -> 51 us on the charged brush, 13,760 charges and 509 rows; the
+// multiply-adds alone, at 16 slots a row, are 23 us of the FP32 pipe).
+template <int QF, int PP>
 __global__ void __launch_bounds__(KS_FB) k_ks_force_dense(const KSpace* __restrict__ Ks) {
   const KSpace K = Ks[blockIdx.z];
-  if (!K.dense || (int)blockIdx.x * KS_FB >= K.nq || (int)blockIdx.y >= K.nkchunks) return;
+  if (!K.dense || (int)blockIdx.x * KS_FB * PP >= K.nq || (int)blockIdx.y >= K.nkchunks) return;
   constexpr int NF = 4 * QF;  // folded slots |n| = 0 .. NF - 1
   extern __shared__ __align__(16) unsigned char shraw[];
   float4* Wd = reinterpret_cast<float4*>(shraw);              // [KS_FR][NF][2]
@@ -555,8 +626,11 @@ __global__ void __launch_bounds__(KS_FB) k_ks_force_dense(const KSpace* __restri
       wp = wsrc[r * nsig + nxm + m];
       if (m > 0) wm = wsrc[r * nsig + nxm - m];
     }
-    Wd[2 * e] = make_float4(wp.x + wm.x, wp.y - wm.y, wp.y + wm.y, wp.x - wm.x);
-    Wd[2 * e + 1] = make_float4(wp.z + wm.z, wp.w - wm.w, wp.w + wm.w, wp.z - wm.z);
+    // slots side by side by two, for the packed multiply-adds: of slots m, m + 1 the words 2 q, 2 q + 1
+    // hold the q-th of (u + u', v - v', v + v', u' - u) and of the same of the Sx columns
+    float* o = reinterpret_cast<float*>(Wd) + 16 * (e >> 1) + (e & 1);
+    o[0] = wp.x + wm.x; o[2] = wp.y - wm.y; o[4] = wp.y + wm.y; o[6] = wm.x - wp.x;
+    o[8] = wp.z + wm.z; o[10] = wp.w - wm.w; o[12] = wp.w + wm.w; o[14] = wm.z - wp.z;
   }
   for (int r = threadIdx.x; r < nr; r += KS_FB) {
     const int4 R = K.rows[K.frow[rbeg + r]];
@@ -564,60 +638,87 @@ __global__ void __launch_bounds__(KS_FB) k_ks_force_dense(const KSpace* __restri
     rc[r] = make_int2(R.z < 0 ? -yc : yc, nxm + K.nym + 2 + R.w);
     ryz[r] = make_float2((float)K.kvec[3 * R.x + 1], (float)K.kvec[3 * R.x + 2]);
   }
-  const int p = blockIdx.x * KS_FB + threadIdx.x;
-  const int pc = min(p, K.nq - 1);
-  const float2* T = K.tabf + pc;
-  float2 X[NF];
+  const int p0 = blockIdx.x * KS_FB * PP + threadIdx.x;
+  const float2* T[PP];
+  float2 Xc[PP][NF / 2], Xd[PP][NF / 2];  // X = c + id of slots 2 j, 2 j + 1 as (c, c'), (d, d')
 #pragma unroll
-  for (int j = 0; j < NF; ++j) {
-    X[j] = make_float2(0.f, 0.f);
-    if (j >= mlo && j <= mhi && j <= nxm) X[j] = T[(size_t)j * K.nq];
+  for (int a = 0; a < PP; ++a) {
+    T[a] = K.tabf + min(p0 + a * KS_FB, K.nq - 1);
+#pragma unroll
+    for (int j = 0; j < NF / 2; ++j) {
+      float2 x = make_float2(0.f, 0.f), y = x;
+      if (2 * j >= mlo && 2 * j <= mhi && 2 * j <= nxm) x = T[a][(size_t)(2 * j) * K.nq];
+      if (2 * j + 1 >= mlo && 2 * j + 1 <= mhi && 2 * j + 1 <= nxm) y = T[a][(size_t)(2 * j + 1) * K.nq];
+      Xc[a][j] = make_float2(x.x, y.x);
+      Xd[a][j] = make_float2(x.y, y.y);
+    }
   }
   __syncthreads();
-  if (p >= K.nq) return;
-  float fx = 0.f, fy = 0.f, fz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
+  if (p0 >= K.nq) return;
+  float F[PP][3], Fc[PP][3];  // sums and compensations
+  float2 Y[PP], Z[PP];
   int2 R = rc[0];
-  float2 Y = T[(size_t)abs(R.x) * K.nq], Z = T[(size_t)R.y * K.nq];
+#pragma unroll
+  for (int a = 0; a < PP; ++a) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) F[a][d] = Fc[a][d] = 0.f;
+    Y[a] = T[a][(size_t)abs(R.x) * K.nq];
+    Z[a] = T[a][(size_t)R.y * K.nq];
+  }
   for (int r = 0; r < nr; ++r) {
     int2 Rn = R;
-    float2 Yn = Y, Zn = Z;
-    if (r + 1 < nr) {
-      Rn = rc[r + 1];
-      Yn = T[(size_t)abs(Rn.x) * K.nq];
-      Zn = T[(size_t)Rn.y * K.nq];
+    float2 YZ[PP];
+#pragma unroll
+    for (int a = 0; a < PP; ++a) {
+      if (R.x < 0) Y[a].y = -Y[a].y;
+      cmul(Y[a], Z[a], YZ[a]);
     }
-    if (R.x < 0) Y.y = -Y.y;
-    float2 YZ;
-    cmul(Y, Z, YZ);
+    if (r + 1 < nr) {  // the next row's factors, while this one is summed
+      Rn = rc[r + 1];
+#pragma unroll
+      for (int a = 0; a < PP; ++a) {
+        Y[a] = T[a][(size_t)abs(Rn.x) * K.nq];
+        Z[a] = T[a][(size_t)Rn.y * K.nq];
+      }
+    }
     const float4* w = Wd + r * NF * 2;
-    float s_re = 0.f, s_im = 0.f, x_re = 0.f, x_im = 0.f;
+    float2 sr[PP], si[PP], xr[PP], xi[PP];  // S and Sx over even and odd slots
+#pragma unroll
+    for (int a = 0; a < PP; ++a) sr[a] = si[a] = xr[a] = xi[a] = make_float2(0.f, 0.f);
 #pragma unroll
     for (int g = 0; g < QF; ++g) {  // groups of four slots; a group outside the window is skipped
       if (4 * g + 3 < mlo || 4 * g > mhi) continue;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float2 x = X[4 * g + i];
-        const float4 a = w[2 * (4 * g + i)], b = w[2 * (4 * g + i) + 1];
-        s_re = fmaf(x.x, a.x, fmaf(x.y, a.y, s_re));
-        s_im = fmaf(x.x, a.z, fmaf(-x.y, a.w, s_im));
-        x_re = fmaf(x.x, b.x, fmaf(x.y, b.y, x_re));
-        x_im = fmaf(x.x, b.z, fmaf(-x.y, b.w, x_im));
+      for (int i = 2 * g; i < 2 * g + 2; ++i) {
+        const float4 u = w[4 * i], v = w[4 * i + 1], ux = w[4 * i + 2], vx = w[4 * i + 3];
+#pragma unroll
+        for (int a = 0; a < PP; ++a) {
+          sr[a] = ffma2(Xc[a][i], make_float2(u.x, u.y), ffma2(Xd[a][i], make_float2(u.z, u.w), sr[a]));
+          si[a] = ffma2(Xc[a][i], make_float2(v.x, v.y), ffma2(Xd[a][i], make_float2(v.z, v.w), si[a]));
+          xr[a] = ffma2(Xc[a][i], make_float2(ux.x, ux.y), ffma2(Xd[a][i], make_float2(ux.z, ux.w), xr[a]));
+          xi[a] = ffma2(Xc[a][i], make_float2(vx.x, vx.y), ffma2(Xd[a][i], make_float2(vx.z, vx.w), xi[a]));
+        }
       }
     }
-    const float srow = YZ.x * s_im - YZ.y * s_re;
-    const float sxrow = YZ.x * x_im - YZ.y * x_re;
     const float2 kyz = ryz[r];
-    ksum<true>(fx, cx, sxrow, K.plain);
-    ksum<true>(fy, cy, kyz.x * srow, K.plain);
-    ksum<true>(fz, cz, kyz.y * srow, K.plain);
+#pragma unroll
+    for (int a = 0; a < PP; ++a) {
+      const float srow = YZ[a].x * (si[a].x + si[a].y) - YZ[a].y * (sr[a].x + sr[a].y);
+      const float sxrow = YZ[a].x * (xi[a].x + xi[a].y) - YZ[a].y * (xr[a].x + xr[a].y);
+      ksum<true>(F[a][0], Fc[a][0], sxrow, K.plain);
+      ksum<true>(F[a][1], Fc[a][1], kyz.x * srow, K.plain);
+      ksum<true>(F[a][2], Fc[a][2], kyz.y * srow, K.plain);
+    }
     R = Rn;
-    Y = Yn;
-    Z = Zn;
   }
-  double* o = K.fpart + ((size_t)blockIdx.y * K.nq + p) * 3;
-  o[0] = (double)fx - (double)cx;
-  o[1] = (double)fy - (double)cy;
-  o[2] = (double)fz - (double)cz;
+#pragma unroll
+  for (int a = 0; a < PP; ++a) {
+    const int p = p0 + a * KS_FB;
+    if (p >= K.nq) return;
+    double* o = K.fpart + ((size_t)blockIdx.y * K.nq + p) * 3;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) o[d] = f2d_fast(F[a][d]) - f2d_fast(Fc[a][d]);
+  }
 }
 
 // F_i = -(8 pi q_i / V) * sum over k-chunks in a fixed order, and the slab term's -4 pi q_i M_z / V
@@ -649,8 +750,10 @@ __global__ void __launch_bounds__(128) k_ks_force_sum(DevState s, const KSpace* 
 }
 
 namespace {
-size_t rho_smem(bool mixed) {
-  return (size_t)KS_TILE * (KS_XS + KS_AS) * (mixed ? sizeof(float2) : sizeof(double2)) +
+// (zc: the most Z columns that the rows of a block use)
+size_t rho_smem(int nym, int zc, bool mixed) {
+  return ((size_t)KS_TILE * KS_AS + 2 * (size_t)(KS_SL + nym + 1 + zc) * KS_CS) *
+             (mixed ? sizeof(float2) : sizeof(double2)) +
          (size_t)KS_RB * sizeof(int2);
 }
 size_t force_smem(const KSpace& K, bool mixed) {
@@ -666,10 +769,11 @@ size_t dense_smem(int qf) {
 constexpr int KS_DENSE_QX_MAX = 8;  // the register-resident X of k_ks_force_dense: nxm <= 15
 
 template <int QF>
-void launch_dense(const KSpace* Ks, size_t shm, dim3 g, cudaStream_t st) {
-  k_ks_force_dense<QF><<<g, KS_FB, shm, st>>>(Ks);
+void launch_dense(const KSpace* Ks, size_t shm, dim3 g, int pp, cudaStream_t st) {
+  if (pp == 2) k_ks_force_dense<QF, 2><<<g, KS_FB, shm, st>>>(Ks);
+  else k_ks_force_dense<QF, 1><<<g, KS_FB, shm, st>>>(Ks);
 }
-typedef void (*dense_launcher)(const KSpace*, size_t, dim3, cudaStream_t);
+typedef void (*dense_launcher)(const KSpace*, size_t, dim3, int, cudaStream_t);
 const dense_launcher kDense[5] = {nullptr, launch_dense<1>, launch_dense<2>, launch_dense<3>, launch_dense<4>};
 bool use_dense(const KSpace& K, bool mixed) { return mixed && K.qx <= KS_DENSE_QX_MAX; }
 }  // namespace
@@ -678,7 +782,7 @@ bool kspace_dense(const KSpace& K, bool mixed) { return use_dense(K, mixed); }
 size_t kspace_force_smem(const KSpace& K, bool mixed) { return force_smem(K, mixed); }
 
 int kspace_prepare(const KSpace& K, bool mixed) {
-  const size_t a = rho_smem(mixed), b = use_dense(K, mixed) ? dense_smem(dense_qf(K)) : force_smem(K, mixed);
+  const size_t a = rho_smem(K.nym, K.zc_max, mixed), b = use_dense(K, mixed) ? dense_smem(dense_qf(K)) : force_smem(K, mixed);
   if (a > KS_SMEM_MAX || b > KS_SMEM_MAX) return (int)cudaErrorInvalidConfiguration;
   // The opt-in is a property of the kernel for the whole process, not of a context: set it to the
   // largest allowed size once, so that no context lowers it below another's needs (occupancy
@@ -691,8 +795,13 @@ int kspace_prepare(const KSpace& K, bool mixed) {
   return (int)e;  // dense_smem stays below 48 KB: 32 rows x 16 folded slots x 32 B + 512 B
 }
 
-KSpaceBatch kspace_batch(const std::vector<KSpace>& Ks, bool mixed) {
+KSpaceBatch kspace_batch(const std::vector<KSpace>& Ks, bool mixed, int nsm) {
   KSpaceBatch B = {};
+  // two particles per thread of the dense force kernel when that leaves every SM two blocks
+  long long two = 0;
+  for (const KSpace& K : Ks)
+    if (use_dense(K, mixed)) two += (long long)((K.nq + 2 * KS_FB - 1) / (2 * KS_FB)) * K.nkchunks;
+  B.pp = two >= 2 * nsm ? 2 : 1;
   B.n = (int)Ks.size();
   for (const KSpace& K : Ks) {
     if (K.nq == 0) continue;  // no charges: every block of this replica leaves
@@ -700,13 +809,14 @@ KSpaceBatch kspace_batch(const std::vector<KSpace>& Ks, bool mixed) {
     B.tab = std::max(B.tab, K.nk ? (K.nq * K.ncol + KS_TAB_T - 1) / KS_TAB_T : 0);
     B.nq = std::max(B.nq, K.nq);
     if (K.nk == 0) continue;
+    B.rho_shm = std::max(B.rho_shm, rho_smem(K.nym, K.zc_max, mixed));
     B.rows = std::max(B.rows, (K.nrows + KS_RB - 1) / KS_RB);
     B.pchunks = std::max(B.pchunks, K.npchunks);
     B.nz = std::max(B.nz, (K.nxm + KS_SL) / KS_SL);
     B.sum = std::max(B.sum, std::min(KS_RED_MAX, (K.nk + 31) / 32));
     const int fb = (K.nq + KS_FB - 1) / KS_FB;
     if (use_dense(K, mixed)) {
-      B.dense_p = std::max(B.dense_p, fb);
+      B.dense_p = std::max(B.dense_p, (fb + B.pp - 1) / B.pp);
       B.dense_k = std::max(B.dense_k, K.nkchunks);
       B.qf = std::max(B.qf, dense_qf(K));
     } else {
@@ -741,18 +851,17 @@ static int launch_ks(const DevState& s, const SimConst& C, KSpaceBatch B, cudaSt
   }
   if (recip) {
     const dim3 g1(B.rows, B.pchunks, B.nz * B.n), g2(B.sum, B.n);
-    const size_t shm1 = rho_smem(s.mixed);
     const double fac_alpha = 1. / (4. * C.alpha_c);
     if (s.mixed) {
-      k_ks_rho<true><<<g1, KS_RHO_T, shm1, st>>>(B.d, B.nz);
+      k_ks_rho<true><<<g1, KS_RHO_T, B.rho_shm, st>>>(B.d, B.nz);
       k_ks_rho_sum<true><<<g2, 256, 0, st>>>(B.d, 4. * pi, fac_alpha, acc, eflag);
     } else {
-      k_ks_rho<false><<<g1, KS_RHO_T, shm1, st>>>(B.d, B.nz);
+      k_ks_rho<false><<<g1, KS_RHO_T, B.rho_shm, st>>>(B.d, B.nz);
       k_ks_rho_sum<false><<<g2, 256, 0, st>>>(B.d, 4. * pi, fac_alpha, acc, eflag);
     }
     launches += 2;
     if (B.dense_p) {
-      kDense[B.qf](B.d, dense_smem(B.qf), dim3(B.dense_p, B.dense_k, B.n), st);
+      kDense[B.qf](B.d, dense_smem(B.qf), dim3(B.dense_p, B.dense_k, B.n), B.pp, st);
       ++launches;
     }
     if (B.force_p) {

@@ -231,7 +231,8 @@ struct KSpace {
   // The dense slot table has 4 qx slots per row, nx = -nxm .. -nxm + 4 qx - 1.
   int qx;
   int pchunk, npchunks;
-  double* rho_part;     // [npchunks][2*nk]
+  int zc_max;           // Z columns that a block of KS_RB rows uses, at most
+  double* rho_part;     // [npchunks][2*nk] (mixed: four FP32 words per k, two per part)
   float4* kdf;          // [nk] (kx, G Re rho, G Im rho, nx + nxm as int bits)   (mixed)
   double2* kdd;         // [nk] (G Re rho, G Im rho)                              (fp64)
   float4* wdense;       // [nrows][4 qx] (W, kx W) per slot, W = G rho, rows in frow order;
@@ -250,6 +251,7 @@ struct KSpace {
   int dense;            // 1: the force in the dense kernel (kspace_dense)
   int plain;            // 1: FP32 sums without Kahan compensation (mfa_options.kspace_plain_sums)
 };
+constexpr int KS_RB = 64;        // rows per rho block
 constexpr int KS_FB = 128;       // particles per force block
 constexpr int KS_FR = 32;        // rows per force chunk
 constexpr int KS_RED_MAX = 256;  // blocks of a grid reduction, at most
@@ -263,10 +265,10 @@ int kspace_prepare(const KSpace& K, bool mixed);
 // The k-spaces of a batch and the largest extents of each kernel's grid over them.
 struct KSpaceBatch {
   const KSpace* d;  // [n] in device memory
-  int n, nq, dip, tab, rows, pchunks, nz, sum, dense_p, dense_k, qf, force_p, force_k;
-  size_t force_shm;
+  int n, pp, nq, dip, tab, rows, pchunks, nz, sum, dense_p, dense_k, qf, force_p, force_k;
+  size_t rho_shm, force_shm;
 };
-KSpaceBatch kspace_batch(const std::vector<KSpace>& Ks, bool mixed);
+KSpaceBatch kspace_batch(const std::vector<KSpace>& Ks, bool mixed, int nsm);
 // ewald_k and dipolar_correction into the FP64 force array; both at once, as the fused step takes
 // them (mixed: into the FP32 force array).  They return the kernels launched.
 int launch_kspace(const DevState& s, const SimConst& C, const KSpaceBatch& B, cudaStream_t st, bool eflag, Acc acc);
