@@ -761,6 +761,200 @@ __global__ void __launch_bounds__(128, PERSIST ? 8 : ((INTEG && !EFLAG) ? 10 : 9
   }
 }
 
+// The mixed pair kernel for few particles: a small system leaves the thread-per-particle kernel four
+// warps on some SMs, and its time is the latency of one thread's walk (19 us at 6400 particles).  Here
+// PL_G lanes take a particle's list side by side and place the kept entries by a ballot; they evaluate
+// a batch side by side too, and one lane per component adds the products of a batch in list order, so
+// the sums are those of k_pair to the bit (batches of PAIR_BATCH kept entries, products and sums
+// rounded apart).  A warp of its own per block evaluates the bonded terms of the 32 particles
+// meanwhile and then integrates them (FUSED, BONDED, UNI, INTEG as in k_pair).
+constexpr int PL_G = 8, PL_P = 32, PL_T = PL_P * PL_G + 32;
+
+template <bool EFLAG, bool FUSED, bool BONDED, bool UNI, bool INTEG>
+__global__ void __launch_bounds__(PL_T) k_pair_lanes(DevState s, SimConst C, Acc acc, int bmask) {
+  __shared__ PairEntry<float> tab[NPAIR];
+  __shared__ int jl[PL_P][PAIR_BATCH + PL_G];
+  __shared__ float prod[3][PL_P][PAIR_BATCH + 1];
+  __shared__ double tot[3][PL_P];
+  __shared__ float wall_e[PL_P], wall_w[PL_P];
+  const unsigned FULL = 0xffffffffu;
+  for (int k = threadIdx.x; k < NPAIR; k += PL_T) tab[k] = s.tabf[k];
+  const int lane = threadIdx.x & 31;
+  const bool tail = threadIdx.x >= PL_P * PL_G;
+  const int pl = tail ? lane : (int)threadIdx.x / PL_G, i = blockIdx.x * PL_P + pl;
+  const bool inside = i < s.N;
+  const int w = inside ? __ldg(&s.info[i]) : 0;
+  const bool active = inside && info_mobile(w);
+  const int rep = info_rep(w);
+  float fb[3] = {0.f, 0.f, 0.f}, eb[4] = {0.f, 0.f, 0.f, 0.f};
+  BondVir<float> bv;
+  if (EFLAG) bv.zero();
+  __syncthreads();
+  if (tail) {
+    if constexpr (BONDED) {
+      if (active) bonded_of<true, EFLAG>(s, C, bmask, i, w, fb, eb, &bv);
+    }
+  } else {
+    const int q8 = lane & (PL_G - 1), grp = lane / PL_G;
+    const RepDesc& R = s.reps[rep];
+    const int ti = info_type(w), p0 = R.p0;
+    float e_w = 0.f, w_wall = 0.f;
+    double sum = 0.;  // lanes 0..2: the component's total, from the external forces on
+    if (FUSED && active) {
+      if (q8 < 3 && C.poiseuille && ti != 0) sum = f2d_fast(C.mass_f[ti] * C.cforce_f[q8]);
+      if (q8 == 2 && C.wall == 2) {  // as k_pair
+        const double zd = s.rz[i];
+        const float zl = d2f_fast(zd), zh = d2f_fast(R.L[2] - zd);
+        float fwb, fwt;
+        wall93f_split(C, ti, zl, zh, fwb, fwt, e_w);
+        const double ez = f2d_fast(fwb) + f2d_fast(fwt);
+        sum = ez + sum;
+        if (EFLAG) w_wall = fwb * zl - fwt * zh;
+      }
+    }
+    if (EFLAG && FUSED && q8 == 2) {
+      wall_e[pl] = e_w;
+      wall_w[pl] = w_wall;
+    }
+    float run = 0.f;  // without FUSED: the component's FP32 sum over the whole list
+    float e_lj = 0.f, e_c = 0.f, wv[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    const long long step = R.s_time + *s.steps_done;
+    const float r2min = C.force_switch_on ? (float)r2min_of(C, step) : 0.f;
+    const uint32_t nkey = pair_key(R.seed, step);
+    const int n = active ? __ldg(&s.nn[i]) : 0;
+    const int* __restrict__ nb = s.nbr + i;
+    const int4 qi = active ? __ldg(&s.pfx[i]) : make_int4(0, 0, 0, 0);
+    const float4 vi = active ? __ldg(&s.vf[i]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int tag_i = __float_as_int(vi.w) - p0;
+    const float ux = R.ufx_f[0], uy = R.ufx_f[1], uz = R.ufx_f[2];
+    const float cx = ux * 512.f, cy = uy * 512.f, cz = uz * 512.f;
+    int m = 0, k = 0;  // kept entries waiting in jl, list position: alike in the lanes of a particle
+    for (;;) {
+      while (__any_sync(FULL, m < PAIR_BATCH && k < n)) {
+        const bool go = m < PAIR_BATCH && k < n;
+        int j = 0;
+        bool hit = false;
+        if (go && k + q8 < n) {
+          j = __ldg(nb + (size_t)(k + q8) * s.Np);
+          const int4 qj = __ldg(&s.pfx[j]);
+          const float dx = i2f_coarse(fx_diff(qi.x, qj.x), 9) * cx;
+          const float dy = i2f_coarse(fx_diff(qi.y, qj.y), 9) * cy;
+          const float dz = i2f_coarse(fx_diff(qi.z, qj.z), 9) * cz;
+          hit = dx * dx + dy * dy + dz * dz < (UNI ? C.scr2_uni_f : tab[ti * MAXT + info_type(qj.w)].screen2);
+        }
+        const unsigned bits = (__ballot_sync(FULL, hit) >> (grp * PL_G)) & ((1u << PL_G) - 1u);
+        if (hit) jl[pl][m + __popc(bits & ((1u << q8) - 1u))] = j;
+        m += __popc(bits);
+        if (go) k += PL_G;
+      }
+      __syncwarp();
+      const int take = min(m, PAIR_BATCH);
+      if (!__any_sync(FULL, take > 0)) break;
+      for (int c = q8; c < take; c += PL_G) {
+        const int j = jl[pl][c];
+        const int4 qj = __ldg(&s.pfx[j]);
+        const float dx = i2f_fast(fx_diff(qi.x, qj.x)) * ux;
+        const float dy = i2f_fast(fx_diff(qi.y, qj.y)) * uy;
+        const float dz = i2f_fast(fx_diff(qi.z, qj.z)) * uz;
+        const PairEntry<float>& e = tab[ti * MAXT + info_type(qj.w)];
+        const float half = info_mobile(qj.w) ? 0.5f : 1.f;
+        const float fs = pair_fs<EFLAG>(s, C, e, dx, dy, dz, j, vi.x, vi.y, vi.z, tag_i, p0, nkey, r2min, half, e_lj,
+                                        e_c);
+        prod[0][pl][c] = __fmul_rn(fs, dx);
+        prod[1][pl][c] = __fmul_rn(fs, dy);
+        prod[2][pl][c] = __fmul_rn(fs, dz);
+        if (EFLAG) sym_add(wv, half * fs, dx, dy, dz);
+      }
+      __syncwarp();
+      if (q8 < 3) {
+        float f = FUSED ? 0.f : run;
+        for (int c = 0; c < take; ++c) f = __fadd_rn(f, prod[q8][pl][c]);
+        if (FUSED) sum += f2d_fast(f); else run = f;
+      }
+      // the entries past the batch to the front
+      const int left = m - take;
+      const int mv = q8 < left ? jl[pl][take + q8] : 0;
+      __syncwarp();
+      if (q8 < left) jl[pl][q8] = mv;
+      m = left;
+      __syncwarp();
+    }
+    if (q8 < 3) tot[q8][pl] = FUSED ? sum : (double)run;
+    if (EFLAG) {
+      int sl[8];
+      float v[8];
+      sl[0] = O_VFF; v[0] = e_lj;
+      sl[1] = O_VCOUL; v[1] = e_c;
+      sym_slots(sl + 2, v + 2, O_VIR + 9 * V_PAIR, wv);
+      obs_push<float, 8>(acc, sl, v, rep, active);
+    }
+  }
+  __syncthreads();
+  if (!tail) return;
+  float ike = 0.f, ikin[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, ifh[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (inside) {
+    double fxd = tot[0][lane], fyd = tot[1][lane], fzd = tot[2][lane];
+    if (BONDED && active) {
+      fxd += f2d_fast(fb[0]);
+      fyd += f2d_fast(fb[1]);
+      fzd += f2d_fast(fb[2]);
+    }
+    if constexpr (INTEG) {
+      if (active) {
+        int_mixed_particle<2, EFLAG>(s, C, i, w, d2f_fast(fxd), d2f_fast(fyd), d2f_fast(fzd), s.pfx_alt, s.vf_alt,
+                                     ike, ikin, ifh);
+      } else if (C.move_walls) {  // a wall bead on a moving wall: its next site
+        double x, y, z;
+        s.pfx_alt[i] = move_wall_bead(s, C, i, w, x, y, z);
+        s.vf_alt[i] = s.vf[i];
+      } else {  // a wall bead: its views as they are
+        s.pfx_alt[i] = s.pfx[i];
+        s.vf_alt[i] = s.vf[i];
+      }
+      if (i == 0) *s.steps_alt = *s.steps_done + 1;
+    } else if constexpr (FUSED) {
+      s.f4[i] = make_float4(d2f_fast(fxd), d2f_fast(fyd), d2f_fast(fzd), 0.f);
+    } else if (active) {
+      s.fx[i] += fxd;
+      s.fy[i] += fyd;
+      s.fz[i] += fzd;
+    }
+  }
+  if constexpr (EFLAG && FUSED) {
+    constexpr int NB = BONDED ? 31 : 0, NI = INTEG ? 13 : 0, NV = NB + 2 + NI;
+    int sl[NV];
+    float v[NV];
+    if constexpr (BONDED) bonded_slots(sl, v, eb, bv);
+    sl[NB] = O_VFW; v[NB] = wall_e[lane];
+    sl[NB + 1] = O_VIR + 9 * V_WALL + 8; v[NB + 1] = wall_w[lane];
+    if constexpr (INTEG) {
+      constexpr int b = NB + 2;
+      const int idx[6] = {0, 4, 8, 1, 2, 5};
+      sl[b] = O_TFLUID; v[b] = ike;
+#pragma unroll
+      for (int c = 0; c < 6; ++c) {
+        sl[b + 1 + c] = O_KIN + idx[c]; v[b + 1 + c] = ikin[c];
+        sl[b + 7 + c] = O_FH + c; v[b + 7 + c] = ifh[c];
+      }
+    }
+    obs_push<float, NV>(acc, sl, v, rep, active);
+  }
+}
+
+template <bool EFLAG>
+static void launch_pair_lanes(const DevState& s, const SimConst& C, cudaStream_t st, bool fused, Acc acc, int mask,
+                              bool uni, bool integ) {
+  using KernT = void (*)(DevState, SimConst, Acc, int);
+  // [integ][bonded][uni]
+  const KernT kf[2][2][2] = {{{k_pair_lanes<EFLAG, true, false, false, false>, k_pair_lanes<EFLAG, true, false, true, false>},
+                              {k_pair_lanes<EFLAG, true, true, false, false>, k_pair_lanes<EFLAG, true, true, true, false>}},
+                             {{k_pair_lanes<EFLAG, true, false, false, true>, k_pair_lanes<EFLAG, true, false, true, true>},
+                              {k_pair_lanes<EFLAG, true, true, false, true>, k_pair_lanes<EFLAG, true, true, true, true>}}};
+  const KernT kd[2] = {k_pair_lanes<EFLAG, false, false, false, false>, k_pair_lanes<EFLAG, false, false, true, false>};
+  const KernT k = fused ? kf[integ ? 1 : 0][mask ? 1 : 0][uni ? 1 : 0] : kd[uni ? 1 : 0];
+  k<<<(s.N + PL_P - 1) / PL_P, PL_T, 0, st>>>(s, C, acc, mask);
+}
+
 // The pair kernel of the FP64 mode.  The FP64 pipe bounds it (an FP64 instruction of a warp holds it
 // for 16 clocks however many lanes are active), so (1) the list is screened in FP32 on the fixed-point
 // view, (2) the kept pairs of a warp's 32 particles are put together and evaluated 32 at a time, a
@@ -924,7 +1118,17 @@ void launch_pair(const DevState& s, const SimConst& C, cudaStream_t st, bool acc
   const int B = (block == 32 || block == 64) ? block : 128;
   const int g = (s.N + B - 1) / B;
   const bool uni = C.scr2_uni_f > 0.f;
-  if (s.mixed && !accumulate) {  // the fused step
+  // Lanes per particle for systems too small to fill the GPU with threads (an explicit block size or
+  // the persistent schedule asks for k_pair).  The line follows the lists' length, for which their
+  // capacity stands (61 entries with the WCA cut-off, 180 with 2.24 sigma, 284 with a Coulomb cut-off
+  // of 3): lanes / thread per particle took 17 / 19 us at 20 k and 24 / 19 at 40 k particles (WCA), 56 / 71
+  // at 42 k and 93 / 86 at 83 k (2.24 sigma), 55 / 68 at 64 k and 94 / 91 at 130 k (charged).
+  const bool lanes = s.mixed && B == 128 && block != 128 && s.N <= 400ll * s.nbr_cap &&
+                     !(s.pair_persist && !accumulate && !eflag);
+  if (lanes) {
+    if (eflag) launch_pair_lanes<true>(s, C, st, !accumulate, acc, bonded_mask, uni, integ);
+    else launch_pair_lanes<false>(s, C, st, !accumulate, acc, bonded_mask, uni, integ);
+  } else if (s.mixed && !accumulate) {  // the fused step
     using KernT = void (*)(DevState, SimConst, bool, Acc, int);
     // [bonded][uni][eflag]
     const KernT ks[2][2][2] = {{{k_pair<false, true>, k_pair<true, true>},
