@@ -112,7 +112,12 @@ int dalloc(mfa_ctx* ctx, T** p, size_t n) {
     if (r_ != MFA_OK) return r_;                   \
   } while (0)
 
-Acc acc_of(double* a, int nrep) { return Acc{a, nrep}; }
+Acc acc_of(double* a, int nrep) { return Acc{a, nrep, 1}; }
+
+// copies of the fused step's accumulators: 16 for a single system down to one from 128 replicas on
+// (adding the copies up costs a record of 256 replicas 20 us with 16 of them)
+int acc_copies(int nrep) { return std::max(1, std::min(16, 128 / nrep)); }
+Acc step_acc(const mfa_ctx* ctx) { return Acc{ctx->acc_step, ctx->nrep, acc_copies(ctx->nrep)}; }
 
 // The list capacity is raised before the next step when the largest list count of the rebuilds
 // so far has passed 85 % of it (or the lists overflowed), so that a density fluctuation later in
@@ -807,7 +812,7 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
   DA(ctx->dreps, n_rep);
   DA(ctx->dtabf, NPAIR);
   DA(ctx->dtabd, NPAIR);
-  DA(ctx->acc_step, NOBS * n_rep);
+  DA(ctx->acc_step, (size_t)NOBS * n_rep * acc_copies(n_rep));
   DA(ctx->acc_call, NOBS * n_rep);
   DA(ctx->rec, NOBS * n_rep);
   DA(ctx->prof, (size_t)n_rep * C.hist_dim * 21);
@@ -862,7 +867,7 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
   CK(cudaMemsetAsync(S.steps_done, 0, sizeof(long long), st));
   CK(cudaMemsetAsync(S.steps_alt, 0, sizeof(long long), st));
   CK(cudaMemsetAsync(S.rebuilds, 0, sizeof(long long), st));
-  CK(cudaMemsetAsync(ctx->acc_step, 0, sizeof(double) * NOBS * n_rep, st));
+  CK(cudaMemsetAsync(ctx->acc_step, 0, sizeof(double) * NOBS * n_rep * acc_copies(n_rep), st));
   CK(cudaMemsetAsync(ctx->acc_call, 0, sizeof(double) * NOBS * n_rep, st));
   CK(cudaMemsetAsync(ctx->rec, 0, sizeof(double) * NOBS * n_rep, st));
   CK(cudaMemsetAsync(ctx->prof, 0, sizeof(double) * n_rep * C.hist_dim * 21, st));
@@ -1220,7 +1225,7 @@ static DevState other_views(const DevState& S) {
 static long long issue_steps(mfa_ctx* ctx, int n, int phase, bool prof, bool obs, bool capturing, int* err) {
   const SimConst& C = ctx->C;
   cudaStream_t st = ctx->st;
-  Acc acc = acc_of(ctx->acc_step, ctx->nrep);
+  Acc acc = step_acc(ctx);
   const int mask = any_chains(ctx) ? bonded_mask(ctx) : 0;
   long long L = 0;
   auto energies_at = [&](int k) { return ((phase + k) % ctx->opt.energy_every == 0) || k == n; };
@@ -1748,7 +1753,7 @@ int mfa_kernel_times(mfa_ctx* ctx, int32_t nsteps, float* mean_ms, int32_t* laun
   const DevState& S = ctx->S;
   const SimConst& C = ctx->C;
   cudaStream_t st = ctx->st;
-  Acc acc = acc_of(ctx->acc_step, ctx->nrep);
+  Acc acc = step_acc(ctx);
   const int mask = any_chains(ctx) ? bonded_mask(ctx) : 0;
   std::vector<cudaEvent_t> evs;
   std::vector<int> fam;

@@ -181,9 +181,9 @@ struct BondVir {
 // terms that i owns, to e4[4] = {FENE, brush bending, melt bending, orientation}.  With EFLAG the
 // virial goes to bv: half of each of i's bonds (-fac d (x) d, the other half comes from the
 // partner), the whole of the angle centred on i (-f_a (x) r_prev + f_c (x) r_next) and of the
-// orientation term of a head (F_1 (x) (r_1 - r_head)).  Returns false when i is in no chain of two
+// orientation term of a head (F_1 (x) (r_1 - r_head)).  FENE_ONLY: mask is 1.  Returns false when i is in no chain of two
 // or more beads.
-template <bool MIXED, bool EFLAG>
+template <bool MIXED, bool EFLAG, bool FENE_ONLY = false>
 __device__ __forceinline__ bool bonded_of(const DevState& s, const SimConst& C, int mask, int i, int w,
                                           real_t<MIXED>* F, real_t<MIXED>* e4, BondVir<real_t<MIXED>>* bv) {
   using real = real_t<MIXED>;
@@ -201,9 +201,9 @@ __device__ __forceinline__ bool bonded_of(const DevState& s, const SimConst& C, 
   if (kind < 0 || n < 2) return false;
   const int t0 = t - m;
   {
-    const bool do_fene = mask & 1;
-    const bool do_bend = (kind == 0 && (mask & 2)) || (kind == 1 && (mask & 4));
-    const bool do_or = kind == 0 && (mask & 8) && m <= 1;
+    const bool do_fene = FENE_ONLY || (mask & 1);
+    const bool do_bend = !FENE_ONLY && ((kind == 0 && (mask & 2)) || (kind == 1 && (mask & 4)));
+    const bool do_or = !FENE_ONLY && kind == 0 && (mask & 8) && m <= 1;
     const int lo = max(0, m - ((do_bend) ? 2 : 1)), hi = min(n - 1, m + ((do_bend) ? 2 : 1));
     BeadPos<MIXED> P[5];  // beads m-2 .. m+2 (fixed slots, so the array stays in registers)
 #pragma unroll
@@ -340,6 +340,17 @@ __device__ __forceinline__ void bonded_slots(int* sl, T* v, const T* e4, const B
 #pragma unroll
   for (int c = 0; c < 9; ++c) { sl[22 + c] = O_VIR + 9 * V_OR + c; v[22 + c] = bv.orient[c]; }
 }
+
+// the FENE ones alone (7 of them)
+template <typename T>
+__device__ __forceinline__ void fene_slots(int* sl, T* v, const T* e4, const BondVir<T>& bv) {
+  sl[0] = O_VINTRA; v[0] = e4[0];
+  sym_slots(sl + 1, v + 1, O_VIR + 9 * V_FENE, bv.fene);
+}
+// bonded terms of the fused mixed kernels: none, FENE alone, all (by the mask)
+constexpr int BOND_NONE = 0, BOND_FENE = 1, BOND_ALL = 2;
+inline int bond_kind(int mask) { return mask == 0 ? BOND_NONE : (mask == 1 ? BOND_FENE : BOND_ALL); }
+constexpr int bond_values(int bonded) { return bonded == BOND_ALL ? 31 : (bonded == BOND_FENE ? 7 : 0); }
 
 template <bool MIXED, bool EFLAG>
 __global__ void __launch_bounds__(128) k_bonded(DevState s, SimConst C, int mask, Acc acc, bool to_f4) {
@@ -489,7 +500,7 @@ __device__ __forceinline__ double pair_fs64(const DevState& s, const SimConst& C
 //           pairs are added to an FP64 per-particle total, together with the bonded, wall and body
 //           forces of the particle, and the total is stored (rounded to FP32) in the force array
 //           that the integrator reads;
-//   BONDED  (FUSED only) the particle's bonded terms (bonded_of) in the same thread, which saves
+//   BONDED  (FUSED only) the particle's bonded terms (bonded_of; FENE alone or all) in the same thread, which saves
 //           the bonded kernel's launch and its read-modify-write of the force;
 //   UNI     one screening cut-off for every type pair (SimConst::scr2_uni_f).
 // Without FUSED the forces are added to (accumulate) or stored in the FP64 force arrays.
@@ -505,12 +516,15 @@ __device__ __forceinline__ double pair_fs64(const DevState& s, const SimConst& C
 //           of blockDim.x particles from a queue (s.pair_q[0], one atomic ticket per tile, no
 //           waiting) and the last block to finish resets the queue for the next launch.  Compiled
 //           for 8 resident blocks per SM (64 registers): at 9 the tile loop spills.
-template <bool EFLAG, bool FUSED = false, bool BONDED = false, bool UNI = false, bool PERSIST = false,
+template <bool EFLAG, bool FUSED = false, int BONDED = BOND_NONE, bool UNI = false, bool PERSIST = false,
           bool INTEG = false>
-// Resident blocks per SM: 10 for the kernel with the integration in its tail (48 registers and a
-// 52-byte spill; 0.558 against 0.584 ms per step at 9 blocks, 56 registers; 11 or 12 blocks leave
-// 40 registers and spill 124 bytes: 0.579 ms), 9 for the other fused forms, 8 for the persistent
-// schedule (its tile loop spills at 9).
+// Resident blocks per SM: 10 for the kernel with the integration in its tail (48 registers, no spill
+// with FENE bonds alone, 52 bytes with every bonded term; 0.537 ms per step on 256 brush replicas,
+// 0.553 at 11 or 12 blocks), 9 for the other fused forms (an energy step of these replicas costs 125 us
+// more than a plain one; 166 at 8 blocks, 210 at 7), 8 for the persistent schedule (its tile loop
+// spills at 9).  FENE bonds alone have a variant of their own: compiled for every bonded term the
+// energy variant spilled 200 bytes and reduced 54 values per warp instead of 30 (235 us more than a
+// plain step), and the plain one took 0.559 ms.
 __global__ void __launch_bounds__(128, PERSIST ? 8 : ((INTEG && !EFLAG) ? 10 : 9)) k_pair(DevState s, SimConst C,
                                                                                           bool accumulate, Acc acc,
                                                                                           int bmask = 0) {
@@ -570,7 +584,7 @@ __global__ void __launch_bounds__(128, PERSIST ? 8 : ((INTEG && !EFLAG) ? 10 : 9
   // variant with bonded terms, of the bonded virial partials after it: the batch is dead once
   // the pair loop ends, and a barrier separates the two uses, so the variant keeps room for L1.
   constexpr int JL_WORDS = PAIR_BATCH * 128;
-  constexpr int BV_WORDS = (EFLAG && BONDED) ? 128 * (int)(sizeof(BondVir<real>) / 4) : 0;
+  constexpr int BV_WORDS = (EFLAG && BONDED == BOND_ALL) ? 128 * (int)(sizeof(BondVir<real>) / 4) : 0;
   __shared__ __align__(16) int pair_pool[JL_WORDS > BV_WORDS ? JL_WORDS : BV_WORDS];
   real fx = 0, fy = 0, fz = 0;        // the current batch (FUSED), else the whole sum
   real e_lj = 0, e_c = 0;
@@ -671,15 +685,12 @@ __global__ void __launch_bounds__(128, PERSIST ? 8 : ((INTEG && !EFLAG) ? 10 : 9
     }
   }
   real eb[4] = {0, 0, 0, 0};
-  // the bonded virial partials of the thread (EFLAG): in shared memory, where the bonded terms'
-  // registers are scarce (27 words per thread: a stride prime to the 32 banks)
-  __shared__ BondVir<real> bv_unused[1];  // the reference the other variants pass and never use
-  BondVir<real>& bv = (EFLAG && BONDED) ? reinterpret_cast<BondVir<real>*>(pair_pool)[threadIdx.x] : bv_unused[0];
-  if (EFLAG && BONDED) {
-    __syncthreads();  // every thread of the block is past its pair loop: the batch area is free
-    bv.zero();
-  }
-  bool hb = false;
+  // the bonded virial partials of the thread (EFLAG): with every term in shared memory, where the
+  // bonded terms' registers are scarce (27 words per thread: a stride prime to the 32 banks)
+  BondVir<real> bv_own;
+  BondVir<real>& bv = (EFLAG && BONDED == BOND_ALL) ? reinterpret_cast<BondVir<real>*>(pair_pool)[threadIdx.x] : bv_own;
+  if (EFLAG && BONDED == BOND_ALL) __syncthreads();  // every thread is past its pair loop: the batch area is free
+  if (EFLAG && BONDED) bv.zero();
   double fxd = 0., fyd = 0., fzd = 0.;
   // INTEG with EFLAG: the integrator's kinetic energy, kinetic tensor and head forces
   float ike = 0.f, ikin[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, ifh[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -690,7 +701,7 @@ __global__ void __launch_bounds__(128, PERSIST ? 8 : ((INTEG && !EFLAG) ? 10 : 9
     if (active) {
       if constexpr (BONDED) {
         real fb[3] = {0, 0, 0};
-        hb = bonded_of<true, EFLAG>(s, C, bmask, i, w, fb, eb, &bv);
+        bonded_of<true, EFLAG, BONDED == BOND_FENE>(s, C, bmask, i, w, fb, eb, &bv);
         fxd += f2d_fast(fb[0]);
         fyd += f2d_fast(fb[1]);
         fzd += f2d_fast(fb[2]);
@@ -726,16 +737,14 @@ __global__ void __launch_bounds__(128, PERSIST ? 8 : ((INTEG && !EFLAG) ? 10 : 9
     }
   }
   if (EFLAG) {  // one warp reduction for every energy and virial component of the kernel
-    constexpr int NB = BONDED ? 31 : 0, NW = FUSED ? 2 : 0, NI = INTEG ? 13 : 0, NV = 8 + NB + NW + NI;
+    constexpr int NB = bond_values(BONDED), NW = FUSED ? 2 : 0, NI = INTEG ? 13 : 0, NV = 8 + NB + NW + NI;
     int sl[NV];
     real v[NV];
     sl[0] = O_VFF; v[0] = e_lj;
     sl[1] = O_VCOUL; v[1] = e_c;
     sym_slots(sl + 2, v + 2, O_VIR + 9 * V_PAIR, wv);
-    if constexpr (BONDED) {
-      (void)hb;
-      bonded_slots(sl + 8, v + 8, eb, bv);
-    }
+    if constexpr (BONDED == BOND_ALL) bonded_slots(sl + 8, v + 8, eb, bv);
+    if constexpr (BONDED == BOND_FENE) fene_slots(sl + 8, v + 8, eb, bv);
     if constexpr (FUSED) {
       sl[8 + NB] = O_VFW; v[8 + NB] = e_w;
       sl[9 + NB] = O_VIR + 9 * V_WALL + 8; v[9 + NB] = w_wall;
@@ -770,7 +779,7 @@ __global__ void __launch_bounds__(128, PERSIST ? 8 : ((INTEG && !EFLAG) ? 10 : 9
 // meanwhile and then integrates them (FUSED, BONDED, UNI, INTEG as in k_pair).
 constexpr int PL_G = 8, PL_P = 32, PL_T = PL_P * PL_G + 32;
 
-template <bool EFLAG, bool FUSED, bool BONDED, bool UNI, bool INTEG>
+template <bool EFLAG, bool FUSED, int BONDED, bool UNI, bool INTEG>
 __global__ void __launch_bounds__(PL_T) k_pair_lanes(DevState s, SimConst C, Acc acc, int bmask) {
   __shared__ PairEntry<float> tab[NPAIR];
   __shared__ int jl[PL_P][PAIR_BATCH + PL_G];
@@ -792,7 +801,7 @@ __global__ void __launch_bounds__(PL_T) k_pair_lanes(DevState s, SimConst C, Acc
   __syncthreads();
   if (tail) {
     if constexpr (BONDED) {
-      if (active) bonded_of<true, EFLAG>(s, C, bmask, i, w, fb, eb, &bv);
+      if (active) bonded_of<true, EFLAG, BONDED == BOND_FENE>(s, C, bmask, i, w, fb, eb, &bv);
     }
   } else {
     const int q8 = lane & (PL_G - 1), grp = lane / PL_G;
@@ -921,10 +930,11 @@ __global__ void __launch_bounds__(PL_T) k_pair_lanes(DevState s, SimConst C, Acc
     }
   }
   if constexpr (EFLAG && FUSED) {
-    constexpr int NB = BONDED ? 31 : 0, NI = INTEG ? 13 : 0, NV = NB + 2 + NI;
+    constexpr int NB = bond_values(BONDED), NI = INTEG ? 13 : 0, NV = NB + 2 + NI;
     int sl[NV];
     float v[NV];
-    if constexpr (BONDED) bonded_slots(sl, v, eb, bv);
+    if constexpr (BONDED == BOND_ALL) bonded_slots(sl, v, eb, bv);
+    if constexpr (BONDED == BOND_FENE) fene_slots(sl, v, eb, bv);
     sl[NB] = O_VFW; v[NB] = wall_e[lane];
     sl[NB + 1] = O_VIR + 9 * V_WALL + 8; v[NB + 1] = wall_w[lane];
     if constexpr (INTEG) {
@@ -946,12 +956,12 @@ static void launch_pair_lanes(const DevState& s, const SimConst& C, cudaStream_t
                               bool uni, bool integ) {
   using KernT = void (*)(DevState, SimConst, Acc, int);
   // [integ][bonded][uni]
-  const KernT kf[2][2][2] = {{{k_pair_lanes<EFLAG, true, false, false, false>, k_pair_lanes<EFLAG, true, false, true, false>},
-                              {k_pair_lanes<EFLAG, true, true, false, false>, k_pair_lanes<EFLAG, true, true, true, false>}},
-                             {{k_pair_lanes<EFLAG, true, false, false, true>, k_pair_lanes<EFLAG, true, false, true, true>},
-                              {k_pair_lanes<EFLAG, true, true, false, true>, k_pair_lanes<EFLAG, true, true, true, true>}}};
-  const KernT kd[2] = {k_pair_lanes<EFLAG, false, false, false, false>, k_pair_lanes<EFLAG, false, false, true, false>};
-  const KernT k = fused ? kf[integ ? 1 : 0][mask ? 1 : 0][uni ? 1 : 0] : kd[uni ? 1 : 0];
+#define LANES(I, B) {k_pair_lanes<EFLAG, true, B, false, I>, k_pair_lanes<EFLAG, true, B, true, I>}
+  const KernT kf[2][3][2] = {{LANES(false, BOND_NONE), LANES(false, BOND_FENE), LANES(false, BOND_ALL)},
+                             {LANES(true, BOND_NONE), LANES(true, BOND_FENE), LANES(true, BOND_ALL)}};
+#undef LANES
+  const KernT kd[2] = {k_pair_lanes<EFLAG, false, BOND_NONE, false, false>, k_pair_lanes<EFLAG, false, BOND_NONE, true, false>};
+  const KernT k = fused ? kf[integ ? 1 : 0][bond_kind(mask)][uni ? 1 : 0] : kd[uni ? 1 : 0];
   k<<<(s.N + PL_P - 1) / PL_P, PL_T, 0, st>>>(s, C, acc, mask);
 }
 
@@ -1130,24 +1140,15 @@ void launch_pair(const DevState& s, const SimConst& C, cudaStream_t st, bool acc
     else launch_pair_lanes<false>(s, C, st, !accumulate, acc, bonded_mask, uni, integ);
   } else if (s.mixed && !accumulate) {  // the fused step
     using KernT = void (*)(DevState, SimConst, bool, Acc, int);
-    // [bonded][uni][eflag]
-    const KernT ks[2][2][2] = {{{k_pair<false, true>, k_pair<true, true>},
-                                {k_pair<false, true, false, true>, k_pair<true, true, false, true>}},
-                               {{k_pair<false, true, true>, k_pair<true, true, true>},
-                                {k_pair<false, true, true, true>, k_pair<true, true, true, true>}}};
-    // the persistent schedule for the steps without energies: [bonded][uni]
-    const KernT kp[2][2] = {{k_pair<false, true, false, false, true>, k_pair<false, true, false, true, true>},
-                            {k_pair<false, true, true, false, true>, k_pair<false, true, true, true, true>}};
-    // with the step's integration in the tail: [eflag][bonded][uni]
-    const KernT ki[2][2][2] = {{{k_pair<false, true, false, false, false, true>,
-                                 k_pair<false, true, false, true, false, true>},
-                                {k_pair<false, true, true, false, false, true>,
-                                 k_pair<false, true, true, true, false, true>}},
-                               {{k_pair<true, true, false, false, false, true>,
-                                 k_pair<true, true, false, true, false, true>},
-                                {k_pair<true, true, true, false, false, true>,
-                                 k_pair<true, true, true, true, false, true>}}};
-    const int bi = bonded_mask ? 1 : 0, ui = uni ? 1 : 0;
+    // [eflag][bonded][uni]: forces alone, the persistent schedule, with the step's integration in the tail
+#define PAIRK(E, B, P, I) {k_pair<E, true, B, false, P, I>, k_pair<E, true, B, true, P, I>}
+#define PAIRB(E, P, I) {PAIRK(E, BOND_NONE, P, I), PAIRK(E, BOND_FENE, P, I), PAIRK(E, BOND_ALL, P, I)}
+    const KernT ks[2][3][2] = {PAIRB(false, false, false), PAIRB(true, false, false)};
+    const KernT kp[3][2] = PAIRB(false, true, false);
+    const KernT ki[2][3][2] = {PAIRB(false, false, true), PAIRB(true, false, true)};
+#undef PAIRB
+#undef PAIRK
+    const int bi = bond_kind(bonded_mask), ui = uni ? 1 : 0;
     if (integ) {
       ki[eflag ? 1 : 0][bi][ui]<<<g, B, 0, st>>>(s, C, false, acc, bonded_mask);
     } else if (s.pair_persist && !eflag) {
@@ -1157,7 +1158,7 @@ void launch_pair(const DevState& s, const SimConst& C, cudaStream_t st, bool acc
       const int grid = std::min(g, std::max(per_sm, 1) * s.nsm);
       k<<<grid, B, 0, st>>>(s, C, false, acc, bonded_mask);
     } else {
-      ks[bi][ui][eflag ? 1 : 0]<<<g, B, 0, st>>>(s, C, false, acc, bonded_mask);
+      ks[eflag ? 1 : 0][bi][ui]<<<g, B, 0, st>>>(s, C, false, acc, bonded_mask);
     }
   } else if (s.mixed) {  // the drop-in: added to the FP64 force
     if (eflag) k_pair<true><<<g, B, 0, st>>>(s, C, true, acc);

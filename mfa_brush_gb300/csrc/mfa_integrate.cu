@@ -294,13 +294,18 @@ void launch_profiles(const DevState& s, const SimConst& C, cudaStream_t st, doub
   k_profiles<<<g, 256, shm, st>>>(s, C, prof, H, chunk);
 }
 
-// energy record: out[k*nrep + r] = acc, acc = 0
+// energy record: out[k*nrep + r] = sum of the copies of acc, acc = 0
 __global__ void k_record(Acc acc, double* out) {
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   int n = NOBS * acc.nrep;
   if (k >= n) return;
-  out[k] = acc.a[k];
-  acc.a[k] = 0.;
+  double t = 0.;
+#pragma unroll 4
+  for (int c = 0; c < acc.copies; ++c) {
+    t += acc.a[(size_t)c * n + k];
+    acc.a[(size_t)c * n + k] = 0.;
+  }
+  out[k] = t;
 }
 
 // Observation quantities (observation.f90): one block per replica.  Rg^2 of each chain from its
