@@ -26,6 +26,8 @@
 
 namespace mfa {
 
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 template <bool MIXED>
 using real_t = typename std::conditional<MIXED, float, double>::type;
 
@@ -394,6 +396,13 @@ __global__ void __launch_bounds__(128) k_bonded(DevState s, SimConst C, int mask
 // 24 / 32 (groups of 2; 12 with groups of 4: 0.585).
 constexpr int PAIR_BATCH = 12;
 constexpr int PAIR_G = 2;
+// Every block prefetches into L2 what the block one per SM later reads from memory: the own-particle
+// arrays and the first list rows (a lane per row; most WCA lists end there).  The kernel is bound by
+// the latency of its loads (7.7 of 15 stall cycles per issue), and these would come from HBM: pair
+// kernel 500 -> 456 us on 256 brush replicas (own-particle streams of the tail alone 490, own block's
+// rows and streams 462, 2 / 4 / 10 blocks per SM ahead 458 / 463 / 490; 16, 20 or 32 rows: alike,
+// alike, 1 us more).
+constexpr int PAIR_ROWS_AHEAD = 18;
 
 // Force factor fs of the pair (i, j) along d = r_i - r_j (LJ with the switch-on clamp, DPD with the
 // pair's Philox noise, real-space Coulomb), fluid_fluid.f90:97-261, dpd_forces.f90:45-115,
@@ -401,7 +410,7 @@ constexpr int PAIR_G = 2;
 // FP64 (pair_fs64) forms.
 template <bool EFLAG>
 __device__ __forceinline__ float pair_fs(const DevState& s, const SimConst& C, const PairEntry<float>& e, float dx,
-                                         float dy, float dz, int j, float vix, float viy, float viz, int tag_i,
+                                         float dy, float dz, float4 vj, float vix, float viy, float viz, int tag_i,
                                          int p0, uint32_t nkey, float r2min, float half, float& e_lj, float& e_c) {
   const float r2raw = dx * dx + dy * dy + dz * dz;
   const int fl = e.flags;
@@ -411,7 +420,7 @@ __device__ __forceinline__ float pair_fs(const DevState& s, const SimConst& C, c
   if (in_lj) {
     r2 = r2raw < r2min ? r2min : r2raw;
     // the hardware reciprocal (2 ulp) instead of the IEEE division sequence
-    const float inv_r2 = __fdividef(1.f, r2);
+    const float inv_r2 = rcp_ftz(r2);
     const float s2 = e.sig2 * inv_r2;
     const float s6 = s2 * s2 * s2;
     const float s12 = s6 * s6;
@@ -420,9 +429,8 @@ __device__ __forceinline__ float pair_fs(const DevState& s, const SimConst& C, c
   }
   const bool dpd = (in_lj && (fl & PF_DPD_LJ)) || ((fl & PF_DPD_OWN) && r2 < e.dpd_rc2);
   if (dpd) {
-    const float4 v4 = __ldg(&s.vf[j]);
-    const int tag_j = __float_as_int(v4.w) - p0;
-    const float ir = rsqrtf(r2);  // one hardware reciprocal square root (2 ulp)
+    const int tag_j = __float_as_int(vj.w) - p0;
+    const float ir = rsqrt_ftz(r2);  // one hardware reciprocal square root (2 ulp)
     const float r = r2 * ir;
     float wr, wd;
     if (C.dpd_weight1) {
@@ -432,7 +440,7 @@ __device__ __forceinline__ float pair_fs(const DevState& s, const SimConst& C, c
       wd = wr * wr;
     }
     const float g = pair_gauss_f(nkey, tag_i, tag_j);
-    const float rdot = ((vix - v4.x) * dx + (viy - v4.y) * dy + (viz - v4.z) * dz) * ir;
+    const float rdot = ((vix - vj.x) * dx + (viy - vj.y) * dy + (viz - vj.z) * dz) * ir;
     fs += (C.sig_f * wr * g - C.gamma_f * wd * rdot) * ir;
   }
   if (fl & PF_COUL) {
@@ -556,6 +564,26 @@ __global__ void __launch_bounds__(128, PERSIST ? 8 : ((INTEG && !EFLAG) ? 10 : 9
   const bool active = inside && info_mobile(w);
   const int rep = info_rep(w);
   float e_w = 0.f, w_wall = 0.f;  // FUSED: wall energy and virial
+  {  // the streams of the block that starts about when this one ends, on their way into L2
+    const int ip = i + s.nsm * (int)blockDim.x, i0 = ip & ~31, row = threadIdx.x & 31;
+    if (i0 < s.N && row < min(PAIR_ROWS_AHEAD, s.nbr_cap)) prefetch_l2(s.nbr + (size_t)row * s.Np + i0);
+    if (ip < s.N) {
+      prefetch_l2(s.info + ip);
+      prefetch_l2(s.nn + ip);
+      prefetch_l2(s.pfx + ip);
+      prefetch_l2(s.vf + ip);
+      if (FUSED) prefetch_l2(s.rz + ip);
+      if (INTEG) {
+        prefetch_l2(s.rx + ip);
+        prefetch_l2(s.ry + ip);
+        prefetch_l2(s.vx + ip);
+        prefetch_l2(s.vy + ip);
+        prefetch_l2(s.vz + ip);
+        prefetch_l2(s.ref + ip);
+        prefetch_l2(s.tag + ip);
+      }
+    }
+  }
   if constexpr (FUSED) {
     // the particle's external forces first: its FP64 total starts from them
     double ez = 0., ex = 0., ey = 0.;
@@ -664,11 +692,12 @@ __global__ void __launch_bounds__(128, PERSIST ? 8 : ((INTEG && !EFLAG) ? 10 : 9
       for (int t = 0; t < m; ++t) {
         const int j = jl[128 * t];
         real dx, dy, dz;
+        const float4 vj = __ldg(&s.vf[j]);  // with the position: behind the cut-off test it would wait again
         const int wj = delta(j, dx, dy, dz);
         const PairEntry<real>& e = tab[ti * MAXT + info_type(wj)];
         // half of each mobile pair (both ends sum it); a fixed wall bead has no list of its own
         const real half = info_mobile(wj) ? (real)0.5 : (real)1;
-        const real fs = pair_fs<EFLAG>(s, C, e, dx, dy, dz, j, vi.x, vi.y, vi.z, tag_i, p0, nkey, r2min, half,
+        const real fs = pair_fs<EFLAG>(s, C, e, dx, dy, dz, vj, vi.x, vi.y, vi.z, tag_i, p0, nkey, r2min, half,
                                        e_lj, e_c);
         // unmerged products and sums: alike with and without energies
         fx = __fadd_rn(fx, __fmul_rn(fs, dx));
@@ -861,13 +890,14 @@ __global__ void __launch_bounds__(PL_T) k_pair_lanes(DevState s, SimConst C, Acc
       if (!__any_sync(FULL, take > 0)) break;
       for (int c = q8; c < take; c += PL_G) {
         const int j = jl[pl][c];
+        const float4 vj = __ldg(&s.vf[j]);
         const int4 qj = __ldg(&s.pfx[j]);
         const float dx = i2f_fast(fx_diff(qi.x, qj.x)) * ux;
         const float dy = i2f_fast(fx_diff(qi.y, qj.y)) * uy;
         const float dz = i2f_fast(fx_diff(qi.z, qj.z)) * uz;
         const PairEntry<float>& e = tab[ti * MAXT + info_type(qj.w)];
         const float half = info_mobile(qj.w) ? 0.5f : 1.f;
-        const float fs = pair_fs<EFLAG>(s, C, e, dx, dy, dz, j, vi.x, vi.y, vi.z, tag_i, p0, nkey, r2min, half, e_lj,
+        const float fs = pair_fs<EFLAG>(s, C, e, dx, dy, dz, vj, vi.x, vi.y, vi.z, tag_i, p0, nkey, r2min, half, e_lj,
                                         e_c);
         prod[0][pl][c] = __fmul_rn(fs, dx);
         prod[1][pl][c] = __fmul_rn(fs, dy);
