@@ -1272,6 +1272,10 @@ static long long issue_steps(mfa_ctx* ctx, int n, int phase, bool prof, bool obs
       if (k < n && !split) {
         launch_integrate(S, C, st, 2, true, ef, acc);
         L += 1;
+      } else if (k < n && prof && !ef && S.mixed) {  // both halves and the profile between them at once
+        launch_integrate_profiles(S, C, st, ctx->prof, C.hist_dim);
+        L += 1;
+        continue;
       } else {
         launch_integrate(S, C, st, 1, true, ef, acc);
         L += 1;

@@ -18,7 +18,8 @@ __device__ __forceinline__ double wrap_bits(double x, double L, long long Lbits)
 
 // The update of one mobile particle i (info word w) in the mixed path, after its force (Fx, Fy, Fz)
 // for MODE >= 1; the views go to (pfx_out, vf_out).  Shared by k_int_mixed and by the pair kernel
-// that fuses MODE 2 into its tail, so both give the same bits.
+// that fuses MODE 2 into its tail, so both give the same bits.  MODE 3 is MODE 1 followed by MODE 0, to
+// the bit, with v(n) in between for the caller (the profiles); it leaves a and F unwritten.
 // verlet_positions.f90:214-247 (WALL 1 with a wall velocity): the sites of the first half of a
 // replica's wall beads move by +va_spring_twall dt per step and the other half by
 // -va_spring_twall dt, wrapped into [0, L) in x and y, and the beads sit on their sites.  Their
@@ -59,7 +60,8 @@ __device__ __forceinline__ int4 move_wall_bead(const DevState& s, const SimConst
 template <int MODE, bool EFLAG>
 __device__ __forceinline__ void int_mixed_particle(const DevState& s, const SimConst& C, int i, int w, float Fx,
                                                    float Fy, float Fz, int4* __restrict__ pfx_out,
-                                                   float4* __restrict__ vf_out, float& ke, float* kin, float* fh) {
+                                                   float4* __restrict__ vf_out, float& ke, float* kin, float* fh,
+                                                   double* vn = nullptr) {
   const int rep = info_rep(w);
   {
     const RepDesc& R = s.reps[rep];
@@ -98,6 +100,12 @@ __device__ __forceinline__ void int_mixed_particle(const DevState& s, const SimC
     vx += f2d_fast(dvx);
     vy += f2d_fast(dvy);
     vz += f2d_fast(dvz);
+    if (MODE == 3) {  // v(n) for the caller, then MODE 0's half kick
+      vn[0] = vx; vn[1] = vy; vn[2] = vz;
+      vx += f2d_fast(dvx);
+      vy += f2d_fast(dvy);
+      vz += f2d_fast(dvz);
+    }
     s.vx[i] = vx; s.vy[i] = vy; s.vz[i] = vz;
     if (MODE == 1) {
       s.ax[i] = f2d_fast(ax); s.ay[i] = f2d_fast(ay); s.az[i] = f2d_fast(az);

@@ -224,74 +224,153 @@ void launch_integrate(const DevState& s, const SimConst& C, cudaStream_t st, int
 }
 
 // ---------------------------------------------------------------------------------------------
-// Profiles: histo(2) + velocity_prof(2) (functions.f90:157-214, 319-365).  Each block takes a
-// contiguous run of slots, accumulates [bin][species][count, sum v, sum v^2] in shared memory
-// and flushes to the replica's global FP64 profile whenever the replica changes.
-// prof layout per replica: [hist][3 species][7] (count, vx, vy, vz, vx^2, vy^2, vz^2).
+// Profiles: histo(2) + velocity_prof(2) (functions.f90:157-214, 319-365).
+// prof layout per replica: [hist][3 species][7] (count, vx, vy, vz, vx^2, vy^2, vz^2), FP64.
+// A block takes a tile of consecutive slots.  Sorted by cell, they fall into few (bin, species) keys,
+// so FP64 shared atomics wait for each other (a step of 1.6 M particles with them and separate
+// integrator passes took 1138 us, with this 993).  Instead
+// the tile's velocities are ordered by key in shared memory (a counting sort: integer atomics give the
+// ranks), four lanes sum each component of a key, and its seven sums go to the global profile.
+//   STEP 0  the profile of the state;
+//   STEP 1  the mixed step with profiles but without energies: velocities(n), the profile, positions
+//           (n+1) in one pass (int_mixed_particle<3>) instead of three.
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_profiles(DevState s, SimConst C, double* __restrict__ prof, int H,
-                                                  int chunk) {
+constexpr int PROF_T = 256;
+
+template <int STEP, int PROF_PER>
+__global__ void __launch_bounds__(PROF_T, 4) k_profiles(DevState s, SimConst C, double* __restrict__ prof, int H) {
+  constexpr int PROF_TILE = PROF_T * PROF_PER;
   extern __shared__ double sh[];
-  const int n_sh = H * 3 * 7;
-  const int b0 = blockIdx.x * chunk, b1 = min(s.N, b0 + chunk);
-  if (b0 >= s.N) return;
-  for (int k = threadIdx.x; k < n_sh; k += blockDim.x) sh[k] = 0.;
-  __syncthreads();
-  int cur = info_rep(s.info[b0]);
-  int pos = b0;
-  while (pos < b1) {
-    // [pos, seg_end): slots of replica `cur` inside this block's chunk
-    int seg_end = b1;
-    if (info_rep(s.info[b1 - 1]) != cur) {
-      int lo = pos, hi = b1 - 1;  // last slot with replica == cur
-      while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (info_rep(s.info[mid]) == cur) lo = mid; else hi = mid - 1;
-      }
-      seg_end = lo + 1;
-    }
-    const RepDesc& R = s.reps[cur];
-    for (int i = pos + threadIdx.x; i < seg_end; i += blockDim.x) {
-      const int w = s.info[i];
-      const int sp = info_species(w);
-      if (!info_mobile(w) || sp == 3) continue;
+  const int nkey = 3 * H;
+  double* vs = sh;                                        // [3][PROF_TILE] velocities in key order
+  int* cnt = reinterpret_cast<int*>(vs + 3 * PROF_TILE);  // [nkey]
+  int* off = cnt + nkey;                                  // [nkey]
+  int* used = off + nkey;                                 // [nkey] keys with particles
+  __shared__ int nused, wsum[PROF_T / 32];
+  const int b0 = blockIdx.x * PROF_TILE, b1 = min(s.N, b0 + PROF_TILE);
+  int key[PROF_PER], rep[PROF_PER];
+  double v[PROF_PER][3];
+#pragma unroll
+  for (int t = 0; t < PROF_PER; ++t) {
+    const int i = b0 + t * PROF_T + threadIdx.x;
+    key[t] = -1;
+    rep[t] = -1;
+    if (i >= b1) continue;
+    const int w = s.info[i], sp = info_species(w);
+    rep[t] = info_rep(w);
+    if (info_mobile(w)) {
+      const RepDesc& R = s.reps[rep[t]];
       int zi = (int)(s.rz[i] * R.hist_inv_dz) + 1;
       zi = min(max(zi, 1), H) - 1;
-      double* h = sh + (zi * 3 + sp) * 7;
-      const double vx = s.vx[i], vy = s.vy[i], vz = s.vz[i];
-      atomicAdd(h + 0, 1.);
-      atomicAdd(h + 1, vx);
-      atomicAdd(h + 2, vy);
-      atomicAdd(h + 3, vz);
-      atomicAdd(h + 4, vx * vx);
-      atomicAdd(h + 5, vy * vy);
-      atomicAdd(h + 6, vz * vz);
+      if (sp != 3) key[t] = zi * 3 + sp;
+      if constexpr (STEP == 1) {
+        const float4 F = s.f4[i];
+        float ke, kin[6], fh[6];
+        int_mixed_particle<3, false>(s, C, i, w, F.x, F.y, F.z, s.pfx, s.vf, ke, kin, fh, v[t]);
+      } else {
+        v[t][0] = s.vx[i]; v[t][1] = s.vy[i]; v[t][2] = s.vz[i];
+      }
+    } else if (STEP == 1 && C.move_walls) {  // a wall bead on a moving wall
+      double x, y, z;
+      s.pfx[i] = move_wall_bead(s, C, i, w, x, y, z);
+    }
+  }
+  if (STEP == 1 && blockIdx.x == 0 && threadIdx.x == 0) *s.steps_done += 1;
+  // the replicas of the tile one after another (usually one)
+  const int r0 = info_rep(s.info[b0]), r1 = info_rep(s.info[b1 - 1]);
+  for (int r = r0; r <= r1; ++r) {
+    for (int k = threadIdx.x; k < nkey; k += PROF_T) cnt[k] = 0;
+    if (threadIdx.x == 0) nused = 0;
+    __syncthreads();
+    int rank[PROF_PER];
+#pragma unroll
+    for (int t = 0; t < PROF_PER; ++t) rank[t] = (rep[t] == r && key[t] >= 0) ? atomicAdd(&cnt[key[t]], 1) : -1;
+    __syncthreads();
+    // starts of the keys: each thread a run of them
+    const int per = (nkey + PROF_T - 1) / PROF_T, k0 = threadIdx.x * per, k1 = min(nkey, k0 + per);
+    int mine = 0;
+    for (int k = k0; k < k1; ++k) mine += cnt[k];
+    int x = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if ((threadIdx.x & 31) >= o) x += y;
+    }
+    if ((threadIdx.x & 31) == 31) wsum[threadIdx.x >> 5] = x;
+    __syncthreads();
+    int at = x - mine;
+    for (int q = 0; q < (int)(threadIdx.x >> 5); ++q) at += wsum[q];
+    for (int k = k0; k < k1; ++k) {
+      off[k] = at;
+      at += cnt[k];
+      if (cnt[k] > 0) used[atomicAdd(&nused, 1)] = k;
     }
     __syncthreads();
-    double* g = prof + (size_t)cur * n_sh;
-    for (int k = threadIdx.x; k < n_sh; k += blockDim.x) {
-      double v = sh[k];
-      if (v != 0.) atomicAdd(g + k, v);
-      sh[k] = 0.;
+#pragma unroll
+    for (int t = 0; t < PROF_PER; ++t)
+      if (rank[t] >= 0) {
+        const int o = off[key[t]] + rank[t];
+        vs[o] = v[t][0];
+        vs[PROF_TILE + o] = v[t][1];
+        vs[2 * PROF_TILE + o] = v[t][2];
+      }
+    __syncthreads();
+    // (key, component, quarter of its particles): four neighbouring lanes share a key's component
+    const int tasks = nused * 12, rounds = (tasks + PROF_T - 1) / PROF_T;
+    for (int q = 0; q < rounds; ++q) {
+      const int task = q * PROF_T + threadIdx.x, part = task & 3, c = (task >> 2) % 3;
+      double a = 0., b = 0.;
+      int k = 0, n = 0;
+      if (task < tasks) {
+        k = used[task / 12];
+        n = cnt[k];
+        const double* u = vs + c * PROF_TILE + off[k];
+        for (int e = part; e < n; e += 4) {
+          const double x1 = u[e];
+          a += x1;
+          b = fma(x1, x1, b);
+        }
+      }
+#pragma unroll
+      for (int o = 1; o <= 2; o <<= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+      }
+      if (task < tasks) {
+        double* g = prof + ((size_t)r * nkey + k) * 7;
+        if (part == 0) atomicAdd(g + 1 + c, a);
+        if (part == 1) atomicAdd(g + 4 + c, b);
+        if (part == 2 && c == 0) atomicAdd(g, (double)n);
+      }
     }
     __syncthreads();
-    pos = seg_end;
-    if (pos < b1) cur = info_rep(s.info[pos]);
   }
 }
 
+template <int STEP, int PER>
+static void launch_prof(const DevState& s, const SimConst& C, cudaStream_t st, double* prof, int H) {
+  const int tile = PROF_T * PER;
+  auto bytes = [&](int h) { return sizeof(double) * 3 * tile + sizeof(int) * 9 * (size_t)h; };
+  // above 48 KB dynamic shared memory needs an explicit opt-in, a property of the kernel for the
+  // whole process: set once to the size of the largest histogram
+  static const cudaError_t opted = cudaFuncSetAttribute(
+      k_profiles<STEP, PER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes(MFA_HIST_DIM_MAX));
+  (void)opted;
+  k_profiles<STEP, PER><<<(s.N + tile - 1) / tile, PROF_T, bytes(H), st>>>(s, C, prof, H);
+}
+
+// Four particles a thread; one when that leaves SMs without a block.  (1.6 M particles: 993 us a step with
+// four and four blocks per SM, 1008 with three, 1020 with eight and two, 995 with two and six.)
+static bool prof_small(const DevState& s) { return s.N < 2 * s.nsm * PROF_T; }
+
 void launch_profiles(const DevState& s, const SimConst& C, cudaStream_t st, double* prof, int H) {
-  // small chunks: enough blocks to fill the GPU for one large replica as for many small ones (a
-  // block of sorted particles touches few bins, so its flush is short)
-  const int chunk = 1024;
-  const int g = (s.N + chunk - 1) / chunk;
-  const size_t shm = sizeof(double) * H * 3 * 7;
-  static size_t shm_set = 48 * 1024;
-  if (shm > shm_set) {  // above 48 KB dynamic shared memory needs an explicit opt-in
-    cudaFuncSetAttribute(k_profiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
-    shm_set = shm;
-  }
-  k_profiles<<<g, 256, shm, st>>>(s, C, prof, H, chunk);
+  if (prof_small(s)) launch_prof<0, 1>(s, C, st, prof, H);
+  else launch_prof<0, 4>(s, C, st, prof, H);
+}
+
+void launch_integrate_profiles(const DevState& s, const SimConst& C, cudaStream_t st, double* prof, int H) {
+  if (prof_small(s)) launch_prof<1, 1>(s, C, st, prof, H);
+  else launch_prof<1, 4>(s, C, st, prof, H);
 }
 
 // energy record: out[k*nrep + r] = sum of the copies of acc, acc = 0

@@ -186,6 +186,8 @@ void launch_const_force(const DevState& s, const SimConst& C, cudaStream_t st);
 void launch_integrate(const DevState& s, const SimConst& C, cudaStream_t st, int mode, bool add_ext,
                       bool eflag, Acc acc);
 void launch_profiles(const DevState& s, const SimConst& C, cudaStream_t st, double* prof, int hist);
+// velocities(n), the profile and positions(n+1) of a mixed step without energies in one pass
+void launch_integrate_profiles(const DevState& s, const SimConst& C, cudaStream_t st, double* prof, int hist);
 void launch_record(Acc acc, double* out, cudaStream_t st);
 // observation quantities per replica: out[9 r + 0..2] brush Rg^2, 3..5 melt Rg^2, 6..8 momentum
 void launch_observe(const DevState& s, const SimConst& C, cudaStream_t st, double* out);
