@@ -43,6 +43,7 @@ struct mfa_ctx {
   bool kspace = false;
   bool fuse_integ = false;  // mfa_step runs the integration of its plain steps in the pair kernel
   unsigned* h_status = nullptr;  // pinned: [0] status bits, [1] largest list count seen
+  double* h_rec = nullptr;       // pinned: [NOBS][nrep] accumulators or record read back by the calls
   cudaEvent_t ev_status = nullptr;  // recorded after each copy of the status words into h_status
   bool grow_pending = false;     // the list capacity is to be raised before the next step
   bool overflow_reported = false;  // the current list overflow was returned to the caller already
@@ -145,6 +146,41 @@ int post_status(mfa_ctx* ctx) {
   CK(cudaMemcpyAsync(ctx->h_status, ctx->S.status, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaEventRecord(ctx->ev_status, ctx->st));
   return MFA_OK;
+}
+
+// n doubles and the status words into page-locked host memory by one kernel: a drop-in call returns
+// its energies to the host, and two copies into pageable memory and their events took longer than
+// its kernel.
+__global__ void k_publish(const double* __restrict__ src, int n, double* __restrict__ dst,
+                          const unsigned* __restrict__ status, unsigned* __restrict__ hstatus) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < n) dst[k] = src[k];
+  if (k < 2) hstatus[k] = status[k];
+}
+
+// slots [slot, slot + n) of the accumulators or record `src` to the same places of ctx->h_rec, with
+// the status checked; large ones (many replicas) by the copy engine
+int read_slots(mfa_ctx* ctx, const double* src, int slot, int n) {
+  const size_t at = (size_t)slot * ctx->nrep, cnt = (size_t)n * ctx->nrep;
+  if (cnt <= 8192) {
+    k_publish<<<(int)(cnt + 255) / 256, 256, 0, ctx->st>>>(src + at, (int)cnt, ctx->h_rec + at, ctx->S.status,
+                                                           ctx->h_status);
+    CK(cudaGetLastError());
+  } else {
+    CK(cudaMemcpyAsync(ctx->h_rec + at, src + at, sizeof(double) * cnt, cudaMemcpyDeviceToHost, ctx->st));
+    RET(post_status(ctx));
+  }
+  return check_status(ctx);
+}
+
+struct SlotRanges {
+  int slot[4], n[4];
+};
+__global__ void k_zero_slots(double* acc, int nrep, SlotRanges r) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    if (k < r.n[q] * nrep) acc[(size_t)r.slot[q] * nrep + k] = 0.;
 }
 
 // Non-blocking look at the status words of the last post_status: when that copy has arrived (no
@@ -766,7 +802,10 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
   S.mixed = ctx->opt.precision == MFA_PREC_MIXED;
   const size_t Nn = ctx->Np;
   double** dst[12] = {&S.rx, &S.ry, &S.rz, &S.vx, &S.vy, &S.vz, &S.ax, &S.ay, &S.az, &S.fx, &S.fy, &S.fz};
-  for (auto d : dst) DA(*d, Nn);
+  for (int k = 0; k < 9; ++k) DA(*dst[k], Nn);
+  DA(S.fx, 3 * Nn);  // (the three together: one memset clears them)
+  S.fy = S.fx + Nn;
+  S.fz = S.fy + Nn;
   for (int k = 0; k < 9; ++k) DA(S.tmp[k], Nn);
   DA(S.tag, Nn); DA(S.info, Nn); DA(S.tmp_tag, Nn); DA(S.tmp_info, Nn); DA(S.slot_of_tag, Nn);
   DA(S.pfx, Nn);  // (the FP64 mode: for the list build and the pair kernel's screening)
@@ -826,6 +865,7 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
   DA(ctx->series_head, 1);
   CK(cudaMallocHost(&ctx->h_status, 2 * sizeof(unsigned)));
   CK(cudaMallocHost(&ctx->h_rebuilds, sizeof(long long)));
+  CK(cudaMallocHost(&ctx->h_rec, sizeof(double) * NOBS * n_rep));
   ctx->h_status[0] = ctx->h_status[1] = 0;
   S.reps = ctx->dreps;
   S.tabf = ctx->dtabf;
@@ -873,7 +913,7 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
   CK(cudaMemsetAsync(ctx->prof, 0, sizeof(double) * n_rep * C.hist_dim * 21, st));
   if (ctx->avg) CK(cudaMemsetAsync(ctx->avg, 0, sizeof(double) * NAVG * n_rep, st));
   CK(cudaMemsetAsync(ctx->series_head, 0, sizeof(long long), st));
-  for (int k = 9; k < 12; ++k) CK(cudaMemsetAsync(*dst[k], 0, sizeof(double) * Nn, st));
+  CK(cudaMemsetAsync(S.fx, 0, sizeof(double) * 3 * Nn, st));
   // ---- state upload (canonical AoS -> slots) --------------------------------------------------
   {
     double *dr = nullptr, *dv = nullptr, *dac = nullptr;
@@ -948,6 +988,7 @@ int mfa_destroy(mfa_ctx* ctx) {
   for (void* p : ctx->allocs) cudaFree(p);
   if (ctx->h_status) cudaFreeHost(ctx->h_status);
   if (ctx->h_rebuilds) cudaFreeHost(ctx->h_rebuilds);
+  if (ctx->h_rec) cudaFreeHost(ctx->h_rec);
   for (int k = 0; k < 16; ++k)
     if (ctx->ev[k]) cudaEventDestroy(ctx->ev[k]);
   if (ctx->st) cudaStreamDestroy(ctx->st);
@@ -978,25 +1019,23 @@ int mfa_n_particles(const mfa_ctx* ctx, int64_t* n_total, int32_t* n_rep) {
 }
 
 // ---- per-routine drop-ins -------------------------------------------------------------------
-// A drop-in clears the accumulator slots it fills; from then on the energy, virial and head-force
-// readers take the per-routine accumulators (until the next mfa_step record).
-static int zero_call_slot(mfa_ctx* ctx, int slot, int n = 1) {
-  CK(cudaMemsetAsync(ctx->acc_call + (size_t)slot * ctx->nrep, 0, sizeof(double) * ctx->nrep * n, ctx->st));
+// A drop-in clears the accumulator slots it fills (its energies and, each replacing its own group,
+// the 9 virial slots); from then on the energy, virial and head-force readers take the per-routine
+// accumulators (until the next mfa_step record).
+static int zero_call_slots(mfa_ctx* ctx, SlotRanges r) {
+  int most = 0;
+  for (int q = 0; q < 4; ++q) most = std::max(most, r.n[q]);
+  k_zero_slots<<<(most * ctx->nrep + 255) / 256, 256, 0, ctx->st>>>(ctx->acc_call, ctx->nrep, r);
+  CK(cudaGetLastError());
   ctx->last_source = 2;
   return MFA_OK;
 }
-// the 9 virial slots of a group (each drop-in replaces its own group)
-static int zero_call_group(mfa_ctx* ctx, int group) { return zero_call_slot(ctx, O_VIR + 9 * group, 9); }
+static SlotRanges energy_and_group(int slot, int group) { return SlotRanges{{slot, O_VIR + 9 * group}, {1, 9}}; }
 
-static int read_call_slot(mfa_ctx* ctx, int slot, double* out, double add_self) {
+static int read_call_slot(mfa_ctx* ctx, int slot, double* out) {
   if (!out) return MFA_OK;
-  CK(cudaMemcpyAsync(out, ctx->acc_call + (size_t)slot * ctx->nrep, sizeof(double) * ctx->nrep,
-                     cudaMemcpyDeviceToHost, ctx->st));
-  RET(post_status(ctx));
-  int r = check_status(ctx);
-  if (r != MFA_OK) return r;
-  if (add_self != 0.)
-    for (int k = 0; k < ctx->nrep; ++k) out[k] += ctx->v_coul_self[k];
+  RET(read_slots(ctx, ctx->acc_call, slot, 1));
+  std::copy_n(ctx->h_rec + (size_t)slot * ctx->nrep, ctx->nrep, out);
   return MFA_OK;
 }
 
@@ -1026,32 +1065,29 @@ int mfa_check_skin(mfa_ctx* ctx, int32_t* rebuilt) {
 
 int mfa_zero_force(mfa_ctx* ctx) {
   if (!ctx) return MFA_ERR_ARG;
-  CK(cudaMemsetAsync(ctx->S.fx, 0, sizeof(double) * ctx->N, ctx->st));
-  CK(cudaMemsetAsync(ctx->S.fy, 0, sizeof(double) * ctx->N, ctx->st));
-  CK(cudaMemsetAsync(ctx->S.fz, 0, sizeof(double) * ctx->N, ctx->st));
+  CK(cudaMemsetAsync(ctx->S.fx, 0, sizeof(double) * 3 * ctx->Np, ctx->st));
   return MFA_OK;
 }
 
 int mfa_fluid_fluid(mfa_ctx* ctx, double* v_ff, double* v_coul) {
   if (!ctx) return MFA_ERR_ARG;
-  int r;
-  if ((r = zero_call_slot(ctx, O_VFF)) || (r = zero_call_slot(ctx, O_VCOUL)) || (r = zero_call_group(ctx, V_PAIR)))
-    return r;
+  RET(zero_call_slots(ctx, SlotRanges{{O_VFF, O_VCOUL, O_VIR + 9 * V_PAIR}, {1, 1, 9}}));
   launch_pair(ctx->S, ctx->C, ctx->st, true, true, acc_of(ctx->acc_call, ctx->nrep), ctx->opt.block_size);
   ctx->launches += 1;
   CK(cudaGetLastError());
-  ctx->last_source = 2;
-  if ((r = read_call_slot(ctx, O_VFF, v_ff, 0.))) return r;
-  if ((r = read_call_slot(ctx, O_VCOUL, v_coul, ctx->C.charged ? 1. : 0.))) return r;
-  if (v_ff)
-    for (int k = 0; k < ctx->nrep; ++k) v_ff[k] += ctx->v_ff_walls[k];
+  if (!v_ff && !v_coul) return MFA_OK;
+  static_assert(O_VFF == 0 && O_VCOUL > O_VFF, "both energies in one read");
+  RET(read_slots(ctx, ctx->acc_call, O_VFF, O_VCOUL + 1));
+  for (int k = 0; k < ctx->nrep; ++k) {
+    if (v_ff) v_ff[k] = ctx->h_rec[(size_t)O_VFF * ctx->nrep + k] + ctx->v_ff_walls[k];
+    if (v_coul) v_coul[k] = ctx->h_rec[(size_t)O_VCOUL * ctx->nrep + k] + (ctx->C.charged ? ctx->v_coul_self[k] : 0.);
+  }
   return MFA_OK;
 }
 
 int mfa_fluid_wall(mfa_ctx* ctx, int32_t wall_type, double* v_fw) {
   if (!ctx) return MFA_ERR_ARG;
-  int r;
-  if ((r = zero_call_slot(ctx, O_VFW)) || (r = zero_call_group(ctx, V_WALL))) return r;
+  RET(zero_call_slots(ctx, energy_and_group(O_VFW, V_WALL)));
   if (wall_type == 2 && ctx->C.wall == 2) {
     launch_wall(ctx->S, ctx->C, ctx->st, true, acc_of(ctx->acc_call, ctx->nrep));
     ctx->launches += 1;
@@ -1059,7 +1095,7 @@ int mfa_fluid_wall(mfa_ctx* ctx, int32_t wall_type, double* v_fw) {
     return fail(ctx, MFA_ERR_UNSUPPORTED, "fluid_wall: only wall types 1 (in the pair kernel) and 2 are built");
   }
   CK(cudaGetLastError());
-  return read_call_slot(ctx, O_VFW, v_fw, 0.);
+  return read_call_slot(ctx, O_VFW, v_fw);
 }
 
 int mfa_wall_wall(mfa_ctx* ctx, int32_t wall_type, double* v_ww) {
@@ -1070,13 +1106,12 @@ int mfa_wall_wall(mfa_ctx* ctx, int32_t wall_type, double* v_ww) {
 }
 
 static int bonded_call(mfa_ctx* ctx, int mask, int slot, double* out) {
-  int r;
   const int group = mask == 1 ? V_FENE : mask == 2 ? V_BEND : mask == 4 ? V_BENDM : V_OR;
-  if ((r = zero_call_slot(ctx, slot)) || (r = zero_call_group(ctx, group))) return r;
+  RET(zero_call_slots(ctx, energy_and_group(slot, group)));
   launch_bonded(ctx->S, ctx->C, ctx->st, mask, true, acc_of(ctx->acc_call, ctx->nrep));
   ctx->launches += 1;
   CK(cudaGetLastError());
-  return read_call_slot(ctx, slot, out, 0.);
+  return read_call_slot(ctx, slot, out);
 }
 
 int mfa_intra_molec(mfa_ctx* ctx, double* v) { return ctx ? bonded_call(ctx, 1, O_VINTRA, v) : MFA_ERR_ARG; }
@@ -1097,21 +1132,19 @@ int mfa_ewald_k(mfa_ctx* ctx, int32_t mode, double* v) {
   if (!ctx) return MFA_ERR_ARG;
   if (mode == 0) return MFA_OK;
   if (!ctx->kspace) return fail(ctx, MFA_ERR_STATE, "ewald_k: not a charged system");
-  int r;
-  if ((r = zero_call_slot(ctx, O_VCOULK)) || (r = zero_call_group(ctx, V_KSPACE))) return r;
+  RET(zero_call_slots(ctx, energy_and_group(O_VCOULK, V_KSPACE)));
   ctx->launches += launch_kspace(ctx->S, ctx->C, ctx->KB, ctx->st, true, acc_of(ctx->acc_call, ctx->nrep));
   CK(cudaGetLastError());
-  return read_call_slot(ctx, O_VCOULK, v, 0.);
+  return read_call_slot(ctx, O_VCOULK, v);
 }
 
 int mfa_dipolar_correction(mfa_ctx* ctx, double* v) {
   if (!ctx) return MFA_ERR_ARG;
   if (!ctx->kspace) return fail(ctx, MFA_ERR_STATE, "dipolar_correction: not a charged system");
-  int r;
-  if ((r = zero_call_slot(ctx, O_VDIP)) || (r = zero_call_group(ctx, V_DIP))) return r;
+  RET(zero_call_slots(ctx, energy_and_group(O_VDIP, V_DIP)));
   ctx->launches += launch_dipolar(ctx->S, ctx->C, ctx->KB, ctx->st, true, acc_of(ctx->acc_call, ctx->nrep));
   CK(cudaGetLastError());
-  return read_call_slot(ctx, O_VDIP, v, 0.);
+  return read_call_slot(ctx, O_VDIP, v);
 }
 
 int mfa_constant_force(mfa_ctx* ctx, int32_t mode) {
@@ -1125,20 +1158,14 @@ int mfa_constant_force(mfa_ctx* ctx, int32_t mode) {
 
 int mfa_verlet_velocities(mfa_ctx* ctx, mfa_energies* e) {
   if (!ctx) return MFA_ERR_ARG;
-  int r;
-  if ((r = zero_call_slot(ctx, O_TFLUID)) || (r = zero_call_slot(ctx, O_FH, 6)) || (r = zero_call_slot(ctx, O_KIN, 9)))
-    return r;
+  RET(zero_call_slots(ctx, SlotRanges{{O_TFLUID, O_FH, O_KIN}, {1, 6, 9}}));
   launch_integrate(ctx->S, ctx->C, ctx->st, 1, false, true, acc_of(ctx->acc_call, ctx->nrep));
   ctx->launches += 1;
   CK(cudaGetLastError());
   ctx->host_steps += 1;
-  ctx->last_source = 2;
   if (e) {
-    std::vector<double> h(NOBS * ctx->nrep);
-    CK(cudaMemcpyAsync(h.data(), ctx->acc_call, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, ctx->st));
-    RET(post_status(ctx));
-    if ((r = check_status(ctx))) return r;
-    for (int k = 0; k < ctx->nrep; ++k) fill_energies(ctx, h.data(), k, &e[k]);
+    RET(read_slots(ctx, ctx->acc_call, 0, NOBS));
+    for (int k = 0; k < ctx->nrep; ++k) fill_energies(ctx, ctx->h_rec, k, &e[k]);
   }
   return MFA_OK;
 }
@@ -1406,6 +1433,16 @@ int mfa_sync_to_host(mfa_ctx* ctx, double* r0, double* v, double* a, double* for
   if (!r0 && !v && !a && !force) return mfa_synchronize(ctx);
   double* buf = nullptr;
   RET(staging(ctx, &buf));
+  if (ctx->N <= 65536) {
+    // a short state: one gather and the copies behind it on one stream (the events that let the copies
+    // of a long one overlap its gathers take longer than these)
+    launch_gather_state(ctx->S, ctx->st, r0 ? buf : nullptr, v ? buf + n3 : nullptr, a ? buf + 2 * n3 : nullptr,
+                        force ? buf + 3 * n3 : nullptr);
+    for (int k = 0; k < 4; ++k)
+      if (host[k]) CK(cudaMemcpyAsync(host[k], buf + k * n3, n3 * 8, cudaMemcpyDeviceToHost, ctx->st));
+    RET(post_status(ctx));
+    return check_status(ctx);
+  }
   // One array at a time: its gather into the staging buffer (device memory, the compute stream),
   // then its copy-engine copy to the host (the copy stream) while the next array is gathered.
   // (A gather kernel writing to host memory directly measured 3x slower than this.)
@@ -1456,13 +1493,8 @@ int mfa_set_state(mfa_ctx* ctx, const double* r0, const double* v, const double*
 
 int mfa_get_energies(mfa_ctx* ctx, mfa_energies* out) {
   if (!ctx || !out) return MFA_ERR_ARG;
-  std::vector<double> h(NOBS * ctx->nrep);
-  const double* src = ctx->last_source == 2 ? ctx->acc_call : ctx->rec;
-  CK(cudaMemcpyAsync(h.data(), src, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, ctx->st));
-  RET(post_status(ctx));
-  int r = check_status(ctx);
-  if (r) return r;
-  for (int k = 0; k < ctx->nrep; ++k) fill_energies(ctx, h.data(), k, &out[k]);
+  RET(read_slots(ctx, ctx->last_source == 2 ? ctx->acc_call : ctx->rec, 0, O_VIR));
+  for (int k = 0; k < ctx->nrep; ++k) fill_energies(ctx, ctx->h_rec, k, &out[k]);
   return MFA_OK;
 }
 
