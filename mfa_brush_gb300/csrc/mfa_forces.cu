@@ -472,7 +472,9 @@ __device__ __forceinline__ double pair_fs64(const DevState& s, const SimConst& C
   if (!(in_lj || dpd || in_c)) return fs;
   const double ir = rsqrt64(r2);  // the only root and division of the pair
   if (in_lj) {
-    const double inv_r2 = ir * ir;
+    // (rounded once: the seventh power below would enlarge the square's own error.  1 % of the step)
+    double inv_r2 = ir * ir;
+    inv_r2 = fma(inv_r2, fma(-inv_r2, r2, 1.), inv_r2);
     const double s2 = e.sig2 * inv_r2;
     const double s6 = s2 * s2 * s2;
     const double s12 = s6 * s6;
