@@ -289,6 +289,71 @@ int upload_noise_tables(mfa_ctx* ctx) {
   return MFA_OK;
 }
 
+// The FP64 mode's table of the real-space Coulomb factors (CoulTab) up to the largest distance at which
+// a charged pair interacts.  It starts at r = 0.7 (closer pairs, rare between beads of 1 sigma, take the
+// functions); interval width 1/30 of its start, at most a tenth of 1 / alpha, at most 4096 intervals.
+int make_coul_table(mfa_ctx* ctx, double r2max) {
+  const SimConst& C = ctx->C;
+  const double lo = 0.49;
+  if (!(r2max > lo) || !(C.alpha_c > 0.)) return MFA_OK;
+  const double h0 = std::min(lo / 30., 0.1 / C.alpha_c);
+  const int n = (int)std::ceil((r2max - lo) / h0);
+  if (n > 4096) return MFA_OK;
+  const double h = (r2max - lo) / n;
+  // monomial coefficients from the values at the 8 Chebyshev points, by the Chebyshev coefficients and
+  // the polynomials' own recursion
+  double cheb[8][8] = {};  // T_k in monomials
+  cheb[0][0] = 1;
+  cheb[1][1] = 1;
+  for (int k = 2; k < 8; ++k)
+    for (int m = 0; m < 8; ++m) cheb[k][m] = (m ? 2 * cheb[k - 1][m - 1] : 0) - cheb[k - 2][m];
+  double node[8], ct[8][8];
+  for (int i = 0; i < 8; ++i) {
+    node[i] = std::cos(M_PI * (i + 0.5) / 8);
+    for (int k = 0; k < 8; ++k) ct[k][i] = std::cos(M_PI * k * (i + 0.5) / 8) * (k ? 2. : 1.) / 8;
+  }
+  std::vector<double> tab(16 * (size_t)n);
+  for (int q = 0; q < n; ++q) {
+    double v[2][8];
+    for (int i = 0; i < 8; ++i) {
+      // the roundings of x, alpha x, sqrt(alpha) r and r, which erfc and exp enlarge, go back in to
+      // first order: 8e-16 relative for alpha x up to 100, where the plain formulas are at 8e-15
+      const double al = C.alpha_c, x = lo + h * (q + 0.5 * (node[i] + 1));
+      const double dx = (double)((long double)lo + (long double)h * (q + 0.5L * ((long double)node[i] + 1)) - x);
+      double r = std::sqrt(x);
+      const double z = C.sqrt_alpha * r, p = al * x, dp = std::fma(al, x, -p) + al * dx;
+      double ex = std::exp(-p);
+      ex -= ex * dp;
+      const double ec = std::erfc(z) - C.inv_sqrt_pi * ex * (std::fma(-z, z, p) + dp) / z;
+      r += 0.5 * (std::fma(-r, r, x) + dx) / r;
+      v[0][i] = (2 * C.sqrt_alpha * C.inv_sqrt_pi * ex / r + ec / (r * r)) / r;
+      v[1][i] = ec / r;
+    }
+    for (int g = 0; g < 2; ++g) {
+      // (the value in the middle of the range taken out first: the small differences then keep their
+      // own rounding)
+      const double v0 = v[g][3];
+      double out[8] = {};
+      for (int k = 0; k < 8; ++k) {
+        double a = 0;
+        for (int i = 0; i < 8; ++i) a += ct[k][i] * (v[g][i] - v0);
+        for (int m = 0; m < 8; ++m) out[m] += a * cheb[k][m];
+      }
+      out[0] += v0;
+      for (int m = 0; m < 8; ++m) tab[((size_t)g * n + q) * 8 + m] = out[m];
+    }
+  }
+  double* d = nullptr;
+  CoulTab* t = nullptr;
+  DA(d, tab.size());
+  DA(t, 1);
+  CoulTab host = {lo, r2max, 1. / h, n, 0, d, d + 8 * (size_t)n};
+  CK(cudaMemcpy(d, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(t, &host, sizeof host, cudaMemcpyHostToDevice));
+  ctx->S.coul = t;
+  return MFA_OK;
+}
+
 // ewald_k(0) (ewald_k.f90:37-124): the k-vectors in the reference's enumeration order, G(k),
 // and the list of charged particles, of replica rep (the particles p0 .. p0 + n_mon_tot - 1 of the
 // batch; a_type holds the whole batch).
@@ -397,10 +462,15 @@ int setup_kspace(mfa_ctx* ctx, const int32_t* a_type, int rep) {
     }
     fwin[c] = make_int2(lo, hi);
   }
+  K.ncolq = K.ncol + nz + 1;
+  K.qmax = 0.;
+  for (double q : qv) K.qmax = std::max(K.qmax, std::fabs(q));
+  K.inv_qmax = K.qmax > 0. ? 1. / K.qmax : 0.;
   // rho particle chunks: one wave of three blocks per SM, chunks a multiple of the 32-particle tile
   const int kb = (K.nrows + 63) / 64 * ((2 * nx + 1 + 31) / 32);  // k_ks_rho: 64 rows x 32 slots
   int pch = std::max(1, std::min(256, (3 * 152 + kb - 1) / kb));
   K.pchunk = std::max(32, ((K.nq + pch - 1) / pch + 31) / 32 * 32);
+  if (!ctx->S.mixed && dense) K.pchunk = std::min(K.pchunk, 2048);  // (the range of its integer totals)
   K.npchunks = std::max(1, (K.nq + K.pchunk - 1) / K.pchunk);
   DA(K.kn, K.nk);
   DA(K.kvec, 3 * K.nk);
@@ -424,7 +494,13 @@ int setup_kspace(mfa_ctx* ctx, const int32_t* a_type, int rep) {
     DA(K.kdf, K.nk);
     DA(K.wdense, (size_t)K.nrows * 4 * K.qx);
   } else {
-    DA(K.tabd, (size_t)K.nq * K.ncol);
+    if (dense) {
+      DA(K.tabq, (size_t)K.nq * K.ncolq);
+      DA(K.wq, (size_t)K.nrows * 16 * 4);
+      DA(K.rowq, 3 * (size_t)K.nrows);
+    } else {
+      DA(K.tabd, (size_t)K.nq * K.ncol);
+    }
     DA(K.kdd, K.nk);
   }
   cudaStream_t st = ctx->st;
@@ -871,6 +947,13 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
   S.tabf = ctx->dtabf;
   S.tabd = ctx->dtabd;
   if (!S.mixed) RET(upload_noise_tables(ctx));
+  if (!S.mixed && charged) {
+    double r2max = p->rc_coul_2;
+    if (r2max <= 0.)
+      for (const PairEntry<double>& e : td)
+        if (e.flags & PF_COUL) r2max = std::max(r2max, e.range2);
+    RET(make_coul_table(ctx, r2max));
+  }
   S.rl2_uni = C.rl2_uni_f;
   S.fx_err = (float)fx_err;
   S.nl_h = nl_h;

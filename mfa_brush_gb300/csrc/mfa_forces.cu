@@ -496,9 +496,21 @@ __device__ __forceinline__ double pair_fs64(const DevState& s, const SimConst& C
     fs += (C.sig * wr * g - C.gamma * wd * rdot) * ir;
   }
   if (in_c) {
-    const double r = r2 * ir, qq = e.qq, ec = erfc(C.sqrt_alpha * r);
-    if (EFLAG) e_c += half * qq * ec * ir;
-    fs += (qq * C.sqrt_alpha * C.inv_sqrt_pi * 2. * exp(-C.alpha_c * r2) * ir + qq * ec * ir * ir) * ir;
+    const CoulTab* T = s.coul;
+    if (T && r2 >= T->lo && r2 < T->hi) {
+      const double x = (r2 - T->lo) * T->inv_h, z = x + 4503599627370496.0;  // 2^52: rounds to an integer
+      int k = __double2loint(z);
+      double t = x - (z - 4503599627370496.0);  // [-1/2, 1/2] from the nearest edge
+      if (t < 0.) --k;
+      k = min(k, T->n - 1);
+      t = fma(2., t, t < 0. ? 1. : -1.);  // [-1, 1] inside the interval
+      fs += e.qq * coul_poly(T->f + 8 * (size_t)k, t);
+      if (EFLAG) e_c += half * e.qq * coul_poly(T->e + 8 * (size_t)k, t);
+    } else {
+      const double r = r2 * ir, qq = e.qq, ec = erfc(C.sqrt_alpha * r);
+      if (EFLAG) e_c += half * qq * ec * ir;
+      fs += (qq * C.sqrt_alpha * C.inv_sqrt_pi * 2. * exp(-C.alpha_c * r2) * ir + qq * ec * ir * ir) * ir;
+    }
   }
   return fs;
 }

@@ -102,6 +102,53 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// ---- the FP64 mode's sums in integers -----------------------------------------------------------
+// An FP64 multiply-add of a warp holds the SM's FP64 pipe for 16 clocks; three 32 x 32 + 64 bit integer
+// ones do the same work in two fifths of that (charged brush, 13,760 charges and 8070 k: rho 903 -> 306
+// us, force 1740 -> 597).  A number v, |v| <= 1, is held in two limbs, v = h 2^-27 +
+// l 2^-57 with |l| <= 2^29 (57 bits behind the point; a double in [1/2, 1) has 53).  A product keeps
+// h h' (in units of 2^-54) and h l' + l h' (2^-84), each summed exactly in 64 bits; l l', at most 2^-56
+// and of either sign, is left out.  The k sets of up to 15 waves per axis (nxm) take this path.
+constexpr double QL_MAGIC = 6755399441055744.0;  // 1.5 * 2^52: the low word of the sum is the integer
+
+__device__ __forceinline__ int2 ql_of(double v) {
+  const double t = fma(v, 134217728.0, QL_MAGIC);
+  const double r = fma(v, 134217728.0, QL_MAGIC - t);
+  return make_int2(__double2loint(t), __double2loint(fma(r, 1073741824.0, QL_MAGIC)));
+}
+struct QlSum {
+  long long h, m;
+  __device__ __forceinline__ void zero() { h = m = 0; }
+  __device__ __forceinline__ void add(int2 a, int2 b) {
+    h += (long long)a.x * b.x;
+    m += (long long)a.x * b.y;
+    m += (long long)a.y * b.x;
+  }
+  __device__ __forceinline__ long long q54() const { return h + ((m + (1ll << 29)) >> 30); }  // units of 2^-54
+  // units of 2^-58, for sums below 16
+  __device__ __forceinline__ long long q58() const { return (h << 4) + ((m + (1ll << 25)) >> 26); }
+};
+__device__ __forceinline__ int2 ql_neg(int2 a) { return make_int2(-a.x, -a.y); }
+// the limbs of t units of 2^-58, |t| <= 2^58
+__device__ __forceinline__ int2 ql_limbs(long long t) {
+  const long long h = (t + (1ll << 30)) >> 31;
+  return make_int2((int)h, ((int)(t - (h << 31)) + 1) >> 1);
+}
+__device__ __forceinline__ int2 ql_re(int4 a) { return make_int2(a.x, a.y); }
+__device__ __forceinline__ int2 ql_im(int4 a) { return make_int2(a.z, a.w); }
+// (a b) of complex numbers of modulus at most 1
+__device__ __forceinline__ int4 ql_cmul(int4 a, int4 b) {
+  QlSum re, im;
+  re.zero();
+  im.zero();
+  re.add(ql_re(a), ql_re(b));
+  re.add(ql_neg(ql_im(a)), ql_im(b));
+  im.add(ql_re(a), ql_im(b));
+  im.add(ql_im(a), ql_re(b));
+  const int2 x = ql_limbs(re.q58()), y = ql_limbs(im.q58());
+  return make_int4(x.x, x.y, y.x, y.y);
+}
+
 constexpr int KS_TILE = 32;  // particles per shared-memory tile of k_ks_rho (one per lane)
 
 // rho(row, nx) = sum_p A(p, row) X(p, nx), A = q Y(ny) Z(nz), with X(p, -n) = conj X(p, n): the
@@ -128,6 +175,7 @@ __global__ void __launch_bounds__(KS_RHO_T, MIXED ? 3 : 1) k_ks_rho(const KSpace
   const KSpace K = Ks[blockIdx.z / nz];
   const int zs = blockIdx.z % nz;
   if ((int)blockIdx.x * KS_RB >= K.nrows || (int)blockIdx.y >= K.npchunks || zs * KS_SL > K.nxm || K.nq == 0) return;
+  if (!MIXED && K.dense) return;  // (k_ks_rho_q)
   using real = kreal<MIXED>;
   using Cx = kcplx<MIXED>;
   extern __shared__ __align__(16) unsigned char shraw[];
@@ -284,6 +332,112 @@ __global__ void __launch_bounds__(KS_RHO_T, MIXED ? 3 : 1) k_ks_rho(const KSpace
   }
 }
 
+// The same in integer limbs (FP64 mode, K.dense): lanes, rows and tiles as k_ks_rho; the tables are
+// those of X, Y and q Z / q_max.  A tile's sums go to 64-bit totals in units of 2^-51 (a chunk holds at most
+// 2048 particles: a total, and the sums of two that a k takes, stay at or below 2^62).
+__global__ void __launch_bounds__(KS_RHO_T, 2) k_ks_rho_q(const KSpace* __restrict__ Ks, int nz) {
+  const KSpace K = Ks[blockIdx.z / nz];
+  const int zs = blockIdx.z % nz;
+  if (!K.dense || (int)blockIdx.x * KS_RB >= K.nrows || (int)blockIdx.y >= K.npchunks || zs > 0 || K.nq == 0) return;
+  extern __shared__ __align__(16) unsigned char shraw[];
+  int4* As = reinterpret_cast<int4*>(shraw);                 // [KS_TILE][KS_RB + 1]
+  int2* rc = reinterpret_cast<int2*>(As + KS_TILE * (KS_RB + 1));
+  int4* cols = reinterpret_cast<int4*>(rc + KS_RB);          // two tiles of columns: 16 X, the Y, the block's Z
+  const int rbeg = blockIdx.x * KS_RB, nr = min(KS_RB, K.nrows - rbeg);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4;
+  constexpr int NW = KS_RHO_T / 32, RL = KS_RW / 2;
+  const int slot = lane & (KS_SL - 1), r0 = warp * KS_RW + half * RL;
+  const bool act = r0 < nr;
+  const int zlo = K.rows[rbeg].w, nzc = K.rows[rbeg + nr - 1].w - zlo + 1, ncols = KS_SL + K.nym + 1 + nzc;
+  for (int r = threadIdx.x; r < nr; r += KS_RHO_T) {
+    const int4 R = K.rows[rbeg + r];
+    const int yc = KS_SL + abs(R.z);
+    rc[r] = make_int2(R.z < 0 ? -yc : yc, KS_SL + K.nym + 1 + R.w - zlo);
+  }
+  const int p_beg = blockIdx.y * K.pchunk, p_end = min(K.nq, p_beg + K.pchunk);
+  auto fetch = [&](int t0, int buf) {
+    const int pq = t0 + lane;
+    if (pq < p_end) {
+      int4* to = cols + buf * ncols * KS_CS + lane;
+      for (int c = warp; c < ncols; c += NW) {
+        const int col = c < KS_SL ? c : (c < KS_SL + K.nym + 1 ? K.nxm + 1 + c - KS_SL
+                                                               : K.ncol + zlo + c - KS_SL - K.nym - 1);
+        if (c >= KS_SL || c <= K.nxm) cp_async(to + c * KS_CS, K.tabq + (size_t)col * K.nq + pq);
+      }
+    }
+    cp_async_commit();
+  };
+  for (int c = K.nxm + 1 + warp; c < KS_SL; c += NW)
+    cols[c * KS_CS + lane] = cols[(ncols + c) * KS_CS + lane] = make_int4(0, 0, 0, 0);
+  long long tot[4][RL];
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int i = 0; i < RL; ++i) tot[a][i] = 0;
+  fetch(p_beg, 0);
+  int buf = 0;
+  for (int t0 = p_beg; t0 < p_end; t0 += KS_TILE, buf ^= 1) {
+    const int nt = min(KS_TILE, p_end - t0);
+    cp_async_wait<0>();
+    __syncthreads();  // this tile's columns are here; the A and columns of the tile before are used up
+    fetch(t0 + KS_TILE, buf ^ 1);
+    const int4* col = cols + buf * ncols * KS_CS;
+    if (lane < nt) {
+#pragma unroll 2
+      for (int h = 0; h < KS_RB / NW; ++h) {
+        const int r = warp + NW * h;
+        if (r < nr) {
+          const int2 R = rc[r];
+          int4 y = col[abs(R.x) * KS_CS + lane];
+          if (R.x < 0) { y.z = -y.z; y.w = -y.w; }
+          As[lane * (KS_RB + 1) + r] = ql_cmul(y, col[R.y * KS_CS + lane]);
+        }
+      }
+    }
+    __syncthreads();
+    if (act) {
+      const int4* xs = col + slot * KS_CS;
+      QlSum t[4][RL];
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int i = 0; i < RL; ++i) t[a][i].zero();
+#pragma unroll 1
+      for (int p = 0; p < nt; ++p) {
+        const int4 x = xs[p];
+#pragma unroll
+        for (int i = 0; i < RL; ++i) {
+          const int4 A = As[p * (KS_RB + 1) + r0 + i];
+          t[0][i].add(ql_re(A), ql_re(x));
+          t[1][i].add(ql_im(A), ql_im(x));
+          t[2][i].add(ql_re(A), ql_im(x));
+          t[3][i].add(ql_im(A), ql_re(x));
+        }
+      }
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int i = 0; i < RL; ++i) tot[a][i] += (t[a][i].q54() + 4) >> 3;
+    }
+  }
+  if (act && slot <= K.nxm) {
+    const double sc = K.qmax * 4.4408920985006262e-16;  // 2^-51
+#pragma unroll
+    for (int i = 0; i < RL; ++i) {
+      const int r = r0 + i;
+      if (r < nr) {
+        const int4 R = K.rows[rbeg + r];
+        const int lo = K.kn[R.x].x, kp = R.x + slot - lo, km = R.x - slot - lo;
+        double2* o = reinterpret_cast<double2*>(K.rho_part) + (size_t)blockIdx.y * K.nk;
+        if (kp >= R.x && kp < R.y)
+          o[kp] = make_double2((double)(tot[0][i] - tot[1][i]) * sc, (double)(tot[2][i] + tot[3][i]) * sc);
+        if (slot > 0 && km >= R.x && km < R.y)
+          o[km] = make_double2((double)(tot[0][i] + tot[1][i]) * sc, (double)(tot[3][i] - tot[2][i]) * sc);
+      }
+    }
+  }
+}
+
 // Block sum of v (all threads, warps in order); the same value in every thread.
 __device__ __forceinline__ double block_sum(double v, double* red) {
   v = warp_sum(v);
@@ -379,9 +533,13 @@ __global__ void __launch_bounds__(KS_TAB_T) k_ks_tables(DevState s, const KSpace
     return;
   }
   const int idx = (blockIdx.x - dblk) * KS_TAB_T + threadIdx.x;
-  if (!(what & KS_RECIP) || K.nk == 0 || idx >= K.nq * K.ncol) return;
-  const int col = idx / K.nq, p = idx - col * K.nq;
+  const int ncol = (!MIXED && K.dense) ? K.ncolq : K.ncol;
+  if (!(what & KS_RECIP) || K.nk == 0 || idx >= K.nq * ncol) return;
+  int col = idx / K.nq;
+  const int p = idx - col * K.nq;
   const int i = s.slot_of_tag[K.qtag[p]];
+  const bool times_q = col >= K.ncol;  // (the limb tables hold q Z / q_max as well)
+  if (times_q) col -= K.nzm + 1;
   int n = col, ax = 0;
   if (col > K.nxm + 1 + K.nym) { n = col - K.nxm - K.nym - 2; ax = 2; }
   else if (col > K.nxm) { n = col - K.nxm - 1; ax = 1; }
@@ -395,6 +553,23 @@ __global__ void __launch_bounds__(KS_TAB_T) k_ks_tables(DevState s, const KSpace
     float sn, cs;
     sincospif(i2f_fast((int)(ph >> 32)) * (2.f / 4294967296.f), &sn, &cs);
     K.tabf[idx] = make_float2(cs, sn);
+  } else if (K.dense) {
+    // the same phase to 64 bits: the nearest of 1024 table angles and the angle from it by the series
+    const unsigned long long ph = (unsigned long long)round_bits(t * 288230376151711744.0) * (unsigned)n << 6;
+    const int k = (int)((ph + (1ull << 53)) >> 54) & 1023;
+    const long long lo = (long long)(ph << 10) >> 10;  // ph mod 2^54, signed
+    const double d = (double)lo * (6.283185307179586476925 / 18446744073709551616.0);  // 2 pi / 2^64
+    const double2 a = __ldg(&s.noise->cs[k]);
+    const double d2 = d * d, c = fma(d2, fma(d2, 1.0 / 24.0, -0.5), 1.0);
+    const double e = d * fma(d2, fma(d2, 1.0 / 120.0, -1.0 / 6.0), 1.0);
+    double re = fma(a.x, c, -(a.y * e)), im = fma(a.y, c, a.x * e);
+    if (times_q) {
+      const double q = K.qval[p] * K.inv_qmax;
+      re *= q;
+      im *= q;
+    }
+    const int2 x = ql_of(re), y = ql_of(im);
+    K.tabq[idx] = make_int4(x.x, x.y, y.x, y.y);
   } else {
     double u = (double)n * t;
     u -= rint(u);  // turns in [-1/2, 1/2]
@@ -721,6 +896,136 @@ __global__ void __launch_bounds__(KS_FB) k_ks_force_dense(const KSpace* __restri
   }
 }
 
+// The folded slot table of the dense force in limbs: a warp per row, lane m = |n|.  Per slot the eight
+// words of k_ks_force_dense (kx as n; its unit goes into the row's factor), each row scaled by powers
+// of two so that the sums over its slots stay within 1, and per row (ky, kz, dk) times its scale and the units of the integer sums.
+__global__ void __launch_bounds__(128) k_ks_fold_q(const KSpace* __restrict__ Ks, int nf) {
+  const KSpace K = Ks[blockIdx.y];
+  const int row = blockIdx.x * 4 + (threadIdx.x >> 5), m = threadIdx.x & 31;  // (row in force order)
+  if (!K.dense || K.nq == 0 || row >= K.nrows) return;
+  const int4 R = K.rows[K.frow[row]];
+  const int lo = K.kn[R.x].x, kp = R.x + m - lo, km = R.x - m - lo;
+  double2 w = make_double2(0., 0.), v = w;
+  if (m <= K.nxm && kp >= R.x && kp < R.y) w = K.kdd[kp];
+  if (m > 0 && m <= K.nxm && km >= R.x && km < R.y) v = K.kdd[km];
+  double a[8] = {w.x + v.x, w.y - v.y, w.y + v.y, v.x - w.x,
+                 m * (w.x - v.x), m * (w.y + v.y), m * (w.y - v.y), -m * (w.x + v.x)};
+  double sc[2];
+#pragma unroll
+  for (int g = 0; g < 2; ++g) {
+    double br = fabs(a[4 * g]) + fabs(a[4 * g + 1]), bi = fabs(a[4 * g + 2]) + fabs(a[4 * g + 3]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      br += __shfl_xor_sync(0xffffffffu, br, o);
+      bi += __shfl_xor_sync(0xffffffffu, bi, o);
+    }
+    const double big = fmax(br, bi);
+    // 2^-e with 2^e > big (1 for a row of zeros)
+    const int e = big > 0. ? ((__double2hiint(big) >> 20) & 0x7FF) - 1022 : 0;
+    const double down = __hiloint2double((1023 - e) << 20, 0);
+    sc[g] = __hiloint2double((1023 + e) << 20, 0);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) a[4 * g + c] *= down;
+  }
+  if (m < nf) {
+    int4* o = K.wq + ((size_t)row * nf + m) * 4;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int2 x = ql_of(a[2 * c]), y = ql_of(a[2 * c + 1]);
+      o[c] = make_int4(x.x, x.y, y.x, y.y);
+    }
+  }
+  if (m == 0) {
+    const double unit = 3.4694469519536142e-18;  // 2^-58
+    K.rowq[3 * row] = (double)(2. * M_PI) * K.cx * sc[1] * unit;
+    K.rowq[3 * row + 1] = K.kvec[3 * R.x + 1] * sc[0] * unit;
+    K.rowq[3 * row + 2] = K.kvec[3 * R.x + 2] * sc[0] * unit;
+  }
+}
+
+// The dense force in integer limbs (FP64 mode): rows, slots, windows and partials as
+// k_ks_force_dense; the sums of a row's 32 products are exact in 64 bits, and only the row's two results go to
+// FP64.  Against 80-bit arithmetic the forces are 3.5e-16 off (r.m.s., of the largest), as the FP64
+// kernels' were (3 to 15 waves, 40 to 4100 charges).
+template <int QF>
+__global__ void __launch_bounds__(KS_FB) k_ks_force_q(const KSpace* __restrict__ Ks, int nf) {
+  const KSpace K = Ks[blockIdx.z];
+  if (!K.dense || (int)blockIdx.x * KS_FB >= K.nq || (int)blockIdx.y >= K.nkchunks) return;
+  constexpr int NF = 4 * QF;
+  extern __shared__ __align__(16) unsigned char shraw[];
+  int4* Wq = reinterpret_cast<int4*>(shraw);                // [KS_FR][NF][4]
+  double* rw = reinterpret_cast<double*>(Wq + KS_FR * NF * 4);  // [KS_FR][3]
+  int2* rc = reinterpret_cast<int2*>(rw + 3 * KS_FR);       // [KS_FR] signed Y column, Z column
+  const int rbeg = blockIdx.y * KS_FR, nr = min(KS_FR, K.nrows - rbeg), nxm = K.nxm;
+  const int2 win = K.fwin[blockIdx.y];
+  const int ax = abs(win.x - nxm), ay = abs(win.y - nxm);
+  const int mlo = (win.x <= nxm && nxm <= win.y) ? 0 : min(ax, ay), mhi = max(ax, ay);
+  for (int e = threadIdx.x; e < nr * NF * 4; e += KS_FB) {
+    const int r = e / (4 * NF), m = (e >> 2) - r * NF;
+    Wq[e] = m < nf ? K.wq[((size_t)(rbeg + r) * nf + m) * 4 + (e & 3)] : make_int4(0, 0, 0, 0);
+  }
+  for (int r = threadIdx.x; r < 3 * nr; r += KS_FB) rw[r] = K.rowq[3 * rbeg + r];
+  for (int r = threadIdx.x; r < nr; r += KS_FB) {
+    const int4 R = K.rows[K.frow[rbeg + r]];
+    const int yc = nxm + 1 + abs(R.z);
+    rc[r] = make_int2(R.z < 0 ? -yc : yc, nxm + K.nym + 2 + R.w);
+  }
+  const int p = blockIdx.x * KS_FB + threadIdx.x;
+  const int4* T = K.tabq + min(p, K.nq - 1);
+  int4 X[NF];
+#pragma unroll
+  for (int j = 0; j < NF; ++j) {
+    X[j] = make_int4(0, 0, 0, 0);
+    if (j >= mlo && j <= mhi && j <= nxm) X[j] = T[(size_t)j * K.nq];
+  }
+  __syncthreads();
+  if (p >= K.nq) return;
+  double fx = 0., fy = 0., fz = 0.;
+  int2 R = rc[0];
+  int4 Y = T[(size_t)abs(R.x) * K.nq], Z = T[(size_t)R.y * K.nq];
+#pragma unroll 1
+  for (int r = 0; r < nr; ++r) {
+    if (R.x < 0) { Y.z = -Y.z; Y.w = -Y.w; }
+    const int4 YZ = ql_cmul(Y, Z);
+    if (r + 1 < nr) {  // the next row's factors, while this one is summed
+      R = rc[r + 1];
+      Y = T[(size_t)abs(R.x) * K.nq];
+      Z = T[(size_t)R.y * K.nq];
+    }
+    const int4* w = Wq + r * NF * 4;
+    QlSum sr, si, xr, xi;
+    sr.zero(); si.zero(); xr.zero(); xi.zero();
+#pragma unroll
+    for (int g = 0; g < QF; ++g) {  // (a branch per slot or two, or more blocks per SM, were 2-7 % slower)
+      if (4 * g + 3 < mlo || 4 * g > mhi) continue;
+#pragma unroll
+      for (int j = 4 * g; j < 4 * g + 4; ++j) {
+        const int4 u = w[4 * j], v = w[4 * j + 1], ux = w[4 * j + 2], vx = w[4 * j + 3];
+        const int2 c = ql_re(X[j]), d = ql_im(X[j]);
+        sr.add(c, ql_re(u)); sr.add(d, ql_im(u));
+        si.add(c, ql_re(v)); si.add(d, ql_im(v));
+        xr.add(c, ql_re(ux)); xr.add(d, ql_im(ux));
+        xi.add(c, ql_re(vx)); xi.add(d, ql_im(vx));
+      }
+    }
+    // Im(conj(Y Z) S) and Im(conj(Y Z) Sx) of the row
+    QlSum a, b;
+    a.zero();
+    b.zero();
+    const int2 yr = ql_re(YZ), yi = ql_neg(ql_im(YZ));
+    a.add(yr, ql_limbs(si.q58())); a.add(yi, ql_limbs(sr.q58()));
+    b.add(yr, ql_limbs(xi.q58())); b.add(yi, ql_limbs(xr.q58()));
+    const double srow = (double)a.q58(), sxrow = (double)b.q58();
+    fx = fma(sxrow, rw[3 * r], fx);
+    fy = fma(srow, rw[3 * r + 1], fy);
+    fz = fma(srow, rw[3 * r + 2], fz);
+  }
+  double* o = K.fpart + ((size_t)blockIdx.y * K.nq + p) * 3;
+  o[0] = fx;
+  o[1] = fy;
+  o[2] = fz;
+}
+
 // F_i = -(8 pi q_i / V) * sum over k-chunks in a fixed order, and the slab term's -4 pi q_i M_z / V
 // along z, added to the FP64 force array or, in the fused mixed-precision step, to the FP32 one.  A
 // thread per component: the partials of a chunk are read in order.
@@ -763,6 +1068,14 @@ size_t force_smem(const KSpace& K, bool mixed) {
 }
 // groups of four folded slots |nx| = 0 .. nxm of k_ks_force_dense
 int dense_qf(const KSpace& K) { return (K.nxm + 4) / 4; }
+// (the limb forms of the FP64 mode)
+size_t rho_q_smem(int nym, int zc) {
+  return ((size_t)KS_TILE * (KS_RB + 1) + 2 * (size_t)(KS_SL + nym + 1 + zc) * KS_CS) * sizeof(int4) +
+         (size_t)KS_RB * sizeof(int2);
+}
+size_t force_q_smem(int qf) {
+  return (size_t)KS_FR * (4 * qf * 4 * sizeof(int4) + 3 * sizeof(double) + sizeof(int2));
+}
 size_t dense_smem(int qf) {
   return (size_t)KS_FR * (4 * qf * 2 * sizeof(float4) + sizeof(int2) + sizeof(float2));
 }
@@ -773,16 +1086,24 @@ void launch_dense(const KSpace* Ks, size_t shm, dim3 g, int pp, cudaStream_t st)
   if (pp == 2) k_ks_force_dense<QF, 2><<<g, KS_FB, shm, st>>>(Ks);
   else k_ks_force_dense<QF, 1><<<g, KS_FB, shm, st>>>(Ks);
 }
+template <int QF>
+void launch_force_q(const KSpace* Ks, dim3 g, cudaStream_t st) {
+  k_ks_force_q<QF><<<g, KS_FB, force_q_smem(QF), st>>>(Ks, 4 * QF);
+}
+typedef void (*force_q_launcher)(const KSpace*, dim3, cudaStream_t);
+const force_q_launcher kForceQ[5] = {nullptr, launch_force_q<1>, launch_force_q<2>, launch_force_q<3>, launch_force_q<4>};
 typedef void (*dense_launcher)(const KSpace*, size_t, dim3, int, cudaStream_t);
 const dense_launcher kDense[5] = {nullptr, launch_dense<1>, launch_dense<2>, launch_dense<3>, launch_dense<4>};
-bool use_dense(const KSpace& K, bool mixed) { return mixed && K.qx <= KS_DENSE_QX_MAX; }
+bool use_dense(const KSpace& K, bool) { return K.qx <= KS_DENSE_QX_MAX; }
 }  // namespace
 
 bool kspace_dense(const KSpace& K, bool mixed) { return use_dense(K, mixed); }
 size_t kspace_force_smem(const KSpace& K, bool mixed) { return force_smem(K, mixed); }
 
 int kspace_prepare(const KSpace& K, bool mixed) {
-  const size_t a = rho_smem(K.nym, K.zc_max, mixed), b = use_dense(K, mixed) ? dense_smem(dense_qf(K)) : force_smem(K, mixed);
+  const bool q = use_dense(K, mixed) && !mixed;
+  const size_t a = q ? rho_q_smem(K.nym, K.zc_max) : rho_smem(K.nym, K.zc_max, mixed);
+  const size_t b = q ? force_q_smem(dense_qf(K)) : (use_dense(K, mixed) ? dense_smem(dense_qf(K)) : force_smem(K, mixed));
   if (a > KS_SMEM_MAX || b > KS_SMEM_MAX) return (int)cudaErrorInvalidConfiguration;
   // The opt-in is a property of the kernel for the whole process, not of a context: set it to the
   // largest allowed size once, so that no context lowers it below another's needs (occupancy
@@ -792,7 +1113,8 @@ int kspace_prepare(const KSpace& K, bool mixed) {
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ks_rho<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ks_force<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ks_force<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  return (int)e;  // dense_smem stays below 48 KB: 32 rows x 16 folded slots x 32 B + 512 B
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ks_rho_q, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
+  return (int)e;  // force_q_smem and dense_smem stay below 48 KB: 32 rows x 16 folded slots x 32 B + 512 B
 }
 
 KSpaceBatch kspace_batch(const std::vector<KSpace>& Ks, bool mixed, int nsm) {
@@ -801,15 +1123,18 @@ KSpaceBatch kspace_batch(const std::vector<KSpace>& Ks, bool mixed, int nsm) {
   long long two = 0;
   for (const KSpace& K : Ks)
     if (use_dense(K, mixed)) two += (long long)((K.nq + 2 * KS_FB - 1) / (2 * KS_FB)) * K.nkchunks;
-  B.pp = two >= 2 * nsm ? 2 : 1;
+  B.pp = mixed && two >= 2 * nsm ? 2 : 1;
   B.n = (int)Ks.size();
   for (const KSpace& K : Ks) {
     if (K.nq == 0) continue;  // no charges: every block of this replica leaves
     B.dip = std::max(B.dip, ks_dipole_blocks(K.nq));
-    B.tab = std::max(B.tab, K.nk ? (K.nq * K.ncol + KS_TAB_T - 1) / KS_TAB_T : 0);
+    const int ncol = (!mixed && use_dense(K, mixed)) ? K.ncolq : K.ncol;
+    B.tab = std::max(B.tab, K.nk ? (K.nq * ncol + KS_TAB_T - 1) / KS_TAB_T : 0);
     B.nq = std::max(B.nq, K.nq);
     if (K.nk == 0) continue;
-    B.rho_shm = std::max(B.rho_shm, rho_smem(K.nym, K.zc_max, mixed));
+    if (!mixed && use_dense(K, mixed)) B.rho_q_shm = std::max(B.rho_q_shm, rho_q_smem(K.nym, K.zc_max));
+    else B.rho_shm = std::max(B.rho_shm, rho_smem(K.nym, K.zc_max, mixed));
+    B.nrows = std::max(B.nrows, K.nrows);
     B.rows = std::max(B.rows, (K.nrows + KS_RB - 1) / KS_RB);
     B.pchunks = std::max(B.pchunks, K.npchunks);
     B.nz = std::max(B.nz, (K.nxm + KS_SL) / KS_SL);
@@ -856,11 +1181,16 @@ static int launch_ks(const DevState& s, const SimConst& C, KSpaceBatch B, cudaSt
       k_ks_rho<true><<<g1, KS_RHO_T, B.rho_shm, st>>>(B.d, B.nz);
       k_ks_rho_sum<true><<<g2, 256, 0, st>>>(B.d, 4. * pi, fac_alpha, acc, eflag);
     } else {
-      k_ks_rho<false><<<g1, KS_RHO_T, B.rho_shm, st>>>(B.d, B.nz);
+      if (B.rho_shm) k_ks_rho<false><<<g1, KS_RHO_T, B.rho_shm, st>>>(B.d, B.nz);
+      if (B.rho_q_shm) k_ks_rho_q<<<g1, KS_RHO_T, B.rho_q_shm, st>>>(B.d, B.nz);
       k_ks_rho_sum<false><<<g2, 256, 0, st>>>(B.d, 4. * pi, fac_alpha, acc, eflag);
     }
     launches += 2;
-    if (B.dense_p) {
+    if (B.dense_p && !s.mixed) {
+      k_ks_fold_q<<<dim3((B.nrows + 3) / 4, B.n), 128, 0, st>>>(B.d, 4 * B.qf);
+      kForceQ[B.qf](B.d, dim3(B.dense_p, B.dense_k, B.n), st);
+      launches += 2;
+    } else if (B.dense_p) {
       kDense[B.qf](B.d, dense_smem(B.qf), dim3(B.dense_p, B.dense_k, B.n), B.pp, st);
       ++launches;
     }

@@ -72,6 +72,7 @@ struct DevState {
   const PairEntry<float>* tabf;
   const PairEntry<double>* tabd;
   const NoiseTab* noise;  // FP64 mode
+  const CoulTab* coul;    // FP64 mode, charged, where a table serves (0: none)
 };
 
 // energy accumulators: slot-major [NOBS][nrep], `copies` of them one after another.  obs_push adds
@@ -224,6 +225,12 @@ struct KSpace {
   double* kfac;         // [nk] exp(-k^2/(4 alpha_c)) / k^2
   float2* tabf;         // [ncol][nq] (mixed): X(0..nxm), Y(0..nym), Z(0..nzm) per particle
   double2* tabd;        // [ncol][nq] (fp64)
+  // FP64 mode, nxm <= 15: the same in integer limbs (mfa_kspace.cu), [ncolq][nq]: X, Y, Z, q Z / qmax;
+  // the folded slots of the force [nrows][slots][4] and its factors per row [nrows][3]
+  int ncolq;
+  double qmax, inv_qmax;  // largest |charge|
+  int4 *tabq, *wq;
+  double* rowq;
   int* qtag;            // [nq] tags of the charged particles
   double* qval;         // [nq] their charges
   float* qvalf;         // [nq] the same in FP32
@@ -255,7 +262,7 @@ struct KSpace {
   double* red_part;     // [8*KS_RED_MAX]: rho_sum energy and virial (7 per block), dipole moment
   unsigned* ticket;     // [2] zero between launches
   int rep;
-  int dense;            // 1: the force in the dense kernel (kspace_dense)
+  int dense;            // 1: the dense kernels (kspace_dense); in the FP64 mode the limb forms
   int plain;            // 1: FP32 sums without Kahan compensation (mfa_options.kspace_plain_sums)
 };
 constexpr int KS_RB = 64;        // rows per rho block
@@ -263,7 +270,7 @@ constexpr int KS_FB = 128;       // particles per force block
 constexpr int KS_FR = 32;        // rows per force chunk
 constexpr int KS_RED_MAX = 256;  // blocks of a grid reduction, at most
 constexpr size_t KS_SMEM_MAX = 227 * 1024;  // dynamic shared memory of one block, at most
-// the dense force kernel (X in registers) serves mixed precision with nxm <= 15
+// the dense force kernels (X in registers) serve nxm <= 15
 bool kspace_dense(const KSpace& K, bool mixed);
 // shared memory of the one-k-at-a-time force kernel for the chunks set in K
 size_t kspace_force_smem(const KSpace& K, bool mixed);
@@ -273,7 +280,8 @@ int kspace_prepare(const KSpace& K, bool mixed);
 struct KSpaceBatch {
   const KSpace* d;  // [n] in device memory
   int n, pp, nq, dip, tab, rows, pchunks, nz, sum, dense_p, dense_k, qf, force_p, force_k;
-  size_t rho_shm, force_shm;
+  int nrows;
+  size_t rho_shm, rho_q_shm, force_shm;
 };
 KSpaceBatch kspace_batch(const std::vector<KSpace>& Ks, bool mixed, int nsm);
 // ewald_k and dipolar_correction into the FP64 force array; both at once, as the fused step takes
