@@ -6,13 +6,16 @@
 //            Philox draw keyed on (seed, step, min tag, max tag) so both sides see the same g and
 //            momentum is conserved exactly in exact arithmetic.  Energies are halved per visit
 //            (a fixed wall bead has no list: its pairs count in full).
-//            MIXED: positions are fixed-point int4 (the int32 difference is the x,y minimum image),
+//            k_pair is the mixed mode's: positions are fixed-point int4 (the int32 difference is the x,y minimum image),
 //            all pair arithmetic is FP32.  In the fused mixed step the FP32 partial sums over each
 //            batch of kept pairs go into an FP64 per-particle total, with the particle's bonded
 //            terms (evaluated by the same thread), its 9-3 wall force and the body force; in the
 //            drop-in the FP32 sum is added to the FP64 force.  With a single cut-off for every
 //            type pair the screening compares against one constant (UNI).  With energies, the
 //            pair, bond, angle and wall virial is summed as well.
+// k_pair_lanes : the same for systems too small to fill the GPU with a thread per particle: eight
+//            lanes per particle, the same bits.
+// k_pair64 : the same in FP64 mode: FP32 screening, kept pairs of a warp put together.
 // k_bonded : intra_molec.f90:16-188 (FENE), bending.f90:19-121 / bending_melt.f90:22-108 and
 //            orientation.f90:24-88.  Owner computes: the thread of bead m evaluates every bond,
 //            angle and orientation term that acts on m (terms centred on m-1, m, m+1) and adds
@@ -541,8 +544,8 @@ __device__ __forceinline__ double pair_fs64(const DevState& s, const SimConst& C
 template <bool EFLAG, bool FUSED = false, int BONDED = BOND_NONE, bool UNI = false, bool PERSIST = false,
           bool INTEG = false>
 // Resident blocks per SM: 10 for the kernel with the integration in its tail (48 registers, no spill
-// with FENE bonds alone, 52 bytes with every bonded term; 0.537 ms per step on 256 brush replicas,
-// 0.553 at 11 or 12 blocks), 9 for the other fused forms (an energy step of these replicas costs 125 us
+// with FENE bonds alone, 52 bytes with every bonded term; 0.456 ms per step on 256 brush replicas;
+// before the loads were moved ahead of their use 0.537, and 0.553 at 11 or 12 blocks), 9 for the other fused forms (an energy step of these replicas costs 125 us
 // more than a plain one; 166 at 8 blocks, 210 at 7), 8 for the persistent schedule (its tile loop
 // spills at 9).  FENE bonds alone have a variant of their own: compiled for every bonded term the
 // energy variant spilled 200 bytes and reduced 54 values per warp instead of 30 (235 us more than a
@@ -820,6 +823,8 @@ __global__ void __launch_bounds__(128, PERSIST ? 8 : ((INTEG && !EFLAG) ? 10 : 9
 // the sums are those of k_pair to the bit (batches of PAIR_BATCH kept entries, products and sums
 // rounded apart).  A warp of its own per block evaluates the bonded terms of the 32 particles
 // meanwhile and then integrates them (FUSED, BONDED, UNI, INTEG as in k_pair).
+// Measured: 17.9 -> 11.5 us at 6400 particles (WCA), 59 -> 22 at 6800 (2.24 sigma), 67 -> 35 at 33,600
+// (charged brush).
 constexpr int PL_G = 8, PL_P = 32, PL_T = PL_P * PL_G + 32;
 
 template <bool EFLAG, bool FUSED, int BONDED, bool UNI, bool INTEG>
@@ -1011,13 +1016,19 @@ static void launch_pair_lanes(const DevState& s, const SimConst& C, cudaStream_t
 
 // The pair kernel of the FP64 mode.  The FP64 pipe bounds it (an FP64 instruction of a warp holds it
 // for 16 clocks however many lanes are active), so (1) the list is screened in FP32 on the fixed-point
-// view, (2) the kept pairs of a warp's 32 particles are put together and evaluated 32 at a time, a
+// view, (2) the kept pairs of a warp's particles are put together and evaluated 32 at a time, a
 // lane per pair whoever owns it (a thread per particle left half of the lanes idle: the kept counts
-// of neighbours differ), and (3) the roots, divisions and noise are those of mfa_dev.cuh.  The
+// of neighbours differ; 16 brush replicas 6648 -> 4146 us a call of 10 steps with (3), and 9700
+// before the screening in FP32), and (3) the roots, divisions and noise are those of mfa_dev.cuh.  The
 // products go back through shared memory and each owner adds its own in list order, so the sums do
 // not depend on which lane evaluated a pair.  A warp on a replica boundary evaluates each lane's own
 // pairs instead, so that the energy sums (by lane) stay with their replica.
-constexpr int P64_BATCH = 8;  // kept pairs per particle and round
+// With G lanes per particle (4 or 8) a warp takes 32 / G particles: their lists are screened side by
+// side, and a small system has G times as many warps, whose serial chain of loads and FP64 results is
+// what its time is then.  The kept pairs and the order of the sums are the same.  G = 1 fills the rounds
+// best (150 pairs of 32 WCA particles instead of 38 of 8).  Pair kernel, us, G = 1 / 4 / 8: WCA, 6400
+// particles 42 / 19 / 19; 2.24 sigma, 6800 213 / 77 / 73; charged, 32.5 k 247 / 138 / 132.
+constexpr int P64_BATCH = 8;  // kept pairs per lane and round
 struct Pair64Warp {           // shared memory of a warp
   double own[6][32];          // its particles' positions and half-step velocities
   double f[3][32 * P64_BATCH];  // force of each kept pair on its owner
@@ -1026,7 +1037,7 @@ struct Pair64Warp {           // shared memory of a warp
   unsigned char who[32 * P64_BATCH];
 };
 
-template <bool EFLAG, bool UNI>
+template <bool EFLAG, bool UNI, int G>
 __global__ void __launch_bounds__(128, 4) k_pair64(DevState s, SimConst C, bool accumulate, Acc acc) {
   extern __shared__ __align__(16) unsigned char sh_raw[];
   __shared__ PairEntry<double> tab[NPAIR];
@@ -1039,7 +1050,9 @@ __global__ void __launch_bounds__(128, 4) k_pair64(DevState s, SimConst C, bool 
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   Pair64Warp& W = reinterpret_cast<Pair64Warp*>(sh_raw)[threadIdx.x >> 5];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr int BATCH = P64_BATCH * G;
+  const int own = lane / G, sub = lane % G;  // the lane's particle of the warp's 32 / G
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) / G;
   const bool inside = i < s.N;
   const int w = __ldg(&s.info[min(i, s.N - 1)]);  // (the lanes past the end take the last replica)
   const bool active = inside && info_mobile(w);
@@ -1056,11 +1069,13 @@ __global__ void __launch_bounds__(128, 4) k_pair64(DevState s, SimConst C, bool 
   int4 qi = make_int4(0, 0, 0, 0);
   if (active) {
     qi = __ldg(&s.pfx[i]);
-    const dbl4 x = s.pd[i], v = s.vd[i];
-    W.own[0][lane] = x.x; W.own[1][lane] = x.y; W.own[2][lane] = x.z;
-    W.own[3][lane] = v.x; W.own[4][lane] = v.y; W.own[5][lane] = v.z;
-    W.tag[lane] = (int)__double_as_longlong(v.w) - p0;
-    W.type[lane] = ti;
+    if (sub == 0) {
+      const dbl4 x = s.pd[i], v = s.vd[i];
+      W.own[0][own] = x.x; W.own[1][own] = x.y; W.own[2][own] = x.z;
+      W.own[3][own] = v.x; W.own[4][own] = v.y; W.own[5][own] = v.z;
+      W.tag[own] = (int)__double_as_longlong(v.w) - p0;
+      W.type[own] = ti;
+    }
   }
   const float cx = R.ufx_f[0] * 512.f, cy = R.ufx_f[1] * 512.f, cz = R.ufx_f[2] * 512.f;
   auto screen = [&](int j) -> bool {  // as the mixed kernel's
@@ -1074,29 +1089,53 @@ __global__ void __launch_bounds__(128, 4) k_pair64(DevState s, SimConst C, bool 
   double wv[6] = {0., 0., 0., 0., 0., 0.};  // EFLAG: pair virial, xx yy zz xy xz yz
   int k = 0;
   while (__any_sync(FULL, k < n)) {
-    // the lane's next kept pairs, at most P64_BATCH, first in its own row of W.j
+    // the particle's next kept pairs, at most BATCH, first in its own row of W.j
     int m = 0;
-    while (k < n && m < P64_BATCH) {
-      constexpr int G = 4;  // entries whose loads are in flight together
-      if (k + G <= n && m <= P64_BATCH - G) {
-        int jg[G];
-        bool hg[G];
+    if constexpr (G == 1) {
+      while (k < n && m < BATCH) {
+        constexpr int F = 4;  // entries whose loads are in flight together
+        if (k + F <= n && m <= BATCH - F) {
+          int jg[F];
+          bool hg[F];
 #pragma unroll
-        for (int u = 0; u < G; ++u) jg[u] = __ldg(nb + (size_t)(k + u) * s.Np);
+          for (int u = 0; u < F; ++u) jg[u] = __ldg(nb + (size_t)(k + u) * s.Np);
 #pragma unroll
-        for (int u = 0; u < G; ++u) hg[u] = screen(jg[u]);
+          for (int u = 0; u < F; ++u) hg[u] = screen(jg[u]);
 #pragma unroll
-        for (int u = 0; u < G; ++u)
-          if (hg[u]) W.j[lane * P64_BATCH + m++] = jg[u];
-        k += G;
-      } else {
-        const int j = __ldg(nb + (size_t)k * s.Np);
-        ++k;
-        if (screen(j)) W.j[lane * P64_BATCH + m++] = j;
+          for (int u = 0; u < F; ++u)
+            if (hg[u]) W.j[lane * BATCH + m++] = jg[u];
+          k += F;
+        } else {
+          const int j = __ldg(nb + (size_t)k * s.Np);
+          ++k;
+          if (screen(j)) W.j[lane * BATCH + m++] = j;
+        }
       }
+    } else {
+      constexpr int F = 2;  // G entries at a time, F of these in flight together
+      while (__any_sync(FULL, k < n && m <= BATCH - F * G)) {
+        const bool room = m <= BATCH - F * G;
+        int jg[F];
+        bool hg[F];
+#pragma unroll
+        for (int u = 0; u < F; ++u) {
+          const int e = k + u * G + sub;
+          jg[u] = room && e < n ? __ldg(nb + (size_t)e * s.Np) : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < F; ++u) hg[u] = jg[u] >= 0 && screen(jg[u]);
+#pragma unroll
+        for (int u = 0; u < F; ++u) {
+          const unsigned bits = (__ballot_sync(FULL, hg[u]) >> (own * G)) & ((1u << G) - 1u);
+          if (hg[u]) W.j[own * BATCH + m + __popc(bits & ((1u << sub) - 1u))] = jg[u];
+          m += __popc(bits);
+        }
+        if (room) k += F * G;
+      }
+      __syncwarp();
     }
     // then together: owner after owner, each in list order
-    int at = m;
+    int at = sub == 0 ? m : 0;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int y = __shfl_up_sync(FULL, at, o);
@@ -1106,19 +1145,19 @@ __global__ void __launch_bounds__(128, 4) k_pair64(DevState s, SimConst C, bool 
     at -= m;
     int mine[P64_BATCH];
 #pragma unroll
-    for (int t = 0; t < P64_BATCH; ++t) mine[t] = (t < m) ? W.j[lane * P64_BATCH + t] : 0;
+    for (int t = 0; t < P64_BATCH; ++t) mine[t] = (t * G + sub < m) ? W.j[own * BATCH + t * G + sub] : 0;
     __syncwarp();
 #pragma unroll
     for (int t = 0; t < P64_BATCH; ++t)
-      if (t < m) {
-        W.j[at + t] = mine[t];
-        W.who[at + t] = (unsigned char)lane;
+      if (t * G + sub < m) {
+        W.j[at + t * G + sub] = mine[t];
+        W.who[at + t * G + sub] = (unsigned char)own;
       }
     __syncwarp();
-    const int rounds = one ? (total + 31) >> 5 : (int)__reduce_max_sync(FULL, (unsigned)m);
+    const int rounds = one ? (total + 31) >> 5 : ((int)__reduce_max_sync(FULL, (unsigned)m) + G - 1) / G;
     for (int t = 0; t < rounds; ++t) {
-      const int q = one ? 32 * t + lane : at + t;
-      if (one ? q < total : t < m) {
+      const int q = one ? 32 * t + lane : at + t * G + sub;
+      if (one ? q < total : t * G + sub < m) {
         const int j = W.j[q], o = W.who[q];
         const dbl4 pj = s.pd[j];
         const double dx = mic_fast(W.own[0][o] - pj.x, L0, iL0);
@@ -1136,23 +1175,33 @@ __global__ void __launch_bounds__(128, 4) k_pair64(DevState s, SimConst C, bool 
       }
     }
     __syncwarp();
-    for (int t = 0; t < m; ++t) {
-      fx += W.f[0][at + t];
-      fy += W.f[1][at + t];
-      fz += W.f[2][at + t];
+    if constexpr (G == 1) {
+      for (int t = 0; t < m; ++t) {
+        fx += W.f[0][at + t];
+        fy += W.f[1][at + t];
+        fz += W.f[2][at + t];
+      }
+    } else if (sub < 3) {  // (a lane per component, in fx)
+      for (int t = 0; t < m; ++t) fx += W.f[sub][at + t];
     }
     __syncwarp();
   }
-  if (inside) {
-    if (!accumulate) {
-      s.fx[i] = fx;
-      s.fy[i] = fy;
-      s.fz[i] = fz;
-    } else if (active) {
-      s.fx[i] += fx;
-      s.fy[i] += fy;
-      s.fz[i] += fz;
+  if constexpr (G == 1) {
+    if (inside) {
+      if (!accumulate) {
+        s.fx[i] = fx;
+        s.fy[i] = fy;
+        s.fz[i] = fz;
+      } else if (active) {
+        s.fx[i] += fx;
+        s.fy[i] += fy;
+        s.fz[i] += fz;
+      }
     }
+  } else if (inside && sub < 3) {
+    double* f = sub == 0 ? s.fx : (sub == 1 ? s.fy : s.fz);
+    if (!accumulate) f[i] = fx;
+    else if (active) f[i] += fx;
   }
   if (EFLAG) {
     int sl[8];
@@ -1209,12 +1258,23 @@ void launch_pair(const DevState& s, const SimConst& C, cudaStream_t st, bool acc
     else k_pair<false><<<g, B, 0, st>>>(s, C, true, acc);
   } else {
     using KernT = void (*)(DevState, SimConst, bool, Acc);
-    const KernT kd[2][2] = {{k_pair64<false, false>, k_pair64<true, false>},
-                            {k_pair64<false, true>, k_pair64<true, true>}};
+#define PAIR64(G) {{k_pair64<false, false, G>, k_pair64<true, false, G>}, {k_pair64<false, true, G>, k_pair64<true, true, G>}}
+    const KernT kd[3][2][2] = {PAIR64(1), PAIR64(4), PAIR64(8)};
+#undef PAIR64
+    // Lanes per particle by the particles and the lists' length (their capacity: 61 entries with the WCA
+    // cut-off, 180 with 2.24 sigma, 284 with a Coulomb cut-off of 3; an explicit block size asks for one).
+    // 4 lanes / one took, us: WCA 35 / 43 at 19.6 k, 62 / 61 at 40 k, 107 / 89 at 78 k; 2.24 sigma 202 / 244
+    // at 21 k, 682 / 716 at 83 k, 2471 / 2485 at 333 k; charged 138 / 247 at 32 k, 384 / 474 at 130 k.
+    // 8 lanes / 4: WCA 12 / 17 at 2.3 k, 19 / 19 at 6.4 k, 42 / 35 at 20 k; 2.24 sigma 73 / 77 at 6.8 k, 207 / 202
+    // at 21 k; charged 80 / 96 at 16 k, 132 / 138 at 32 k, 223 / 216 at 64 k;
+    // explicit walls 23 / 21 at 7200.
+    const bool given = block == 32 || block == 64 || block == 128;
+    const int lg = given || s.N > 10ll * s.nbr_cap * s.nbr_cap ? 0 : (s.N > 60ll * s.nbr_cap ? 1 : 2);
+    const long long threads = (long long)s.N * (lg == 0 ? 1 : (lg == 1 ? 4 : 8));
     // the warps are independent: one per block while that leaves SMs without a full block of four
-    const int B64 = (block == 32 || block == 64 || block == 128) ? block : (s.N < 128 * 4 * s.nsm ? 32 : 128);
-    kd[uni ? 1 : 0][eflag ? 1 : 0]<<<(s.N + B64 - 1) / B64, B64, B64 / 32 * sizeof(Pair64Warp), st>>>(s, C, accumulate,
-                                                                                                   acc);
+    const int B64 = given ? block : (threads < 128ll * 4 * s.nsm ? 32 : 128);
+    kd[lg][uni ? 1 : 0][eflag ? 1 : 0]<<<(int)((threads + B64 - 1) / B64), B64, B64 / 32 * sizeof(Pair64Warp), st>>>(
+        s, C, accumulate, acc);
   }
 }
 
