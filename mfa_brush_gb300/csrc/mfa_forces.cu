@@ -71,8 +71,8 @@ __device__ __forceinline__ void bead_delta(const BeadPos<MIXED>& a, const BeadPo
     d[1] = i2f_fast(fx_diff(a.q.y, b.q.y)) * R.ufx_f[1];
     d[2] = i2f_fast(fx_diff(a.q.z, b.q.z)) * R.ufx_f[2];
   } else {
-    d[0] = mic_ref(a.x - b.x, R.L[0], R.invL[0]);
-    d[1] = mic_ref(a.y - b.y, R.L[1], R.invL[1]);
+    d[0] = mic_fast(a.x - b.x, R.L[0], R.invL[0]);
+    d[1] = mic_fast(a.y - b.y, R.L[1], R.invL[1]);
     d[2] = a.z - b.z;
   }
 }
@@ -190,11 +190,12 @@ struct BondVir {
 // or more beads.
 template <bool MIXED, bool EFLAG, bool FENE_ONLY = false>
 __device__ __forceinline__ bool bonded_of(const DevState& s, const SimConst& C, int mask, int i, int w,
-                                          real_t<MIXED>* F, real_t<MIXED>* e4, BondVir<real_t<MIXED>>* bv) {
+                                          real_t<MIXED>* F, real_t<MIXED>* e4, BondVir<real_t<MIXED>>* bv,
+                                          int tag = -1) {
   using real = real_t<MIXED>;
   const RepDesc& R = s.reps[info_rep(w)];
   int kind = -1, m = 0, n = 0;
-  const int t = __ldg(&s.tag[i]);
+  const int t = tag >= 0 ? tag : __ldg(&s.tag[i]);
   const int lt = t - R.p0;
   if (lt < R.part_init_d) {
     kind = 0; n = R.n_mon; m = lt % n;
@@ -357,18 +358,24 @@ constexpr int BOND_NONE = 0, BOND_FENE = 1, BOND_ALL = 2;
 inline int bond_kind(int mask) { return mask == 0 ? BOND_NONE : (mask == 1 ? BOND_FENE : BOND_ALL); }
 constexpr int bond_values(int bonded) { return bonded == BOND_ALL ? 31 : (bonded == BOND_FENE ? 7 : 0); }
 
+// A thread per tag (by_tag) in larger systems: the beads of a chain are consecutive tags, so the warps
+// that work are full and those of the solvent leave (by slot nearly every warp holds a few chain beads,
+// and an FP64 instruction takes the same time for them).  16 brush replicas in FP64, 291 k particles, by
+// slot / by tag: 42 / 30 us; charged brush, 33.6 k: 12.7 / 11.2.  A small system waits for the longer chain
+// of loads instead (its slot comes first): 7200 particles 45.5 / 47.5 us a step.
 template <bool MIXED, bool EFLAG>
-__global__ void __launch_bounds__(128) k_bonded(DevState s, SimConst C, int mask, Acc acc, bool to_f4) {
+__global__ void __launch_bounds__(128) k_bonded(DevState s, SimConst C, int mask, Acc acc, bool to_f4,
+                                                   bool by_tag) {
   using real = real_t<MIXED>;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool inside = i < s.N;
-  const int w = inside ? __ldg(&s.info[i]) : 0;
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool inside = g < s.N;
+  const int i = inside ? (by_tag ? __ldg(&s.slot_of_tag[g]) : g) : 0, w = inside ? __ldg(&s.info[i]) : 0;
   const int rep = info_rep(w);
   real F[3] = {0, 0, 0};
   real e4[4] = {0, 0, 0, 0};
   BondVir<real> bv;
   if (EFLAG) bv.zero();
-  const bool has = inside && info_mobile(w) && bonded_of<MIXED, EFLAG>(s, C, mask, i, w, F, e4, &bv);
+  const bool has = inside && info_mobile(w) && bonded_of<MIXED, EFLAG>(s, C, mask, i, w, F, e4, &bv, by_tag ? g : -1);
   if (has) {
     if (MIXED && to_f4) {  // fused step: FP32 force array
       float4 f = s.f4[i];
@@ -1282,12 +1289,13 @@ void launch_bonded(const DevState& s, const SimConst& C, cudaStream_t st, int ma
                    bool fused) {
   if (!mask) return;
   int B = 128, g = (s.N + B - 1) / B;
+  const bool by_tag = s.N > B * s.nsm;  // (more than four warps per SM)
   if (s.mixed) {
-    if (eflag) k_bonded<true, true><<<g, B, 0, st>>>(s, C, mask, acc, fused);
-    else k_bonded<true, false><<<g, B, 0, st>>>(s, C, mask, acc, fused);
+    if (eflag) k_bonded<true, true><<<g, B, 0, st>>>(s, C, mask, acc, fused, by_tag);
+    else k_bonded<true, false><<<g, B, 0, st>>>(s, C, mask, acc, fused, by_tag);
   } else {
-    if (eflag) k_bonded<false, true><<<g, B, 0, st>>>(s, C, mask, acc, false);
-    else k_bonded<false, false><<<g, B, 0, st>>>(s, C, mask, acc, false);
+    if (eflag) k_bonded<false, true><<<g, B, 0, st>>>(s, C, mask, acc, false, by_tag);
+    else k_bonded<false, false><<<g, B, 0, st>>>(s, C, mask, acc, false, by_tag);
   }
 }
 
