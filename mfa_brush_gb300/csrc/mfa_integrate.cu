@@ -15,6 +15,8 @@
 //           the mixed step adds them in the pair kernel).  With energies: the kinetic energy and
 //           the kinetic tensor sum m v (x) v (viscosity.f90:20-27) of v(n).
 // All integration is FP64 in both precision modes.
+// k_profiles: histo(2), velocity_prof(2) (functions.f90:157-214,319-365), a counting sort per tile, in
+//   one pass with the step's integration when a mixed step takes both.
 #include "mfa_obs.cuh"
 #include "mfa_integ.cuh"
 

@@ -22,7 +22,9 @@
 //                 slots folded together: per row S = sum conj(X) G rho and
 //                 S_x = sum conj(X) kx G rho, then Im(conj(Y Z) S_x) to F_x and ky, kz times
 //                 Im(conj(Y Z) S) to F_y, F_z; rows added with Kahan compensation;
-//   k_ks_force:   the same per row, one k at a time from shared memory (FP64, or nxm > 15);
+//   k_ks_force:   the same per row, one k at a time from shared memory (nxm > 15);
+//   k_ks_rho_q, k_ks_fold_q, k_ks_force_q: rho, the folded table and the dense force of the FP64 mode
+//                 for nxm <= 15, in two-limb integers;
 //   k_ks_force_sum: the chunk partials in a fixed order, times -8 pi q / V, into the force array.
 // dipolar_correction.f90:20-33 (Yeh-Berkowitz slab term), FP64: the moment in blocks of its own of
 // k_ks_tables, the force in k_ks_force_sum.
