@@ -360,7 +360,7 @@ constexpr int bond_values(int bonded) { return bonded == BOND_ALL ? 31 : (bonded
 
 // A thread per tag (by_tag) in larger systems: the beads of a chain are consecutive tags, so the warps
 // that work are full and those of the solvent leave (by slot nearly every warp holds a few chain beads,
-// and an FP64 instruction takes the same time for them).  16 brush replicas in FP64, 291 k particles, by
+// and an FP64 instruction takes the same time for them).  16 brush replicas in FP64, 243 k particles, by
 // slot / by tag: 42 / 30 us; charged brush, 33.6 k: 12.7 / 11.2.  A small system waits for the longer chain
 // of loads instead (its slot comes first): 7200 particles 45.5 / 47.5 us a step.
 template <bool MIXED, bool EFLAG>
@@ -1026,7 +1026,7 @@ static void launch_pair_lanes(const DevState& s, const SimConst& C, cudaStream_t
 // view, (2) the kept pairs of a warp's particles are put together and evaluated 32 at a time, a
 // lane per pair whoever owns it (a thread per particle left half of the lanes idle: the kept counts
 // of neighbours differ; 16 brush replicas 6648 -> 4146 us a call of 10 steps with (3), and 9700
-// before the screening in FP32), and (3) the roots, divisions and noise are those of mfa_dev.cuh.  The
+// before the screening in FP32; 3824 now), and (3) the roots, divisions and noise are those of mfa_dev.cuh.  The
 // products go back through shared memory and each owner adds its own in list order, so the sums do
 // not depend on which lane evaluated a pair.  A warp on a replica boundary evaluates each lane's own
 // pairs instead, so that the energy sums (by lane) stay with their replica.
@@ -1278,8 +1278,9 @@ void launch_pair(const DevState& s, const SimConst& C, cudaStream_t st, bool acc
     const bool given = block == 32 || block == 64 || block == 128;
     const int lg = given || s.N > 10ll * s.nbr_cap * s.nbr_cap ? 0 : (s.N > 60ll * s.nbr_cap ? 1 : 2);
     const long long threads = (long long)s.N * (lg == 0 ? 1 : (lg == 1 ? 4 : 8));
-    // the warps are independent: one per block while that leaves SMs without a full block of four
-    const int B64 = given ? block : (threads < 128ll * 4 * s.nsm ? 32 : 128);
+    // the warps are independent, so one per block: with four the slowest holds the others' place (16 brush
+    // replicas, 128 / 64 / 32 threads: 243 / 238 / 237 us; 1 M particles 911 / 890 / 886)
+    const int B64 = given ? block : 32;
     kd[lg][uni ? 1 : 0][eflag ? 1 : 0]<<<(int)((threads + B64 - 1) / B64), B64, B64 / 32 * sizeof(Pair64Warp), st>>>(
         s, C, accumulate, acc);
   }
