@@ -419,14 +419,30 @@ int setup_kspace(mfa_ctx* ctx, const int32_t* a_type, int rep) {
     krow[k] = (int)rows.size() - 1;
   }
   K.nrows = (int)rows.size();
-  for (int r = 0; r < K.nrows; r += KS_RB)
-    K.zc_max = std::max(K.zc_max, rows[std::min(r + KS_RB, K.nrows) - 1].w - rows[r].w + 1);
   // slots of a row: nx = -nxm .. -nxm + 4 qx - 1 (the dense slot table of the force kernel)
   K.qx = (2 * nx + 1 + 3) / 4;
   // force chunks of whole rows: KS_FR for the dense kernel; for the one-k-at-a-time kernel as
   // many as let its shared-memory tables fit (the X table alone grows with nxm)
   const bool dense = kspace_dense(K, ctx->S.mixed);
   K.dense = dense ? 1 : 0;
+  // the Y and Z columns of each rho block (in the limb tables Z is q Z, behind the others)
+  const int nblk = (K.nrows + KS_RB - 1) / KS_RB, zcol = (!ctx->S.mixed && dense) ? K.ncol : nx + ny + 2;
+  std::vector<int> bcol((size_t)nblk * KS_BC), bncol(nblk);
+  std::vector<int2> rloc(K.nrows);
+  for (int b = 0; b < nblk; ++b) {
+    std::map<int, int> at;  // column -> place among the block's
+    auto place = [&](int col) {
+      const auto it = at.emplace(col, (int)at.size()).first;
+      bcol[(size_t)b * KS_BC + it->second] = col;
+      return KS_SL + it->second;
+    };
+    for (int r = b * KS_RB; r < std::min(K.nrows, (b + 1) * KS_RB); ++r) {
+      const int y = place(nx + 1 + std::abs(rows[r].z));
+      rloc[r] = make_int2(rows[r].z < 0 ? -y : y, place(zcol + rows[r].w));
+    }
+    bncol[b] = (int)at.size();
+    K.yz_max = std::max(K.yz_max, bncol[b]);
+  }
   std::vector<int> chunk_row;
   for (int frows = KS_FR;; frows /= 2) {
     chunk_row.clear();
@@ -482,6 +498,9 @@ int setup_kspace(mfa_ctx* ctx, const int32_t* a_type, int rep) {
   DA(K.frow, K.nrows);
   DA(K.fpos, K.nrows);
   DA(K.fwin, K.nkchunks);
+  DA(K.bcol, bcol.size());
+  DA(K.bncol, nblk);
+  DA(K.rloc, K.nrows);
   DA(K.rho_part, (size_t)K.npchunks * 2 * K.nk);
   DA(K.fpart, (size_t)K.nkchunks * std::max(K.nq, 1) * 3);
   DA(K.red_part, 8 * KS_RED_MAX);
@@ -513,6 +532,9 @@ int setup_kspace(mfa_ctx* ctx, const int32_t* a_type, int rep) {
   CK(cudaMemcpyAsync(K.frow, frow.data(), sizeof(int) * K.nrows, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(K.fpos, fpos.data(), sizeof(int) * K.nrows, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(K.fwin, fwin.data(), sizeof(int2) * K.nkchunks, cudaMemcpyHostToDevice, st));
+  CK(cudaMemcpyAsync(K.bcol, bcol.data(), sizeof(int) * bcol.size(), cudaMemcpyHostToDevice, st));
+  CK(cudaMemcpyAsync(K.bncol, bncol.data(), sizeof(int) * nblk, cudaMemcpyHostToDevice, st));
+  CK(cudaMemcpyAsync(K.rloc, rloc.data(), sizeof(int2) * K.nrows, cudaMemcpyHostToDevice, st));
   CK(cudaMemsetAsync(K.ticket, 0, 2 * sizeof(unsigned), st));
   if (K.wdense) CK(cudaMemsetAsync(K.wdense, 0, sizeof(float4) * K.nrows * 4 * K.qx, st));
   if (K.nq) {

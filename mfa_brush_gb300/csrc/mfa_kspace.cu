@@ -164,10 +164,10 @@ constexpr int KS_TILE = 32;  // particles per shared-memory tile of k_ks_rho (on
 // Slots outside a row's k-range are computed and not stored.  The table columns that the block's
 // rows and slots use are copied a tile ahead (cp.async); the A of a tile is formed from them.  (Read
 // from global memory when the tile began, their latency stood before every tile: with the packed
-// sums 57 -> 39 us on the charged brush.)
+// sums 57 -> 39 us on the charged brush.)  The Y and Z columns are those that the 64 rows name (K.bcol),
+// at most 128: they fit in shared memory however long the box is.
 constexpr int KS_RHO_T = 256;  // threads of a k_ks_rho block (8 warps)
 constexpr int KS_RW = 8;       // rows per warp (four per half-warp)
-constexpr int KS_SL = 16;      // |nx| slots per block
 constexpr int KS_CS = KS_TILE + 1;  // column stride (odd: 16 slots of one particle are 16 banks apart)
 constexpr int KS_AS = KS_RB + 2;  // A row stride (16-byte aligned rows)
 static_assert(KS_TILE * KS_AS * sizeof(float2) % 16 == 0, "the columns follow the A rows 16-byte aligned");
@@ -183,7 +183,8 @@ __global__ void __launch_bounds__(KS_RHO_T, MIXED ? 3 : 1) k_ks_rho(const KSpace
   extern __shared__ __align__(16) unsigned char shraw[];
   Cx* As = reinterpret_cast<Cx*>(shraw);              // [KS_TILE][KS_AS]
   int2* rc = reinterpret_cast<int2*>(As + KS_TILE * KS_AS);  // [KS_RB] signed Y column, Z column (of a tile)
-  Cx* cols = reinterpret_cast<Cx*>(rc + KS_RB);       // two tiles of columns: 16 X, the Y, the block's Z
+  int* bc = reinterpret_cast<int*>(rc + KS_RB);       // [KS_BC] the block's Y and Z columns
+  Cx* cols = reinterpret_cast<Cx*>(bc + KS_BC);       // two tiles of columns: 16 X, the block's Y and Z
   const Cx* tab = ktab<MIXED>(K);
   const int rbeg = blockIdx.x * KS_RB, nr = min(KS_RB, K.nrows - rbeg);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4;
@@ -192,13 +193,10 @@ __global__ void __launch_bounds__(KS_RHO_T, MIXED ? 3 : 1) k_ks_rho(const KSpace
   const int slot = zs * KS_SL + (lane & (KS_SL - 1));  // |nx| of the lane
   const int r0 = warp * KS_RW + half * RL;             // the lane's first row
   const bool act = r0 < nr;
-  // (rows come kz outer: the block's Z columns are one range)
-  const int zlo = K.rows[rbeg].w, nzc = K.rows[rbeg + nr - 1].w - zlo + 1, ncols = KS_SL + K.nym + 1 + nzc;
-  for (int r = threadIdx.x; r < nr; r += KS_RHO_T) {
-    const int4 R = K.rows[rbeg + r];
-    const int yc = KS_SL + abs(R.z);
-    rc[r] = make_int2(R.z < 0 ? -yc : yc, KS_SL + K.nym + 1 + R.w - zlo);
-  }
+  const int ncols = KS_SL + K.bncol[blockIdx.x];
+  for (int c = threadIdx.x; c < ncols - KS_SL; c += KS_RHO_T) bc[c] = K.bcol[blockIdx.x * KS_BC + c];
+  for (int r = threadIdx.x; r < nr; r += KS_RHO_T) rc[r] = K.rloc[rbeg + r];
+  __syncthreads();
   const int p_beg = blockIdx.y * K.pchunk, p_end = min(K.nq, p_beg + K.pchunk);
   auto fetch = [&](int t0, int buf) {
     const int pq = t0 + lane;
@@ -206,8 +204,7 @@ __global__ void __launch_bounds__(KS_RHO_T, MIXED ? 3 : 1) k_ks_rho(const KSpace
       Cx* to = cols + buf * ncols * KS_CS + lane;
       for (int c = warp; c < ncols; c += NW) {
         const int n = zs * KS_SL + c;  // X column
-        const int col = c < KS_SL ? n : (c < KS_SL + K.nym + 1 ? K.nxm + 1 + c - KS_SL
-                                                               : K.nxm + K.nym + 2 + zlo + c - KS_SL - K.nym - 1);
+        const int col = c < KS_SL ? n : bc[c - KS_SL];
         if (c >= KS_SL || n <= K.nxm) cp_async(to + c * KS_CS, tab + (size_t)col * K.nq + pq);
       }
     }
@@ -344,26 +341,24 @@ __global__ void __launch_bounds__(KS_RHO_T, 2) k_ks_rho_q(const KSpace* __restri
   extern __shared__ __align__(16) unsigned char shraw[];
   int4* As = reinterpret_cast<int4*>(shraw);                 // [KS_TILE][KS_RB + 1]
   int2* rc = reinterpret_cast<int2*>(As + KS_TILE * (KS_RB + 1));
-  int4* cols = reinterpret_cast<int4*>(rc + KS_RB);          // two tiles of columns: 16 X, the Y, the block's Z
+  int* bc = reinterpret_cast<int*>(rc + KS_RB);              // [KS_BC]
+  int4* cols = reinterpret_cast<int4*>(bc + KS_BC);          // two tiles of columns: 16 X, the block's Y and Z
   const int rbeg = blockIdx.x * KS_RB, nr = min(KS_RB, K.nrows - rbeg);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4;
   constexpr int NW = KS_RHO_T / 32, RL = KS_RW / 2;
   const int slot = lane & (KS_SL - 1), r0 = warp * KS_RW + half * RL;
   const bool act = r0 < nr;
-  const int zlo = K.rows[rbeg].w, nzc = K.rows[rbeg + nr - 1].w - zlo + 1, ncols = KS_SL + K.nym + 1 + nzc;
-  for (int r = threadIdx.x; r < nr; r += KS_RHO_T) {
-    const int4 R = K.rows[rbeg + r];
-    const int yc = KS_SL + abs(R.z);
-    rc[r] = make_int2(R.z < 0 ? -yc : yc, KS_SL + K.nym + 1 + R.w - zlo);
-  }
+  const int ncols = KS_SL + K.bncol[blockIdx.x];
+  for (int c = threadIdx.x; c < ncols - KS_SL; c += KS_RHO_T) bc[c] = K.bcol[blockIdx.x * KS_BC + c];
+  for (int r = threadIdx.x; r < nr; r += KS_RHO_T) rc[r] = K.rloc[rbeg + r];
+  __syncthreads();
   const int p_beg = blockIdx.y * K.pchunk, p_end = min(K.nq, p_beg + K.pchunk);
   auto fetch = [&](int t0, int buf) {
     const int pq = t0 + lane;
     if (pq < p_end) {
       int4* to = cols + buf * ncols * KS_CS + lane;
       for (int c = warp; c < ncols; c += NW) {
-        const int col = c < KS_SL ? c : (c < KS_SL + K.nym + 1 ? K.nxm + 1 + c - KS_SL
-                                                               : K.ncol + zlo + c - KS_SL - K.nym - 1);
+        const int col = c < KS_SL ? c : bc[c - KS_SL];
         if (c >= KS_SL || c <= K.nxm) cp_async(to + c * KS_CS, K.tabq + (size_t)col * K.nq + pq);
       }
     }
@@ -1057,11 +1052,11 @@ __global__ void __launch_bounds__(128) k_ks_force_sum(DevState s, const KSpace* 
 }
 
 namespace {
-// (zc: the most Z columns that the rows of a block use)
-size_t rho_smem(int nym, int zc, bool mixed) {
-  return ((size_t)KS_TILE * KS_AS + 2 * (size_t)(KS_SL + nym + 1 + zc) * KS_CS) *
+// (yz: the most Y and Z columns that the rows of a block use)
+size_t rho_smem(int yz, bool mixed) {
+  return ((size_t)KS_TILE * KS_AS + 2 * (size_t)(KS_SL + yz) * KS_CS) *
              (mixed ? sizeof(float2) : sizeof(double2)) +
-         (size_t)KS_RB * sizeof(int2);
+         (size_t)KS_RB * sizeof(int2) + (size_t)KS_BC * sizeof(int);
 }
 size_t force_smem(const KSpace& K, bool mixed) {
   const size_t cx = mixed ? sizeof(float2) : sizeof(double2);
@@ -1071,9 +1066,9 @@ size_t force_smem(const KSpace& K, bool mixed) {
 // groups of four folded slots |nx| = 0 .. nxm of k_ks_force_dense
 int dense_qf(const KSpace& K) { return (K.nxm + 4) / 4; }
 // (the limb forms of the FP64 mode)
-size_t rho_q_smem(int nym, int zc) {
-  return ((size_t)KS_TILE * (KS_RB + 1) + 2 * (size_t)(KS_SL + nym + 1 + zc) * KS_CS) * sizeof(int4) +
-         (size_t)KS_RB * sizeof(int2);
+size_t rho_q_smem(int yz) {
+  return ((size_t)KS_TILE * (KS_RB + 1) + 2 * (size_t)(KS_SL + yz) * KS_CS) * sizeof(int4) +
+         (size_t)KS_RB * sizeof(int2) + (size_t)KS_BC * sizeof(int);
 }
 size_t force_q_smem(int qf) {
   return (size_t)KS_FR * (4 * qf * 4 * sizeof(int4) + 3 * sizeof(double) + sizeof(int2));
@@ -1104,7 +1099,7 @@ size_t kspace_force_smem(const KSpace& K, bool mixed) { return force_smem(K, mix
 
 int kspace_prepare(const KSpace& K, bool mixed) {
   const bool q = use_dense(K, mixed) && !mixed;
-  const size_t a = q ? rho_q_smem(K.nym, K.zc_max) : rho_smem(K.nym, K.zc_max, mixed);
+  const size_t a = q ? rho_q_smem(K.yz_max) : rho_smem(K.yz_max, mixed);
   const size_t b = q ? force_q_smem(dense_qf(K)) : (use_dense(K, mixed) ? dense_smem(dense_qf(K)) : force_smem(K, mixed));
   if (a > KS_SMEM_MAX || b > KS_SMEM_MAX) return (int)cudaErrorInvalidConfiguration;
   // The opt-in is a property of the kernel for the whole process, not of a context: set it to the
@@ -1134,8 +1129,8 @@ KSpaceBatch kspace_batch(const std::vector<KSpace>& Ks, bool mixed, int nsm) {
     B.tab = std::max(B.tab, K.nk ? (K.nq * ncol + KS_TAB_T - 1) / KS_TAB_T : 0);
     B.nq = std::max(B.nq, K.nq);
     if (K.nk == 0) continue;
-    if (!mixed && use_dense(K, mixed)) B.rho_q_shm = std::max(B.rho_q_shm, rho_q_smem(K.nym, K.zc_max));
-    else B.rho_shm = std::max(B.rho_shm, rho_smem(K.nym, K.zc_max, mixed));
+    if (!mixed && use_dense(K, mixed)) B.rho_q_shm = std::max(B.rho_q_shm, rho_q_smem(K.yz_max));
+    else B.rho_shm = std::max(B.rho_shm, rho_smem(K.yz_max, mixed));
     B.nrows = std::max(B.nrows, K.nrows);
     B.rows = std::max(B.rows, (K.nrows + KS_RB - 1) / KS_RB);
     B.pchunks = std::max(B.pchunks, K.npchunks);

@@ -245,7 +245,11 @@ struct KSpace {
   // The dense slot table has 4 qx slots per row, nx = -nxm .. -nxm + 4 qx - 1.
   int qx;
   int pchunk, npchunks;
-  int zc_max;           // Z columns that a block of KS_RB rows uses, at most
+  // the Y and Z table columns that a block of KS_RB rows of k_ks_rho uses [blocks][KS_BC], their number
+  // (at most yz_max), and each row's two of them [nrows] (behind the KS_SL X slots; Y signed as ny)
+  int *bcol, *bncol;
+  int2* rloc;
+  int yz_max;
   double* rho_part;     // [npchunks][2*nk] (mixed: four FP32 words per k, two per part)
   float4* kdf;          // [nk] (kx, G Re rho, G Im rho, nx + nxm as int bits)   (mixed)
   double2* kdd;         // [nk] (G Re rho, G Im rho)                              (fp64)
@@ -266,6 +270,8 @@ struct KSpace {
   int plain;            // 1: FP32 sums without Kahan compensation (mfa_options.kspace_plain_sums)
 };
 constexpr int KS_RB = 64;        // rows per rho block
+constexpr int KS_SL = 16;        // |nx| slots per rho block
+constexpr int KS_BC = 2 * KS_RB;  // Y and Z columns of its rows, at most
 constexpr int KS_FB = 128;       // particles per force block
 constexpr int KS_FR = 32;        // rows per force chunk
 constexpr int KS_RED_MAX = 256;  // blocks of a grid reduction, at most
