@@ -447,6 +447,10 @@ const char* mfa_kernel_name(int32_t fam);
    FMA chains per thread on 8 warps per SM sub-partition, best of 10 timed launches: the roof
    for the FP32-issue-bound kernels.  No counterpart in the reference (a measurement aid).    */
 int mfa_fp32_fma_peak(int32_t device, double* tflops);
+/* How often a block of the cell sort looks at the grid barrier before the sort gives up (2^21 by
+   default, about a second).  When it does, the state is lost: the call that next reads the status and
+   every later step return MFA_ERR_CUDA.  A small limit lets that path be tested. */
+int mfa_set_barrier_limit(mfa_ctx* ctx, int32_t looks);
 /* Number of kernel launches issued by the library since the context was created. */
 int mfa_launch_count(mfa_ctx* ctx, int64_t* n);
 /* Number of cell-sort + neighbour-list rebuilds since the context was created (synchronises):

@@ -207,6 +207,7 @@ SIGNATURES = {
     "mfa_kernel_times": (i32, [vp, i32, P(C.c_float), ip]),
     "mfa_kernel_name": (C.c_char_p, [i32]),
     "mfa_fp32_fma_peak": (i32, [i32, dp]),
+    "mfa_set_barrier_limit": (i32, [vp, i32]),
     "mfa_launch_count": (i32, [vp, P(i64)]),
     "mfa_rebuild_count": (i32, [vp, P(i64)]),
     "mfa_replica_rebuild_counts": (i32, [vp, P(i64)]),

@@ -128,11 +128,16 @@ void note_list_count(mfa_ctx* ctx) {
     ctx->grow_pending = true;
 }
 
+// A sort that gave up leaves the slots half-way: the context's state is lost, and nothing clears the bit.
+int sort_lost(mfa_ctx* ctx) {
+  return fail(ctx, MFA_ERR_CUDA, "the cell sort's grid barrier timed out; the context's state is lost");
+}
+
 int check_status(mfa_ctx* ctx) {
   CK(cudaStreamSynchronize(ctx->st));
   unsigned s = ctx->h_status[0];
+  if (s & ST_BARRIER) return sort_lost(ctx);
   note_list_count(ctx);
-  if (s & ST_BARRIER) return fail(ctx, MFA_ERR_CUDA, "the cell sort's grid barrier timed out");
   if (s & ST_NAN) return fail(ctx, MFA_ERR_NAN, "non-finite position detected");
   if (s & ST_OUT_OF_BOX) return fail(ctx, MFA_ERR_OUT_OF_BOX, "a particle left the channel");
   if (s & ST_NLIST_OVERFLOW) {
@@ -191,6 +196,7 @@ int poll_status(mfa_ctx* ctx) {
   const cudaError_t q = cudaEventQuery(ctx->ev_status);
   if (q == cudaErrorNotReady) return MFA_OK;
   CK(q);
+  if (ctx->h_status[0] & ST_BARRIER) return sort_lost(ctx);
   note_list_count(ctx);
   if (ctx->h_status[0] & ST_NLIST_OVERFLOW) return MFA_ERR_NLIST_OVERFLOW;
   return MFA_OK;
@@ -202,9 +208,10 @@ __global__ void k_clear_overflow(unsigned* status) {
 }
 
 // rebuild of the flagged replicas (all of them when forced); counts and clears the flags
-void rebuild(mfa_ctx* ctx, bool force) {
-  launch_rebuild(ctx->S, ctx->st, force);
+int rebuild(mfa_ctx* ctx, bool force) {
+  CK(launch_rebuild(ctx->S, ctx->st, force));
   ctx->launches += rebuild_launches();
+  return MFA_OK;
 }
 
 // Graph form of the skin check: the IF body (the rebuild kernels) runs only on steps whose
@@ -233,9 +240,11 @@ int capture_conditional_rebuild(mfa_ctx* ctx, const DevState& S) {
   CK(cudaGraphAddNode(&node, graph, deps, nullptr, nd, &cp));
   cudaGraph_t body = cp.conditional.phGraph_out[0];
   CK(cudaStreamBeginCaptureToGraph(ctx->st2, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-  launch_rebuild(S, ctx->st2, false);  // the flagged replicas (the flags stay set until its last kernel)
+  // the flagged replicas (the flags stay set until its last kernel)
+  const cudaError_t launched = launch_rebuild(S, ctx->st2, false);
   cudaGraph_t captured;
   CK(cudaStreamEndCapture(ctx->st2, &captured));
+  CK(launched);
   CK(cudaStreamUpdateCaptureDependencies(st, &node, nullptr, 1, cudaStreamSetCaptureDependencies));
   return MFA_OK;
 }
@@ -941,6 +950,7 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
   DA(S.wl_k, n_rep + 1);
   DA(S.wl_y, n_rep + 1);
   DA(S.wl_n, 5);
+  S.barrier_spins = 1 << 21;
   CK(cudaDeviceGetAttribute(&S.nsm, cudaDevAttrMultiProcessorCount, ctx->device));
   DA(S.rebuilds, 1);
   DA(S.rep_rebuilds, n_rep);
@@ -1004,6 +1014,8 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
   CK(cudaMemsetAsync(S.cell_count, 0, sizeof(int) * (cell_off + 1), st));
   CK(cudaMemsetAsync(S.pair_q, 0, sizeof(int) * 2, st));
   CK(cudaMemsetAsync(S.wl_n, 0, sizeof(int) * 5, st));
+  CK(cudaMemsetAsync(S.wl_k, 0, sizeof(int) * (n_rep + 1), st));
+  CK(cudaMemsetAsync(S.nn, 0, sizeof(int) * ctx->N, st));
   CK(cudaMemsetAsync(S.row_count, 0, sizeof(int) * row_off, st));
   CK(cudaMemsetAsync(S.plane_count, 0, sizeof(int) * plane_off, st));
   CK(cudaMemcpyAsync(S.cell_start + cell_off, &ctx->N, sizeof(int), cudaMemcpyHostToDevice, st));  // the last cell's end
@@ -1055,7 +1067,7 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
   // the pair kernel's), one block per tile
   ctx->fuse_integ = S.mixed && !ctx->kspace && !ctx->opt.separate_integrator && !S.pair_persist;
   // ---- initial sort + list, then size the list from the observed maximum ------------------------
-  rebuild(ctx, true);
+  RET(rebuild(ctx, true));
   RET(post_status(ctx));
   int rc = check_status(ctx);
   if (rc == MFA_ERR_NLIST_OVERFLOW || rc == MFA_OK) {
@@ -1075,7 +1087,7 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
       DA(S.nbr, (size_t)newcap * Nn);
       CK(cudaMemsetAsync(S.status, 0, 2 * sizeof(unsigned), st));
       ctx->h_status[0] = ctx->h_status[1] = 0;
-      rebuild(ctx, true);
+      RET(rebuild(ctx, true));
       RET(post_status(ctx));
       rc = check_status(ctx);
     }
@@ -1153,14 +1165,13 @@ int mfa_verlet_positions(mfa_ctx* ctx) {
   RET(prepare_step(ctx));
   launch_integrate(ctx->S, ctx->C, ctx->st, 0, false, false, acc_of(ctx->acc_call, ctx->nrep));
   ctx->launches += 1;
-  rebuild(ctx, false);
-  CK(cudaGetLastError());
+  RET(rebuild(ctx, false));
   return MFA_OK;
 }
 
 int mfa_check_skin(mfa_ctx* ctx, int32_t* rebuilt) {
   if (!ctx) return MFA_ERR_ARG;
-  rebuild(ctx, false);
+  RET(rebuild(ctx, false));
   CK(cudaMemcpyAsync(ctx->h_rebuilds, ctx->S.rebuilds, sizeof(long long), cudaMemcpyDeviceToHost, ctx->st));
   CK(cudaStreamSynchronize(ctx->st));
   if (rebuilt) *rebuilt = (*ctx->h_rebuilds != ctx->last_rebuilds) ? 1 : 0;
@@ -1295,12 +1306,15 @@ static int grow_lists(mfa_ctx* ctx) {
   const int seen = (int)ctx->h_status[1];
   const int newcap = std::min(NL_CAP_MAX, std::max(S.nbr_cap * 3 / 2, seen * 3 / 2 + 16));
   if (newcap <= S.nbr_cap) return MFA_OK;
+  RET(post_status(ctx));
   CK(cudaStreamSynchronize(ctx->st));
+  if (ctx->h_status[0] & ST_BARRIER) return sort_lost(ctx);  // (no list would be built)
   auto it = std::find(ctx->allocs.begin(), ctx->allocs.end(), (void*)S.nbr);
   if (it != ctx->allocs.end()) { cudaFree(*it); ctx->allocs.erase(it); }
   S.nbr = nullptr;
   DA(S.nbr, (size_t)newcap * S.Np);
   S.nbr_cap = newcap;
+  CK(cudaMemsetAsync(S.nn, 0, sizeof(int) * ctx->N, ctx->st));  // (nothing reads the new array before it is built)
   for (auto& g : ctx->graphs) cudaGraphExecDestroy(g.second.first);
   ctx->graphs.clear();
   // the overflow of the old capacity is over once the lists are rebuilt with the new one (the
@@ -1309,8 +1323,7 @@ static int grow_lists(mfa_ctx* ctx) {
   ctx->h_status[0] &= ~ST_NLIST_OVERFLOW;
   ctx->h_status[1] = 0;
   ctx->overflow_reported = false;
-  rebuild(ctx, true);
-  return MFA_OK;
+  return rebuild(ctx, true);
 }
 
 // Start of mfa_step / mfa_verlet_positions: the status of earlier calls (when it has arrived)
@@ -1387,7 +1400,11 @@ static long long issue_steps(mfa_ctx* ctx, int n, int phase, bool prof, bool obs
       }
       L += 1;  // the rebuild body's launches are not counted: they run only when triggered
     } else {
-      launch_rebuild(Sr, st, false);
+      const cudaError_t e = launch_rebuild(Sr, st, false);
+      if (e != cudaSuccess) {
+        *err = fail(ctx, MFA_ERR_CUDA, std::string("rebuild: ") + cudaGetErrorString(e));
+        return L;
+      }
       L += rebuild_launches();
     }
     const bool split = prof || (obs && ef);
@@ -1508,6 +1525,7 @@ int mfa_step(mfa_ctx* ctx, int32_t nsteps) {
   } else {
     int err = MFA_OK;
     L = issue_steps(ctx, nsteps, phase, prof, obs, false, &err);
+    if (err != MFA_OK) return err;
     CK(cudaGetLastError());
   }
   ctx->launches += L;
@@ -1592,7 +1610,7 @@ int mfa_set_state(mfa_ctx* ctx, const double* r0, const double* v, const double*
   }
   // the lists stay valid unless some particle moved more than skin/2 from the last rebuild
   launch_refresh_views(ctx->S, ctx->C, ctx->st);
-  rebuild(ctx, false);
+  RET(rebuild(ctx, false));
   return mfa_synchronize(ctx);
 }
 
@@ -1925,7 +1943,7 @@ int mfa_kernel_times(mfa_ctx* ctx, int32_t nsteps, float* mean_ms, int32_t* laun
     // the rebuild as the fused step runs it: the replicas whose skin test fired, if any
     DevState Sr = Sk;
     Sr.permute_accel = 0;
-    launch_rebuild(Sr, st, false);
+    CK(launch_rebuild(Sr, st, false));
     mark(0);
     if (ctx->fuse_integ && !ef) {
       launch_pair(Sk, C, st, false, false, acc, ctx->opt.block_size, mask, true);
@@ -1946,7 +1964,7 @@ int mfa_kernel_times(mfa_ctx* ctx, int32_t nsteps, float* mean_ms, int32_t* laun
   }
   // then a rebuild of every replica, three times
   for (int k = 0; k < 3; ++k) {
-    launch_rebuild(S, st, true);
+    CK(launch_rebuild(S, st, true));
     mark(8);
   }
   CK(cudaStreamSynchronize(st));
@@ -1966,6 +1984,16 @@ int mfa_kernel_times(mfa_ctx* ctx, int32_t nsteps, float* mean_ms, int32_t* laun
   ctx->host_steps += nsteps;
   ctx->last_source = 1;
   return post_status(ctx);
+}
+
+int mfa_set_barrier_limit(mfa_ctx* ctx, int32_t looks) {
+  if (!ctx) return MFA_ERR_ARG;
+  if (looks < 0) return fail(ctx, MFA_ERR_ARG, "set_barrier_limit: looks < 0");
+  CK(cudaStreamSynchronize(ctx->st));
+  ctx->S.barrier_spins = looks;
+  for (auto& g : ctx->graphs) cudaGraphExecDestroy(g.second.first);
+  ctx->graphs.clear();
+  return MFA_OK;
 }
 
 int mfa_launch_count(mfa_ctx* ctx, int64_t* n) {

@@ -212,8 +212,11 @@ __device__ __forceinline__ void copyback_slot(const DevState& s, int i) {
 }
 
 // Grid barrier of a cooperative launch: every block arrives at the k-th barrier (k = 1, 2, ..) on a
-// counter that the list builder's end sets back to zero.  The wait is bounded (about a second):
-// then the status word gets ST_BARRIER and the kernel returns.
+// counter that the list builder's end sets back to zero.  The wait is bounded (about a second): then
+// the status word gets ST_BARRIER and the block leaves.  A block goes on only when all have arrived, so
+// whatever a block does rests on finished phases.  The counts and the slots may then be half-way, so
+// from that on every sort and list builder leaves at once (sort_failed): the lists stay those of the
+// last complete rebuild, whose slots are in range, and the host refuses further steps.
 __device__ __forceinline__ bool grid_barrier(const DevState& s, int k) {
   __shared__ bool ok;
   __syncthreads();
@@ -224,7 +227,7 @@ __device__ __forceinline__ bool grid_barrier(const DevState& s, int k) {
     __threadfence();
     asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(cnt) : "memory");
     seen = old + 1;
-    for (int t = 0; t < (1 << 21) && seen < target; ++t)
+    for (int t = 0; t < s.barrier_spins && seen < target; ++t)
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(cnt) : "memory");
     ok = seen >= target;
     if (!ok) atomicOr(s.status, ST_BARRIER);
@@ -232,6 +235,10 @@ __device__ __forceinline__ bool grid_barrier(const DevState& s, int k) {
   }
   __syncthreads();
   return ok;
+}
+
+__device__ __forceinline__ unsigned sort_failed(const DevState& s) {
+  return *(volatile const unsigned*)s.status & ST_BARRIER;
 }
 
 // block-wide exclusive scan of v; the block's total in `total`
@@ -292,10 +299,12 @@ __device__ __forceinline__ void make_worklist(const DevState& s, bool force, Wor
 // from 79 to 36 us, of 32 brush replicas (447 k particles) from 188 to 159, of 256 (4.66 M) from 1451
 // to 1336, and a step's rebuild of the flagged ones of these 256 from 229 to 197 us.
 __global__ void __launch_bounds__(SORT_T, SORT_PER_SM) k_sort(DevState s, bool force) {
+  const unsigned failed = sort_failed(s);
   if (!force && s.rebuild_flag[0] == 0) {  // (the same for every block: the list builder's end clears it)
     if (blockIdx.x == 0 && threadIdx.x == 0) s.wl_n[0] = s.wl_k[0] = 0;
     return;
   }
+  if (__syncthreads_or(failed)) return;  // (another block of this launch may set it meanwhile)
   __shared__ int wl[5][WL_SHARED + 1];
   __shared__ int sh[SORT_T / 32];
   WorkList L;
@@ -485,6 +494,7 @@ __device__ __forceinline__ NlRow nl_row(const DevState& s, const RepDesc& R, int
 template <bool UNI, int H, int HX = H>
 __global__ void __launch_bounds__(NL_T, 8) k_nlist(DevState s) {
   constexpr int NR = (2 * H + 1) * (2 * H + 1);
+  if (sort_failed(s)) return;  // (no kernel that sets it runs beside this one: the same for every thread)
   const int nwl = s.wl_n[0], nchunks = s.wl_k[nwl];
   const int lane = threadIdx.x & 31, warp = (blockIdx.x * NL_T + threadIdx.x) >> 5, nwarps = gridDim.x * (NL_T / 32);
   __shared__ int nl_sh[NL_T * (NL_STAGE | 1)];
@@ -648,7 +658,7 @@ __global__ void __launch_bounds__(NL_T, 8) k_nlist(DevState s) {
 
 int rebuild_launches() { return 2; }
 
-void launch_rebuild(const DevState& s, cudaStream_t st, bool force) {
+cudaError_t launch_rebuild(const DevState& s, cudaStream_t st, bool force) {
   // two blocks per SM at most (what is resident together), no more than the particles fill
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(std::min((s.N + SORT_T - 1) / SORT_T, s.nsm * SORT_PER_SM));
@@ -659,7 +669,8 @@ void launch_rebuild(const DevState& s, cudaStream_t st, bool force) {
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, k_sort, s, force);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_sort, s, force);
+  if (e != cudaSuccess) return e;
   const int uni = s.rl2_uni > 0.f ? 1 : 0;
   using KernT = void (*)(DevState);
   const KernT kerns[3][2] = {{k_nlist<false, 1>, k_nlist<true, 1>},
@@ -670,6 +681,7 @@ void launch_rebuild(const DevState& s, cudaStream_t st, bool force) {
   const KernT kern = (s.nl_hx != s.nl_h) ? kx[s.nl_hx - 2][uni] : kerns[s.nl_h - 1][uni];
   const int gl = std::min((s.N * NL_G + NL_T - 1) / NL_T, s.nsm * 8);
   kern<<<gl, NL_T, 0, st>>>(s);
+  return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------------------------

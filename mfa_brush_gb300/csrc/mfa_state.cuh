@@ -62,6 +62,7 @@ struct DevState {
   // [nrep + 1]; wl_n: their number, the list builder's chunk queue and its finished blocks, whether
   // a cell is denser than its bucket, the sort's barrier counter (the last three 0 between rebuilds)
   int *wl_rep, *wl_p, *wl_c, *wl_y, *wl_k, *wl_n;
+  int barrier_spins;          // looks at the sort's grid barrier before a block gives up
   int nsm;                    // streaming multiprocessors of the device (grids of the rebuild)
   long long* rebuilds;        // [1] rebuild events (any replica)
   long long* rep_rebuilds;    // [nrep] rebuilds of each replica
@@ -158,7 +159,7 @@ __device__ __forceinline__ void sym_add(T* w6, T c, T dx, T dy, T dz) {
 // ---- rebuild (cell sort + neighbour list) --------------------------------------------------------
 // Rebuilds the replicas whose flag is set (every replica when `force`), then counts the rebuild
 // and clears the flags.
-void launch_rebuild(const DevState& s, cudaStream_t st, bool force);
+cudaError_t launch_rebuild(const DevState& s, cudaStream_t st, bool force);
 int rebuild_launches();  // kernels of one rebuild
 // The skin test's outcome for replica `rep` (check_skin.f90:11-24 decides per system).
 __device__ __forceinline__ void flag_rebuild(const DevState& s, int rep) {
