@@ -511,9 +511,10 @@ __device__ __forceinline__ double pair_fs64(const DevState& s, const SimConst& C
       const double x = (r2 - T->lo) * T->inv_h, z = x + 4503599627370496.0;  // 2^52: rounds to an integer
       int k = __double2loint(z);
       double t = x - (z - 4503599627370496.0);  // [-1/2, 1/2] from the nearest edge
-      if (t < 0.) --k;
-      k = min(k, T->n - 1);
-      t = fma(2., t, t < 0. ? 1. : -1.);  // [-1, 1] inside the interval
+      // (the last doubles below hi may round onto the table's end, edge n: the interval left of it as well)
+      const bool left = t < 0. || k >= T->n;
+      if (left) --k;
+      t = fma(2., t, left ? 1. : -1.);  // [-1, 1] inside the interval
       fs += e.qq * coul_poly(T->f + 8 * (size_t)k, t);
       if (EFLAG) e_c += half * e.qq * coul_poly(T->e + 8 * (size_t)k, t);
     } else {
