@@ -130,6 +130,10 @@ struct QlSum {
   // units of 2^-58, for sums below 16
   __device__ __forceinline__ long long q58() const { return (h << 4) + ((m + (1ll << 25)) >> 26); }
 };
+// The high limb of a number that is not finite: in a q Z column it marks the particle, and what its
+// chunk sums (k_ks_rho_q) is then NaN, as a sum in floating point would be.
+constexpr int QL_NAN = (int)0x80000000;
+__device__ __forceinline__ bool nonfinite(double v) { return (__double2hiint(v) & 0x7FF00000) == 0x7FF00000; }
 __device__ __forceinline__ int2 ql_neg(int2 a) { return make_int2(-a.x, -a.y); }
 // the limbs of t units of 2^-58, |t| <= 2^58
 __device__ __forceinline__ int2 ql_limbs(long long t) {
@@ -371,6 +375,7 @@ __global__ void __launch_bounds__(KS_RHO_T, 2) k_ks_rho_q(const KSpace* __restri
   for (int a = 0; a < 4; ++a)
 #pragma unroll
     for (int i = 0; i < RL; ++i) tot[a][i] = 0;
+  int bad = 0;  // a particle that is not finite (every particle of the chunk comes by with the first row)
   fetch(p_beg, 0);
   int buf = 0;
   for (int t0 = p_beg; t0 < p_end; t0 += KS_TILE, buf ^= 1) {
@@ -387,7 +392,9 @@ __global__ void __launch_bounds__(KS_RHO_T, 2) k_ks_rho_q(const KSpace* __restri
           const int2 R = rc[r];
           int4 y = col[abs(R.x) * KS_CS + lane];
           if (R.x < 0) { y.z = -y.z; y.w = -y.w; }
-          As[lane * (KS_RB + 1) + r] = ql_cmul(y, col[R.y * KS_CS + lane]);
+          const int4 z = col[R.y * KS_CS + lane];
+          bad |= z.x == QL_NAN;
+          As[lane * (KS_RB + 1) + r] = ql_cmul(y, z);
         }
       }
     }
@@ -417,8 +424,9 @@ __global__ void __launch_bounds__(KS_RHO_T, 2) k_ks_rho_q(const KSpace* __restri
         for (int i = 0; i < RL; ++i) tot[a][i] += (t[a][i].q54() + 4) >> 3;
     }
   }
+  bad = __syncthreads_or(bad);
   if (act && slot <= K.nxm) {
-    const double sc = K.qmax * 4.4408920985006262e-16;  // 2^-51
+    const double sc = bad ? nan("") : K.qmax * 4.4408920985006262e-16;  // 2^-51
 #pragma unroll
     for (int i = 0; i < RL; ++i) {
       const int r = r0 + i;
@@ -544,12 +552,13 @@ __global__ void __launch_bounds__(KS_TAB_T) k_ks_tables(DevState s, const KSpace
   // bits are the phase in [-1/2, 1/2) turns.  One FP64 product; in FP64 the products, the reduction
   // and the conversions of a column bound this kernel.
   double t = (ax == 0 ? K.cx * s.rx[i] : (ax == 1 ? K.cy * s.ry[i] : K.cz * s.rz[i]));
+  bool bad = nonfinite(t);  // (the integers below know no NaN)
   if ((__double2hiint(t) & 0x7FFFFFFF) >= 0x40200000) t -= rint(t);  // (8 turns away: not wrapped yet)
   if constexpr (MIXED) {
     const unsigned long long ph = (unsigned long long)round_bits(t * 288230376151711744.0) * (unsigned)n << 6;
     float sn, cs;
     sincospif(i2f_fast((int)(ph >> 32)) * (2.f / 4294967296.f), &sn, &cs);
-    K.tabf[idx] = make_float2(cs, sn);
+    K.tabf[idx] = bad ? make_float2(nanf(""), nanf("")) : make_float2(cs, sn);
   } else if (K.dense) {
     // the same phase to 64 bits: the nearest of 1024 table angles and the angle from it by the series
     const unsigned long long ph = (unsigned long long)round_bits(t * 288230376151711744.0) * (unsigned)n << 6;
@@ -564,9 +573,10 @@ __global__ void __launch_bounds__(KS_TAB_T) k_ks_tables(DevState s, const KSpace
       const double q = K.qval[p] * K.inv_qmax;
       re *= q;
       im *= q;
+      bad = bad || nonfinite(s.rx[i]) || nonfinite(s.ry[i]);
     }
     const int2 x = ql_of(re), y = ql_of(im);
-    K.tabq[idx] = make_int4(x.x, x.y, y.x, y.y);
+    K.tabq[idx] = make_int4(bad ? QL_NAN : x.x, x.y, y.x, y.y);
   } else {
     double u = (double)n * t;
     u -= rint(u);  // turns in [-1/2, 1/2]
@@ -598,8 +608,8 @@ __global__ void __launch_bounds__(256) k_ks_rho_sum(const KSpace* __restrict__ K
       for (int c = g; c < K.npchunks; c += 8) {
         if constexpr (MIXED) {
           const float4 v = reinterpret_cast<const float4*>(K.rho_part)[(size_t)c * K.nk + k];
-          re += f2d_fast(v.x) + f2d_fast(v.y);
-          im += f2d_fast(v.z) + f2d_fast(v.w);
+          re += f2d_nan(v.x) + f2d_nan(v.y);
+          im += f2d_nan(v.z) + f2d_nan(v.w);
         } else {
           const double2 v = reinterpret_cast<const double2*>(K.rho_part)[(size_t)c * K.nk + k];
           re += v.x;
@@ -889,7 +899,7 @@ __global__ void __launch_bounds__(KS_FB) k_ks_force_dense(const KSpace* __restri
     if (p >= K.nq) return;
     double* o = K.fpart + ((size_t)blockIdx.y * K.nq + p) * 3;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) o[d] = f2d_fast(F[a][d]) - f2d_fast(Fc[a][d]);
+    for (int d = 0; d < 3; ++d) o[d] = f2d_nan(F[a][d]) - f2d_nan(Fc[a][d]);
   }
 }
 
@@ -920,7 +930,7 @@ __global__ void __launch_bounds__(128) k_ks_fold_q(const KSpace* __restrict__ Ks
     // 2^-e with 2^e > big (1 for a row of zeros)
     const int e = big > 0. ? ((__double2hiint(big) >> 20) & 0x7FF) - 1022 : 0;
     const double down = __hiloint2double((1023 - e) << 20, 0);
-    sc[g] = __hiloint2double((1023 + e) << 20, 0);
+    sc[g] = big == big ? __hiloint2double((1023 + e) << 20, 0) : big;  // (a NaN goes on in the row's factors)
 #pragma unroll
     for (int c = 0; c < 4; ++c) a[4 * g + c] *= down;
   }
