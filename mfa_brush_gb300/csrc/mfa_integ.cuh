@@ -128,8 +128,9 @@ __device__ __forceinline__ void int_mixed_particle(const DevState& s, const SimC
       const float dz = i2f_fast(fx_diff(q.z, q0.z)) * R.ufx_f[2];
       // rounded unmerged, so that the decision is the same in every kernel that makes it
       if (__fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx))) > C.skin_half2_f) flag_rebuild(s, rep);
-      const long long bx = __double_as_longlong(x), bz = __double_as_longlong(z);
-      if (((bx >> 52) & 0x7FF) == 0x7FF || ((bz >> 52) & 0x7FF) == 0x7FF) atomicOr(s.status, ST_NAN);
+      const int all1 = 0x7FF00000;  // an exponent of ones: not finite
+      if ((__double2hiint(x) & all1) == all1 || (__double2hiint(y) & all1) == all1 || (__double2hiint(z) & all1) == all1)
+        atomicOr(s.status, ST_NAN);
     }
   }
 }

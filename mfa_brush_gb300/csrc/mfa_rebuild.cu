@@ -68,9 +68,9 @@ __device__ __forceinline__ void bin_particle(const DevState& s, int i) {
     // check in FP32, as FP64 compares and the cell-height division issue on the FP64 pipe
     const double zd = s.rz[i];
     const float z = d2f_fast(zd);
-    if (!(z >= R.zlim_f[0] && z <= R.zlim_f[1]))  // also false for NaN
-      atomicOr(s.status, (__double_as_longlong(zd) & 0x7FF0000000000000ll) == 0x7FF0000000000000ll ? ST_NAN
-                                                                                                : ST_OUT_OF_BOX);
+    const int ez = (__double2hiint(zd) >> 20) & 0x7FF;  // (the conversion is right below 2^127)
+    if (ez >= 1023 + 127 || !(z >= R.zlim_f[0] && z <= R.zlim_f[1]))
+      atomicOr(s.status, ez == 0x7FF ? ST_NAN : ST_OUT_OF_BOX);
   } else {
     const double lz = 1. / R.inv_lc[2];
     const double x = s.rx[i], y = s.ry[i], z = s.rz[i];
