@@ -366,7 +366,7 @@ int make_coul_table(mfa_ctx* ctx, double r2max) {
 // ewald_k(0) (ewald_k.f90:37-124): the k-vectors in the reference's enumeration order, G(k),
 // and the list of charged particles, of replica rep (the particles p0 .. p0 + n_mon_tot - 1 of the
 // batch; a_type holds the whole batch).
-int setup_kspace(mfa_ctx* ctx, const int32_t* a_type, int rep) {
+int setup_kspace(mfa_ctx* ctx, const int32_t* a_type, int rep, std::vector<KsRowBlock>& rblk) {
   const mfa_system& s = ctx->sys[rep];
   const int p0 = ctx->hreps[rep].p0;
   const mfa_params& p = ctx->P;
@@ -434,24 +434,25 @@ int setup_kspace(mfa_ctx* ctx, const int32_t* a_type, int rep) {
   // many as let its shared-memory tables fit (the X table alone grows with nxm)
   const bool dense = kspace_dense(K, ctx->S.mixed);
   K.dense = dense ? 1 : 0;
-  // the Y and Z columns of each rho block (in the limb tables Z is q Z, behind the others)
-  const int nblk = (K.nrows + KS_RB - 1) / KS_RB, zcol = (!ctx->S.mixed && dense) ? K.ncol : nx + ny + 2;
-  std::vector<int> bcol((size_t)nblk * KS_BC), bncol(nblk);
-  std::vector<int2> rloc(K.nrows);
-  for (int b = 0; b < nblk; ++b) {
-    std::map<int, int> at;  // column -> place among the block's
-    auto place = [&](int col) {
-      const auto it = at.emplace(col, (int)at.size()).first;
-      bcol[(size_t)b * KS_BC + it->second] = col;
-      return KS_SL + it->second;
-    };
-    for (int r = b * KS_RB; r < std::min(K.nrows, (b + 1) * KS_RB); ++r) {
-      const int y = place(nx + 1 + std::abs(rows[r].z));
-      rloc[r] = make_int2(rows[r].z < 0 ? -y : y, place(zcol + rows[r].w));
+  // the row blocks of k_ks_rho
+  for (int r = 0; r < K.nrows;) {
+    KsRowBlock b = {};
+    b.row = r;
+    b.zlo = rows[r].w;
+    int lo = std::abs(rows[r].z), hi = lo;
+    for (; r < K.nrows && b.nr < KS_RB; ++r, ++b.nr) {
+      const int y = std::abs(rows[r].z), l = std::min(lo, y), h = std::max(hi, y), z = rows[r].w - b.zlo + 1;
+      if (h - l + 1 + z > KS_BC) break;
+      lo = l;
+      hi = h;
+      b.nz = z;
     }
-    bncol[b] = (int)at.size();
-    K.yz_max = std::max(K.yz_max, bncol[b]);
+    b.ylo = lo;
+    b.ny = hi - lo + 1;
+    K.yz_max = std::max(K.yz_max, b.ny + b.nz);
+    rblk.push_back(b);
   }
+  K.nrblk = (int)rblk.size();
   std::vector<int> chunk_row;
   for (int frows = KS_FR;; frows /= 2) {
     chunk_row.clear();
@@ -507,9 +508,6 @@ int setup_kspace(mfa_ctx* ctx, const int32_t* a_type, int rep) {
   DA(K.frow, K.nrows);
   DA(K.fpos, K.nrows);
   DA(K.fwin, K.nkchunks);
-  DA(K.bcol, bcol.size());
-  DA(K.bncol, nblk);
-  DA(K.rloc, K.nrows);
   DA(K.rho_part, (size_t)K.npchunks * 2 * K.nk);
   DA(K.fpart, (size_t)K.nkchunks * std::max(K.nq, 1) * 3);
   DA(K.red_part, 8 * KS_RED_MAX);
@@ -541,9 +539,6 @@ int setup_kspace(mfa_ctx* ctx, const int32_t* a_type, int rep) {
   CK(cudaMemcpyAsync(K.frow, frow.data(), sizeof(int) * K.nrows, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(K.fpos, fpos.data(), sizeof(int) * K.nrows, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(K.fwin, fwin.data(), sizeof(int2) * K.nkchunks, cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(K.bcol, bcol.data(), sizeof(int) * bcol.size(), cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(K.bncol, bncol.data(), sizeof(int) * nblk, cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(K.rloc, rloc.data(), sizeof(int2) * K.nrows, cudaMemcpyHostToDevice, st));
   CK(cudaMemsetAsync(K.ticket, 0, 2 * sizeof(unsigned), st));
   if (K.wdense) CK(cudaMemsetAsync(K.wdense, 0, sizeof(float4) * K.nrows * 4 * K.qx, st));
   if (K.nq) {
@@ -1051,11 +1046,16 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
   // ---- k-space --------------------------------------------------------------------------------
   if (charged && p->n_kmax > 0) {
     ctx->Ks.assign(n_rep, KSpace{});
-    for (int rep = 0; rep < n_rep; ++rep) {
-      int r = setup_kspace(ctx, a_type, rep);
-      if (r != MFA_OK) return r;
-    }
+    std::vector<std::vector<KsRowBlock>> rblk(n_rep);
+    for (int rep = 0; rep < n_rep; ++rep) RET(setup_kspace(ctx, a_type, rep, rblk[rep]));
     ctx->KB = kspace_batch(ctx->Ks, S.mixed, S.nsm);
+    std::vector<KsRowBlock> flat((size_t)n_rep * ctx->KB.rows, KsRowBlock{});
+    for (int rep = 0; rep < n_rep; ++rep)
+      if (ctx->Ks[rep].nq) std::copy(rblk[rep].begin(), rblk[rep].end(), flat.begin() + (size_t)rep * ctx->KB.rows);
+    KsRowBlock* drb = nullptr;
+    DA(drb, flat.size());
+    CK(cudaMemcpy(drb, flat.data(), sizeof(KsRowBlock) * flat.size(), cudaMemcpyHostToDevice));
+    ctx->KB.rblk = drb;
     KSpace* dks = nullptr;
     DA(dks, n_rep);
     CK(cudaMemcpy(dks, ctx->Ks.data(), sizeof(KSpace) * n_rep, cudaMemcpyHostToDevice));

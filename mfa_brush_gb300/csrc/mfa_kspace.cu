@@ -168,8 +168,10 @@ constexpr int KS_TILE = 32;  // particles per shared-memory tile of k_ks_rho (on
 // Slots outside a row's k-range are computed and not stored.  The table columns that the block's
 // rows and slots use are copied a tile ahead (cp.async); the A of a tile is formed from them.  (Read
 // from global memory when the tile began, their latency stood before every tile: with the packed
-// sums 57 -> 39 us on the charged brush.)  The Y and Z columns are those that the 64 rows name (K.bcol),
-// at most 128: they fit in shared memory however long the box is.
+// sums 57 -> 39 us on the charged brush.)  The Y and Z columns are the ranges
+// that the block's rows use, at most KS_BC of them (KsRowBlock): they fit however long the box is.  (A block
+// of one or two tiles waits mostly for its first loads: with the ranges read one load behind K, or a list of
+// columns behind a barrier, twelve small charged channels took 21.8 us, now 20.7.)
 constexpr int KS_RHO_T = 256;  // threads of a k_ks_rho block (8 warps)
 constexpr int KS_RW = 8;       // rows per warp (four per half-warp)
 constexpr int KS_CS = KS_TILE + 1;  // column stride (odd: 16 slots of one particle are 16 banks apart)
@@ -177,30 +179,27 @@ constexpr int KS_AS = KS_RB + 2;  // A row stride (16-byte aligned rows)
 static_assert(KS_TILE * KS_AS * sizeof(float2) % 16 == 0, "the columns follow the A rows 16-byte aligned");
 
 template <bool MIXED>
-__global__ void __launch_bounds__(KS_RHO_T, MIXED ? 3 : 1) k_ks_rho(const KSpace* __restrict__ Ks, int nz) {
+__global__ void __launch_bounds__(KS_RHO_T, MIXED ? 3 : 1) k_ks_rho(const KSpace* __restrict__ Ks,
+                                                                             const KsRowBlock* __restrict__ rblk, int nz) {
   const KSpace K = Ks[blockIdx.z / nz];
+  const KsRowBlock Q = rblk[blockIdx.z / nz * gridDim.x + blockIdx.x];  // (beside K, not behind it)
   const int zs = blockIdx.z % nz;
-  if ((int)blockIdx.x * KS_RB >= K.nrows || (int)blockIdx.y >= K.npchunks || zs * KS_SL > K.nxm || K.nq == 0) return;
+  if (Q.nr == 0 || (int)blockIdx.y >= K.npchunks || zs * KS_SL > K.nxm || K.nq == 0) return;
   if (!MIXED && K.dense) return;  // (k_ks_rho_q)
   using real = kreal<MIXED>;
   using Cx = kcplx<MIXED>;
   extern __shared__ __align__(16) unsigned char shraw[];
   Cx* As = reinterpret_cast<Cx*>(shraw);              // [KS_TILE][KS_AS]
   int2* rc = reinterpret_cast<int2*>(As + KS_TILE * KS_AS);  // [KS_RB] signed Y column, Z column (of a tile)
-  int* bc = reinterpret_cast<int*>(rc + KS_RB);       // [KS_BC] the block's Y and Z columns
-  Cx* cols = reinterpret_cast<Cx*>(bc + KS_BC);       // two tiles of columns: 16 X, the block's Y and Z
+  Cx* cols = reinterpret_cast<Cx*>(rc + KS_RB);       // two tiles of columns: 16 X, the block's Y and Z
   const Cx* tab = ktab<MIXED>(K);
-  const int rbeg = blockIdx.x * KS_RB, nr = min(KS_RB, K.nrows - rbeg);
+  const int rbeg = Q.row, nr = Q.nr, ncols = KS_SL + Q.ny + Q.nz;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4;
   constexpr int NW = KS_RHO_T / 32;
   constexpr int RL = KS_RW / 2;  // rows per lane
   const int slot = zs * KS_SL + (lane & (KS_SL - 1));  // |nx| of the lane
   const int r0 = warp * KS_RW + half * RL;             // the lane's first row
   const bool act = r0 < nr;
-  const int ncols = KS_SL + K.bncol[blockIdx.x];
-  for (int c = threadIdx.x; c < ncols - KS_SL; c += KS_RHO_T) bc[c] = K.bcol[blockIdx.x * KS_BC + c];
-  for (int r = threadIdx.x; r < nr; r += KS_RHO_T) rc[r] = K.rloc[rbeg + r];
-  __syncthreads();
   const int p_beg = blockIdx.y * K.pchunk, p_end = min(K.nq, p_beg + K.pchunk);
   auto fetch = [&](int t0, int buf) {
     const int pq = t0 + lane;
@@ -208,7 +207,8 @@ __global__ void __launch_bounds__(KS_RHO_T, MIXED ? 3 : 1) k_ks_rho(const KSpace
       Cx* to = cols + buf * ncols * KS_CS + lane;
       for (int c = warp; c < ncols; c += NW) {
         const int n = zs * KS_SL + c;  // X column
-        const int col = c < KS_SL ? n : bc[c - KS_SL];
+        const int col = c < KS_SL ? n : (c < KS_SL + Q.ny ? K.nxm + 1 + Q.ylo + c - KS_SL
+                                                          : K.nxm + K.nym + 2 + Q.zlo + c - KS_SL - Q.ny);
         if (c >= KS_SL || n <= K.nxm) cp_async(to + c * KS_CS, tab + (size_t)col * K.nq + pq);
       }
     }
@@ -226,6 +226,11 @@ __global__ void __launch_bounds__(KS_RHO_T, MIXED ? 3 : 1) k_ks_rho(const KSpace
 #pragma unroll
     for (int i = 0; i < RL; ++i) s[a][i] = c[a][i] = 0;
   fetch(p_beg, 0);
+  for (int r = threadIdx.x; r < nr; r += KS_RHO_T) {
+    const int4 R = K.rows[rbeg + r];
+    const int yc = KS_SL + abs(R.z) - Q.ylo;
+    rc[r] = make_int2(R.z < 0 ? -yc : yc, KS_SL + Q.ny + R.w - Q.zlo);
+  }
   int buf = 0;
   for (int t0 = p_beg; t0 < p_end; t0 += KS_TILE, buf ^= 1) {
     const int nt = min(KS_TILE, p_end - t0);
@@ -338,31 +343,29 @@ __global__ void __launch_bounds__(KS_RHO_T, MIXED ? 3 : 1) k_ks_rho(const KSpace
 // The same in integer limbs (FP64 mode, K.dense): lanes, rows and tiles as k_ks_rho; the tables are
 // those of X, Y and q Z / q_max.  A tile's sums go to 64-bit totals in units of 2^-51 (a chunk holds at most
 // 2048 particles: a total, and the sums of two that a k takes, stay at or below 2^62).
-__global__ void __launch_bounds__(KS_RHO_T, 2) k_ks_rho_q(const KSpace* __restrict__ Ks, int nz) {
+__global__ void __launch_bounds__(KS_RHO_T, 2) k_ks_rho_q(const KSpace* __restrict__ Ks, const KsRowBlock* __restrict__ rblk,
+                                                           int nz) {
   const KSpace K = Ks[blockIdx.z / nz];
+  const KsRowBlock Q = rblk[blockIdx.z / nz * gridDim.x + blockIdx.x];
   const int zs = blockIdx.z % nz;
-  if (!K.dense || (int)blockIdx.x * KS_RB >= K.nrows || (int)blockIdx.y >= K.npchunks || zs > 0 || K.nq == 0) return;
+  if (!K.dense || Q.nr == 0 || (int)blockIdx.y >= K.npchunks || zs > 0 || K.nq == 0) return;
   extern __shared__ __align__(16) unsigned char shraw[];
   int4* As = reinterpret_cast<int4*>(shraw);                 // [KS_TILE][KS_RB + 1]
   int2* rc = reinterpret_cast<int2*>(As + KS_TILE * (KS_RB + 1));
-  int* bc = reinterpret_cast<int*>(rc + KS_RB);              // [KS_BC]
-  int4* cols = reinterpret_cast<int4*>(bc + KS_BC);          // two tiles of columns: 16 X, the block's Y and Z
-  const int rbeg = blockIdx.x * KS_RB, nr = min(KS_RB, K.nrows - rbeg);
+  int4* cols = reinterpret_cast<int4*>(rc + KS_RB);          // two tiles of columns: 16 X, the block's Y and Z
+  const int rbeg = Q.row, nr = Q.nr, ncols = KS_SL + Q.ny + Q.nz;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = lane >> 4;
   constexpr int NW = KS_RHO_T / 32, RL = KS_RW / 2;
   const int slot = lane & (KS_SL - 1), r0 = warp * KS_RW + half * RL;
   const bool act = r0 < nr;
-  const int ncols = KS_SL + K.bncol[blockIdx.x];
-  for (int c = threadIdx.x; c < ncols - KS_SL; c += KS_RHO_T) bc[c] = K.bcol[blockIdx.x * KS_BC + c];
-  for (int r = threadIdx.x; r < nr; r += KS_RHO_T) rc[r] = K.rloc[rbeg + r];
-  __syncthreads();
   const int p_beg = blockIdx.y * K.pchunk, p_end = min(K.nq, p_beg + K.pchunk);
   auto fetch = [&](int t0, int buf) {
     const int pq = t0 + lane;
     if (pq < p_end) {
       int4* to = cols + buf * ncols * KS_CS + lane;
       for (int c = warp; c < ncols; c += NW) {
-        const int col = c < KS_SL ? c : bc[c - KS_SL];
+        const int col = c < KS_SL ? c : (c < KS_SL + Q.ny ? K.nxm + 1 + Q.ylo + c - KS_SL
+                                                          : K.ncol + Q.zlo + c - KS_SL - Q.ny);
         if (c >= KS_SL || c <= K.nxm) cp_async(to + c * KS_CS, K.tabq + (size_t)col * K.nq + pq);
       }
     }
@@ -377,6 +380,11 @@ __global__ void __launch_bounds__(KS_RHO_T, 2) k_ks_rho_q(const KSpace* __restri
     for (int i = 0; i < RL; ++i) tot[a][i] = 0;
   int bad = 0;  // a particle that is not finite (every particle of the chunk comes by with the first row)
   fetch(p_beg, 0);
+  for (int r = threadIdx.x; r < nr; r += KS_RHO_T) {
+    const int4 R = K.rows[rbeg + r];
+    const int yc = KS_SL + abs(R.z) - Q.ylo;
+    rc[r] = make_int2(R.z < 0 ? -yc : yc, KS_SL + Q.ny + R.w - Q.zlo);
+  }
   int buf = 0;
   for (int t0 = p_beg; t0 < p_end; t0 += KS_TILE, buf ^= 1) {
     const int nt = min(KS_TILE, p_end - t0);
@@ -1066,7 +1074,7 @@ namespace {
 size_t rho_smem(int yz, bool mixed) {
   return ((size_t)KS_TILE * KS_AS + 2 * (size_t)(KS_SL + yz) * KS_CS) *
              (mixed ? sizeof(float2) : sizeof(double2)) +
-         (size_t)KS_RB * sizeof(int2) + (size_t)KS_BC * sizeof(int);
+         (size_t)KS_RB * sizeof(int2);
 }
 size_t force_smem(const KSpace& K, bool mixed) {
   const size_t cx = mixed ? sizeof(float2) : sizeof(double2);
@@ -1078,7 +1086,7 @@ int dense_qf(const KSpace& K) { return (K.nxm + 4) / 4; }
 // (the limb forms of the FP64 mode)
 size_t rho_q_smem(int yz) {
   return ((size_t)KS_TILE * (KS_RB + 1) + 2 * (size_t)(KS_SL + yz) * KS_CS) * sizeof(int4) +
-         (size_t)KS_RB * sizeof(int2) + (size_t)KS_BC * sizeof(int);
+         (size_t)KS_RB * sizeof(int2);
 }
 size_t force_q_smem(int qf) {
   return (size_t)KS_FR * (4 * qf * 4 * sizeof(int4) + 3 * sizeof(double) + sizeof(int2));
@@ -1142,7 +1150,7 @@ KSpaceBatch kspace_batch(const std::vector<KSpace>& Ks, bool mixed, int nsm) {
     if (!mixed && use_dense(K, mixed)) B.rho_q_shm = std::max(B.rho_q_shm, rho_q_smem(K.yz_max));
     else B.rho_shm = std::max(B.rho_shm, rho_smem(K.yz_max, mixed));
     B.nrows = std::max(B.nrows, K.nrows);
-    B.rows = std::max(B.rows, (K.nrows + KS_RB - 1) / KS_RB);
+    B.rows = std::max(B.rows, K.nrblk);
     B.pchunks = std::max(B.pchunks, K.npchunks);
     B.nz = std::max(B.nz, (K.nxm + KS_SL) / KS_SL);
     B.sum = std::max(B.sum, std::min(KS_RED_MAX, (K.nk + 31) / 32));
@@ -1168,6 +1176,7 @@ static int launch_ks(const DevState& s, const SimConst& C, KSpaceBatch B, cudaSt
     KSpaceBatch A = B;
     A.n = most;
     B.d += most;
+    B.rblk += (size_t)most * B.rows;
     B.n -= most;
     return launch_ks(s, C, A, st, what, eflag, acc, to_f4) + launch_ks(s, C, B, st, what, eflag, acc, to_f4);
   }
@@ -1185,11 +1194,11 @@ static int launch_ks(const DevState& s, const SimConst& C, KSpaceBatch B, cudaSt
     const dim3 g1(B.rows, B.pchunks, B.nz * B.n), g2(B.sum, B.n);
     const double fac_alpha = 1. / (4. * C.alpha_c);
     if (s.mixed) {
-      k_ks_rho<true><<<g1, KS_RHO_T, B.rho_shm, st>>>(B.d, B.nz);
+      k_ks_rho<true><<<g1, KS_RHO_T, B.rho_shm, st>>>(B.d, B.rblk, B.nz);
       k_ks_rho_sum<true><<<g2, 256, 0, st>>>(B.d, 4. * pi, fac_alpha, acc, eflag);
     } else {
-      if (B.rho_shm) k_ks_rho<false><<<g1, KS_RHO_T, B.rho_shm, st>>>(B.d, B.nz);
-      if (B.rho_q_shm) k_ks_rho_q<<<g1, KS_RHO_T, B.rho_q_shm, st>>>(B.d, B.nz);
+      if (B.rho_shm) k_ks_rho<false><<<g1, KS_RHO_T, B.rho_shm, st>>>(B.d, B.rblk, B.nz);
+      if (B.rho_q_shm) k_ks_rho_q<<<g1, KS_RHO_T, B.rho_q_shm, st>>>(B.d, B.rblk, B.nz);
       k_ks_rho_sum<false><<<g2, 256, 0, st>>>(B.d, 4. * pi, fac_alpha, acc, eflag);
     }
     launches += 2;

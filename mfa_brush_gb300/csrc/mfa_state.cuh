@@ -219,6 +219,11 @@ void launch_pair_list(const DevState& s, const SimConst& C, cudaStream_t st, int
 // The k-vectors come in the reference's order: kz outer, ky, kx inner, so every (ky, kz) pair
 // owns one contiguous run of k ("row") whose phases share the factor Y Z: a (k, particle) term
 // then costs one complex product instead of a sin/cos of a large argument.
+// Rows of one rho block: the first of them, their number, and the ranges of |ny| and nz that they use (KS_RB
+// rows, fewer where the ranges would be more than KS_BC columns together: rows of one nz never are).
+struct alignas(16) KsRowBlock {
+  int row, nr, ylo, ny, zlo, nz, pad[2];
+};
 struct KSpace {
   int nk, nq, nxm, nym, nzm, ncol;
   int4* kn;             // [nk] (nx, ny, nz, 0) in the reference's enumeration order
@@ -246,11 +251,7 @@ struct KSpace {
   // The dense slot table has 4 qx slots per row, nx = -nxm .. -nxm + 4 qx - 1.
   int qx;
   int pchunk, npchunks;
-  // the Y and Z table columns that a block of KS_RB rows of k_ks_rho uses [blocks][KS_BC], their number
-  // (at most yz_max), and each row's two of them [nrows] (behind the KS_SL X slots; Y signed as ny)
-  int *bcol, *bncol;
-  int2* rloc;
-  int yz_max;
+  int nrblk, yz_max;    // k_ks_rho's blocks of rows; the Y and Z columns that one of them uses, at most
   double* rho_part;     // [npchunks][2*nk] (mixed: four FP32 words per k, two per part)
   float4* kdf;          // [nk] (kx, G Re rho, G Im rho, nx + nxm as int bits)   (mixed)
   double2* kdd;         // [nk] (G Re rho, G Im rho)                              (fp64)
@@ -270,9 +271,9 @@ struct KSpace {
   int dense;            // 1: the dense kernels (kspace_dense); in the FP64 mode the limb forms
   int plain;            // 1: FP32 sums without Kahan compensation (mfa_options.kspace_plain_sums)
 };
-constexpr int KS_RB = 64;        // rows per rho block
+constexpr int KS_RB = 64;        // rows per rho block, at most
 constexpr int KS_SL = 16;        // |nx| slots per rho block
-constexpr int KS_BC = 2 * KS_RB;  // Y and Z columns of its rows, at most
+constexpr int KS_BC = 128;       // Y and Z columns of its rows, at most
 constexpr int KS_FB = 128;       // particles per force block
 constexpr int KS_FR = 32;        // rows per force chunk
 constexpr int KS_RED_MAX = 256;  // blocks of a grid reduction, at most
@@ -286,6 +287,7 @@ int kspace_prepare(const KSpace& K, bool mixed);
 // The k-spaces of a batch and the largest extents of each kernel's grid over them.
 struct KSpaceBatch {
   const KSpace* d;  // [n] in device memory
+  const KsRowBlock* rblk;  // [n][rows] row blocks of k_ks_rho; nr is 0 past a replica's own
   int n, pp, nq, dip, tab, rows, pchunks, nz, sum, dense_p, dense_k, qf, force_p, force_k;
   int nrows;
   size_t rho_shm, rho_q_shm, force_shm;
