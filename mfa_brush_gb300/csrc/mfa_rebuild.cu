@@ -215,8 +215,8 @@ __device__ __forceinline__ void copyback_slot(const DevState& s, int i) {
 // counter that the list builder's end sets back to zero.  The wait is bounded (about a second): then
 // the status word gets ST_BARRIER and the block leaves.  A block goes on only when all have arrived, so
 // whatever a block does rests on finished phases.  The counts and the slots may then be half-way, so
-// from that on every sort and list builder leaves at once (sort_failed): the lists stay those of the
-// last complete rebuild, whose slots are in range, and the host refuses further steps.
+// from that on every sort leaves at once (sort_failed) and the list builder finds no work: the lists stay
+// those of the last complete rebuild, whose slots are in range, and the host refuses further steps.
 __device__ __forceinline__ bool grid_barrier(const DevState& s, int k) {
   __shared__ bool ok;
   __syncthreads();
@@ -230,7 +230,10 @@ __device__ __forceinline__ bool grid_barrier(const DevState& s, int k) {
     for (int t = 0; t < s.barrier_spins && seen < target; ++t)
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(cnt) : "memory");
     ok = seen >= target;
-    if (!ok) atomicOr(s.status, ST_BARRIER);
+    if (!ok) {
+      atomicOr(s.status, ST_BARRIER);
+      s.wl_n[0] = s.wl_k[0] = 0;  // (block 0 wrote its own before it arrived here, or gives up later)
+    }
     __threadfence();
   }
   __syncthreads();
@@ -238,7 +241,7 @@ __device__ __forceinline__ bool grid_barrier(const DevState& s, int k) {
 }
 
 __device__ __forceinline__ unsigned sort_failed(const DevState& s) {
-  return *(volatile const unsigned*)s.status & ST_BARRIER;
+  return s.status[0] & ST_BARRIER;
 }
 
 // block-wide exclusive scan of v; the block's total in `total`
@@ -396,7 +399,7 @@ __device__ __forceinline__ void rebuild_done(const DevState& s) {
   __syncthreads();
   if (!last) return;
   int* flag = s.rebuild_flag;
-  const bool any = flag[0] != 0;
+  const bool failed = sort_failed(s), any = flag[0] != 0 && !failed;
   __syncthreads();
   for (int r = threadIdx.x; r < s.nrep && any; r += blockDim.x) {
     if (flag[1 + r]) {
@@ -405,7 +408,8 @@ __device__ __forceinline__ void rebuild_done(const DevState& s) {
     }
   }
   if (threadIdx.x == 0) {
-    s.wl_n[2] = s.wl_n[3] = s.wl_n[4] = 0;
+    s.wl_n[2] = 0;
+    if (!failed) s.wl_n[3] = s.wl_n[4] = 0;
     if (any) {
       *s.rebuilds += 1;
       flag[0] = 0;
@@ -494,7 +498,6 @@ __device__ __forceinline__ NlRow nl_row(const DevState& s, const RepDesc& R, int
 template <bool UNI, int H, int HX = H>
 __global__ void __launch_bounds__(NL_T, 8) k_nlist(DevState s) {
   constexpr int NR = (2 * H + 1) * (2 * H + 1);
-  if (sort_failed(s)) return;  // (no kernel that sets it runs beside this one: the same for every thread)
   const int nwl = s.wl_n[0], nchunks = s.wl_k[nwl];
   const int lane = threadIdx.x & 31, warp = (blockIdx.x * NL_T + threadIdx.x) >> 5, nwarps = gridDim.x * (NL_T / 32);
   __shared__ int nl_sh[NL_T * (NL_STAGE | 1)];
