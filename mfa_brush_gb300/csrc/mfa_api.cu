@@ -981,6 +981,7 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
         if (e.flags & PF_COUL) r2max = std::max(r2max, e.range2);
     RET(make_coul_table(ctx, r2max));
   }
+  CK((cudaError_t)profiles_prepare(S, C.hist_dim));
   S.rl2_uni = C.rl2_uni_f;
   S.fx_err = (float)fx_err;
   S.nl_h = nl_h;

@@ -349,21 +349,28 @@ __global__ void __launch_bounds__(PROF_T, 4) k_profiles(DevState s, SimConst C, 
   }
 }
 
+static size_t prof_bytes(int per, int H) { return sizeof(double) * 3 * PROF_T * per + sizeof(int) * 9 * (size_t)H; }
+
 template <int STEP, int PER>
 static void launch_prof(const DevState& s, const SimConst& C, cudaStream_t st, double* prof, int H) {
   const int tile = PROF_T * PER;
-  auto bytes = [&](int h) { return sizeof(double) * 3 * tile + sizeof(int) * 9 * (size_t)h; };
-  // above 48 KB dynamic shared memory needs an explicit opt-in, a property of the kernel for the
-  // whole process: set once to the size of the largest histogram
-  static const cudaError_t opted = cudaFuncSetAttribute(
-      k_profiles<STEP, PER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes(MFA_HIST_DIM_MAX));
-  (void)opted;
-  k_profiles<STEP, PER><<<(s.N + tile - 1) / tile, PROF_T, bytes(H), st>>>(s, C, prof, H);
+  k_profiles<STEP, PER><<<(s.N + tile - 1) / tile, PROF_T, prof_bytes(PER, H), st>>>(s, C, prof, H);
 }
 
 // Four particles a thread; one when that leaves SMs without a block.  (1.6 M particles: 993 us a step with
 // four and four blocks per SM, 1008 with three, 1020 with eight and two, 995 with two and six.)
 static bool prof_small(const DevState& s) { return s.N < 2 * s.nsm * PROF_T; }
+
+// Above 48 KB dynamic shared memory needs an explicit opt-in, a property of the kernel on one device for every
+// context there: set to the size of the largest histogram, so that no context lowers it below another's.
+int profiles_prepare(const DevState& s, int H) {
+  if (prof_small(s) || prof_bytes(4, H) <= 48 * 1024) return (int)cudaSuccess;
+  static_assert(sizeof(double) * 3 * PROF_T + sizeof(int) * 9 * MFA_HIST_DIM_MAX <= 48 * 1024, "one a thread: never");
+  const int mx = (int)prof_bytes(4, MFA_HIST_DIM_MAX);
+  cudaError_t e = cudaFuncSetAttribute(k_profiles<0, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_profiles<1, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
+  return (int)e;
+}
 
 void launch_profiles(const DevState& s, const SimConst& C, cudaStream_t st, double* prof, int H) {
   if (prof_small(s)) launch_prof<0, 1>(s, C, st, prof, H);

@@ -190,6 +190,8 @@ void launch_integrate(const DevState& s, const SimConst& C, cudaStream_t st, int
 void launch_profiles(const DevState& s, const SimConst& C, cudaStream_t st, double* prof, int hist);
 // velocities(n), the profile and positions(n+1) of a mixed step without energies in one pass
 void launch_integrate_profiles(const DevState& s, const SimConst& C, cudaStream_t st, double* prof, int hist);
+// host-side preparation of both for a histogram of `hist` bins; returns a CUDA error
+int profiles_prepare(const DevState& s, int hist);
 void launch_record(Acc acc, double* out, cudaStream_t st);
 // observation quantities per replica: out[9 r + 0..2] brush Rg^2, 3..5 melt Rg^2, 6..8 momentum
 void launch_observe(const DevState& s, const SimConst& C, cudaStream_t st, double* out);
