@@ -227,6 +227,9 @@ int capture_conditional_rebuild(mfa_ctx* ctx, const DevState& S) {
   const cudaGraphNode_t* deps = nullptr;
   size_t nd = 0;
   CK(cudaStreamGetCaptureInfo(st, &cs, nullptr, &graph, &deps, nullptr, &nd));
+  if (cs != cudaStreamCaptureStatusActive)  // (an invalidated capture has no graph)
+    return fail(ctx, MFA_ERR_CUDA, std::string("a launch failed while a step was captured: ") +
+                                       cudaGetErrorString(cudaGetLastError()));
   cudaGraphConditionalHandle h;
   CK(cudaGraphConditionalHandleCreate(&h, graph, 0, 0));
   k_cond_rebuild<<<1, 1, 0, st>>>(S.rebuild_flag, h);
@@ -1509,16 +1512,18 @@ int mfa_step(mfa_ctx* ctx, int32_t nsteps) {
     auto key = std::make_tuple(nsteps, phase, (int)prof, (int)obs);
     auto it = ctx->graphs.find(key);
     if (it == ctx->graphs.end()) {
-      cudaGraph_t g;
+      cudaGraph_t g = nullptr;
       int err = MFA_OK;
       CK(cudaStreamBeginCapture(ctx->st, cudaStreamCaptureModeThreadLocal));
       L = issue_steps(ctx, nsteps, phase, prof, obs, true, &err);
       cudaError_t ec = cudaStreamEndCapture(ctx->st, &g);
+      const cudaError_t el = cudaGetLastError();  // (a refused launch does not end every capture)
+      if (ec == cudaSuccess) ec = el;
+      cudaGraphExec_t ge = nullptr;
+      if (err == MFA_OK && ec == cudaSuccess) ec = cudaGraphInstantiate(&ge, g, 0);
+      if (g) cudaGraphDestroy(g);
       if (err != MFA_OK) return err;
       CK(ec);
-      cudaGraphExec_t ge;
-      CK(cudaGraphInstantiate(&ge, g, 0));
-      cudaGraphDestroy(g);
       it = ctx->graphs.emplace(key, std::make_pair(ge, L)).first;
     }
     CK(cudaGraphLaunch(it->second.first, ctx->st));

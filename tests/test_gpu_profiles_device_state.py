@@ -16,7 +16,9 @@ FAKE = r"""
 #include <stdlib.h>
 int cudaFuncSetAttribute(const void* f, int attr, int value) {
   const char* refuse = getenv("FAKE_REFUSE");
+  const char* lie = getenv("FAKE_LIE");
   fprintf(stderr, "opt-in %d\n", value);
+  if (lie && atoi(lie) == value) return 0; /* and does nothing: the launches will fail */
   if (refuse && atoi(refuse) == value) return 1; /* cudaErrorInvalidValue */
   void* rt = dlopen("libcudart.so.13", RTLD_LAZY | RTLD_NOLOAD); /* the one that the library brought in */
   return rt ? ((int (*)(const void*, int, int))dlsym(rt, "cudaFuncSetAttribute"))(f, attr, value) : 999;
@@ -65,3 +67,9 @@ def test_every_context_opts_in(gpu, tmp_path):
 def test_a_refused_opt_in_fails_the_context(gpu, tmp_path):
     r = _run(tmp_path, FAKE_REFUSE=str(BYTES))
     assert r.returncode != 0 and "MFA_ERR_CUDA" in r.stderr
+
+
+def test_a_launch_that_fails_is_an_error_of_the_call(gpu, tmp_path):
+    """The steps are captured as a graph: the failed launch must not be left out of it, nor end the process."""
+    r = _run(tmp_path, FAKE_LIE=str(BYTES))
+    assert r.returncode == 1 and "MFA_ERR_CUDA" in r.stderr, (r.returncode, r.stderr)
