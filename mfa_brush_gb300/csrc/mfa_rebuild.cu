@@ -20,8 +20,7 @@
 // and its lists name only its own slots).
 // In a captured CUDA graph the sequence sits in the body of a conditional node that runs only on
 // steps where some replica is flagged.
-#include <algorithm>
-
+#include "mfa_grid.h"
 #include "mfa_state.cuh"
 
 namespace mfa {
@@ -39,8 +38,6 @@ __device__ __forceinline__ void cell_coords(const RepDesc& R, const int4& q, int
 // ---- work list ------------------------------------------------------------------------------
 // particles per chunk of the list builder (a warp's, consecutive slots of one replica)
 constexpr int NL_CHUNK = 32;
-constexpr int SORT_T = 512;      // threads per block of k_sort
-constexpr int SORT_PER_SM = 2;   // its blocks per SM (3 or 4: 0.5-2 % slower steps, fewer registers)
 constexpr int WL_SHARED = 1024;  // replicas whose work list fits in shared memory
 
 // The replicas to rebuild (n of them) in ascending order and the prefix sums over them of their
@@ -441,9 +438,7 @@ __device__ __forceinline__ void rebuild_done(const DevState& s) {
 // Each lane (group) stages its first NL_STAGE entries in shared memory and the warp writes them out
 // row by row: the k-th neighbours of 32 consecutive particles are 32 consecutive ints of nbr
 // (scattered 4-byte stores into the column-major list cost read-modify-writes in HBM).
-constexpr int NL_T = 128;    // threads per block
 constexpr int NL_STAGE = 32;  // staged entries per particle (later ones go straight to the list)
-constexpr int NL_G = 8;      // lanes per particle of the second form
 
 struct NlRow {  // slot ranges of a row, the second when it wraps in x
   int b0, e0, b1, e1;
@@ -496,7 +491,7 @@ __device__ __forceinline__ NlRow nl_row(const DevState& s, const RepDesc& R, int
 }
 
 template <bool UNI, int H, int HX = H>
-__global__ void __launch_bounds__(NL_T, 8) k_nlist(DevState s) {
+__global__ void __launch_bounds__(NL_T, NL_PER_SM) k_nlist(DevState s) {
   constexpr int NR = (2 * H + 1) * (2 * H + 1);
   const int nwl = s.wl_n[0], nchunks = s.wl_k[nwl];
   const int lane = threadIdx.x & 31, warp = (blockIdx.x * NL_T + threadIdx.x) >> 5, nwarps = gridDim.x * (NL_T / 32);
@@ -662,9 +657,8 @@ __global__ void __launch_bounds__(NL_T, 8) k_nlist(DevState s) {
 int rebuild_launches() { return 2; }
 
 cudaError_t launch_rebuild(const DevState& s, cudaStream_t st, bool force) {
-  // two blocks per SM at most (what is resident together), no more than the particles fill
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(std::min((s.N + SORT_T - 1) / SORT_T, s.nsm * SORT_PER_SM));
+  cfg.gridDim = dim3(sort_blocks(s.N, s.nsm));
   cfg.blockDim = dim3(SORT_T);
   cfg.stream = st;
   cudaLaunchAttribute at[1];
@@ -682,8 +676,7 @@ cudaError_t launch_rebuild(const DevState& s, cudaStream_t st, bool force) {
   // cells finer along x alone (with 3x3 rows in y, z)
   const KernT kx[2][2] = {{k_nlist<false, 1, 2>, k_nlist<true, 1, 2>}, {k_nlist<false, 1, 3>, k_nlist<true, 1, 3>}};
   const KernT kern = (s.nl_hx != s.nl_h) ? kx[s.nl_hx - 2][uni] : kerns[s.nl_h - 1][uni];
-  const int gl = std::min((s.N * NL_G + NL_T - 1) / NL_T, s.nsm * 8);
-  kern<<<gl, NL_T, 0, st>>>(s);
+  kern<<<list_blocks(s.N, s.nsm), NL_T, 0, st>>>(s);
   return cudaGetLastError();
 }
 
