@@ -993,13 +993,9 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
     return fail(ctx, MFA_ERR_ARG, "pair_schedule must be 0 or 1");
   S.pair_persist = ctx->opt.pair_schedule;
   // neighbour capacity: 2x the mean count of the densest replica + 32, at least 48
-  int cap = ctx->opt.nbr_capacity;
-  if (cap <= 0) {
-    double est = 4. / 3. * M_PI * rl_max * rl_max * rl_max * dens_max;
-    cap = (int)std::ceil(2.0 * est) + 32;
-    cap = std::max(cap, 48);
-  }
-  cap = std::min(cap, NL_CAP_MAX);
+  const double est = 4. / 3. * M_PI * rl_max * rl_max * rl_max * dens_max;
+  const int est_cap = (int)std::min((double)NL_CAP_MAX, std::max(std::ceil(2.0 * est) + 32, 48.));
+  const int cap = ctx->opt.nbr_capacity > 0 ? std::min(ctx->opt.nbr_capacity, NL_CAP_MAX) : est_cap;
   S.nbr_cap = cap;
   DA(S.nbr, (size_t)cap * Nn);
   cudaStream_t st = ctx->st;
@@ -1097,6 +1093,11 @@ int mfa_batch_init(const mfa_params* p, int32_t n_rep, const mfa_system* sysv, c
     }
   }
   if (rc != MFA_OK) return rc;
+  S.list_len = S.nbr_cap;
+  if (ctx->opt.nbr_capacity > 0) {
+    const int mx = (int)ctx->h_status[1];
+    S.list_len = std::min(S.nbr_cap, mx * 3 / 2 + 16 > est_cap ? std::max(est_cap * 2, mx * 3 / 2 + 32) : est_cap);
+  }
   CK(cudaMemcpy(ctx->h_rebuilds, ctx->S.rebuilds, sizeof(long long), cudaMemcpyDeviceToHost));
   ctx->last_rebuilds = *ctx->h_rebuilds;
   return MFA_OK;
@@ -1318,6 +1319,7 @@ static int grow_lists(mfa_ctx* ctx) {
   S.nbr = nullptr;
   DA(S.nbr, (size_t)newcap * S.Np);
   S.nbr_cap = newcap;
+  S.list_len = ctx->opt.nbr_capacity > 0 ? std::min(newcap, std::max(S.list_len, seen * 3 / 2 + 16)) : newcap;
   CK(cudaMemsetAsync(S.nn, 0, sizeof(int) * ctx->N, ctx->st));  // (nothing reads the new array before it is built)
   for (auto& g : ctx->graphs) cudaGraphExecDestroy(g.second.first);
   ctx->graphs.clear();

@@ -1230,11 +1230,12 @@ void launch_pair(const DevState& s, const SimConst& C, cudaStream_t st, bool acc
   const int g = (s.N + B - 1) / B;
   const bool uni = C.scr2_uni_f > 0.f;
   // Lanes per particle for systems too small to fill the GPU with threads (an explicit block size or
-  // the persistent schedule asks for k_pair).  The line follows the lists' length, for which their
-  // capacity stands (61 entries with the WCA cut-off, 180 with 2.24 sigma, 284 with a Coulomb cut-off
-  // of 3): lanes / thread per particle took 17 / 19 us at 20 k and 24 / 19 at 40 k particles (WCA), 56 / 71
-  // at 42 k and 93 / 86 at 83 k (2.24 sigma), 55 / 68 at 64 k and 94 / 91 at 130 k (charged).
-  const bool lanes = s.mixed && B == 128 && block != 128 && s.N <= 400ll * s.nbr_cap &&
+  // the persistent schedule asks for k_pair).  The line follows the lists' length, for which the capacity
+  // that the library chooses stands (61 entries with the WCA cut-off, 180 with 2.24 sigma, 284 with a Coulomb
+  // cut-off of 3): lanes / thread per particle took 17 / 19 us at 20 k and 24 / 19 at 40 k particles (WCA), 56 / 71
+  // at 42 k and 93 / 86 at 83 k (2.24 sigma), 55 / 68 at 64 k and 94 / 91 at 130 k (charged).  (A capacity of
+  // 420 given by the caller put WCA channels of up to 168 k particles on the wrong side.)
+  const bool lanes = s.mixed && B == 128 && block != 128 && s.N <= 400ll * s.list_len &&
                      !(s.pair_persist && !accumulate && !eflag);
   if (lanes) {
     if (eflag) launch_pair_lanes<true>(s, C, st, !accumulate, acc, bonded_mask, uni, integ);
@@ -1269,7 +1270,7 @@ void launch_pair(const DevState& s, const SimConst& C, cudaStream_t st, bool acc
 #define PAIR64(G) {{k_pair64<false, false, G>, k_pair64<true, false, G>}, {k_pair64<false, true, G>, k_pair64<true, true, G>}}
     const KernT kd[3][2][2] = {PAIR64(1), PAIR64(4), PAIR64(8)};
 #undef PAIR64
-    // Lanes per particle by the particles and the lists' length (their capacity: 61 entries with the WCA
+    // Lanes per particle by the particles and the lists' length (as above: 61 entries with the WCA
     // cut-off, 180 with 2.24 sigma, 284 with a Coulomb cut-off of 3; an explicit block size asks for one).
     // 4 lanes / one took, us: WCA 35 / 43 at 19.6 k, 62 / 61 at 40 k, 107 / 89 at 78 k; 2.24 sigma 202 / 244
     // at 21 k, 682 / 716 at 83 k, 2471 / 2485 at 333 k; charged 138 / 247 at 32 k, 384 / 474 at 130 k.
@@ -1277,7 +1278,7 @@ void launch_pair(const DevState& s, const SimConst& C, cudaStream_t st, bool acc
     // at 21 k; charged 80 / 96 at 16 k, 132 / 138 at 32 k, 223 / 216 at 64 k;
     // explicit walls 23 / 21 at 7200.
     const bool given = block == 32 || block == 64 || block == 128;
-    const int lg = given || s.N > 10ll * s.nbr_cap * s.nbr_cap ? 0 : (s.N > 60ll * s.nbr_cap ? 1 : 2);
+    const int lg = given || s.N > 10ll * s.list_len * s.list_len ? 0 : (s.N > 60ll * s.list_len ? 1 : 2);
     const long long threads = (long long)s.N * (lg == 0 ? 1 : (lg == 1 ? 4 : 8));
     // the warps are independent, so one per block: with four the slowest holds the others' place (16 brush
     // replicas, 128 / 64 / 32 threads: 243 / 238 / 237 us; 1 M particles 911 / 890 / 886)

@@ -43,6 +43,8 @@ struct DevState {
   // neighbour list
   int *nn, *nbr;
   int nbr_cap;
+  int list_len;  // the lists' length for the pair kernels' layout rules: the capacity that the library chooses, or
+                 // a smaller one that the caller gave (a larger one makes the lists no longer)
   // cells
   int *cell_of, *rank, *perm, *cell_count, *cell_start;
   int *row_count, *plane_count;  // particles per row (y, z) and plane (z) of list cells (0 between rebuilds)
