@@ -556,8 +556,8 @@ __global__ void __launch_bounds__(KS_TAB_T) k_ks_tables(DevState s, const KSpace
   int n = col, ax = 0;
   if (col > K.nxm + 1 + K.nym) { n = col - K.nxm - K.nym - 2; ax = 2; }
   else if (col > K.nxm) { n = col - K.nxm - 1; ax = 1; }
-  // the phase of n = 1 in turns as a 64-bit fixed point (2^-58), times n with wrap-around: its top 32
-  // bits are the phase in [-1/2, 1/2) turns.  One FP64 product; in FP64 the products, the reduction
+  // the phase of n = 1 in turns as a 64-bit fixed point (2^-58), times n with wrap-around: as a signed
+  // number of 2^-64 it is the phase in [-1/2, 1/2) turns.  One FP64 product; in FP64 the products, the reduction
   // and the conversions of a column bound this kernel.
   double t = (ax == 0 ? K.cx * s.rx[i] : (ax == 1 ? K.cy * s.ry[i] : K.cz * s.rz[i]));
   bool bad = nonfinite(t);  // (the integers below know no NaN)
@@ -565,7 +565,12 @@ __global__ void __launch_bounds__(KS_TAB_T) k_ks_tables(DevState s, const KSpace
   if constexpr (MIXED) {
     const unsigned long long ph = (unsigned long long)round_bits(t * 288230376151711744.0) * (unsigned)n << 6;
     float sn, cs;
-    sincospif(i2f_fast((int)(ph >> 32)) * (2.f / 4294967296.f), &sn, &cs);
+    // 2 ph / 2^64 from all of its bits: the upper half in two exact parts, the lower half rounded (below the
+    // rounding of the sum)
+    const int hi = (int)(ph >> 32);
+    const float low = fmaf(__int_as_float(0x4B000000 | (hi & 0xFFFF)) - 8388608.0f, 4294967296.0f, __uint2float_rn((unsigned)ph));
+    sincospif(fmaf(__int_as_float(0x4B400000 + (hi >> 16)) - 12582912.0f, 3.0517578125e-05f,
+                   low * 1.08420217248550443401e-19f), &sn, &cs);
     K.tabf[idx] = bad ? make_float2(nanf(""), nanf("")) : make_float2(cs, sn);
   } else if (K.dense) {
     // the same phase to 64 bits: the nearest of 1024 table angles and the angle from it by the series
