@@ -498,7 +498,9 @@ __device__ __forceinline__ double pair_fs64(const DevState& s, const SimConst& C
     if (C.dpd_weight1) {
       wr = wd = 1;
     } else {
-      wr = 1. - r2 * ir * ((fl & PF_DPD_OWN) ? e.inv_dpd_rc : e.inv_rc);
+      // (r corrected as the root it stands for: r2 ir rounds twice, 0.1 % of the forces' error)
+      const double q = r2 * ir, r = fma(fma(-q, q, r2), half_of(ir), q);
+      wr = 1. - r * ((fl & PF_DPD_OWN) ? e.inv_dpd_rc : e.inv_rc);
       wd = wr * wr;
     }
     const double g = pair_gauss_d(s.noise, nkey, tag_i, tag_j);
@@ -1028,8 +1030,9 @@ static void launch_pair_lanes(const DevState& s, const SimConst& C, cudaStream_t
 // lane per pair whoever owns it (a thread per particle left half of the lanes idle: the kept counts
 // of neighbours differ; 16 brush replicas 6648 -> 4146 us a call of 10 steps with (3), and 9700
 // before the screening in FP32; 3824 now), and (3) the roots, divisions and noise are those of mfa_dev.cuh.  The
-// products go back through shared memory and each owner adds its own in list order, so the sums do
-// not depend on which lane evaluated a pair.  A warp on a replica boundary evaluates each lane's own
+// factors and distances go back through shared memory and each owner adds its own in list order, so the
+// sums do not depend on which lane evaluated a pair (multiply-adds: products rounded before the sums were
+// 0.5 % further from 64-bit-exact forces).  A warp on a replica boundary evaluates each lane's own
 // pairs instead, so that the energy sums (by lane) stay with their replica.
 // With G lanes per particle (4 or 8) a warp takes 32 / G particles: their lists are screened side by
 // side, and a small system has G times as many warps, whose serial chain of loads and FP64 results is
@@ -1039,7 +1042,8 @@ static void launch_pair_lanes(const DevState& s, const SimConst& C, cudaStream_t
 constexpr int P64_BATCH = 8;  // kept pairs per lane and round
 struct Pair64Warp {           // shared memory of a warp
   double own[6][32];          // its particles' positions and half-step velocities
-  double f[3][32 * P64_BATCH];  // force of each kept pair on its owner
+  double f[32 * P64_BATCH];     // force factor of each kept pair
+  double d[3][32 * P64_BATCH];  // and its distance from the owner
   int tag[32], type[32];
   int j[32 * P64_BATCH];
   unsigned char who[32 * P64_BATCH];
@@ -1176,21 +1180,23 @@ __global__ void __launch_bounds__(128, 4) k_pair64(DevState s, SimConst C, bool 
         const double half = info_mobile(wj) ? 0.5 : 1.;
         const double fs = pair_fs64<EFLAG>(s, C, tab[W.type[o] * MAXT + info_type(wj)], dx, dy, dz, j, W.own[3][o],
                                            W.own[4][o], W.own[5][o], W.tag[o], p0, nkey, r2min, half, e_lj, e_c);
-        W.f[0][q] = fs * dx;
-        W.f[1][q] = fs * dy;
-        W.f[2][q] = fs * dz;
+        W.f[q] = fs;
+        W.d[0][q] = dx;
+        W.d[1][q] = dy;
+        W.d[2][q] = dz;
         if (EFLAG) sym_add(wv, half * fs, dx, dy, dz);
       }
     }
     __syncwarp();
     if constexpr (G == 1) {
       for (int t = 0; t < m; ++t) {
-        fx += W.f[0][at + t];
-        fy += W.f[1][at + t];
-        fz += W.f[2][at + t];
+        const double fs = W.f[at + t];
+        fx = fma(fs, W.d[0][at + t], fx);
+        fy = fma(fs, W.d[1][at + t], fy);
+        fz = fma(fs, W.d[2][at + t], fz);
       }
     } else if (sub < 3) {  // (a lane per component, in fx)
-      for (int t = 0; t < m; ++t) fx += W.f[sub][at + t];
+      for (int t = 0; t < m; ++t) fx = fma(W.f[at + t], W.d[sub][at + t], fx);
     }
     __syncwarp();
   }
