@@ -11,6 +11,7 @@
 
 #include "../../include/mfa_gpu.h"
 #include "mfa_obs.cuh"
+#include "mfa_grid.h"
 #include "mfa_state.cuh"
 
 using namespace mfa;
@@ -495,6 +496,8 @@ int setup_kspace(mfa_ctx* ctx, const int32_t* a_type, int rep, std::vector<KsRow
   K.qmax = 0.;
   for (double q : qv) K.qmax = std::max(K.qmax, std::fabs(q));
   K.inv_qmax = K.qmax > 0. ? 1. / K.qmax : 0.;
+  if (table_blocks(K.nq, (!ctx->S.mixed && dense) ? K.ncolq : K.ncol) < 0)
+    return fail(ctx, MFA_ERR_CAPACITY, "ewald_k: more than 2^32 table entries");
   // rho particle chunks: one wave of three blocks per SM, chunks a multiple of the 32-particle tile
   const int kb = (K.nrows + 63) / 64 * ((2 * nx + 1 + 31) / 32);  // k_ks_rho: 64 rows x 32 slots
   int pch = std::max(1, std::min(256, (3 * 152 + kb - 1) / kb));

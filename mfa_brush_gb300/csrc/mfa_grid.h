@@ -1,4 +1,4 @@
-// mfa_grid.h -- launch shapes of the rebuild kernels (plain C++).
+// mfa_grid.h -- launch shapes of the rebuild kernels and of the k-space tables (plain C++).
 #pragma once
 #include <algorithm>
 #include <cstdint>
@@ -18,6 +18,14 @@ inline int sort_blocks(int64_t n, int nsm) {
 }
 inline int list_blocks(int64_t n, int nsm) {
   return (int)std::min<int64_t>((n * NL_G + NL_T - 1) / NL_T, (int64_t)nsm * NL_PER_SM);
+}
+
+constexpr int KS_TAB_T = 256;  // threads of a k_ks_tables block
+// Blocks of the tables of nq charges, a thread per entry, up to the 2^32 entries that the kernel's unsigned index
+// holds (the FP64 mode's, with the q Z columns, pass 2^31 from 16 million charges on); -1 beyond.
+inline int table_blocks(int64_t nq, int ncol) {
+  const int64_t entries = nq * ncol;
+  return entries <= 0xFFFFFFFFll - KS_TAB_T ? (int)((entries + KS_TAB_T - 1) / KS_TAB_T) : -1;
 }
 
 }  // namespace mfa

@@ -36,6 +36,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "mfa_grid.h"
 #include "mfa_state.cuh"
 
 namespace mfa {
@@ -522,7 +523,6 @@ __device__ __forceinline__ bool grid_sum_last_n(const double* v, double* part, u
 
 // parts of the sum that a launch covers
 constexpr int KS_RECIP = 1, KS_DIPOLE = 2;
-constexpr int KS_TAB_T = 256;  // threads of a k_ks_tables block
 __host__ __device__ inline int ks_dipole_blocks(int nq) {
   return nq > 0 ? (nq + KS_TAB_T - 1) / KS_TAB_T < KS_RED_MAX ? (nq + KS_TAB_T - 1) / KS_TAB_T : KS_RED_MAX : 0;
 }
@@ -545,11 +545,11 @@ __global__ void __launch_bounds__(KS_TAB_T) k_ks_tables(DevState s, const KSpace
     }
     return;
   }
-  const int idx = (blockIdx.x - dblk) * KS_TAB_T + threadIdx.x;
+  const unsigned idx = (blockIdx.x - dblk) * KS_TAB_T + threadIdx.x, nq = K.nq;
   const int ncol = (!MIXED && K.dense) ? K.ncolq : K.ncol;
-  if (!(what & KS_RECIP) || K.nk == 0 || idx >= K.nq * ncol) return;
-  int col = idx / K.nq;
-  const int p = idx - col * K.nq;
+  if (!(what & KS_RECIP) || K.nk == 0 || idx >= nq * ncol) return;
+  int col = idx / nq;
+  const int p = idx - col * nq;
   const int i = s.slot_of_tag[K.qtag[p]];
   const bool times_q = col >= K.ncol;  // (the limb tables hold q Z / q_max as well)
   if (times_q) col -= K.nzm + 1;
@@ -1149,7 +1149,7 @@ KSpaceBatch kspace_batch(const std::vector<KSpace>& Ks, bool mixed, int nsm) {
     if (K.nq == 0) continue;  // no charges: every block of this replica leaves
     B.dip = std::max(B.dip, ks_dipole_blocks(K.nq));
     const int ncol = (!mixed && use_dense(K, mixed)) ? K.ncolq : K.ncol;
-    B.tab = std::max(B.tab, K.nk ? (K.nq * ncol + KS_TAB_T - 1) / KS_TAB_T : 0);
+    B.tab = std::max(B.tab, K.nk ? table_blocks(K.nq, ncol) : 0);
     B.nq = std::max(B.nq, K.nq);
     if (K.nk == 0) continue;
     if (!mixed && use_dense(K, mixed)) B.rho_q_shm = std::max(B.rho_q_shm, rho_q_smem(K.yz_max));
