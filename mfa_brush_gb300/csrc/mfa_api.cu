@@ -154,6 +154,16 @@ int post_status(mfa_ctx* ctx) {
   return MFA_OK;
 }
 
+// a launch with its own result (the thread's last error may be one that the caller left)
+template <typename... P, typename... A>
+cudaError_t launch(void (*kernel)(P...), int grid, int block, cudaStream_t st, A... a) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.stream = st;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(a)...);
+}
+
 // n doubles and the status words into page-locked host memory by one kernel: a drop-in call returns
 // its energies to the host, and two copies into pageable memory and their events took longer than
 // its kernel.
@@ -169,9 +179,8 @@ __global__ void k_publish(const double* __restrict__ src, int n, double* __restr
 int read_slots(mfa_ctx* ctx, const double* src, int slot, int n) {
   const size_t at = (size_t)slot * ctx->nrep, cnt = (size_t)n * ctx->nrep;
   if (cnt <= 8192) {
-    k_publish<<<(int)(cnt + 255) / 256, 256, 0, ctx->st>>>(src + at, (int)cnt, ctx->h_rec + at, ctx->S.status,
-                                                           ctx->h_status);
-    CK(cudaGetLastError());
+    CK(launch(k_publish, (int)(cnt + 255) / 256, 256, ctx->st, src + at, (int)cnt, ctx->h_rec + at, ctx->S.status,
+              ctx->h_status));
   } else {
     CK(cudaMemcpyAsync(ctx->h_rec + at, src + at, sizeof(double) * cnt, cudaMemcpyDeviceToHost, ctx->st));
     RET(post_status(ctx));
@@ -1150,8 +1159,7 @@ int mfa_n_particles(const mfa_ctx* ctx, int64_t* n_total, int32_t* n_rep) {
 static int zero_call_slots(mfa_ctx* ctx, SlotRanges r) {
   int most = 0;
   for (int q = 0; q < 4; ++q) most = std::max(most, r.n[q]);
-  k_zero_slots<<<(most * ctx->nrep + 255) / 256, 256, 0, ctx->st>>>(ctx->acc_call, ctx->nrep, r);
-  CK(cudaGetLastError());
+  CK(launch(k_zero_slots, (most * ctx->nrep + 255) / 256, 256, ctx->st, ctx->acc_call, ctx->nrep, r));
   ctx->last_source = 2;
   return MFA_OK;
 }
@@ -1174,6 +1182,7 @@ int mfa_verlet_positions(mfa_ctx* ctx) {
   launch_integrate(ctx->S, ctx->C, ctx->st, 0, false, false, acc_of(ctx->acc_call, ctx->nrep));
   ctx->launches += 1;
   RET(rebuild(ctx, false));
+  CK(cudaGetLastError());
   return MFA_OK;
 }
 
@@ -1519,11 +1528,12 @@ int mfa_step(mfa_ctx* ctx, int32_t nsteps) {
     if (it == ctx->graphs.end()) {
       cudaGraph_t g = nullptr;
       int err = MFA_OK;
+      const cudaError_t before = cudaPeekAtLastError();  // (an error of the caller's own is not the capture's)
       CK(cudaStreamBeginCapture(ctx->st, cudaStreamCaptureModeThreadLocal));
       L = issue_steps(ctx, nsteps, phase, prof, obs, true, &err);
       cudaError_t ec = cudaStreamEndCapture(ctx->st, &g);
-      const cudaError_t el = cudaGetLastError();  // (a refused launch does not end every capture)
-      if (ec == cudaSuccess) ec = el;
+      const cudaError_t el = cudaPeekAtLastError();
+      if (ec == cudaSuccess && el != before) ec = cudaGetLastError();  // (a refused launch does not end every capture)
       cudaGraphExec_t ge = nullptr;
       if (err == MFA_OK && ec == cudaSuccess) ec = cudaGraphInstantiate(&ge, g, 0);
       if (g) cudaGraphDestroy(g);

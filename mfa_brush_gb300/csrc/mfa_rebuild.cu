@@ -666,6 +666,7 @@ cudaError_t launch_rebuild(const DevState& s, cudaStream_t st, bool force) {
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
+  // (the launches' own results: the thread's last error may be the caller's)
   const cudaError_t e = cudaLaunchKernelEx(&cfg, k_sort, s, force);
   if (e != cudaSuccess) return e;
   const int uni = s.rl2_uni > 0.f ? 1 : 0;
@@ -676,8 +677,10 @@ cudaError_t launch_rebuild(const DevState& s, cudaStream_t st, bool force) {
   // cells finer along x alone (with 3x3 rows in y, z)
   const KernT kx[2][2] = {{k_nlist<false, 1, 2>, k_nlist<true, 1, 2>}, {k_nlist<false, 1, 3>, k_nlist<true, 1, 3>}};
   const KernT kern = (s.nl_hx != s.nl_h) ? kx[s.nl_hx - 2][uni] : kerns[s.nl_h - 1][uni];
-  kern<<<list_blocks(s.N, s.nsm), NL_T, 0, st>>>(s);
-  return cudaGetLastError();
+  cfg.gridDim = dim3(list_blocks(s.N, s.nsm));
+  cfg.blockDim = dim3(NL_T);
+  cfg.numAttrs = 0;
+  return cudaLaunchKernelEx(&cfg, kern, s);
 }
 
 // ---------------------------------------------------------------------------------------------
