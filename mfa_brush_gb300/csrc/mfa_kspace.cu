@@ -563,7 +563,7 @@ __global__ void __launch_bounds__(KS_TAB_T) k_ks_tables(DevState s, const KSpace
   bool bad = nonfinite(t);  // (the integers below know no NaN)
   if ((__double2hiint(t) & 0x7FFFFFFF) >= 0x40200000) t -= rint(t);  // (8 turns away: not wrapped yet)
   if constexpr (MIXED) {
-    const unsigned long long ph = (unsigned long long)round_bits(t * 288230376151711744.0) * (unsigned)n << 6;
+    const unsigned long long ph = (unsigned long long)round_bits<58>(t) * (unsigned)n << 6;
     float sn, cs;
     // 2 ph / 2^64 from all of its bits: the upper half in two exact parts, the lower half rounded (below the
     // rounding of the sum)
@@ -574,7 +574,7 @@ __global__ void __launch_bounds__(KS_TAB_T) k_ks_tables(DevState s, const KSpace
     K.tabf[idx] = bad ? make_float2(nanf(""), nanf("")) : make_float2(cs, sn);
   } else if (K.dense) {
     // the same phase to 64 bits: the nearest of 1024 table angles and the angle from it by the series
-    const unsigned long long ph = (unsigned long long)round_bits(t * 288230376151711744.0) * (unsigned)n << 6;
+    const unsigned long long ph = (unsigned long long)round_bits<58>(t) * (unsigned)n << 6;
     const int k = (int)((ph + (1ull << 53)) >> 54) & 1023;
     const long long lo = (long long)(ph << 10) >> 10;  // ph mod 2^54, signed
     const double d = (double)lo * (6.283185307179586476925 / 18446744073709551616.0);  // 2 pi / 2^64
