@@ -480,8 +480,7 @@ __device__ __forceinline__ double pair_fs64(const DevState& s, const SimConst& C
   const bool in_c = (fl & PF_COUL) && ((C.coul_rc2 > 0) ? (r2raw < C.coul_rc2) : in_lj);
   double fs = 0;
   if (!(in_lj || dpd || in_c)) return fs;
-  // the only root and division of the pair (pairs closer than 1e-19 sigma are outside the approximation's range)
-  const double ir = __double2hiint(r2) >= 0x38100000 ? rsqrt64(r2) : 1. / sqrt(r2);
+  const double ir = rsqrt64(r2);  // the only root and division of the pair
   if (in_lj) {
     // (rounded once: the seventh power below would enlarge the square's own error.  1 % of the step)
     double inv_r2 = ir * ir;
