@@ -50,7 +50,10 @@ extern "C" {
 #define MFA_ERR_CAPACITY (-12)       /* request exceeds a fixed, documented maximum            */
 
 /* ---- precision modes ------------------------------------------------------------------- */
-#define MFA_PREC_FP64 0   /* plain FP64: every pair/bond/integration operation in double     */
+#define MFA_PREC_FP64 0   /* every energy, force, virial and position in 64 bits: doubles, and for the
+                             k-space sums of up to 15 waves along x 57-bit fixed point, whose
+                             sums are as close to exact ones.  Which pairs to look at is decided
+                             in FP32 with a margin, whether they interact in double           */
 #define MFA_PREC_MIXED 1  /* FP32 pair/bond arithmetic on fixed-point positions, FP32 per-pair
                              accumulation, FP64 per-particle totals, FP64 integration and
                              FP64 energy reductions                                           */

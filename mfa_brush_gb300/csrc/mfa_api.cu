@@ -445,7 +445,7 @@ int setup_kspace(mfa_ctx* ctx, const int32_t* a_type, int rep, std::vector<KsRow
   K.qx = (2 * nx + 1 + 3) / 4;
   // force chunks of whole rows: KS_FR for the dense kernel; for the one-k-at-a-time kernel as
   // many as let its shared-memory tables fit (the X table alone grows with nxm)
-  const bool dense = kspace_dense(K, ctx->S.mixed);
+  const bool dense = kspace_dense(K);
   K.dense = dense ? 1 : 0;
   // the row blocks of k_ks_rho
   for (int r = 0; r < K.nrows;) {

@@ -16,10 +16,6 @@ __device__ __forceinline__ double wrap_bits(double x, double L, long long Lbits)
   return x + __longlong_as_double(ob);  // x + 0 keeps x (and -0.0 + 0 = +0, a zero all the same)
 }
 
-// The update of one mobile particle i (info word w) in the mixed path, after its force (Fx, Fy, Fz)
-// for MODE >= 1; the views go to (pfx_out, vf_out).  Shared by k_int_mixed and by the pair kernel
-// that fuses MODE 2 into its tail, so both give the same bits.  MODE 3 is MODE 1 followed by MODE 0, to
-// the bit, with v(n) in between for the caller (the profiles); it leaves a and F unwritten.
 // verlet_positions.f90:214-247 (WALL 1 with a wall velocity): the sites of the first half of a
 // replica's wall beads move by +va_spring_twall dt per step and the other half by
 // -va_spring_twall dt, wrapped into [0, L) in x and y, and the beads sit on their sites.  Their
@@ -57,6 +53,10 @@ __device__ __forceinline__ int4 move_wall_bead(const DevState& s, const SimConst
   return q;
 }
 
+// The update of one mobile particle i (info word w) in the mixed path, after its force (Fx, Fy, Fz)
+// for MODE >= 1; the views go to (pfx_out, vf_out).  Shared by k_int_mixed and by the pair kernel
+// that fuses MODE 2 into its tail, so both give the same bits.  MODE 3 is MODE 1 followed by MODE 0, to
+// the bit, with v(n) in between for the caller (the profiles); it leaves a and F unwritten.
 template <int MODE, bool EFLAG>
 __device__ __forceinline__ void int_mixed_particle(const DevState& s, const SimConst& C, int i, int w, float Fx,
                                                    float Fy, float Fz, int4* __restrict__ pfx_out,

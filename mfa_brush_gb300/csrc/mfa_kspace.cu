@@ -6,10 +6,10 @@
 // phase array.  Here nothing of size N x N_k is stored.  The k-vectors come kz outer, ky, kx
 // inner, so a (ky, kz) "row" of k shares the factor Y(ky) Z(kz) and only X(kx) varies along it:
 //   k_ks_tables:  per charged particle, X(nx) = exp(i nx dkx x), Y(ny), Z(nz) for n >= 0, each
-//                 from an FP64 phase reduced to [-1/2, 1/2) turns (sincospi); stored column-major
+//                 from a phase in 64-bit turns (plain FP64 form: reduced in FP64); stored column-major
 //                 ([column][particle]) so that a warp reads 32 particles of one column at once;
 //   k_ks_rho:     rho(row, nx) = sum_p (q Y Z)(p, row) X(p, nx) as a complex matrix product per
-//                 block of 64 rows x 16 |nx| slots x a particle chunk, +nx and -nx from the same
+//                 block of up to 64 rows x 16 |nx| slots x a particle chunk, +nx and -nx from the same
 //                 four real sums (X(-n) = conj X(n)): lane = slot, half-warp = 4 rows, tiles of
 //                 32 particles in shared memory; plain sums over a tile and Kahan-compensated
 //                 sums across tiles in FP32 (MIXED), or FP64 sums; one partial per particle
@@ -1114,16 +1114,15 @@ typedef void (*force_q_launcher)(const KSpace*, dim3, cudaStream_t);
 const force_q_launcher kForceQ[5] = {nullptr, launch_force_q<1>, launch_force_q<2>, launch_force_q<3>, launch_force_q<4>};
 typedef void (*dense_launcher)(const KSpace*, size_t, dim3, int, cudaStream_t);
 const dense_launcher kDense[5] = {nullptr, launch_dense<1>, launch_dense<2>, launch_dense<3>, launch_dense<4>};
-bool use_dense(const KSpace& K, bool) { return K.qx <= KS_DENSE_QX_MAX; }
 }  // namespace
 
-bool kspace_dense(const KSpace& K, bool mixed) { return use_dense(K, mixed); }
+bool kspace_dense(const KSpace& K) { return K.qx <= KS_DENSE_QX_MAX; }
 size_t kspace_force_smem(const KSpace& K, bool mixed) { return force_smem(K, mixed); }
 
 int kspace_prepare(const KSpace& K, bool mixed) {
-  const bool q = use_dense(K, mixed) && !mixed;
+  const bool q = kspace_dense(K) && !mixed;
   const size_t a = q ? rho_q_smem(K.yz_max) : rho_smem(K.yz_max, mixed);
-  const size_t b = q ? force_q_smem(dense_qf(K)) : (use_dense(K, mixed) ? dense_smem(dense_qf(K)) : force_smem(K, mixed));
+  const size_t b = q ? force_q_smem(dense_qf(K)) : (kspace_dense(K) ? dense_smem(dense_qf(K)) : force_smem(K, mixed));
   if (a > KS_SMEM_MAX || b > KS_SMEM_MAX) return (int)cudaErrorInvalidConfiguration;
   // The opt-in is a property of the kernel for the whole process, not of a context: set it to the
   // largest allowed size once, so that no context lowers it below another's needs (occupancy
@@ -1134,7 +1133,7 @@ int kspace_prepare(const KSpace& K, bool mixed) {
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ks_force<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ks_force<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_ks_rho_q, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-  return (int)e;  // force_q_smem and dense_smem stay below 48 KB: 32 rows x 16 folded slots x 32 B + 512 B
+  return (int)e;  // force_q_smem and dense_smem stay below 48 KB: 32 rows x 16 folded slots x 64 or 32 B + 1 KB
 }
 
 KSpaceBatch kspace_batch(const std::vector<KSpace>& Ks, bool mixed, int nsm) {
@@ -1142,17 +1141,17 @@ KSpaceBatch kspace_batch(const std::vector<KSpace>& Ks, bool mixed, int nsm) {
   // two particles per thread of the dense force kernel when that leaves every SM two blocks
   long long two = 0;
   for (const KSpace& K : Ks)
-    if (use_dense(K, mixed)) two += (long long)((K.nq + 2 * KS_FB - 1) / (2 * KS_FB)) * K.nkchunks;
+    if (kspace_dense(K)) two += (long long)((K.nq + 2 * KS_FB - 1) / (2 * KS_FB)) * K.nkchunks;
   B.pp = mixed && two >= 2 * nsm ? 2 : 1;
   B.n = (int)Ks.size();
   for (const KSpace& K : Ks) {
     if (K.nq == 0) continue;  // no charges: every block of this replica leaves
     B.dip = std::max(B.dip, ks_dipole_blocks(K.nq));
-    const int ncol = (!mixed && use_dense(K, mixed)) ? K.ncolq : K.ncol;
+    const int ncol = (!mixed && kspace_dense(K)) ? K.ncolq : K.ncol;
     B.tab = std::max(B.tab, K.nk ? table_blocks(K.nq, ncol) : 0);
     B.nq = std::max(B.nq, K.nq);
     if (K.nk == 0) continue;
-    if (!mixed && use_dense(K, mixed)) B.rho_q_shm = std::max(B.rho_q_shm, rho_q_smem(K.yz_max));
+    if (!mixed && kspace_dense(K)) B.rho_q_shm = std::max(B.rho_q_shm, rho_q_smem(K.yz_max));
     else B.rho_shm = std::max(B.rho_shm, rho_smem(K.yz_max, mixed));
     B.nrows = std::max(B.nrows, K.nrows);
     B.rows = std::max(B.rows, K.nrblk);
@@ -1160,7 +1159,7 @@ KSpaceBatch kspace_batch(const std::vector<KSpace>& Ks, bool mixed, int nsm) {
     B.nz = std::max(B.nz, (K.nxm + KS_SL) / KS_SL);
     B.sum = std::max(B.sum, std::min(KS_RED_MAX, (K.nk + 31) / 32));
     const int fb = (K.nq + KS_FB - 1) / KS_FB;
-    if (use_dense(K, mixed)) {
+    if (kspace_dense(K)) {
       B.dense_p = std::max(B.dense_p, (fb + B.pp - 1) / B.pp);
       B.dense_k = std::max(B.dense_k, K.nkchunks);
       B.qf = std::max(B.qf, dense_qf(K));

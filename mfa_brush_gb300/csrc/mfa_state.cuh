@@ -283,7 +283,7 @@ constexpr int KS_FR = 32;        // rows per force chunk
 constexpr int KS_RED_MAX = 256;  // blocks of a grid reduction, at most
 constexpr size_t KS_SMEM_MAX = 227 * 1024;  // dynamic shared memory of one block, at most
 // the dense force kernels (X in registers) serve nxm <= 15
-bool kspace_dense(const KSpace& K, bool mixed);
+bool kspace_dense(const KSpace& K);
 // shared memory of the one-k-at-a-time force kernel for the chunks set in K
 size_t kspace_force_smem(const KSpace& K, bool mixed);
 // host-side preparation of the kernels (shared-memory opt-in); returns a CUDA error

@@ -13,7 +13,8 @@ SKIN, INSIDE, SHORT = 0.4, 4e-5, 5e-6
 
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("uniform", [True, False])
-@pytest.mark.parametrize("L,D,few", [(30.0, 20.0, True), (30.0, 20.0, False), (2500.0, 60.0, True)])
+@pytest.mark.parametrize("L,D,few", [(30.0, 20.0, True), (30.0, 20.0, False), (2500.0, 60.0, True),
+                                       (30.0, 2500.0, True)])
 def test_pairs_at_the_list_cut_off(precision, uniform, L, D, few):
     inp = configs.two_liquid_inputs(f_x=0.0)
     f = inp.flags
