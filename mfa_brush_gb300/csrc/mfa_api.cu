@@ -294,11 +294,18 @@ NoiseTab noise_tables() {
   for (int k = 0; k < 256; ++k) {
     const long double f = (1.L + (k + 0.5L) / 256.L) / (k < 128 ? 1.L : 2.L);
     const long double c = (k == 0 || k == 255) ? 1.L : roundl(2048.L / f) / 2048.L;
-    t.lg[k] = make_double2((double)c, (double)(2.L * logl(c)));
+    const long double v = 2.L * logl(c), hi = roundl(ldexpl(v, 46)) / ldexpl(1.L, 46);
+    t.lg[k] = NoiseLog{(float)c, (float)(v - hi), (double)hi};
   }
-  for (int e = 0; e < 32; ++e) t.ln2[e] = (double)(2.L * e * logl(2.L));
-  for (int k = 0; k < 1024; ++k)
-    t.cs[k] = make_double2((double)cosl(2.L * pi * k / 1024.L), (double)sinl(2.L * pi * k / 1024.L));
+  for (int e = 0; e < 32; ++e) {
+    const long double v = 2.L * e * logl(2.L), hi = roundl(ldexpl(v, 46)) / ldexpl(1.L, 46);
+    t.ln2[e] = NoiseLn2{(double)hi, (float)(v - hi), 0.f};
+  }
+  for (int k = 0; k < 1024; ++k) {
+    const long double c = cosl(2.L * pi * k / 1024.L), n = sinl(2.L * pi * k / 1024.L);
+    t.cs[k] = make_double2((double)c, (double)n);
+    t.cslo[k] = make_float2((float)(c - (double)c), (float)(n - (double)n));
+  }
   return t;
 }
 
