@@ -129,7 +129,7 @@ __device__ __forceinline__ void int_mixed_particle(const DevState& s, const SimC
       // rounded unmerged, so that the decision is the same in every kernel that makes it
       if (__fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx))) > C.skin_half2_f) flag_rebuild(s, rep);
       const int all1 = 0x7FF00000;  // an exponent of ones: not finite
-      if ((__double2hiint(x) & all1) == all1 || (__double2hiint(y) & all1) == all1 || (__double2hiint(z) & all1) == all1)
+      if (max(max(__double2hiint(x) & all1, __double2hiint(y) & all1), __double2hiint(z) & all1) == all1)
         atomicOr(s.status, ST_NAN);
     }
   }
