@@ -1029,7 +1029,7 @@ static void launch_pair_lanes(const DevState& s, const SimConst& C, cudaStream_t
 // view, (2) the kept pairs of a warp's particles are put together and evaluated 32 at a time, a
 // lane per pair whoever owns it (a thread per particle left half of the lanes idle: the kept counts
 // of neighbours differ; 16 brush replicas 6648 -> 4146 us a call of 10 steps with (3), and 9700
-// before the screening in FP32; 3824 now), and (3) the roots, divisions and noise are those of mfa_dev.cuh.  The
+// before the screening in FP32; 3830 now), and (3) the roots, divisions and noise are those of mfa_dev.cuh.  The
 // factors and distances go back through shared memory and each owner adds its own in list order, so the
 // sums do not depend on which lane evaluated a pair (multiply-adds: products rounded before the sums were
 // 0.5 % further from 64-bit-exact forces).  A warp on a replica boundary evaluates each lane's own
